@@ -206,7 +206,7 @@ def _run_job(s):
         sizes, total = job.output_plan()
         total = job.output_to(s.out.data_ptr(), s.out.numel())
         files = s.out if c["work"] == "ragged" else s.out[:total]  # ragged reads: the whole buffer, zero past the files
-    return [cnt.hist.astype(np.int64), cnt.chunk_reads.astype(np.int64), bounds.astype(np.int64), sizes.astype(np.int64), files]
+    return [cnt.hist.view(np.int64), cnt.chunk_reads.view(np.int64), bounds.view(np.int64), sizes.view(np.int64), files]
 
 
 def run(s):

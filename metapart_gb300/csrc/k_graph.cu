@@ -280,60 +280,6 @@ __global__ void k_apply_zero(uint64_t *lo, uint8_t *hi, uint64_t n, const uint32
 
 // ---------------------------------------------------------- union-find
 
-// The roots of x and of y, the two walks advanced together so that their parent loads are in flight at
-// the same time.  A walk stops at a node that is its own parent or whose parent is BAD (a BAD read is
-// its own root, unionfind.h:25-32), and halves its path as it goes (a node is pointed at its
-// grandparent).  When the walks meet (the same node on both) the two are in one component: x and y come
-// back equal without the rest of the walk (callers use the results as roots only when they differ).
-__device__ __forceinline__ void uf_find2(uint32_t *parent, uint32_t &x, uint32_t &y)
-{
-    bool dx = false, dy = false;
-    for (;;) {
-        const uint32_t px = dx ? x : parent[x];
-        const uint32_t py = dy ? y : parent[y];
-        if (px == py && px != BAD) {
-            x = y = px;
-            return;
-        }
-        dx = dx || px == x || px == BAD;
-        dy = dy || py == y || py == BAD;
-        if (dx && dy) return;
-        const uint32_t gx = dx ? x : parent[px];
-        const uint32_t gy = dy ? y : parent[py];
-        if (!dx) {
-            if (gx == px || gx == BAD) {
-                x = px;
-                dx = true;
-            } else {
-                parent[x] = gx;  // path halving: gx is an ancestor of x
-                x = gx;
-            }
-        }
-        if (!dy) {
-            if (gy == py || gy == BAD) {
-                y = py;
-                dy = true;
-            } else {
-                parent[y] = gy;
-                y = gy;
-            }
-        }
-        if (dx && dy) return;
-    }
-}
-
-__device__ __forceinline__ void uf_union(uint32_t *parent, uint32_t a, uint32_t b, uint32_t *err, uint32_t cap)
-{
-    for (uint32_t it = 0; it < cap; it++) {
-        uint32_t ra = a, rb = b;
-        uf_find2(parent, ra, rb);
-        if (ra == rb) return;
-        const uint32_t hi = ra > rb ? ra : rb, lo = ra > rb ? rb : ra;
-        if (atomicCAS(&parent[lo], lo, hi) == lo) return;
-    }
-    atomicOr(err, DERR_SPIN);
-}
-
 // First tuple of each thread range whose k-mer is not zero (nor zero-marked) and whose read is not BAD.
 __global__ void k_range_first_valid(const uint64_t *lo, const uint8_t *hi, const uint32_t *id, const uint32_t *z,
                                     const uint64_t *range_bounds, int T, const uint32_t *parent, uint64_t *first)

@@ -1,0 +1,78 @@
+#pragma once
+#include <vector>
+
+#include "k_graph.cuh"
+#include "k_sort.cuh"
+
+namespace mp {
+
+// A scan without the order of its tuples: what the mischief filter and the unions need of the sorted scan is
+// only which tuples share a k-mer, so the tuples are split into units of consecutive m-mer buckets (one or two
+// unstable multi-split passes) and grouped by k-mer in shared-memory hash tables.  Results equal filter_scan +
+// union_scan over the sorted scan: the same BAD marks, the same components.
+//
+// A tuple between the passes is K = (bucket - first bucket of its bin) << (2 (k - 10) + 6) | low k-mer bits << 6 |
+// the six adjacency bits the filter reads, and the read id.
+
+constexpr uint64_t GROUP_MAX_TUPLES = 4000000000ull;  // tuple positions are 32 bits
+constexpr uint64_t GROUP_MAX_READS = 0x7FFFFFFFull;   // a grouped id keeps its top bit for the group's first tuple
+
+// One scan (or every sample's scan of a batch, as segments) to split and group.
+struct GroupScan {
+    int k = 0;
+    uint64_t n = 0;                    // tuples
+    const uint64_t *d_hist = nullptr;  // bucket prefix; the scan's buckets are [lo, hi), nseg * NB with segments
+    uint64_t lo = 0, hi = 0;
+    std::vector<uint64_t> bounds;      // thread ranges' tuple bounds, every segment's after the other (ascending)
+    std::vector<uint64_t> seg_tstart;  // nseg + 1 tuple offsets ({0, n} for one scan)
+
+    // the plan (device), from group_plan
+    bool two_level = false;
+    int unit_shift = 0, bin_shift = 0;
+    uint32_t max_units = 0, max_bins = 0, max_tiles = 0;
+    uint32_t *ustart = nullptr, *ub0 = nullptr, *ucur = nullptr;  // units: first tuple, first bucket | range start << 31, fill
+    uint32_t *bstart = nullptr, *bb0 = nullptr, *bu0 = nullptr, *bcur = nullptr;  // bins: first tuple, bucket, unit; fill
+    uint32_t *seg_bin0 = nullptr, *tile_bin = nullptr, *tile_first = nullptr;
+    uint32_t *mid = nullptr, *big = nullptr;  // units above a small block's and above a large block's capacity
+    uint32_t *lrs = nullptr;                  // per segment: first tuple of its last range with tuples
+    uint32_t *ctr = nullptr;                  // GC_* counters
+    uint32_t *qlist = nullptr;                // grouped stretches of the segments' last ranges
+    uint32_t *quirk = nullptr;                // per segment: QW words (see k_gp_quirk)
+    uint32_t hctr[16] = {};                   // the counters on the host
+    std::vector<uint32_t> h_lrs, h_tiles;     // sources of uploads still queued
+};
+
+enum GroupCounter : int {
+    GC_UNITS = 0, GC_BINS, GC_TILES, GC_MID, GC_BIG, GC_BIG_TUPLES,  // the plan's counts
+    GC_WORK_S, GC_WORK_L, GC_OUT, GC_QLIST, GC_ERR, GC_N = 16
+};
+
+// What a scan's unions left open, per segment: the segment's last run is to be united with the segment's first
+// read (the sweeps' initial state, metapart.c:2539-2548); anchor is a read of that run.
+struct GroupQuirk {
+    int seg;
+    uint32_t anchor;
+};
+
+bool group_fits(uint64_t n, uint64_t n_reads, const SortSegments *segs);
+// Plans g (its inputs set) on the device, its counts copied into g.hctr in stream order.
+int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st);
+// Splits the tuples of (lo, hi, id) (enumeration order, segment-major) into units; the result is in
+// (k2, id2) with one level, back in (lo, id) with two.
+int group_split(GroupScan &g, uint64_t *lo, const uint8_t *hi, uint32_t *id, uint64_t *k2, uint32_t *id2, DeviceArena &arena,
+                cudaStream_t st);
+// The mischief filter over the split tuples (kk, ids), and every k-mer's reads side by side in out (n ids).
+int group_filter(GroupScan &g, const uint64_t *kk, const uint32_t *ids, uint32_t *out, uint32_t *parent, uint8_t *filtered,
+                 DeviceArena &arena, cudaStream_t st);
+// The unions over the grouped ids and the compression; open: what the caller has to finish (group_finish).
+int group_union(GroupScan &g, const uint32_t *out, uint32_t *parent, const uint8_t *filtered, uint64_t n_reads,
+                DeviceArena &arena, cudaStream_t st, std::vector<GroupQuirk> &open);
+// The first of the tuples (lo, hi, id)[0, n) by (k-mer, adjacency, position): its id.
+int first_tuple_id(const uint64_t *lo, const uint8_t *hi, const uint32_t *id, uint64_t n, DeviceArena &arena, cudaStream_t st,
+                   uint32_t *out);
+// Unites a segment's last run (a read of it: anchor) with the segment's first read (or hooks that read below it
+// when it is BAD, as union_scan does; *hooked as there) and compresses again.
+int group_finish(uint32_t *parent, uint64_t n_reads, uint32_t first, uint32_t anchor, DeviceArena &arena, cudaStream_t st,
+                 uint32_t *hooked);
+
+}  // namespace mp

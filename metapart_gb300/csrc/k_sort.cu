@@ -933,6 +933,12 @@ static SortTuning sort_tuning(int k, uint64_t n)
     return t;
 }
 
+bool sort_plan_chosen(int k, uint64_t n)
+{
+    const SortTuning t = sort_tuning(k, n), d;
+    return t.byte_digits != d.byte_digits || t.unit_bits != d.unit_bits;
+}
+
 // Prefetch distance of the device-wide sort (no k or scan plan): MP_ONESWEEP_PF_WAVES or one wave.
 static uint32_t onesweep_prefetch_tiles()
 {

@@ -38,6 +38,9 @@ int count_unsorted(const uint64_t *lo, const uint8_t *hi, uint64_t n, unsigned l
 // Stable sort of b[cur][0, n) by (hi, lo); on return b.cur names the sorted buffer.
 int radix_sort(SortBufs &b, uint64_t n, bool has_hi, DeviceArena &arena, cudaStream_t st, SortStats *stats);
 
+// The tuning table or the environment shapes the bucket sort of a scan of n tuples (other digits than the default).
+bool sort_plan_chosen(int k, uint64_t n);
+
 // Independent tuple sets (samples) one after another in one tuple array: segment q holds the tuples
 // [tstart[q], tstart[q + 1]) and the m-mer buckets q * NB .. q * NB + NB - 1 of a segmented histogram.
 struct SortSegments {

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "k_graph.cuh"
+#include "k_group.cuh"
 #include "k_kmers.cuh"
 #include "k_output.cuh"
 #include "k_reads.cuh"
@@ -1018,6 +1019,47 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
     return 0;
 }
 
+// Whether a scan of n tuples is grouped instead of sorted (k_group.cuh).  The sorted scan is for who looks at
+// it or shapes its making: stage dumps, the self-checks, a tuning row or a limit of the sort's look-back; a read
+// that the previous scan hooked below a component (its label changes as this scan's unions begin) takes it too.
+static bool scan_is_grouped(const mp_job *j, int k, uint64_t n)
+{
+    return j->dump_dir.empty() && !j->checks && j->arena.lim.lookback_spins == WaitLimits{}.lookback_spins &&
+           j->hooked_bad == ~0u && !sort_plan_chosen(k, n) && group_fits(n, j->pr.n_reads, nullptr);
+}
+
+// The read (component label) of the scan's first tuple in sorted order, from the reads: only when a scan's unions
+// need it (the sweeps' initial state), so its tuples are enumerated again.
+static int scan_first_read(mp_job *j, int k, int min3, uint64_t lo, uint64_t hi, const uint64_t *hist, bool labels,
+                           uint32_t *err, uint32_t *first)
+{
+    const uint64_t N = j->pr.n_reads;
+    uint64_t b0 = lo, b1 = hi;
+    if (!min3) {  // the first populated bucket (the 3-minimizer choice depends on the whole range)
+        b0 = (uint64_t)(std::upper_bound(hist + lo, hist + hi, hist[lo]) - hist) - 1;
+        b1 = b0 + 1;
+    }
+    uint32_t *cnt = j->arena.alloc<uint32_t>(N + 1);
+    uint64_t *off = j->arena.alloc<uint64_t>(N + 2), *ntot = j->arena.alloc<uint64_t>(1);
+    const size_t tb = scan_tmp_bytes(N + 1);
+    void *tmp = j->arena.alloc<uint8_t>(tb);
+    if (!cnt || !off || !ntot || !tmp) return set_error(MP_ENOMEM, "device memory for enumeration offsets");
+    launch_enum_count(j->d_fq, j->pr, k, min3, (uint32_t)b0, (uint32_t)b1, cnt, err, j->st);
+    MP_CUDA(cudaMemsetAsync(cnt + N, 0, 4, j->st));
+    scan_u32_to_u64(cnt, off, N + 1, ntot, tmp, tb, j->st);
+    uint64_t n = 0;
+    MP_CUDA(cudaMemcpyAsync(&n, ntot, 8, cudaMemcpyDeviceToHost, j->st));
+    MP_CUDA(cudaStreamSynchronize(j->st));
+    const bool has_hi = 2 * k + 8 > 64;
+    uint64_t *tl = j->arena.alloc<uint64_t>(n + 1);
+    uint8_t *th = has_hi ? j->arena.alloc<uint8_t>(n + 1) : nullptr;
+    uint32_t *ti = j->arena.alloc<uint32_t>(n + 1);
+    if (!tl || !ti || (has_hi && !th)) return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)n);
+    launch_enum_write(j->d_fq, j->pr, k, min3, (uint32_t)b0, (uint32_t)b1, labels ? j->d_parent : nullptr, off, tl, th, ti, err,
+                      j->st);
+    return first_tuple_id(tl, th, ti, n, j->arena, j->st, first);
+}
+
 int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_starts, const uint64_t *chunk_first_read,
                      int nchunks, const uint64_t *hist, uint64_t *bounds_out)
 {
@@ -1144,6 +1186,21 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         SortBufs sb;
         int lo_buf = 0, hi_buf = 0;
         uint64_t n = 0;
+        // a refused thread-range plan is reported once the tuples are counted
+        std::vector<uint64_t> rb;
+        const int rb_rc = range_bounds(hist, thrR.data() + (size_t)s * T, T, lo, hi, rb);
+        const std::string rb_msg = rb_rc ? g_err : std::string();
+        const bool grouped = !rb_rc && scan_is_grouped(j, k, expect);
+        GroupScan gs;
+        if (grouped) {
+            gs.k = k;
+            gs.n = expect;
+            gs.d_hist = d_hist;
+            gs.lo = lo;
+            gs.hi = hi;
+            gs.bounds = rb;
+            gs.seg_tstart = {0, expect};
+        }
         {
             StageTimer tm(j->st, j->stage_ms, 2);
             if (!cnt_all) {
@@ -1154,6 +1211,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             uint32_t cerr = 0;
             MP_CUDA(cudaMemcpyAsync(&n, ntot, 8, cudaMemcpyDeviceToHost, j->st));
             MP_CUDA(cudaMemcpyAsync(&cerr, err, 4, cudaMemcpyDeviceToHost, j->st));
+            if (grouped && (rc = group_plan(gs, j->arena, j->st))) return rc;
             MP_CUDA(cudaStreamSynchronize(j->st));
             if (cerr & DERR_LONG_READ) return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
             if (cerr & DERR_TOO_MANY)
@@ -1165,8 +1223,8 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             for (int b = 0; b < 2; b++) {
                 sb.lo[b] = j->arena.alloc<uint64_t>(n + 1);
                 sb.id[b] = j->arena.alloc<uint32_t>(n + 1);
-                sb.hi[b] = has_hi ? j->arena.alloc<uint8_t>(n + 1) : nullptr;
-                if (!sb.lo[b] || !sb.id[b] || (has_hi && !sb.hi[b]))
+                sb.hi[b] = has_hi && !(grouped && b) ? j->arena.alloc<uint8_t>(n + 1) : nullptr;
+                if (!sb.lo[b] || !sb.id[b] || (has_hi && !(grouped && b) && !sb.hi[b]))
                     return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)n);
             }
             if (use_kc && cnt_all)
@@ -1185,6 +1243,40 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             return set_error(MP_EUNSUP, "a read has 256 or more k-mers in scan %d (the reference counts them in 8 bits, "
                                         "enumerateKmers.c:152)", s);
         if (herr) return set_error(MP_EDEVICE, "enumeration flags 0x%x", herr);
+        if (rb_rc) return set_error(rb_rc, "%s", rb_msg.c_str());
+        if (grouped) {
+            const int fin = gs.two_level ? 0 : 1;  // the buffers that hold the split tuples
+            const double ms0 = j->stage_ms[3];
+            {
+                StageTimer tm(j->st, j->stage_ms, 3);
+                if ((rc = group_split(gs, sb.lo[0], sb.hi[0], sb.id[0], sb.lo[1], sb.id[1], j->arena, j->st))) return rc;
+            }
+            {
+                StageTimer tm(j->st, j->stage_ms, 4);
+                if ((rc = group_filter(gs, sb.lo[fin], sb.id[fin], sb.id[fin ^ 1], j->d_parent, j->d_filtered, j->arena, j->st)))
+                    return rc;
+            }
+            {
+                StageTimer tm(j->st, j->stage_ms, 5);
+                std::vector<GroupQuirk> open;
+                if ((rc = group_union(gs, sb.id[fin ^ 1], j->d_parent, j->d_filtered, N, j->arena, j->st, open))) return rc;
+                for (const GroupQuirk &q : open) {
+                    uint32_t first = 0;
+                    if ((rc = scan_first_read(j, k, p->min3, lo, hi, hist, s > 0, err, &first))) return rc;
+                    if ((rc = group_finish(j->d_parent, N, first, q.anchor, j->arena, j->st, &j->hooked_bad))) return rc;
+                }
+            }
+            SortStats ss;
+            ss.passes = gs.two_level ? 2 : 1;
+            ss.pass_ms = j->stage_ms[3] - ms0;
+            ss.bytes = n * (uint64_t)((has_hi ? 25 : 24) + (gs.two_level ? 24 : 0));
+            ss.units = gs.hctr[GC_UNITS];
+            ss.big_buckets = gs.hctr[GC_BIG];
+            ss.big_tuples = gs.hctr[GC_BIG_TUPLES];
+            add_sort_stats(j, ss, n);
+            j->arena.release_scratch();
+            continue;
+        }
         snprintf(name, sizeof name, "scan%d_enum.bin", s);
         if ((rc = dump_tuples(j, name, sb.lo[0], sb.hi[0], sb.id[0], n))) return rc;
         {
@@ -1201,8 +1293,6 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         if ((rc = check_sorted(j, tp.lo, tp.hi, n, s))) return rc;
         snprintf(name, sizeof name, "scan%d_sorted.bin", s);
         if ((rc = dump_tuples(j, name, tp.lo, tp.hi, tp.id, n))) return rc;
-        std::vector<uint64_t> rb;
-        if ((rc = range_bounds(hist, thrR.data() + (size_t)s * T, T, lo, hi, rb))) return rc;
         {
             StageTimer tm(j->st, j->stage_ms, 4);
             if ((rc = filter_scan(tp, rb, j->d_parent, j->d_filtered, j->arena, j->st, !j->dump_dir.empty()))) return rc;

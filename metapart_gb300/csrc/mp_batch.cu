@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "k_graph.cuh"
+#include "k_group.cuh"
 #include "k_kmers.cuh"
 #include "k_output.cuh"
 #include "k_reads.cuh"
@@ -172,6 +173,36 @@ static void retire(mp_batch *b, PendingIO &x)
     b->io.free_persistent(x.fq);
     b->io.free_persistent(x.out);
     x = PendingIO{};
+}
+
+// The read (global id) of a sample's first tuple in sorted order, from the reads [r0, r1): only when its unions
+// need it (the sweeps' initial state).
+static int sample_first_read(const uint8_t *d_fq, const ParsedReads &all, uint64_t r0, uint64_t r1, int k, const uint64_t *shist,
+                             uint32_t *err, DeviceArena &A, cudaStream_t st, uint32_t *first)
+{
+    std::vector<uint64_t> h(NB + 1);
+    MP_CUDA(cudaMemcpyAsync(h.data(), shist, (NB + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaStreamSynchronize(st));
+    const uint64_t b0 = (uint64_t)(std::upper_bound(h.begin(), h.end(), h[0]) - h.begin()) - 1, n = h[b0 + 1] - h[b0];
+    ParsedReads pr = all;
+    pr.n_reads = r1 - r0;
+    pr.rec_start += r0;
+    pr.seq_off += r0;
+    pr.seq_len += r0;
+    const bool has_hi = 2 * k + 8 > 64;
+    uint32_t *cnt = A.alloc<uint32_t>(pr.n_reads + 1), *ti = A.alloc<uint32_t>(n + 1);
+    uint64_t *off = A.alloc<uint64_t>(pr.n_reads + 2), *tl = A.alloc<uint64_t>(n + 1);
+    uint8_t *th = has_hi ? A.alloc<uint8_t>(n + 1) : nullptr;
+    const size_t tb = scan_tmp_bytes(pr.n_reads + 1);
+    void *tmp = A.alloc<uint8_t>(tb);
+    if (!cnt || !ti || !off || !tl || !tmp || (has_hi && !th)) return set_error(MP_ENOMEM, "device memory for a sample's first tuple");
+    launch_enum_count(d_fq, pr, k, 0, (uint32_t)b0, (uint32_t)b0 + 1, cnt, err, st);
+    MP_CUDA(cudaMemsetAsync(cnt + pr.n_reads, 0, 4, st));
+    scan_u32_to_u64(cnt, off, pr.n_reads + 1, nullptr, tmp, tb, st);
+    launch_enum_write(d_fq, pr, k, 0, (uint32_t)b0, (uint32_t)b0 + 1, nullptr, off, tl, th, ti, err, st);
+    const int rc = first_tuple_id(tl, th, ti, n, A, st, first);
+    *first += (uint32_t)r0;
+    return rc;
 }
 
 // One group of samples through every stage.  Its partition files' copies to the host are queued at the end
@@ -355,6 +386,10 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     for (int q = 0; q < nseg; q++) segs.tstart[q] = rb[hrb0[q]];
     segs.tstart[nseg] = rb[Rn];
     const uint64_t T_all = rb[Rn];
+    // grouped instead of sorted (k_group.cuh), as a job's scan: unless the sort's plan or its look-back limit is chosen
+    const bool grouped = A.lim.lookback_spins == WaitLimits{}.lookback_spins && !sort_plan_chosen(k, T_all) &&
+                         group_fits(T_all, N, &segs);
+    GroupScan gs;
     // ---- enumeration: every k-mer of every read (one scan per sample), read order
     SortBufs sb;
     {
@@ -385,8 +420,8 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
         for (int x = 0; x < 2; x++) {
             sb.lo[x] = A.alloc_persistent<uint64_t>(n + 1);
             sb.id[x] = A.alloc_persistent<uint32_t>(n + 1);
-            sb.hi[x] = has_hi ? A.alloc_persistent<uint8_t>(n + 1) : nullptr;
-            if (!sb.lo[x] || !sb.id[x] || (has_hi && !sb.hi[x]))
+            sb.hi[x] = has_hi && !(grouped && x) ? A.alloc_persistent<uint8_t>(n + 1) : nullptr;
+            if (!sb.lo[x] || !sb.id[x] || (has_hi && !(grouped && x) && !sb.hi[x]))
                 return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)n);
         }
         for (const KcPiece &q : kc)
@@ -394,9 +429,29 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
         for (auto &x : kc) free_kc_piece(A, x);
         A.release_scratch();
     }
-    // ---- sort: every sample's tuples by (k-mer, adjacency), within the sample's range
+    // ---- sort: every sample's tuples by (k-mer, adjacency), within the sample's range, or split into units
     int lo_buf = 0, hi_buf = 0;
-    {
+    if (grouped) {
+        const double ms0 = b->stage_ms[3];
+        gs.k = k;
+        gs.n = T_all;
+        gs.d_hist = shist;
+        gs.lo = 0;
+        gs.hi = (uint64_t)nseg * NB;
+        gs.bounds = rb;
+        gs.seg_tstart = segs.tstart;
+        {
+            StageTimer tm(st, b->stage_ms, 3);
+            if ((rc = group_plan(gs, A, st))) return rc;
+            if ((rc = group_split(gs, sb.lo[0], sb.hi[0], sb.id[0], sb.lo[1], sb.id[1], A, st))) return rc;
+        }
+        lo_buf = gs.two_level ? 0 : 1;
+        hi_buf = 1;
+        b->sort_pass_ms += b->stage_ms[3] - ms0;
+        b->sort_bytes += T_all * (uint64_t)((has_hi ? 25 : 24) + (gs.two_level ? 24 : 0));
+        b->sort_passes += gs.two_level ? 2 : 1;
+        b->sort_tuples += T_all;
+    } else {
         StageTimer tm(st, b->stage_ms, 3);
         SortStats ss;
         if ((rc = bucket_sort(sb, T_all, has_hi, k, shist, 0, (uint64_t)nseg * NB, A, st, &ss, &lo_buf, &hi_buf, &segs)))
@@ -414,7 +469,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     tp.n = T_all;
     // free the other buffer's big arrays (the filter and the union read only the sorted ones)
     A.free_persistent(sb.lo[lo_buf ^ 1]);
-    A.free_persistent(sb.id[lo_buf ^ 1]);
+    if (!grouped) A.free_persistent(sb.id[lo_buf ^ 1]);  // (the grouped ids go there)
     if (has_hi) A.free_persistent(sb.hi[hi_buf ^ 1]);
     // ---- filter and unions over every thread range of every sample
     uint32_t *parent = A.alloc_persistent<uint32_t>(N + 1), *size = A.alloc_persistent<uint32_t>(N + 1);
@@ -422,11 +477,26 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     if (!parent || !size || !filtered) return set_error(MP_ENOMEM, "device memory for the forest");
     launch_init_parent(parent, N, st);
     MP_CUDA(cudaMemsetAsync(filtered, 0, N + 1, st));
-    {
-        StageTimer tm(st, b->stage_ms, 4);
-        if ((rc = filter_scan(tp, rb, parent, filtered, A, st, false, true))) return rc;
-    }
-    {
+    if (grouped) {
+        {
+            StageTimer tm(st, b->stage_ms, 4);
+            if ((rc = group_filter(gs, tp.lo, tp.id, sb.id[lo_buf ^ 1], parent, filtered, A, st))) return rc;
+        }
+        StageTimer tm(st, b->stage_ms, 5);
+        std::vector<GroupQuirk> open;
+        if ((rc = group_union(gs, sb.id[lo_buf ^ 1], parent, filtered, N, A, st, open))) return rc;
+        for (const GroupQuirk &q : open) {
+            uint32_t first = 0, hooked = 0;
+            if ((rc = sample_first_read(d_fq, pr, R[q.seg], R[q.seg + 1], k, shist + (size_t)q.seg * NB, err, A, st, &first)))
+                return rc;
+            if ((rc = group_finish(parent, N, first, q.anchor, A, st, &hooked))) return rc;
+        }
+        A.free_persistent(sb.id[lo_buf ^ 1]);
+    } else {
+        {
+            StageTimer tm(st, b->stage_ms, 4);
+            if ((rc = filter_scan(tp, rb, parent, filtered, A, st, false, true))) return rc;
+        }
         std::vector<uint32_t> rseg(Rn);
         for (int q = 0; q < nseg; q++)
             for (uint32_t t = hrb0[q]; t < hrb0[q + 1]; t++) rseg[t] = (uint32_t)q;
@@ -436,7 +506,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     A.release_scratch();
     A.free_persistent(sb.lo[lo_buf]);
     A.free_persistent(sb.id[lo_buf]);
-    if (has_hi) A.free_persistent(sb.hi[hi_buf]);
+    if (has_hi && !grouped) A.free_persistent(sb.hi[hi_buf]);
     A.free_persistent(shist);
     // ---- mate union and every sample's partitions
     std::vector<uint64_t> bounds((size_t)nseg * 17);

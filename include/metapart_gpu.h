@@ -103,8 +103,8 @@ int mp_job_count(mp_job *job, int k, int min3, const uint64_t *chunk_starts, int
 int mp_job_load_count(mp_job *job, const char *bytes, uint64_t nbytes, const uint64_t *file_sizes, int nfiles,
                       int interleaved, int k, int min3, const uint64_t *chunk_starts, int nchunks, uint64_t *hist_out,
                       uint64_t *chunk_reads_out);
-/* Pieces the job's k-mer cache is held in: 0 (no cache), 1 (mp_job_count), or one per upload segment
- * of mp_job_load_count.  Tracing only; no counterpart in the reference. */
+/* Pieces the last count took the job's reads in: 0 (no read store, or the 3-minimizer variant), 1 (mp_job_count), or one
+ * per upload segment of mp_job_load_count.  Tracing only; no counterpart in the reference. */
 int mp_job_kmer_cache_pieces(const mp_job *job);
 
 typedef struct {
@@ -225,9 +225,8 @@ typedef struct {
     int k, min3, num_scans, num_threads;  /* as mp_part_params */
     int num_chunks;                       /* genFastqIdx chunks; a multiple of num_threads */
     int interleaved;                      /* 1: interleaved pairs, 0: single end */
-    int read_store;                       /* MP_STORE_*: what the request's count pass keeps for its partition
-                                             (MP_STORE_PACKED admits the most requests at once: 0.375 bytes per
-                                             base against the k-mer cache's 9 per position) */
+    int read_store;                       /* MP_STORE_*: sets the admission footprint (MP_STORE_PACKED reserves 0.375
+                                             bytes per base, MP_STORE_KMER_CACHE 9 per position) */
 } mp_request_params;
 
 typedef struct {
@@ -271,25 +270,18 @@ int mp_server_stats(mp_server *s, mp_server_stats_t *st);
 /* Runs the queued requests to completion, then stops the workers. */
 void mp_server_destroy(mp_server *s);
 
-/* k-mer cache (default on): mp_job_count of the plain variant keeps every read position's canonical
- * k-mer and adjacency byte (9 bytes per position) in the job, and the next mp_job_partition with the
- * same k filters it per scan instead of recomputing k-mers from the reads; the partition releases it.
- * Skipped without error when device memory or the budget does not allow it.  Turn it off for a
- * count-only job (the drop-in genHistograms).  No counterpart in the reference, whose stages are
- * separate processes. */
+/* mp_job_set_read_store(job, MP_STORE_KMER_CACHE) and (job, MP_STORE_FASTQ).  No counterpart in the reference. */
 int mp_job_set_kmer_cache(mp_job *job, int enable);
 
-/* What the count pass of the plain variant keeps of the reads for the next mp_job_partition of the same k
- * (mp_job_count, mp_job_load_count):
- *   MP_STORE_KMER_CACHE (default): every position's canonical k-mer and adjacency byte, 9 bytes per
- *     position (21.6 GB for 20M reads of 150 bp); the partition's enumeration only filters it;
- *   MP_STORE_PACKED: the reads 2 bits per base with an N mask, 0.375 bytes per base (1.1 GB for the same
- *     reads); the enumeration recomputes the k-mers from them, so it takes longer;
- *   MP_STORE_FASTQ: nothing; the enumeration recomputes the k-mers from the FASTQ bytes.
- * An input with any sequence byte other than A, C, G, T, N keeps no packed copy (the FASTQ path runs); a
- * store that does not fit the budget or the device is skipped.  mp_job_set_kmer_cache(job, 1 / 0) is
- * MP_STORE_KMER_CACHE / MP_STORE_FASTQ.  mp_job_read_store tells which store the job holds now.  No
- * counterpart in the reference, whose stages are separate processes that re-read the FASTQ files. */
+/* The read store that the job's count and partition are asked for:
+ *   MP_STORE_KMER_CACHE (default), MP_STORE_PACKED, or MP_STORE_FASTQ.
+ * The job's FASTQ bytes stay in device memory for its output, and every pass over the k-mers takes them from those
+ * bytes, packing the bases on chip; that is faster than reading stored k-mers (9 bytes per position) or packed reads
+ * was, so no store holds device memory beside the FASTQ bytes.  The choice still sets a request's admission footprint
+ * (mp_request_footprint) and what mp_job_read_store reports: MP_STORE_FASTQ without a count, after a count whose input
+ * MP_STORE_PACKED cannot hold (any sequence byte other than A, C, G, T, N), for the 3-minimizer variant, and after the
+ * partition.  The results are the same with all three.  No counterpart in the reference, whose stages are separate
+ * processes that re-read the FASTQ files. */
 #define MP_STORE_FASTQ 0
 #define MP_STORE_KMER_CACHE 1
 #define MP_STORE_PACKED 2

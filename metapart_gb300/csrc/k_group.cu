@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "k_group.cuh"
+#include "k_readtile.cuh"
 
 namespace mp {
 
@@ -218,39 +219,73 @@ __global__ void __launch_bounds__(1024) k_gp_tiles(const uint32_t *bstart, uint3
     if (threadIdx.x == 0) ctr[GC_TILES] = (uint32_t)carry;
 }
 
-template <int DIGITS> struct SplitSmem {
-    uint64_t key[SP_TILE];
-    uint32_t id[SP_TILE];
-    uint16_t dig[SP_TILE];
-    uint32_t b0[DIGITS];     // first bucket of every digit (the last ones repeat ~0)
-    uint32_t hist[DIGITS];   // tuples per digit, then the digit's first place in the tile
-    uint32_t delta[DIGITS];  // global place of a digit's first tuple less its place in the tile
-    uint32_t ws[SP_THREADS / 32];
-};
-static_assert(2 * (sizeof(SplitSmem<GP_MAX_UNITS>) + 1024) <= 228 * 1024, "two split blocks per SM");
+// Digit lookup: a segment's (or a bin's) bucket range in CELLS cells of 2^shift buckets, each with the digits of its first
+// and its last bucket (low and high half); where they differ, a search between them.  One shared-memory read per tuple
+// in nearly all cases: a binary search over the digits' first buckets instead (10 dependent reads) held the passes to
+// 2.6 TB/s with the shared-memory pipe 83 % busy.
+constexpr uint32_t CELLS_1 = 2048, CELLS_2 = 1024;
 
-// The largest i with b0[i] <= x (b0 ascending, padded with ~0 to a power of two above `top`).
-__device__ __forceinline__ uint32_t digit_at(const uint32_t *b0, uint32_t top, uint32_t x)
+__host__ __device__ __forceinline__ int cell_shift(uint64_t span, uint32_t cells)
 {
-    uint32_t p = 0;
-    for (uint32_t st = top; st; st >>= 1)
-        if (b0[p + st] <= x) p += st;
-    return p;
+    int s = 0;
+    while (((span - 1) >> s) >= cells) s++;
+    return s;
 }
 
-// Unstable, so there are no ballots and no look-back; tiles of 6144 tuples keep a digit's stores at 100 bytes and
-// more.  Two passes take 59.4 ms at 20M x 150 bp, 2 scans (2.39 G tuples, 49 bytes each).
-//
-// From per-thread tuples (key, digit, valid) to contiguous runs per digit: ranks by shared-memory atomics, places
-// by one global atomic per digit and tile (the order of a digit's tuples is free), a shared-memory reorder so that
-// the stores of a digit's tuples are contiguous.
-template <int DIGITS, class LoadId>
-__device__ __forceinline__ void split_tile(SplitSmem<DIGITS> &sm, const uint64_t (&key)[SP_ITEMS], uint32_t (&rd)[SP_ITEMS],
-                                           uint32_t nv, uint32_t *cur, LoadId load_id, uint64_t *out_k,
-                                           uint32_t *out_id, uint32_t n)
+__global__ void __launch_bounds__(256) k_gp_cells(const uint32_t *bb0, const uint32_t *seg_bin0, uint32_t b_lo, uint32_t b_hi,
+                                                  int shift, uint32_t *cells)
+{
+    const uint32_t seg = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= CELLS_1) return;
+    const uint32_t d0 = seg_bin0[seg], nd = seg_bin0[seg + 1] - d0;
+    uint32_t v[2];
+    for (int q = 0; q < 2; q++) {
+        const uint64_t x = min((uint64_t)b_hi - 1, b_lo + ((uint64_t)(c + q) << shift) - q);
+        uint32_t a = 0, z = nd - 1;  // the last bin whose first bucket is at or below x
+        while (a < z) {
+            const uint32_t m = (a + z + 1) >> 1;
+            if ((bb0[d0 + m] & (NB - 1)) <= x) a = m; else z = m - 1;
+        }
+        v[q] = a;
+    }
+    cells[(size_t)seg * CELLS_1 + c] = v[0] | (v[1] << 16);
+}
+
+template <class B>
+__device__ __forceinline__ uint32_t cell_digit(const uint32_t *cells, const B *b0, int shift, uint32_t rel, uint32_t b)
+{
+    const uint32_t v = cells[rel >> shift];
+    uint32_t a = v & 0xFFFFu, z = v >> 16;
+    while (a < z) {
+        const uint32_t m = (a + z + 1) >> 1;
+        if (b0[m] <= b) a = m; else z = m - 1;
+    }
+    return a;
+}
+
+template <int DIGITS, class B, uint32_t CELLS> struct SplitSmem {
+    uint64_t key[SP_TILE];   // (the packed reads of k_enum_bins before)
+    uint32_t id[SP_TILE];
+    uint16_t dig[SP_TILE];
+    B b0[DIGITS];            // first bucket of every digit
+    uint32_t hist[DIGITS];   // tuples per digit, then the digit's first place in the tile
+    uint32_t delta[DIGITS];  // global place of a digit's first tuple less its place in the tile
+    uint32_t cells[CELLS];
+    uint32_t ws[SP_THREADS / 32];
+};
+typedef SplitSmem<GP_MAX_BINS, uint32_t, CELLS_1> BinSmem;
+template <int DIGITS> using UnitSmem = SplitSmem<DIGITS, uint16_t, CELLS_2>;
+static_assert(2 * (sizeof(BinSmem) + 1024) <= 228 * 1024 && 2 * (sizeof(UnitSmem<GP_MAX_UNITS>) + 1024) <= 228 * 1024,
+              "two split blocks per SM");
+
+// Unstable, so there are no ballots and no look-back: ranks by shared-memory atomics, places by one global atomic per
+// digit and tile (the order of a digit's tuples is free), a shared-memory reorder so that a digit's tuples are stored
+// side by side.  rd: digit in (0xFFFF = no tuple).
+template <class Smem, int DIGITS, class LoadId>
+__device__ __forceinline__ void split_tile(Smem &sm, const uint64_t (&key)[SP_ITEMS], uint32_t (&rd)[SP_ITEMS], uint32_t *cur,
+                                           uint32_t nd, LoadId load_id, uint64_t *out_k, uint32_t *out_id, uint32_t n)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // rd: digit in (0xFFFF = none), digit | rank << 16 out
 #pragma unroll
     for (int j = 0; j < SP_ITEMS; j++)
         if (rd[j] != 0xFFFFu) rd[j] |= atomicAdd(&sm.hist[rd[j]], 1u) << 16;
@@ -265,6 +300,9 @@ __device__ __forceinline__ void split_tile(SplitSmem<DIGITS> &sm, const uint64_t
         c[q] = sm.hist[tid * PER + q];
         s += c[q];
     }
+    uint32_t g[PER];
+#pragma unroll
+    for (int q = 0; q < PER; q++) g[q] = c[q] && tid * PER + q < nd ? atomicAdd(&cur[tid * PER + q], c[q]) : 0u;
     uint32_t x = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -272,12 +310,13 @@ __device__ __forceinline__ void split_tile(SplitSmem<DIGITS> &sm, const uint64_t
         if (lane >= o) x += y;
     }
     if (lane == 31) sm.ws[warp] = x;
-    uint32_t g[PER];
-#pragma unroll
-    for (int q = 0; q < PER; q++) g[q] = c[q] ? atomicAdd(&cur[tid * PER + q], c[q]) : 0u;
     __syncthreads();
-    uint32_t before = x - s;
-    for (int w = 0; w < warp; w++) before += sm.ws[w];
+    uint32_t before = x - s, nv = 0;
+    for (int w = 0; w < SP_THREADS / 32; w++) {
+        const uint32_t v = sm.ws[w];
+        before += w < warp ? v : 0u;
+        nv += v;
+    }
 #pragma unroll
     for (int q = 0; q < PER; q++) {
         sm.hist[tid * PER + q] = before;
@@ -303,10 +342,14 @@ __device__ __forceinline__ void split_tile(SplitSmem<DIGITS> &sm, const uint64_t
             out_id[o] = sm.id[p];
         }
     }
+#pragma unroll
+    for (int q = 0; q < PER; q++) sm.hist[tid * PER + q] = 0;  // (read last before the barrier above)
 }
 
+// The tiles of a pass over segments: tile0[q] the segment's first tile, start[q] its first read or tuple, tile_seg the
+// segment of every tile; null for one segment.
 struct SegTiles {
-    const uint32_t *tile_seg = nullptr, *tile0 = nullptr, *tstart = nullptr;  // null: one segment from tuple 0
+    const uint32_t *tile_seg = nullptr, *tile0 = nullptr, *start = nullptr;
 };
 
 __global__ void k_gp_segtiles(const uint32_t *tile0, int nseg, uint32_t *tile_seg)
@@ -315,93 +358,186 @@ __global__ void k_gp_segtiles(const uint32_t *tile0, int nseg, uint32_t *tile_se
     for (uint32_t t = tile0[q] + threadIdx.x; t < tile0[q + 1]; t += blockDim.x) tile_seg[t] = (uint32_t)q;
 }
 
-// First pass: enumerated tuples (lo = k-mer << 8 | adj, hi = k-mer >> 56) into bins.
-__global__ void __launch_bounds__(SP_THREADS, 2) k_split_bins(const uint64_t *__restrict__ lo, const uint8_t *__restrict__ hi,
-                                                              const uint32_t *__restrict__ id, uint32_t n, int bsh,
-                                                              const uint32_t *__restrict__ bb0, uint32_t *bcur,
-                                                              const uint32_t *__restrict__ seg_bin0, SegTiles sg,
-                                                              uint64_t *out_k, uint32_t *out_id)
+// First pass, one of two sources: the reads (k_readtile.cuh; the tuples of the buckets [b_lo, b_hi)), or tuples enumerated
+// before (lo = k-mer << 8 | adj, hi = k-mer >> 56; the 3-minimizer variant).
+struct BinCtx {
+    ReadTiles t;
+    uint32_t n_reads = 0, check_many = 0;
+    const uint32_t *label = nullptr;
+    const uint64_t *lo = nullptr;
+    const uint8_t *hi = nullptr;
+    const uint32_t *id = nullptr;
+    uint32_t tiles = 0, n = 0, b_lo = 0, b_hi = 0;
+    int bsh = 0, shift = 0;
+    const uint32_t *bb0 = nullptr, *seg_bin0 = nullptr, *cells = nullptr;
+    uint32_t *bcur = nullptr, *err = nullptr;
+    SegTiles sg;
+    uint64_t *out_k = nullptr;
+    uint32_t *out_id = nullptr;
+};
+
+template <bool READS>
+__global__ void __launch_bounds__(SP_THREADS, 2) k_split_bins(BinCtx c)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    SplitSmem<GP_MAX_BINS> &sm = *reinterpret_cast<SplitSmem<GP_MAX_BINS> *>(smraw);
+    BinSmem &sm = *reinterpret_cast<BinSmem *>(smraw);
+    __shared__ uint32_t many[READS ? SP_THREADS : 1];
     const int tid = threadIdx.x;
-    uint32_t base = blockIdx.x * SP_TILE, end = n, seg = 0;
-    if (sg.tile_seg) {
-        seg = sg.tile_seg[blockIdx.x];
-        base = sg.tstart[seg] + (blockIdx.x - sg.tile0[seg]) * SP_TILE;
-        end = sg.tstart[seg + 1];
-    }
-    const uint32_t nv = min((uint32_t)SP_TILE, end - base);
-    const uint32_t d0 = seg_bin0[seg], nd = seg_bin0[seg + 1] - d0;
-    for (uint32_t d = tid; d < GP_MAX_BINS; d += SP_THREADS) {
-        sm.b0[d] = d < nd ? bb0[d0 + d] & (NB - 1) : ~0u;
-        sm.hist[d] = 0;
-    }
-    uint64_t key[SP_ITEMS];
-    uint32_t rd[SP_ITEMS];
+    const uint64_t lowmask = (1ull << c.bsh) - 1;
+    uint32_t have = ~0u, d0 = 0, nd = 0;  // the segment whose digits are in shared memory
+    for (uint32_t d = tid; d < GP_MAX_BINS; d += SP_THREADS) sm.hist[d] = 0;
+    for (uint32_t tile = blockIdx.x; tile < c.tiles; tile += gridDim.x) {
+        const uint32_t seg = c.sg.tile_seg ? c.sg.tile_seg[tile] : 0u;
+        const uint32_t per = READS ? c.t.rpt : (uint32_t)SP_TILE;
+        uint32_t base = tile * per, end = READS ? c.n_reads : c.n;
+        if (c.sg.tile_seg) {
+            base = c.sg.start[seg] + (tile - c.sg.tile0[seg]) * per;
+            end = c.sg.start[seg + 1];
+        }
+        __syncthreads();  // the tile before is stored
+        if (seg != have) {
+            have = seg;
+            d0 = c.seg_bin0[seg];
+            nd = c.seg_bin0[seg + 1] - d0;
+            for (uint32_t d = tid; d < nd; d += SP_THREADS) sm.b0[d] = c.bb0[d0 + d] & (NB - 1);
+            for (uint32_t d = tid; d < CELLS_1; d += SP_THREADS) sm.cells[d] = c.cells[(size_t)seg * CELLS_1 + d];
+        }
+        uint64_t key[SP_ITEMS];
+        uint32_t rd[SP_ITEMS];
+        if constexpr (READS) {
+            uint32_t *packed = reinterpret_cast<uint32_t *>(sm.key);
+            const uint32_t r1 = min(end, base + per);
+            if (c.check_many) many[tid] = 0;
+            rt_pack(c.t, base, r1, packed);
+            __syncthreads();
 #pragma unroll
-    for (int j = 0; j < SP_ITEMS; j++) {
-        const uint32_t e = j * SP_THREADS + tid;
-        key[j] = e < nv ? lo[base + e] : 0ull;
-        rd[j] = (hi && e < nv) ? (uint32_t)hi[base + e] : 0u;
-    }
-    __syncthreads();
-    const uint32_t top = nd > 1 ? 1u << (31 - __clz(nd - 1)) : 0u;
-    const uint64_t lowmask = (1ull << bsh) - 1;
+            for (int j = 0; j < SP_ITEMS; j++) rd[j] = 0xFFFFu;
+            const uint32_t rr = tid / c.t.spr, i0 = (tid - rr * c.t.spr) * c.t.P, r = base + rr;
+            const uint32_t L = rr < per && r < r1 ? c.t.seq_len[r] : 0u;
+            uint32_t id = r;
+            if (L > (uint32_t)c.t.k && i0 <= L - (uint32_t)c.t.k) {
+                if (c.label) {
+                    const uint32_t p = c.label[r];
+                    id = p == BAD ? r : p;  // findRoot after full compression (metapart.c:543-568)
+                }
+                KmerRoll s;
+                kr_init(s, c.t, packed + rr * rt_stride(c.t), L, i0);
+                const uint32_t m = min(c.t.P, s.last + 1 - i0);
+                uint32_t got = 0;
 #pragma unroll
-    for (int j = 0; j < SP_ITEMS; j++) {
-        const uint64_t km = (key[j] >> 8) | ((uint64_t)rd[j] << 56);
-        const uint32_t b = (uint32_t)(km >> bsh);
-        const uint32_t d = digit_at(sm.b0, top, b);
-        key[j] = ((((uint64_t)(b - sm.b0[d]) << bsh) | (km & lowmask)) << 6) | (key[j] & 63u);
-        rd[j] = j * SP_THREADS + tid < nv ? d : 0xFFFFu;
+                for (int j = 0; j < SP_ITEMS; j++) {
+                    if (j < m) {
+                        uint64_t km;
+                        const bool v = kr_get(s, c.t.k, km);
+                        const uint32_t b = (uint32_t)(km >> c.bsh);
+                        if (v && b >= c.b_lo && b < c.b_hi) {
+                            const uint32_t d = cell_digit(sm.cells, sm.b0, c.shift, b - c.b_lo, b);
+                            key[j] = ((((uint64_t)(b - sm.b0[d]) << c.bsh) | (km & lowmask)) << 6) | kr_adj6(s);
+                            rd[j] = d;
+                            got++;
+                        }
+                        kr_next(s, c.t.k);
+                    }
+                }
+                // the reference counts a read's k-mers of one scan in 8 bits (enumerateKmers.c:152)
+                if (c.check_many && atomicAdd(&many[rr], got) + got > 255u) atomicOr(c.err, 4u);
+            }
+            split_tile<BinSmem, GP_MAX_BINS>(sm, key, rd, c.bcur + d0, nd, [&](int) { return id; }, c.out_k, c.out_id, c.n);
+        } else {
+            const uint32_t nv = min((uint32_t)SP_TILE, end - base);
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < SP_ITEMS; j++) {
+                const uint32_t e = j * SP_THREADS + tid;
+                rd[j] = 0xFFFFu;
+                if (e < nv) {
+                    const uint64_t v = c.lo[base + e], km = (v >> 8) | (c.hi ? (uint64_t)c.hi[base + e] << 56 : 0ull);
+                    const uint32_t b = min(max((uint32_t)(km >> c.bsh), c.b_lo), c.b_hi - 1);
+                    const uint32_t d = cell_digit(sm.cells, sm.b0, c.shift, b - c.b_lo, b);
+                    key[j] = ((((uint64_t)(b - sm.b0[d]) << c.bsh) | (km & lowmask)) << 6) | (v & 63u);
+                    rd[j] = d;
+                }
+            }
+            split_tile<BinSmem, GP_MAX_BINS>(
+                sm, key, rd, c.bcur + d0, nd,
+                [&](int j) { const uint32_t e = j * SP_THREADS + tid; return e < nv ? c.id[base + e] : 0u; }, c.out_k, c.out_id, c.n);
+        }
     }
-    split_tile<GP_MAX_BINS>(sm, key, rd, nv, bcur + d0,
-                            [&](int j) { const uint32_t e = j * SP_THREADS + tid; return e < nv ? id[base + e] : 0u; }, out_k,
-                            out_id, n);
 }
 
-// Second pass: a bin's tuples into its units.
-template <uint32_t DIGITS, int BLOCKS>
+// Second pass: a bin's tuples into its units.  A block takes consecutive tiles, so it sets up a bin's digits once.
+template <int DIGITS, int BLOCKS>
 __global__ void __launch_bounds__(SP_THREADS, BLOCKS) k_split_units(const uint64_t *__restrict__ kk, const uint32_t *__restrict__ id,
-                                                               uint32_t n, int bsh, const uint32_t *__restrict__ ctr,
-                                                               const uint32_t *__restrict__ bstart,
-                                                               const uint32_t *__restrict__ bb0,
-                                                               const uint32_t *__restrict__ bu0,
-                                                               const uint32_t *__restrict__ bcur,
-                                                               const uint32_t *__restrict__ ub0, uint32_t *ucur,
-                                                               const uint32_t *__restrict__ tile_bin,
-                                                               const uint32_t *__restrict__ tile_first, uint64_t *out_k,
-                                                               uint32_t *out_id)
+                                                                    uint32_t n, int bsh, const uint32_t *__restrict__ ctr,
+                                                                    const uint32_t *__restrict__ bstart,
+                                                                    const uint32_t *__restrict__ bb0,
+                                                                    const uint32_t *__restrict__ bu0,
+                                                                    const uint32_t *__restrict__ bcur,
+                                                                    const uint32_t *__restrict__ ub0, uint32_t *ucur,
+                                                                    const uint32_t *__restrict__ tile_bin,
+                                                                    const uint32_t *__restrict__ tile_first, uint64_t *out_k,
+                                                                    uint32_t *out_id)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    SplitSmem<DIGITS> &sm = *reinterpret_cast<SplitSmem<DIGITS> *>(smraw);
-    if (blockIdx.x >= ctr[GC_TILES]) return;
+    UnitSmem<DIGITS> &sm = *reinterpret_cast<UnitSmem<DIGITS> *>(smraw);
     const int tid = threadIdx.x;
-    const uint32_t bin = tile_bin[blockIdx.x];
-    if (bcur[bin] != bstart[bin + 1]) return;  // the histogram is not the tuples' (its units stay short: k_group)
-    const uint32_t base = bstart[bin] + (blockIdx.x - tile_first[bin]) * SP_TILE;
-    const uint32_t nv = min((uint32_t)SP_TILE, bstart[bin + 1] - base);
-    const uint32_t d0 = bu0[bin], nd = min(bu0[bin + 1] - d0, DIGITS), first = bb0[bin];
-    for (uint32_t d = tid; d < DIGITS; d += SP_THREADS) {
-        sm.b0[d] = d < nd ? (ub0[d0 + d] & 0x7FFFFFFFu) - first : ~0u;
-        sm.hist[d] = 0;
-    }
-    uint64_t key[SP_ITEMS];
-    uint32_t rd[SP_ITEMS];
+    const uint32_t tiles = ctr[GC_TILES], per = (tiles + gridDim.x - 1) / gridDim.x;
+    const uint32_t t0 = blockIdx.x * per, t1 = min(tiles, t0 + per);
+    uint32_t have = ~0u, d0 = 0, nd = 0, bin_start = 0, bin_end = 0, first_tile = 0;
+    int shift = 0;
+    bool whole = false;
+    for (uint32_t d = tid; d < DIGITS; d += SP_THREADS) sm.hist[d] = 0;
+    for (uint32_t tile = t0; tile < t1; tile++) {
+        const uint32_t bin = tile_bin[tile];
+        __syncthreads();  // the tile before is stored
+        if (bin != have) {
+            have = bin;
+            bin_start = bstart[bin];
+            bin_end = bstart[bin + 1];
+            whole = bcur[bin] == bin_end;  // else the histogram is not the tuples' (the bin's units stay short: k_group)
+            first_tile = tile_first[bin];
+            d0 = bu0[bin];
+            nd = min(bu0[bin + 1] - d0, (uint32_t)DIGITS);
+            const uint32_t first = bb0[bin];
+            for (uint32_t d = tid; d < nd; d += SP_THREADS) sm.b0[d] = (uint16_t)((ub0[d0 + d] & 0x7FFFFFFFu) - first);
+            __syncthreads();
+            const uint32_t span = (uint32_t)sm.b0[nd - 1] + 1;  // buckets from the last unit's first on are its own
+            shift = cell_shift(span, CELLS_2);
+            for (uint32_t c = tid; c < CELLS_2; c += SP_THREADS) {
+                uint32_t v[2];
 #pragma unroll
-    for (int j = 0; j < SP_ITEMS; j++) {
-        const uint32_t e = j * SP_THREADS + tid;
-        key[j] = e < nv ? kk[base + e] : 0ull;
-    }
-    __syncthreads();
-    const uint32_t top = nd > 1 ? 1u << (31 - __clz(nd - 1)) : 0u;
+                for (int q = 0; q < 2; q++) {
+                    const uint32_t x = ((c + q) << shift) - q;
+                    uint32_t a = 0, z = nd - 1;
+                    while (a < z) {
+                        const uint32_t m = (a + z + 1) >> 1;
+                        if (sm.b0[m] <= x) a = m; else z = m - 1;
+                    }
+                    v[q] = a;
+                }
+                sm.cells[c] = v[0] | (v[1] << 16);
+            }
+            __syncthreads();
+        }
+        if (!whole) continue;
+        const uint32_t base = bin_start + (tile - first_tile) * SP_TILE, nv = min((uint32_t)SP_TILE, bin_end - base);
+        const uint32_t top = (uint32_t)sm.b0[nd - 1];
+        uint64_t key[SP_ITEMS];
+        uint32_t rd[SP_ITEMS];
 #pragma unroll
-    for (int j = 0; j < SP_ITEMS; j++)
-        rd[j] = j * SP_THREADS + tid < nv ? digit_at(sm.b0, top, (uint32_t)(key[j] >> (bsh + 6))) : 0xFFFFu;
-    split_tile<DIGITS>(sm, key, rd, nv, ucur + d0,
-                             [&](int j) { const uint32_t e = j * SP_THREADS + tid; return e < nv ? id[base + e] : 0u; }, out_k,
-                             out_id, n);
+        for (int j = 0; j < SP_ITEMS; j++) {
+            const uint32_t e = j * SP_THREADS + tid;
+            key[j] = e < nv ? kk[base + e] : 0ull;
+        }
+#pragma unroll
+        for (int j = 0; j < SP_ITEMS; j++) {
+            const uint32_t b = min((uint32_t)(key[j] >> (bsh + 6)), top);
+            rd[j] = j * SP_THREADS + tid < nv ? cell_digit(sm.cells, sm.b0, shift, b, b) : 0xFFFFu;
+        }
+        split_tile<UnitSmem<DIGITS>, DIGITS>(
+            sm, key, rd, ucur + d0, nd, [&](int j) { const uint32_t e = j * SP_THREADS + tid; return e < nv ? id[base + e] : 0u; },
+            out_k, out_id, n);
+    }
 }
 
 // ------------------------------------------------------------------ group and filter
@@ -856,11 +992,12 @@ static void group_kernel_attrs()
     int dev = 0;
     cudaGetDevice(&dev);
     std::call_once(once[dev & 63], [] {
-        cudaFuncSetAttribute(k_split_bins, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SplitSmem<GP_MAX_BINS>));
+        cudaFuncSetAttribute(k_split_bins<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinSmem));
+        cudaFuncSetAttribute(k_split_bins<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinSmem));
         cudaFuncSetAttribute(k_split_units<GP_MAX_UNITS, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(SplitSmem<GP_MAX_UNITS>));
+                             (int)sizeof(UnitSmem<GP_MAX_UNITS>));
         cudaFuncSetAttribute(k_split_units<GP_MAX_UNITS_L, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(SplitSmem<GP_MAX_UNITS_L>));
+                             (int)sizeof(UnitSmem<GP_MAX_UNITS_L>));
         cudaFuncSetAttribute(k_group<512, 12, 13>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmemS));
         cudaFuncSetAttribute(k_group<1024, 12, 14>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmemL));
     });
@@ -886,6 +1023,8 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
     g.max_bins = g.two_level ? bins_bound(g.n, nseg, g.bin_shift) : g.max_units;
     if (g.two_level) g.max_units += g.max_bins;
     g.max_tiles = (uint32_t)(g.n / SP_TILE) + g.max_bins + 1;
+    g.cell_shift = cell_shift(nseg > 1 ? (uint64_t)NB : nbk, CELLS_1);
+    g.cells = arena.alloc<uint32_t>((size_t)nseg * CELLS_1);
     const uint32_t nblk = blocks_of(nbk, GP_COUNT_BLOCK);
     const size_t brk_words = nbk / 32 + 1;
     uint32_t *brk = arena.alloc<uint32_t>(brk_words + GC_N + (size_t)nseg * QW);
@@ -896,7 +1035,7 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
     g.tile_bin = arena.alloc<uint32_t>((size_t)g.max_tiles + g.max_bins);
     g.mid = arena.alloc<uint32_t>(2 * (size_t)(g.n / GP_CAP_S + 1));
     g.qlist = arena.alloc<uint32_t>(3 * (size_t)(g.max_units + 1));
-    if (!brk || !blk || !d_bounds || !g.ustart || !g.bstart || !g.seg_bin0 || !g.tile_bin || !g.mid || !g.qlist)
+    if (!brk || !blk || !d_bounds || !g.ustart || !g.bstart || !g.seg_bin0 || !g.tile_bin || !g.mid || !g.qlist || !g.cells)
         return set_error(MP_ENOMEM, "device memory for the scan's plan");
     g.ub0 = g.ustart + g.max_units + 1;
     g.ucur = g.ub0 + g.max_units + 1;
@@ -924,44 +1063,91 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
     (count_launch(), k_gp_scan<<<1, 1024, 0, st>>>(blk, nblk, (uint32_t)g.n, nseg, g.ctr, g.ustart, g.bstart, g.bu0, g.seg_bin0));
     (count_launch(), k_gp_write<<<nblk, GP_COUNT_THREADS, 0, st>>>(c, blk, g.ctr, g.ustart, g.ub0, g.ucur, g.bstart, g.bb0, g.bu0,
                                                                   g.bcur, g.seg_bin0, g.mid, g.big));
+    (count_launch(), k_gp_cells<<<dim3(CELLS_1 / 256, nseg), 256, 0, st>>>(g.bb0, g.seg_bin0, nseg > 1 ? 0u : (uint32_t)g.lo,
+                                                                          nseg > 1 ? NB : (uint32_t)g.hi, g.cell_shift, g.cells));
     if (g.two_level) (count_launch(), k_gp_tiles<<<1, 1024, 0, st>>>(g.bstart, g.ctr, g.tile_first, g.tile_bin));
     MP_CUDA(cudaMemcpyAsync(g.hctr, g.ctr, GC_N * 4, cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaGetLastError());
     return 0;
 }
 
-int group_split(GroupScan &g, uint64_t *lo, const uint8_t *hi, uint32_t *id, uint64_t *k2, uint32_t *id2, DeviceArena &arena,
-                cudaStream_t st)
+static int launch_bins(GroupScan &g, BinCtx &c, const std::vector<uint64_t> &seg_start, DeviceArena &arena, cudaStream_t st)
 {
     group_kernel_attrs();
-    const int nseg = (int)g.seg_tstart.size() - 1, bsh = 2 * (g.k - 10);
-    SegTiles sg;
-    uint32_t tiles = blocks_of(g.n, SP_TILE);
+    const int nseg = (int)g.seg_tstart.size() - 1;
+    const bool reads = c.lo == nullptr;
+    const uint32_t per = reads ? c.t.rpt : (uint32_t)SP_TILE;
+    c.tiles = blocks_of(reads ? c.n_reads : g.n, (int)per);
     if (nseg > 1) {
         std::vector<uint32_t> &h = g.h_tiles;
         h.assign(2 * (size_t)nseg + 2, 0);
-        tiles = 0;
+        c.tiles = 0;
         for (int q = 0; q <= nseg; q++) {
-            h[q] = tiles;
-            h[nseg + 1 + q] = (uint32_t)g.seg_tstart[q];
-            if (q < nseg) tiles += blocks_of(g.seg_tstart[q + 1] - g.seg_tstart[q], SP_TILE);
+            h[q] = c.tiles;
+            h[nseg + 1 + q] = (uint32_t)seg_start[q];
+            if (q < nseg) c.tiles += blocks_of(seg_start[q + 1] - seg_start[q], (int)per);
         }
-        uint32_t *d = arena.alloc<uint32_t>(h.size() + tiles);
+        uint32_t *d = arena.alloc<uint32_t>(h.size() + c.tiles);
         if (!d) return set_error(MP_ENOMEM, "device memory for the scan's tiles");
         MP_CUDA(cudaMemcpyAsync(d, h.data(), h.size() * 4, cudaMemcpyHostToDevice, st));
-        sg.tile0 = d;
-        sg.tstart = d + nseg + 1;
-        sg.tile_seg = d + h.size();
+        c.sg.tile0 = d;
+        c.sg.start = d + nseg + 1;
+        c.sg.tile_seg = d + h.size();
         (count_launch(), k_gp_segtiles<<<nseg, 256, 0, st>>>(d, nseg, d + h.size()));
     }
-    (count_launch(), k_split_bins<<<tiles, SP_THREADS, sizeof(SplitSmem<GP_MAX_BINS>), st>>>(
-        lo, hi, id, (uint32_t)g.n, bsh, g.bb0, g.bcur, g.seg_bin0, sg, k2, id2));
-    if (g.two_level && g.bin_shift <= 21)
-        (count_launch(), k_split_units<GP_MAX_UNITS, 2><<<g.max_tiles, SP_THREADS, sizeof(SplitSmem<GP_MAX_UNITS>), st>>>(
-            k2, id2, (uint32_t)g.n, bsh, g.ctr, g.bstart, g.bb0, g.bu0, g.bcur, g.ub0, g.ucur, g.tile_bin, g.tile_first, lo, id));
-    else if (g.two_level)
-        (count_launch(), k_split_units<GP_MAX_UNITS_L, 1><<<g.max_tiles, SP_THREADS, sizeof(SplitSmem<GP_MAX_UNITS_L>), st>>>(
-            k2, id2, (uint32_t)g.n, bsh, g.ctr, g.bstart, g.bb0, g.bu0, g.bcur, g.ub0, g.ucur, g.tile_bin, g.tile_first, lo, id));
+    c.n = (uint32_t)g.n;
+    c.b_lo = nseg > 1 ? 0u : (uint32_t)g.lo;
+    c.b_hi = nseg > 1 ? NB : (uint32_t)g.hi;
+    c.bsh = 2 * (g.k - 10);
+    c.shift = g.cell_shift;
+    c.bb0 = g.bb0;
+    c.seg_bin0 = g.seg_bin0;
+    c.cells = g.cells;
+    c.bcur = g.bcur;
+    c.err = g.ctr + GC_ERR;
+    const unsigned blocks = std::min<unsigned>(c.tiles, 2u * (unsigned)sm_count());
+    if (blocks)
+        (count_launch(), (reads ? k_split_bins<true> : k_split_bins<false>)<<<blocks, SP_THREADS, sizeof(BinSmem), st>>>(c));
+    MP_CUDA(cudaGetLastError());
+    return 0;
+}
+
+int group_bins_reads(GroupScan &g, const uint8_t *fq, const ParsedReads &pr, const std::vector<uint64_t> &seg_reads,
+                     const uint32_t *label, uint64_t *k1, uint32_t *id1, DeviceArena &arena, cudaStream_t st)
+{
+    BinCtx c;
+    c.t = read_tiles(fq, pr, g.k, pr.max_len, SP_THREADS);
+    c.n_reads = (uint32_t)pr.n_reads;
+    c.check_many = pr.max_len > (uint32_t)g.k + 254u;  // a read with 256 positions or more
+    c.label = label;
+    c.out_k = k1;
+    c.out_id = id1;
+    return launch_bins(g, c, seg_reads, arena, st);
+}
+
+int group_bins_tuples(GroupScan &g, const uint64_t *lo, const uint8_t *hi, const uint32_t *id, uint64_t *k1, uint32_t *id1,
+                      DeviceArena &arena, cudaStream_t st)
+{
+    BinCtx c;
+    c.lo = lo;
+    c.hi = hi;
+    c.id = id;
+    c.out_k = k1;
+    c.out_id = id1;
+    return launch_bins(g, c, g.seg_tstart, arena, st);
+}
+
+int group_units(GroupScan &g, const uint64_t *k1, const uint32_t *id1, uint64_t *k2, uint32_t *id2, cudaStream_t st)
+{
+    if (!g.two_level) return 0;
+    const int bsh = 2 * (g.k - 10);
+    const unsigned sms = (unsigned)sm_count();
+    if (g.bin_shift <= 21)
+        (count_launch(), k_split_units<GP_MAX_UNITS, 2><<<std::min(g.max_tiles, 2 * sms), SP_THREADS, sizeof(UnitSmem<GP_MAX_UNITS>), st>>>(
+            k1, id1, (uint32_t)g.n, bsh, g.ctr, g.bstart, g.bb0, g.bu0, g.bcur, g.ub0, g.ucur, g.tile_bin, g.tile_first, k2, id2));
+    else
+        (count_launch(), k_split_units<GP_MAX_UNITS_L, 1><<<std::min(g.max_tiles, sms), SP_THREADS, sizeof(UnitSmem<GP_MAX_UNITS_L>), st>>>(
+            k1, id1, (uint32_t)g.n, bsh, g.ctr, g.bstart, g.bb0, g.bu0, g.bcur, g.ub0, g.ucur, g.tile_bin, g.tile_first, k2, id2));
     MP_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1060,6 +1246,9 @@ int group_union(GroupScan &g, const uint32_t *out, uint32_t *parent, const uint8
     MP_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
     MP_CUDA(cudaGetLastError());
+    if (h[GC_ERR] & 4u)
+        return set_error(MP_EUNSUP, "a read has 256 or more k-mers in one scan (the reference counts them in 8 bits, "
+                                    "enumerateKmers.c:152)");
     if (h[GC_ERR] & 2u) return set_error(MP_EFMT, "the histogram does not match the scan's tuples");
     if (herr) return set_error(MP_EDEVICE, "union-find retry limit reached (flags 0x%x)", herr);
     for (int q = 0; q < nseg; q++) {

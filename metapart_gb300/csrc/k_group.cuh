@@ -28,11 +28,11 @@ struct GroupScan {
 
     // the plan (device), from group_plan
     bool two_level = false;
-    int unit_shift = 0, bin_shift = 0;
+    int unit_shift = 0, bin_shift = 0, cell_shift = 0;
     uint32_t max_units = 0, max_bins = 0, max_tiles = 0;
     uint32_t *ustart = nullptr, *ub0 = nullptr, *ucur = nullptr;  // units: first tuple, first bucket | range start << 31, fill
     uint32_t *bstart = nullptr, *bb0 = nullptr, *bu0 = nullptr, *bcur = nullptr;  // bins: first tuple, bucket, unit; fill
-    uint32_t *seg_bin0 = nullptr, *tile_bin = nullptr, *tile_first = nullptr;
+    uint32_t *seg_bin0 = nullptr, *tile_bin = nullptr, *tile_first = nullptr, *cells = nullptr;
     uint32_t *mid = nullptr, *big = nullptr;  // units above a small block's and above a large block's capacity
     uint32_t *lrs = nullptr;                  // per segment: first tuple of its last range with tuples
     uint32_t *ctr = nullptr;                  // GC_* counters
@@ -57,10 +57,15 @@ struct GroupQuirk {
 bool group_fits(uint64_t n, uint64_t n_reads, const SortSegments *segs);
 // Plans g (its inputs set) on the device, its counts copied into g.hctr in stream order.
 int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st);
-// Splits the tuples of (lo, hi, id) (enumeration order, segment-major) into units; the result is in
-// (k2, id2) with one level, back in (lo, id) with two.
-int group_split(GroupScan &g, uint64_t *lo, const uint8_t *hi, uint32_t *id, uint64_t *k2, uint32_t *id2, DeviceArena &arena,
-                cudaStream_t st);
+// First split pass, into bins (into units when one level does: g.two_level false), of n tuples to (k1, id1): enumerated
+// from the reads (seg_reads: nseg + 1 read offsets; label: the reads' components, null in the first scan; every read at
+// most 300 positions), or of tuples enumerated before, segment-major.
+int group_bins_reads(GroupScan &g, const uint8_t *fq, const ParsedReads &pr, const std::vector<uint64_t> &seg_reads,
+                     const uint32_t *label, uint64_t *k1, uint32_t *id1, DeviceArena &arena, cudaStream_t st);
+int group_bins_tuples(GroupScan &g, const uint64_t *lo, const uint8_t *hi, const uint32_t *id, uint64_t *k1, uint32_t *id1,
+                      DeviceArena &arena, cudaStream_t st);
+// Second pass, with two levels: the bins' tuples into units.
+int group_units(GroupScan &g, const uint64_t *k1, const uint32_t *id1, uint64_t *k2, uint32_t *id2, cudaStream_t st);
 // The mischief filter over the split tuples (kk, ids), and every k-mer's reads side by side in out (n ids).
 int group_filter(GroupScan &g, const uint64_t *kk, const uint32_t *ids, uint32_t *out, uint32_t *parent, uint8_t *filtered,
                  DeviceArena &arena, cudaStream_t st);

@@ -203,10 +203,15 @@ __global__ void __launch_bounds__(NL_THREADS) k_nl_write(const uint8_t *buf, uin
 }
 
 // Record table from the newline positions; flags quality/sequence length mismatches.
+// stat: [0] first record with a mismatch, [1] the longest sequence.
 __global__ void k_records(const uint64_t *nl, uint64_t n_rec, uint64_t *rec_start, uint64_t *seq_off, uint32_t *seq_len,
-                          unsigned long long *first_bad)
+                          unsigned long long *stat)
 {
     uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t here = r < n_rec ? (uint32_t)min(nl[4 * r + 1] - nl[4 * r] - 1, (uint64_t)0xFFFFFFFFull) : 0u;
+    const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, here);
+    if ((threadIdx.x & 31) == 0 && most > (uint32_t)*(volatile unsigned long long *)&stat[1])
+        atomicMax(&stat[1], (unsigned long long)most);
     if (r >= n_rec) return;
     uint64_t s = r ? nl[4 * r - 1] + 1 : 0;
     uint64_t sq = nl[4 * r] + 1;
@@ -216,7 +221,7 @@ __global__ void k_records(const uint64_t *nl, uint64_t n_rec, uint64_t *rec_star
     rec_start[r] = s;
     seq_off[r] = sq;
     seq_len[r] = (uint32_t)sl;
-    if (ql != sl || sl > 0xFFFFFFFFull) atomicMin(first_bad, (unsigned long long)r);
+    if (ql != sl || sl > 0xFFFFFFFFull) atomicMin(&stat[0], (unsigned long long)r);
     if (r == n_rec - 1) rec_start[n_rec] = nl[4 * r + 3] + 1;
 }
 
@@ -270,17 +275,19 @@ int parse_fastq_range(const uint8_t *d_base, uint64_t begin, uint64_t end, Parse
     pr->rec_start = arena.alloc_persistent<uint64_t>(n_rec + 1);
     pr->seq_off = arena.alloc_persistent<uint64_t>(n_rec);
     pr->seq_len = arena.alloc_persistent<uint32_t>(n_rec);
-    unsigned long long *bad = arena.alloc<unsigned long long>(1);
+    unsigned long long *bad = arena.alloc<unsigned long long>(2);
     if (!pr->rec_start || !pr->seq_off || !pr->seq_len || !bad) return set_error(MP_ENOMEM, "device memory for the record table");
     MP_CUDA(cudaMemsetAsync(bad, 0xFF, sizeof *bad, st));
+    MP_CUDA(cudaMemsetAsync(bad + 1, 0, sizeof *bad, st));
     (mp::count_launch(), k_records<<<(unsigned)((n_rec + 255) / 256), 256, 0, st>>>(nl, n_rec, pr->rec_start, pr->seq_off, pr->seq_len, bad));
-    unsigned long long hb = 0;
+    unsigned long long hb[2] = {0, 0};
     uint64_t last_end = 0;
-    MP_CUDA(cudaMemcpyAsync(&hb, bad, sizeof hb, cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaMemcpyAsync(hb, bad, sizeof hb, cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaMemcpyAsync(&last_end, pr->rec_start + n_rec, sizeof last_end, cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
     MP_CUDA(cudaGetLastError());
-    if (hb != ~0ull) return set_error(MP_EFMT, "FASTQ record %llu: quality length differs from the sequence length", hb);
+    if (hb[0] != ~0ull) return set_error(MP_EFMT, "FASTQ record %llu: quality length differs from the sequence length", hb[0]);
+    pr->max_len = (uint32_t)hb[1];
     if (last_end != n) return set_error(MP_EFMT, "FASTQ input does not end with a complete record");
     arena.release_scratch();
     return 0;

@@ -99,6 +99,7 @@ struct ParsedReads {
     uint64_t *rec_start = nullptr;  // n_reads + 1 record start offsets (last = input size)
     uint64_t *seq_off = nullptr;    // sequence line offset of each record
     uint32_t *seq_len = nullptr;    // sequence length of each record
+    uint32_t max_len = 0;           // the longest
 };
 
 int parse_fastq(const uint8_t *d_buf, uint64_t n, ParsedReads *pr, DeviceArena &arena, cudaStream_t st);

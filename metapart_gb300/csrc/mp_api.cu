@@ -68,110 +68,6 @@ void launch_init_parent(uint32_t *parent, uint64_t n, cudaStream_t st)
     if (n) (count_launch(), k_init_parent<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(parent, n));
 }
 
-void free_kc_piece(DeviceArena &arena, KcPiece &q)
-{
-    arena.free_persistent(q.off);
-    arena.free_persistent(q.lo);
-    arena.free_persistent(q.hi);
-    arena.free_persistent(q.poff);
-    arena.free_persistent(q.pw);
-    arena.free_persistent(q.pn);
-    q = KcPiece{};
-}
-
-bool make_pk_piece(DeviceArena &arena, cudaStream_t st, const ParsedReads &pr, uint64_t r0, int k, KcPiece *out)
-{
-    const uint64_t N = pr.n_reads;
-    KcPiece q;
-    q.r0 = r0;
-    q.n = N;
-    uint32_t *nr = arena.alloc<uint32_t>(N + 1);
-    uint64_t *tot = arena.alloc<uint64_t>(1);
-    size_t tb = scan_tmp_bytes(N + 1);
-    void *tmp = arena.alloc<uint8_t>(tb);
-    q.poff = arena.alloc_persistent<uint64_t>(N + 2);
-    uint64_t P = 0;
-    bool ok = nr && tot && tmp && q.poff;
-    if (ok) {
-        launch_pk_rounds(pr, k, nr, st);
-        ok = cudaMemsetAsync(nr + N, 0, 4, st) == cudaSuccess;
-    }
-    if (ok) {
-        scan_u32_to_u64(nr, q.poff, N + 1, tot, tmp, tb, st);
-        ok = cudaMemcpyAsync(&P, tot, 8, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
-             cudaStreamSynchronize(st) == cudaSuccess;
-    }
-    if (ok) {
-        q.pw = arena.alloc_persistent<uint64_t>(P + 1);
-        q.pn = arena.alloc_persistent<uint32_t>(P + 1);
-        ok = q.pw && q.pn;
-    }
-    arena.free_scratch(nr);
-    arena.free_scratch(tot);
-    arena.free_scratch(tmp);
-    if (!ok) {
-        free_kc_piece(arena, q);
-        return false;
-    }
-    *out = q;
-    return true;
-}
-
-// The enumeration over one piece of the count pass's copy of the reads (either form): every scan's
-// per-read tuple counts (cnt indexed by global read id), and one bucket range's tuples at off.
-int store_count_scans(const KcPiece &q, const uint32_t *seq_len, int k, const uint32_t *bounds, int S, uint32_t *cnt,
-                      uint64_t stride, uint32_t *err, cudaStream_t st)
-{
-    if (!q.n) return 0;
-    if (q.pw) return launch_pk_count_scans(q.poff, q.pw, q.pn, q.r0, q.n, seq_len, k, bounds, S, cnt, stride, err, st);
-    return launch_kc_count_scans(q.off, q.lo, q.hi, q.n, k, bounds, S, cnt + q.r0, stride, err, st);
-}
-
-void store_write(const KcPiece &q, const uint32_t *seq_len, int k, uint32_t lo, uint32_t hi, const uint32_t *label,
-                 const uint64_t *off, uint64_t *o_lo, uint8_t *o_hi, uint32_t *o_id, uint32_t *err, cudaStream_t st)
-{
-    if (q.pw) launch_pk_write(q.poff, q.pw, q.pn, q.r0, q.n, seq_len, k, lo, hi, label, off, o_lo, o_hi, o_id, err, st);
-    else launch_kc_write(q.off, q.lo, q.hi, q.r0, q.n, k, lo, hi, label, off, o_lo, o_hi, o_id, st);
-}
-
-bool make_kc_piece(DeviceArena &arena, cudaStream_t st, const ParsedReads &pr, uint64_t r0, int k, KcPiece *out)
-{
-    const uint64_t N = pr.n_reads;
-    KcPiece q;
-    q.r0 = r0;
-    q.n = N;
-    uint32_t *npos = arena.alloc<uint32_t>(N + 1);
-    uint64_t *tot = arena.alloc<uint64_t>(1);
-    size_t tb = scan_tmp_bytes(N + 1);
-    void *tmp = arena.alloc<uint8_t>(tb);
-    q.off = arena.alloc_persistent<uint64_t>(N + 2);
-    uint64_t P = 0;
-    bool ok = npos && tot && tmp && q.off;
-    if (ok) {
-        launch_kc_positions(pr, k, npos, st);
-        ok = cudaMemsetAsync(npos + N, 0, 4, st) == cudaSuccess;
-    }
-    if (ok) {
-        scan_u32_to_u64(npos, q.off, N + 1, tot, tmp, tb, st);
-        ok = cudaMemcpyAsync(&P, tot, 8, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
-             cudaStreamSynchronize(st) == cudaSuccess;
-    }
-    if (ok) {
-        q.lo = arena.alloc_persistent<uint64_t>(P + 1);
-        q.hi = arena.alloc_persistent<uint8_t>(P + 1);
-        ok = q.lo && q.hi;
-    }
-    arena.free_scratch(npos);
-    arena.free_scratch(tot);
-    arena.free_scratch(tmp);
-    if (!ok) {
-        free_kc_piece(arena, q);
-        return false;
-    }
-    *out = q;
-    return true;
-}
-
 }  // namespace mp
 
 using namespace mp;
@@ -203,11 +99,8 @@ struct mp_job {
     uint32_t *d_parent = nullptr;
     uint32_t *d_size = nullptr;
     uint8_t *d_filtered = nullptr;
-    // k-mer cache written by the count pass (plain variant), in pieces of consecutive reads (one piece,
-    // or one per input segment of mp_job_load_count)
-    int store = STORE_KMER_CACHE;  // what the count pass keeps of the reads for the partition (mp_job_set_read_store)
-    int kc_k = 0;
-    std::vector<KcPiece> kc;
+    int store = STORE_KMER_CACHE;  // mp_job_set_read_store
+    int kc_pieces = 0;  // pieces the plain variant's last count took the reads in (0: none, or a byte its store cannot hold)
     cudaStream_t copy_st = nullptr;  // uploads of mp_job_load_count
     int T = 0, nchunks = 0;
     std::vector<uint64_t> chunk_rec;
@@ -374,30 +267,6 @@ int range_bounds(const uint64_t *hist, const uint64_t *ltr, int T, uint64_t scan
     return 0;
 }
 
-void drop_kmer_cache(mp_job *j)
-{
-    for (KcPiece &q : j->kc) free_kc_piece(j->arena, q);
-    j->kc.clear();
-    j->kc_k = 0;
-}
-
-// The store of the reads for the plain variant's count pass (the job's choice: the k-mer cache or the packed
-// reads), one piece for all reads; false (and no store) when the job keeps none or device memory or the
-// budget does not allow it -- the partition then computes its k-mers from the FASTQ bytes.
-bool make_kmer_cache(mp_job *j, int k)
-{
-    KcPiece q;
-    const bool made = j->store == STORE_PACKED ? make_pk_piece(j->arena, j->st, j->pr, 0, k, &q)
-                                               : make_kc_piece(j->arena, j->st, j->pr, 0, k, &q);
-    if (!made) {
-        drop_kmer_cache(j);
-        return false;
-    }
-    j->kc.assign(1, q);
-    j->kc_k = k;
-    return true;
-}
-
 int chunk_records(mp_job *j, const uint64_t *chunk_starts, int nchunks, std::vector<uint64_t> &rec)
 {
     rec.assign(nchunks + 1, 0);
@@ -553,8 +422,7 @@ int mp_job_reset(mp_job *j)
     j->d_filtered = nullptr;
     j->d_out = nullptr;
     j->out_plan = OutputPlan{};
-    j->kc.clear();
-    j->kc_k = 0;
+    j->kc_pieces = 0;
     j->partitioned = j->output_ready = false;
     return 0;
 }
@@ -572,6 +440,10 @@ int mp_job_count(mp_job *j, int k, int min3, const uint64_t *chunk_starts, int n
     std::vector<uint64_t> rec;
     int rc = chunk_records(j, chunk_starts, nchunks, rec);
     if (rc) return rc;
+    if (!min3 && j->pr.max_len > (uint32_t)k && j->pr.max_len > (uint32_t)MAX_READ_COUNT) {
+        j->kc_pieces = 0;
+        return set_error(MP_EUNSUP, "a read is longer than %d bases", MAX_READ_COUNT);
+    }
     j->stage_ms[1] = 0;
     uint64_t *d_rec = j->arena.alloc<uint64_t>(nchunks + 1);
     unsigned long long *glob = j->arena.alloc<unsigned long long>(NB);
@@ -582,12 +454,10 @@ int mp_job_count(mp_job *j, int k, int min3, const uint64_t *chunk_starts, int n
     MP_CUDA(cudaMemsetAsync(glob, 0, NB * 8, j->st));
     MP_CUDA(cudaMemsetAsync(err, 0, 4, j->st));
     if (cc) MP_CUDA(cudaMemsetAsync(cc, 0, (size_t)nchunks * NB * 4, j->st));
-    drop_kmer_cache(j);
     {
         StageTimer tm(j->st, j->stage_ms, 1);
-        const bool kc = j->store != STORE_FASTQ && !min3 && make_kmer_cache(j, k);
-        const KcPiece q = kc ? j->kc[0] : KcPiece{};
-        launch_count(j->d_fq, j->pr, k, min3, d_rec, nchunks, cc, glob, err, j->st, q.off, q.lo, q.hi, q.poff, q.pw, q.pn);
+        launch_count(j->d_fq, j->pr, k, min3, d_rec, nchunks, cc, glob, err, j->st, j->store == STORE_PACKED);
+        j->kc_pieces = j->store != STORE_FASTQ && !min3 ? 1 : 0;
     }
     std::vector<unsigned long long> g(NB);
     uint32_t herr = 0;
@@ -598,10 +468,10 @@ int mp_job_count(mp_job *j, int k, int min3, const uint64_t *chunk_starts, int n
     MP_CUDA(cudaGetLastError());
     j->arena.release_scratch();
     if (herr & DERR_LONG_READ) {
-        drop_kmer_cache(j);
+        j->kc_pieces = 0;
         return set_error(MP_EUNSUP, "a read is longer than %d bases", MAX_READ_COUNT);
     }
-    if (herr & DERR_NONACGT) drop_kmer_cache(j);  // a byte the packed reads cannot hold: the FASTQ path
+    if (herr & DERR_NONACGT) j->kc_pieces = 0;  // a byte that packed reads cannot hold
     hist_out[0] = 0;
     for (uint32_t b = 1; b <= NB; b++) hist_out[b] = hist_out[b - 1] + g[b - 1];
     if (chunk_reads_out)
@@ -661,7 +531,7 @@ int load_count_pipelined(mp_job *j, const char *bytes, uint64_t nbytes, const ui
     if (!glob || !err) return MP_ENOMEM;
     MP_CUDA(cudaMemsetAsync(glob, 0, NB * 8, j->st));
     MP_CUDA(cudaMemsetAsync(err, 0, 4, j->st));
-    drop_kmer_cache(j);
+    j->kc_pieces = 0;
     std::vector<ParsedReads> prs(S);
     std::vector<uint64_t> R(S + 1, 0);
     for (int i = 0; i < S; i++) {
@@ -671,16 +541,12 @@ int load_count_pipelined(mp_job *j, const char *bytes, uint64_t nbytes, const ui
             if (parse_fastq_range(j->d_fq, seg[i], seg[i + 1], &prs[i], j->arena, j->st)) return MP_EFMT;
         }
         R[i + 1] = R[i] + prs[i].n_reads;
+        j->pr.max_len = std::max(j->pr.max_len, prs[i].max_len);
+        if (prs[i].max_len > (uint32_t)MAX_READ_COUNT) return MP_EUNSUP;
         StageTimer tm(j->st, j->stage_ms, 1);
-        KcPiece q;
-        const bool made = j->store == STORE_PACKED ? make_pk_piece(j->arena, j->st, prs[i], R[i], k, &q)
-                                                   : make_kc_piece(j->arena, j->st, prs[i], R[i], k, &q);
-        if (!made) return MP_ENOMEM;
-        j->kc.push_back(q);
-        launch_count(j->d_fq + seg[i], prs[i], k, 0, nullptr, 0, nullptr, glob, err, j->st, q.off, q.lo, q.hi, q.poff, q.pw,
-                     q.pn);
+        launch_count(j->d_fq + seg[i], prs[i], k, 0, nullptr, 0, nullptr, glob, err, j->st, j->store == STORE_PACKED);
     }
-    j->kc_k = k;
+    j->kc_pieces = S;
     const uint64_t N = R[S];
     if (N >= UMAX32 || (interleaved && (N & 1))) return MP_EFMT;
     {
@@ -716,7 +582,7 @@ int load_count_pipelined(mp_job *j, const char *bytes, uint64_t nbytes, const ui
     j->arena.free_persistent(glob);
     j->arena.free_persistent(err);
     j->arena.release_scratch();
-    if (herr & DERR_NONACGT) drop_kmer_cache(j);  // a byte the packed reads cannot hold: the FASTQ path
+    if (herr & DERR_NONACGT) j->kc_pieces = 0;  // a byte that packed reads cannot hold
     if (herr & ~DERR_NONACGT) return MP_EUNSUP;
     hist_out[0] = 0;
     for (uint32_t b = 1; b <= NB; b++) hist_out[b] = hist_out[b - 1] + g[b - 1];
@@ -846,8 +712,7 @@ static int check_sorted(mp_job *j, const uint64_t *lo, const uint8_t *hi, uint64
 }
 
 static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uint64_t hi, const std::vector<uint64_t> &pcs,
-                          const std::vector<uint64_t> &rb, const uint64_t *hist, const uint64_t *d_hist, bool use_kc,
-                          uint32_t *err)
+                          const std::vector<uint64_t> &rb, const uint64_t *hist, const uint64_t *d_hist, uint32_t *err)
 {
     const uint64_t N = j->pr.n_reads, scan0 = hist[lo];
     const int P = (int)pcs.size() - 1, T = (int)rb.size() - 1;
@@ -861,7 +726,7 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
         if (!roots) return set_error(MP_ENOMEM, "device memory for the scan's roots");
         MP_CUDA(cudaMemcpyAsync(roots, j->d_parent, (N + 1) * 4, cudaMemcpyDeviceToDevice, j->st));
     }
-    uint32_t *cnt = j->arena.alloc<uint32_t>(N + 1), *d_b = j->arena.alloc<uint32_t>(2 * P);
+    uint32_t *cnt = j->arena.alloc<uint32_t>(N + 1);
     uint64_t *off = j->arena.alloc<uint64_t>(N + 2), *ntot = j->arena.alloc<uint64_t>(1);
     const size_t tb = scan_tmp_bytes(N + 1);
     void *tmp = j->arena.alloc<uint8_t>(tb);
@@ -873,12 +738,7 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
         if (!sb0.lo[b] || !sb0.id[b] || (has_hi && !sb0.hi[b]))
             return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)maxn);
     }
-    if (!cnt || !d_b || !off || !ntot || !tmp) return set_error(MP_ENOMEM, "device memory for enumeration offsets");
-    {
-        std::vector<uint32_t> hb(2 * P);
-        for (int i = 0; i < P; i++) hb[2 * i] = (uint32_t)pcs[i], hb[2 * i + 1] = (uint32_t)pcs[i + 1];
-        MP_CUDA(cudaMemcpyAsync(d_b, hb.data(), hb.size() * 4, cudaMemcpyHostToDevice, j->st));
-    }
+    if (!cnt || !off || !ntot || !tmp) return set_error(MP_ENOMEM, "device memory for enumeration offsets");
     // piece i's tuples in enumeration order into sb0.*[0], then sorted; tp views the sorted piece
     auto piece_tuples = [&](int i, Tuples &tp) -> int {
         const uint64_t b0 = pcs[i], b1 = pcs[i + 1], expect = hist[b1] - hist[b0];
@@ -886,12 +746,7 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
         uint64_t n = 0;
         {
             StageTimer tm(j->st, j->stage_ms, 2);
-            int lrc = 0;
-            if (use_kc)
-                for (const KcPiece &q : j->kc) lrc |= store_count_scans(q, j->pr.seq_len, k, d_b + 2 * i, 1, cnt, N + 1, err, j->st);
-            else
-                launch_enum_count(j->d_fq, j->pr, k, 0, (uint32_t)b0, (uint32_t)b1, cnt, err, j->st);
-            if (lrc) return set_error(MP_EARG, "enumeration count of a scan piece");
+            launch_enum_count(j->d_fq, j->pr, k, 0, (uint32_t)b0, (uint32_t)b1, cnt, err, j->st);
             MP_CUDA(cudaMemsetAsync(cnt + N, 0, 4, j->st));
             scan_u32_to_u64(cnt, off, N + 1, ntot, tmp, tb, j->st);
             MP_CUDA(cudaMemcpyAsync(&n, ntot, 8, cudaMemcpyDeviceToHost, j->st));
@@ -899,13 +754,8 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
             if (n != expect)
                 return set_error(MP_EFMT, "scan %d piece %d: %llu tuples but the histogram holds %llu", s, i,
                                  (unsigned long long)n, (unsigned long long)expect);
-            if (use_kc)
-                for (const KcPiece &q : j->kc)
-                    store_write(q, j->pr.seq_len, k, (uint32_t)b0, (uint32_t)b1, roots, off, sb.lo[0], sb.hi[0], sb.id[0], err,
-                                j->st);
-            else
-                launch_enum_write(j->d_fq, j->pr, k, 0, (uint32_t)b0, (uint32_t)b1, roots, off, sb.lo[0], sb.hi[0],
-                                  sb.id[0], err, j->st);
+            launch_enum_write(j->d_fq, j->pr, k, 0, (uint32_t)b0, (uint32_t)b1, roots, off, sb.lo[0], sb.hi[0], sb.id[0], err,
+                              j->st);
         }
         uint32_t herr = 0;
         MP_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, j->st));
@@ -1060,6 +910,62 @@ static int scan_first_read(mp_job *j, int k, int min3, uint64_t lo, uint64_t hi,
     return first_tuple_id(tl, th, ti, n, j->arena, j->st, first);
 }
 
+// One scan, grouped: from the reads, or (the 3-minimizer variant) from its enumerated tuples lo, hi, id.
+static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo, uint8_t *hi, uint32_t *id, uint32_t *err,
+                        const uint64_t *hist)
+{
+    const uint64_t N = j->pr.n_reads, n = gs.n;
+    int rc = 0;
+    const double ms0 = j->stage_ms[2] + j->stage_ms[3];
+    uint64_t *k1 = j->arena.alloc<uint64_t>(n + 1), *k2 = nullptr;
+    uint32_t *id1 = j->arena.alloc<uint32_t>(n + 1), *id2 = nullptr;
+    {
+        StageTimer tm(j->st, j->stage_ms, min3 ? 3 : 2);
+        if ((rc = group_plan(gs, j->arena, j->st))) return rc;
+        if (min3) {
+            k2 = lo;
+            id2 = id;
+        } else {
+            if (gs.two_level) k2 = j->arena.alloc<uint64_t>(n + 1);
+            id2 = j->arena.alloc<uint32_t>(n + 1);
+        }
+        if (!k1 || !id1 || (gs.two_level && !k2) || !id2)
+            return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)n);
+        rc = min3 ? group_bins_tuples(gs, lo, hi, id, k1, id1, j->arena, j->st)
+                  : group_bins_reads(gs, j->d_fq, j->pr, {0, N}, s ? j->d_parent : nullptr, k1, id1, j->arena, j->st);
+        if (rc) return rc;
+    }
+    {
+        StageTimer tm(j->st, j->stage_ms, 3);
+        if ((rc = group_units(gs, k1, id1, k2, id2, j->st))) return rc;
+    }
+    SortStats ss;
+    ss.passes = gs.two_level ? 2 : 1;
+    ss.pass_ms = j->stage_ms[2] + j->stage_ms[3] - ms0;
+    ss.bytes = n * (uint64_t)(12 + (min3 ? (hi ? 13 : 12) : 0) + (gs.two_level ? 24 : 0));
+    uint32_t *out = gs.two_level ? id1 : id2;
+    {
+        StageTimer tm(j->st, j->stage_ms, 4);
+        if ((rc = group_filter(gs, gs.two_level ? k2 : k1, gs.two_level ? id2 : id1, out, j->d_parent, j->d_filtered, j->arena, j->st)))
+            return rc;
+    }
+    {
+        StageTimer tm(j->st, j->stage_ms, 5);
+        std::vector<GroupQuirk> open;
+        if ((rc = group_union(gs, out, j->d_parent, j->d_filtered, N, j->arena, j->st, open))) return rc;
+        for (const GroupQuirk &q : open) {
+            uint32_t first = 0;
+            if ((rc = scan_first_read(j, gs.k, min3, gs.lo, gs.hi, hist, s > 0, err, &first))) return rc;
+            if ((rc = group_finish(j->d_parent, N, first, q.anchor, j->arena, j->st, &j->hooked_bad))) return rc;
+        }
+    }
+    ss.units = gs.hctr[GC_UNITS];
+    ss.big_buckets = gs.hctr[GC_BIG];
+    ss.big_tuples = gs.hctr[GC_BIG_TUPLES];
+    add_sort_stats(j, ss, n);
+    return 0;
+}
+
 int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_starts, const uint64_t *chunk_first_read,
                      int nchunks, const uint64_t *hist, uint64_t *bounds_out)
 {
@@ -1119,33 +1025,30 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
     MP_CUDA(cudaMemsetAsync(err, 0, 4, j->st));
     const bool has_hi = 2 * k + 8 > 64;
     char name[64], name2[64];
-    // tuples per read of every scan in one pass (plain variant, monotone scan bounds)
     // the histogram prefix on the device, for the sort's planning kernels
     uint64_t *d_hist = j->arena.alloc_persistent<uint64_t>(NB + 1);
     if (!d_hist) return set_error(MP_ENOMEM, "device memory for the histogram");
     MP_CUDA(cudaMemcpyAsync(d_hist, hist, (NB + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, j->st));
     uint32_t *cnt_all = nullptr, *d_b = nullptr;
-    // the count pass's k-mer cache serves this partition when it holds the same k (plain variant)
-    const bool use_kc = !j->kc.empty() && j->kc_k == k && !p->min3 && S <= 8;
-    {
+    bool counted = false;
+    // tuples per read of every scan in one pass (plain variant, monotone scan bounds), once a scan is sorted
+    auto count_scans = [&]() -> int {
+        if (counted) return 0;
+        counted = true;
         bool mono = !p->min3 && S <= 8;
         for (int s = 0; s < S && mono; s++) mono = scanR[s] <= scanR[s + 1];
-        if (mono) {
-            cnt_all = j->arena.alloc_persistent<uint32_t>((size_t)S * (N + 1));
-            d_b = j->arena.alloc_persistent<uint32_t>(S + 1);
-            if (!cnt_all || !d_b) return set_error(MP_ENOMEM, "device memory for enumeration counts");
-            std::vector<uint32_t> hb(scanR.begin(), scanR.end());
-            StageTimer tm(j->st, j->stage_ms, 2);
-            MP_CUDA(cudaMemcpyAsync(d_b, hb.data(), (S + 1) * 4, cudaMemcpyHostToDevice, j->st));
-            int lrc = 0;
-            if (use_kc)
-                for (const KcPiece &q : j->kc) lrc |= store_count_scans(q, j->pr.seq_len, k, d_b, S, cnt_all, N + 1, err, j->st);
-            else
-                lrc = launch_enum_count_scans(j->d_fq, j->pr, k, d_b, S, cnt_all, N + 1, err, j->st);
-            if (lrc) return set_error(MP_EARG, "enumeration count over %d scans", S);
-            for (int s = 0; s < S; s++) MP_CUDA(cudaMemsetAsync(cnt_all + (size_t)s * (N + 1) + N, 0, 4, j->st));
-        }
-    }
+        if (!mono) return 0;
+        cnt_all = j->arena.alloc_persistent<uint32_t>((size_t)S * (N + 1));
+        d_b = j->arena.alloc_persistent<uint32_t>(S + 1);
+        if (!cnt_all || !d_b) return set_error(MP_ENOMEM, "device memory for enumeration counts");
+        std::vector<uint32_t> hb(scanR.begin(), scanR.end());
+        StageTimer tm(j->st, j->stage_ms, 2);
+        MP_CUDA(cudaMemcpyAsync(d_b, hb.data(), (S + 1) * 4, cudaMemcpyHostToDevice, j->st));
+        if (launch_enum_count_scans(j->d_fq, j->pr, k, d_b, S, cnt_all, N + 1, err, j->st))
+            return set_error(MP_EARG, "enumeration count over %d scans", S);
+        for (int s = 0; s < S; s++) MP_CUDA(cudaMemsetAsync(cnt_all + (size_t)s * (N + 1) + N, 0, 4, j->st));
+        return 0;
+    };
     j->pieces_total = 0;
     j->hooked_bad = ~0u;
     const uint64_t piece_cap = p->min3 ? ~0ull : scan_piece_cap(j);  // the 3-minimizer choice depends on the range
@@ -1155,6 +1058,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         if (expect > piece_cap) {
             const std::vector<uint64_t> pcs = plan_pieces(hist, lo, hi, piece_cap);
             if (pcs.size() > 2) {
+                if ((rc = count_scans())) return rc;
                 {  // the per-read checks of the whole scan (its counts, when the pass over all scans did not make them)
                     uint32_t cerr = 0, *c1 = cnt_all ? nullptr : j->arena.alloc<uint32_t>(N + 1);
                     if (!cnt_all && !c1) return set_error(MP_ENOMEM, "device memory for enumeration counts");
@@ -1170,7 +1074,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
                 }
                 std::vector<uint64_t> rb;
                 if ((rc = range_bounds(hist, thrR.data() + (size_t)s * T, T, lo, hi, rb))) return rc;
-                if ((rc = scan_in_pieces(j, s, k, has_hi, lo, hi, pcs, rb, hist, d_hist, use_kc, err))) return rc;
+                if ((rc = scan_in_pieces(j, s, k, has_hi, lo, hi, pcs, rb, hist, d_hist, err))) return rc;
                 j->arena.release_scratch();
                 snprintf(name, sizeof name, "stats%d_parent.bin", s);
                 if ((rc = dump_state(j, name, nullptr))) return rc;
@@ -1178,14 +1082,6 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             }
         }
         j->pieces_total += 1;
-        uint32_t *cnt = cnt_all ? cnt_all + (size_t)s * (N + 1) : j->arena.alloc<uint32_t>(N + 1);
-        uint64_t *off = j->arena.alloc<uint64_t>(N + 2), *ntot = j->arena.alloc<uint64_t>(1);
-        size_t tb = scan_tmp_bytes(N + 1);
-        void *tmp = j->arena.alloc<uint8_t>(tb);
-        if (!cnt || !off || !ntot || !tmp) return set_error(MP_ENOMEM, "device memory for enumeration offsets");
-        SortBufs sb;
-        int lo_buf = 0, hi_buf = 0;
-        uint64_t n = 0;
         // a refused thread-range plan is reported once the tuples are counted
         std::vector<uint64_t> rb;
         const int rb_rc = range_bounds(hist, thrR.data() + (size_t)s * T, T, lo, hi, rb);
@@ -1201,6 +1097,22 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             gs.bounds = rb;
             gs.seg_tstart = {0, expect};
         }
+        if (grouped && !p->min3) {
+            if (j->pr.max_len > (uint32_t)k && j->pr.max_len - (uint32_t)k >= 300u)
+                return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
+            if ((rc = grouped_scan(j, gs, 0, s, nullptr, nullptr, nullptr, err, hist))) return rc;
+            j->arena.release_scratch();
+            continue;
+        }
+        if ((rc = count_scans())) return rc;
+        uint32_t *cnt = cnt_all ? cnt_all + (size_t)s * (N + 1) : j->arena.alloc<uint32_t>(N + 1);
+        uint64_t *off = j->arena.alloc<uint64_t>(N + 2), *ntot = j->arena.alloc<uint64_t>(1);
+        size_t tb = scan_tmp_bytes(N + 1);
+        void *tmp = j->arena.alloc<uint8_t>(tb);
+        if (!cnt || !off || !ntot || !tmp) return set_error(MP_ENOMEM, "device memory for enumeration offsets");
+        SortBufs sb;
+        int lo_buf = 0, hi_buf = 0;
+        uint64_t n = 0;
         {
             StageTimer tm(j->st, j->stage_ms, 2);
             if (!cnt_all) {
@@ -1211,7 +1123,6 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             uint32_t cerr = 0;
             MP_CUDA(cudaMemcpyAsync(&n, ntot, 8, cudaMemcpyDeviceToHost, j->st));
             MP_CUDA(cudaMemcpyAsync(&cerr, err, 4, cudaMemcpyDeviceToHost, j->st));
-            if (grouped && (rc = group_plan(gs, j->arena, j->st))) return rc;
             MP_CUDA(cudaStreamSynchronize(j->st));
             if (cerr & DERR_LONG_READ) return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
             if (cerr & DERR_TOO_MANY)
@@ -1220,20 +1131,15 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             if (n != expect)
                 return set_error(MP_EFMT, "scan %d: %llu tuples but the histogram holds %llu", s, (unsigned long long)n,
                                  (unsigned long long)expect);
-            for (int b = 0; b < 2; b++) {
+            for (int b = 0; b < (grouped ? 1 : 2); b++) {
                 sb.lo[b] = j->arena.alloc<uint64_t>(n + 1);
                 sb.id[b] = j->arena.alloc<uint32_t>(n + 1);
-                sb.hi[b] = has_hi && !(grouped && b) ? j->arena.alloc<uint8_t>(n + 1) : nullptr;
-                if (!sb.lo[b] || !sb.id[b] || (has_hi && !(grouped && b) && !sb.hi[b]))
+                sb.hi[b] = has_hi ? j->arena.alloc<uint8_t>(n + 1) : nullptr;
+                if (!sb.lo[b] || !sb.id[b] || (has_hi && !sb.hi[b]))
                     return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)n);
             }
-            if (use_kc && cnt_all)
-                for (const KcPiece &q : j->kc)
-                    store_write(q, j->pr.seq_len, k, (uint32_t)lo, (uint32_t)hi, s ? j->d_parent : nullptr, off, sb.lo[0],
-                                sb.hi[0], sb.id[0], err, j->st);
-            else
-                launch_enum_write(j->d_fq, j->pr, k, p->min3, (uint32_t)lo, (uint32_t)hi, s ? j->d_parent : nullptr, off,
-                                  sb.lo[0], sb.hi[0], sb.id[0], err, j->st);
+            launch_enum_write(j->d_fq, j->pr, k, p->min3, (uint32_t)lo, (uint32_t)hi, s ? j->d_parent : nullptr, off, sb.lo[0],
+                              sb.hi[0], sb.id[0], err, j->st);
         }
         uint32_t herr = 0;
         MP_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, j->st));
@@ -1245,35 +1151,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         if (herr) return set_error(MP_EDEVICE, "enumeration flags 0x%x", herr);
         if (rb_rc) return set_error(rb_rc, "%s", rb_msg.c_str());
         if (grouped) {
-            const int fin = gs.two_level ? 0 : 1;  // the buffers that hold the split tuples
-            const double ms0 = j->stage_ms[3];
-            {
-                StageTimer tm(j->st, j->stage_ms, 3);
-                if ((rc = group_split(gs, sb.lo[0], sb.hi[0], sb.id[0], sb.lo[1], sb.id[1], j->arena, j->st))) return rc;
-            }
-            {
-                StageTimer tm(j->st, j->stage_ms, 4);
-                if ((rc = group_filter(gs, sb.lo[fin], sb.id[fin], sb.id[fin ^ 1], j->d_parent, j->d_filtered, j->arena, j->st)))
-                    return rc;
-            }
-            {
-                StageTimer tm(j->st, j->stage_ms, 5);
-                std::vector<GroupQuirk> open;
-                if ((rc = group_union(gs, sb.id[fin ^ 1], j->d_parent, j->d_filtered, N, j->arena, j->st, open))) return rc;
-                for (const GroupQuirk &q : open) {
-                    uint32_t first = 0;
-                    if ((rc = scan_first_read(j, k, p->min3, lo, hi, hist, s > 0, err, &first))) return rc;
-                    if ((rc = group_finish(j->d_parent, N, first, q.anchor, j->arena, j->st, &j->hooked_bad))) return rc;
-                }
-            }
-            SortStats ss;
-            ss.passes = gs.two_level ? 2 : 1;
-            ss.pass_ms = j->stage_ms[3] - ms0;
-            ss.bytes = n * (uint64_t)((has_hi ? 25 : 24) + (gs.two_level ? 24 : 0));
-            ss.units = gs.hctr[GC_UNITS];
-            ss.big_buckets = gs.hctr[GC_BIG];
-            ss.big_tuples = gs.hctr[GC_BIG_TUPLES];
-            add_sort_stats(j, ss, n);
+            if ((rc = grouped_scan(j, gs, 1, s, sb.lo[0], sb.hi[0], sb.id[0], err, hist))) return rc;
             j->arena.release_scratch();
             continue;
         }
@@ -1319,7 +1197,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
     j->arena.free_persistent(cnt_all);
     j->arena.free_persistent(d_b);
     j->arena.free_persistent(d_hist);
-    drop_kmer_cache(j);  // its HBM goes back before the mate union and the output
+    j->kc_pieces = 0;
     {
         StageTimer tm(j->st, j->stage_ms, 6);
         if (!j->dump_dir.empty()) {
@@ -1465,13 +1343,13 @@ int mp_job_output_device(mp_job *j, const void **d_out, uint64_t *file_sizes, ui
     return 0;
 }
 
-int mp_job_kmer_cache_pieces(const mp_job *j) { return j ? (int)j->kc.size() : 0; }
+int mp_job_kmer_cache_pieces(const mp_job *j) { return j ? j->kc_pieces : 0; }
 
 int mp_job_set_kmer_cache(mp_job *j, int enable)
 {
     if (!j) return set_error(MP_EARG, "null job");
     j->store = enable ? STORE_KMER_CACHE : STORE_FASTQ;
-    if (!enable) drop_kmer_cache(j);
+    if (!enable) j->kc_pieces = 0;
     return 0;
 }
 
@@ -1480,7 +1358,7 @@ int mp_job_set_read_store(mp_job *j, int store)
     if (!j) return set_error(MP_EARG, "null job");
     if (store != MP_STORE_FASTQ && store != MP_STORE_KMER_CACHE && store != MP_STORE_PACKED)
         return set_error(MP_EARG, "unknown read store %d", store);
-    if (store != j->store) drop_kmer_cache(j);
+    if (store != j->store) j->kc_pieces = 0;
     j->store = store;
     return 0;
 }
@@ -1488,8 +1366,7 @@ int mp_job_set_read_store(mp_job *j, int store)
 int mp_job_read_store(const mp_job *j)
 {
     if (!j) return set_error(MP_EARG, "null job");
-    if (j->kc.empty()) return MP_STORE_FASTQ;
-    return j->kc[0].pw ? MP_STORE_PACKED : MP_STORE_KMER_CACHE;
+    return j->kc_pieces ? j->store : MP_STORE_FASTQ;
 }
 
 int mp_job_set_wait_limits(mp_job *j, uint32_t lookback_spins, uint32_t union_retries, uint32_t mate_rounds)

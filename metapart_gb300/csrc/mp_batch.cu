@@ -267,8 +267,8 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     MP_CUDA(cudaMemsetAsync(cc, 0, (size_t)nseg * NB * sizeof(uint32_t), st));
     MP_CUDA(cudaMemsetAsync(err, 0, 4, st));
     std::vector<ParsedReads> prs(nu);
-    std::vector<KcPiece> kc(nu);
     std::vector<uint64_t> R(nseg + 1, 0), RU(nu + 1, 0);
+    uint32_t max_len = 0;
     for (int u = 0; u < nu; u++) {
         const int qa = useg[u], qb = useg[u + 1];
         const uint64_t b0 = g[qa].byte0, b1 = g[qb - 1].byte0 + smp[g[qb - 1].idx].nbytes;
@@ -316,14 +316,14 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
         if (rc) return rc;
         RU[u + 1] = R[qb];
         StageTimer tm(st, b->stage_ms, 1);
-        if (!make_kc_piece(A, st, prs[u], RU[u], k, &kc[u]))
-            return set_error(MP_ENOMEM, "device memory for the k-mer cache of samples %d..%d", g[qa].idx, g[qb - 1].idx);
+        if (prs[u].max_len > (uint32_t)MAX_READ_COUNT && prs[u].max_len > (uint32_t)k)
+            return set_error(MP_EUNSUP, "a read is longer than %d bases", MAX_READ_COUNT);
+        max_len = std::max(max_len, prs[u].max_len);
         std::vector<uint64_t> loc(qb - qa + 1);
         for (int q = qa; q <= qb; q++) loc[q - qa] = R[q] - RU[u];
         uint64_t *dl = d_srec + qa + u;
         MP_CUDA(cudaMemcpyAsync(dl, loc.data(), loc.size() * 8, cudaMemcpyHostToDevice, st));
-        launch_count(d_fq + b0, prs[u], k, 0, dl, qb - qa, cc + (size_t)qa * NB, nullptr, err, st, kc[u].off, kc[u].lo,
-                     kc[u].hi);
+        launch_count(d_fq + b0, prs[u], k, 0, dl, qb - qa, cc + (size_t)qa * NB, nullptr, err, st);
     }
     const uint64_t N = R[nseg];
     if (N >= UMAX32B) return set_error(MP_EUNSUP, "a group of more than 2^32 - 2 reads");
@@ -332,6 +332,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     {
         StageTimer tm(st, b->stage_ms, 0);
         pr.n_reads = N;
+        pr.max_len = max_len;
         pr.rec_start = A.alloc_persistent<uint64_t>(N + 1);
         pr.seq_off = A.alloc_persistent<uint64_t>(N + 1);
         pr.seq_len = A.alloc_persistent<uint32_t>(N + 1);
@@ -390,49 +391,12 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     const bool grouped = A.lim.lookback_spins == WaitLimits{}.lookback_spins && !sort_plan_chosen(k, T_all) &&
                          group_fits(T_all, N, &segs);
     GroupScan gs;
-    // ---- enumeration: every k-mer of every read (one scan per sample), read order
+    if (max_len > (uint32_t)k && max_len - (uint32_t)k >= 300u) return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
     SortBufs sb;
-    {
-        StageTimer tm(st, b->stage_ms, 2);
-        uint32_t *cnt = A.alloc<uint32_t>(N + 1), *d_b = A.alloc<uint32_t>(2);
-        uint64_t *off = A.alloc<uint64_t>(N + 2), *ntot = A.alloc<uint64_t>(1);
-        const size_t tb = scan_tmp_bytes(N + 1);
-        void *tmp = A.alloc<uint8_t>(tb);
-        if (!cnt || !d_b || !off || !ntot || !tmp) return set_error(MP_ENOMEM, "device memory for enumeration offsets");
-        const uint32_t hb[2] = {0, NB};
-        MP_CUDA(cudaMemcpyAsync(d_b, hb, 8, cudaMemcpyHostToDevice, st));
-        for (const KcPiece &q : kc)
-            if (q.n && launch_kc_count_scans(q.off, q.lo, q.hi, q.n, k, d_b, 1, cnt + q.r0, N + 1, err, st))
-                return set_error(MP_EARG, "enumeration count");
-        MP_CUDA(cudaMemsetAsync(cnt + N, 0, 4, st));
-        scan_u32_to_u64(cnt, off, N + 1, ntot, tmp, tb, st);
-        uint64_t n = 0;
-        MP_CUDA(cudaMemcpyAsync(&n, ntot, 8, cudaMemcpyDeviceToHost, st));
-        MP_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
-        MP_CUDA(cudaStreamSynchronize(st));
-        if (herr & DERR_LONG_READ) return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
-        if (herr & DERR_TOO_MANY)
-            return set_error(MP_EUNSUP, "a read has 256 or more k-mers (the reference counts them in 8 bits, "
-                                        "enumerateKmers.c:152)");
-        if (n != T_all)
-            return set_error(MP_EFMT, "the group enumerates %llu tuples but its histograms hold %llu", (unsigned long long)n,
-                             (unsigned long long)T_all);
-        for (int x = 0; x < 2; x++) {
-            sb.lo[x] = A.alloc_persistent<uint64_t>(n + 1);
-            sb.id[x] = A.alloc_persistent<uint32_t>(n + 1);
-            sb.hi[x] = has_hi && !(grouped && x) ? A.alloc_persistent<uint8_t>(n + 1) : nullptr;
-            if (!sb.lo[x] || !sb.id[x] || (has_hi && !(grouped && x) && !sb.hi[x]))
-                return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)n);
-        }
-        for (const KcPiece &q : kc)
-            launch_kc_write(q.off, q.lo, q.hi, q.r0, q.n, k, 0, NB, nullptr, off, sb.lo[0], sb.hi[0], sb.id[0], st);
-        for (auto &x : kc) free_kc_piece(A, x);
-        A.release_scratch();
-    }
-    // ---- sort: every sample's tuples by (k-mer, adjacency), within the sample's range, or split into units
     int lo_buf = 0, hi_buf = 0;
     if (grouped) {
-        const double ms0 = b->stage_ms[3];
+        // ---- enumeration into bins and units of every sample's buckets
+        const double ms0 = b->stage_ms[2] + b->stage_ms[3];
         gs.k = k;
         gs.n = T_all;
         gs.d_hist = shist;
@@ -440,18 +404,59 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
         gs.hi = (uint64_t)nseg * NB;
         gs.bounds = rb;
         gs.seg_tstart = segs.tstart;
+        for (int x = 0; x < 2; x++) {
+            sb.lo[x] = A.alloc_persistent<uint64_t>(T_all + 1);
+            sb.id[x] = A.alloc_persistent<uint32_t>(T_all + 1);
+            if (!sb.lo[x] || !sb.id[x]) return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)T_all);
+        }
+        {
+            StageTimer tm(st, b->stage_ms, 2);
+            if ((rc = group_plan(gs, A, st))) return rc;
+            if ((rc = group_bins_reads(gs, d_fq, pr, R, nullptr, sb.lo[1], sb.id[1], A, st))) return rc;
+        }
         {
             StageTimer tm(st, b->stage_ms, 3);
-            if ((rc = group_plan(gs, A, st))) return rc;
-            if ((rc = group_split(gs, sb.lo[0], sb.hi[0], sb.id[0], sb.lo[1], sb.id[1], A, st))) return rc;
+            if ((rc = group_units(gs, sb.lo[1], sb.id[1], sb.lo[0], sb.id[0], st))) return rc;
         }
         lo_buf = gs.two_level ? 0 : 1;
-        hi_buf = 1;
-        b->sort_pass_ms += b->stage_ms[3] - ms0;
-        b->sort_bytes += T_all * (uint64_t)((has_hi ? 25 : 24) + (gs.two_level ? 24 : 0));
+        b->sort_pass_ms += b->stage_ms[2] + b->stage_ms[3] - ms0;
+        b->sort_bytes += T_all * (uint64_t)(12 + (gs.two_level ? 24 : 0));
         b->sort_passes += gs.two_level ? 2 : 1;
         b->sort_tuples += T_all;
     } else {
+        // ---- enumeration: every k-mer of every read (one scan per sample), read order
+        {
+            StageTimer tm(st, b->stage_ms, 2);
+            uint32_t *cnt = A.alloc<uint32_t>(N + 1);
+            uint64_t *off = A.alloc<uint64_t>(N + 2), *ntot = A.alloc<uint64_t>(1);
+            const size_t tb = scan_tmp_bytes(N + 1);
+            void *tmp = A.alloc<uint8_t>(tb);
+            if (!cnt || !off || !ntot || !tmp) return set_error(MP_ENOMEM, "device memory for enumeration offsets");
+            launch_enum_count(d_fq, pr, k, 0, 0, NB, cnt, err, st);
+            MP_CUDA(cudaMemsetAsync(cnt + N, 0, 4, st));
+            scan_u32_to_u64(cnt, off, N + 1, ntot, tmp, tb, st);
+            uint64_t n = 0;
+            MP_CUDA(cudaMemcpyAsync(&n, ntot, 8, cudaMemcpyDeviceToHost, st));
+            MP_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
+            MP_CUDA(cudaStreamSynchronize(st));
+            if (herr & DERR_LONG_READ) return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
+            if (herr & DERR_TOO_MANY)
+                return set_error(MP_EUNSUP, "a read has 256 or more k-mers (the reference counts them in 8 bits, "
+                                            "enumerateKmers.c:152)");
+            if (n != T_all)
+                return set_error(MP_EFMT, "the group enumerates %llu tuples but its histograms hold %llu", (unsigned long long)n,
+                                 (unsigned long long)T_all);
+            for (int x = 0; x < 2; x++) {
+                sb.lo[x] = A.alloc_persistent<uint64_t>(n + 1);
+                sb.id[x] = A.alloc_persistent<uint32_t>(n + 1);
+                sb.hi[x] = has_hi ? A.alloc_persistent<uint8_t>(n + 1) : nullptr;
+                if (!sb.lo[x] || !sb.id[x] || (has_hi && !sb.hi[x]))
+                    return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)n);
+            }
+            launch_enum_write(d_fq, pr, k, 0, 0, NB, nullptr, off, sb.lo[0], sb.hi[0], sb.id[0], err, st);
+            A.release_scratch();
+        }
+        // ---- sort: every sample's tuples by (k-mer, adjacency), within the sample's range
         StageTimer tm(st, b->stage_ms, 3);
         SortStats ss;
         if ((rc = bucket_sort(sb, T_all, has_hi, k, shist, 0, (uint64_t)nseg * NB, A, st, &ss, &lo_buf, &hi_buf, &segs)))
@@ -470,7 +475,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     // free the other buffer's big arrays (the filter and the union read only the sorted ones)
     A.free_persistent(sb.lo[lo_buf ^ 1]);
     if (!grouped) A.free_persistent(sb.id[lo_buf ^ 1]);  // (the grouped ids go there)
-    if (has_hi) A.free_persistent(sb.hi[hi_buf ^ 1]);
+    if (has_hi && !grouped) A.free_persistent(sb.hi[hi_buf ^ 1]);
     // ---- filter and unions over every thread range of every sample
     uint32_t *parent = A.alloc_persistent<uint32_t>(N + 1), *size = A.alloc_persistent<uint32_t>(N + 1);
     uint8_t *filtered = A.alloc_persistent<uint8_t>(N + 1);

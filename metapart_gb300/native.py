@@ -219,13 +219,13 @@ class Job:
         return lib().mp_job_num_reads(self.h)
 
     def set_kmer_cache(self, enable: bool):
-        """Keep the count pass's k-mers for the next partition of the same k (default on)."""
+        """set_read_store("kmer_cache") or ("fastq")."""
         _check(lib().mp_job_set_kmer_cache(self.h, int(enable)), "set_kmer_cache")
 
     STORES = {"fastq": 0, "kmer_cache": 1, "packed": 2}
 
     def set_read_store(self, store: str):
-        """What the count pass keeps of the reads for the partition: "kmer_cache" (default), "packed" or "fastq"."""
+        """The read store asked for: "kmer_cache" (default), "packed" or "fastq" (mp_job_set_read_store)."""
         _check(lib().mp_job_set_read_store(self.h, self.STORES[store]), "set_read_store")
 
     @property

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "k_group.cuh"
@@ -24,20 +25,31 @@ constexpr unsigned FULLG = 0xFFFFFFFFu;
 constexpr int GP_UNIT_SHIFT = 12;        // units end where the tuple prefix crosses a multiple of 4096
 constexpr int GP_CAP_S = 6128;           // most tuples of a unit for the 512-thread blocks (two per SM)
 constexpr int GP_CAP_L = 12288;          // and for the 1024-thread blocks; a larger bucket takes the device-wide sort
-constexpr uint32_t GP_MAX_BINS = 1024;   // digits of the first split pass
-constexpr uint32_t GP_MAX_UNITS = 2048;  // digits of the second (units of a bin), up to a bin shift of 21
-constexpr uint32_t GP_MAX_UNITS_L = 4096;  // and above it (scans of more than 2^31 tuples; one block per SM)
+constexpr uint32_t GP_DIGITS = 1024;     // digits of a split pass: bins of a segment, units of a bin
+constexpr uint64_t GP_SMALL = 1500000;   // tuples of a segment that fit GP_DIGITS units however they are spread
 constexpr int GP_COUNT_ITEMS = 8, GP_COUNT_THREADS = 256, GP_COUNT_BLOCK = GP_COUNT_ITEMS * GP_COUNT_THREADS;
 constexpr uint32_t GP_NONE = 0x7FFFFFFFu;  // a grouped id that stands for no read
 constexpr int QW = 8;  // words per segment: tuples found before the last run, last run's, its read, the run's place
 
 struct PlanCtx {
     const uint64_t *hist;
-    uint64_t lo, hi;         // buckets of the scan
-    const uint32_t *brk;     // a bit per bucket (from lo): a thread range starts there
-    int unit_shift, bin_shift;
-    bool two_level;
+    uint64_t lo, hi;          // buckets of the scan
+    const uint32_t *brk;      // a bit per bucket (from lo): a thread range starts there
+    const uint32_t *seg_sh;   // per segment: its bins hold 2^seg_sh buckets
+    const uint32_t *seg_bin0; // per segment: its first bin
+    uint32_t seg_lo;          // first bucket of a segment (lo, or 0 with several)
 };
+
+// The bin width of a segment of n tuples over `span` buckets.  A bin of at most 1024 buckets has at most 1024 units, so
+// the second pass finds a tuple's unit in a table of the bin's buckets; a segment of at most GP_SMALL tuples has at most
+// 1024 units in all and takes bins of about 16384 tuples instead, which fill the second pass's tiles.
+static int bin_width(uint64_t n, uint64_t span)
+{
+    const uint64_t want = n <= GP_SMALL ? std::max<uint64_t>(1, n >> 14) : GP_DIGITS;
+    int s = 0;
+    while (s < 16 && ((span - 1) >> s) + 1 > want) s++;  // a bucket within its bin takes 16 bits
+    return s;
+}
 
 // The populated bucket before b within b's segment: its index, or ~0 when b is the segment's first.
 __device__ __forceinline__ uint64_t prev_bucket(const PlanCtx &c, uint64_t b)
@@ -55,23 +67,22 @@ __device__ __forceinline__ uint64_t prev_bucket(const PlanCtx &c, uint64_t b)
     return a - 1;
 }
 
-// Whether bucket b (populated, prefix [s, e) from the scan's start) starts a unit (bit 0), a bin (bit 1), its
-// segment (bit 2), or a thread range (bit 3).  Units never cross a thread range, a segment, a multiple of 2^16
-// buckets (the bucket within a bin takes 16 bits) or a multiple of 2^unit_shift tuples, except that a bucket which
+// Whether bucket b (populated, prefix [s, e) from the scan's start) starts a unit (bit 0) and a thread range (bit 3).
+// Units never cross a thread range, a segment, a bin or a multiple of 2^GP_UNIT_SHIFT tuples, except that a bucket which
 // would make its unit larger than GP_CAP_S is a unit of its own: every decision is local to the bucket and its
 // predecessor, so the plan is two parallel passes (a greedy packing by one thread per 256 buckets took 140-210 us).
 __device__ __forceinline__ uint32_t plan_flags(const PlanCtx &c, uint64_t b, uint64_t s, uint64_t e)
 {
     const uint64_t p = prev_bucket(c, b);
-    if (p == ~0ull) return 15u;
+    if (p == ~0ull) return 9u;
     const uint64_t sp = c.hist[p] - c.hist[c.lo];
     const uint64_t rel = b - c.lo;
     const bool brk = (c.brk[rel >> 5] >> (rel & 31)) & 1u;
-    const bool far = (p >> 16) != (b >> 16);
-    const uint64_t q = s >> c.unit_shift;
-    const bool unit = brk || far || q != (sp >> c.unit_shift) || e - (q << c.unit_shift) > (uint64_t)GP_CAP_S;
-    const bool bin = c.two_level ? far || (s >> c.bin_shift) != (sp >> c.bin_shift) : unit;
-    return (unit || bin ? 1u : 0u) | (bin ? 2u : 0u) | (brk ? 8u : 0u);
+    const uint32_t sh = c.seg_sh[b / NB];
+    const bool bin = (((uint32_t)b & (NB - 1)) - c.seg_lo) >> sh != (((uint32_t)p & (NB - 1)) - c.seg_lo) >> sh;
+    const uint64_t q = s >> GP_UNIT_SHIFT;
+    const bool unit = brk || bin || q != (sp >> GP_UNIT_SHIFT) || e - (q << GP_UNIT_SHIFT) > (uint64_t)GP_CAP_S;
+    return (unit ? 1u : 0u) | (brk ? 8u : 0u);
 }
 
 // The bucket that starts at each thread range's first tuple.
@@ -110,7 +121,7 @@ __device__ __forceinline__ uint64_t block_scan_excl(uint64_t v, uint64_t *total,
     return before + x - v;
 }
 
-// Units (low word) and bins (high word) starting in each block of GP_COUNT_BLOCK buckets.
+// Units starting in each block of GP_COUNT_BLOCK buckets.
 __global__ void __launch_bounds__(GP_COUNT_THREADS) k_gp_count(PlanCtx c, uint64_t *blk)
 {
     __shared__ uint64_t ws[GP_COUNT_THREADS / 32];
@@ -120,9 +131,7 @@ __global__ void __launch_bounds__(GP_COUNT_THREADS) k_gp_count(PlanCtx c, uint64
         const uint64_t b = c.lo + (uint64_t)blockIdx.x * GP_COUNT_BLOCK + (uint64_t)i * GP_COUNT_THREADS + threadIdx.x;
         if (b >= c.hi) break;
         const uint64_t s = c.hist[b], e = c.hist[b + 1];
-        if (s == e) continue;
-        const uint32_t f = plan_flags(c, b, s - h0, e - h0);
-        v += (f & 1u) | ((uint64_t)((f >> 1) & 1u) << 32);
+        if (s != e) v += plan_flags(c, b, s - h0, e - h0) & 1u;
     }
     uint64_t tot;
     block_scan_excl(v, &tot, ws);
@@ -130,8 +139,8 @@ __global__ void __launch_bounds__(GP_COUNT_THREADS) k_gp_count(PlanCtx c, uint64
 }
 
 // Exclusive scan of the blocks' counts by one block; the sentinels past the last unit and bin.
-__global__ void __launch_bounds__(1024) k_gp_scan(uint64_t *blk, uint32_t nblk, uint32_t n, int nseg, uint32_t *ctr,
-                                                  uint32_t *ustart, uint32_t *bstart, uint32_t *bu0, uint32_t *seg_bin0)
+__global__ void __launch_bounds__(1024) k_gp_scan(uint64_t *blk, uint32_t nblk, uint32_t n, uint32_t nbins, uint32_t *ctr,
+                                                  uint32_t *ustart, uint32_t *bstart, uint32_t *bu0)
 {
     __shared__ uint64_t ws[32];
     uint64_t carry = 0;
@@ -143,21 +152,19 @@ __global__ void __launch_bounds__(1024) k_gp_scan(uint64_t *blk, uint32_t nblk, 
         carry += tot;
     }
     if (threadIdx.x == 0) {
-        const uint32_t nu = (uint32_t)carry, nb = (uint32_t)(carry >> 32);
-        ctr[GC_UNITS] = nu;
-        ctr[GC_BINS] = nb;
-        ustart[nu] = n;
-        bstart[nb] = n;
-        bu0[nb] = nu;
-        seg_bin0[nseg] = nb;
+        ctr[GC_UNITS] = (uint32_t)carry;
+        ustart[carry] = n;
+        bstart[nbins] = n;
+        bu0[nbins] = (uint32_t)carry;
     }
 }
 
 // The unit and bin arrays.  A bucket above GP_CAP_S tuples is a unit of its own (plan_flags), so its size is known here.
 __global__ void __launch_bounds__(GP_COUNT_THREADS) k_gp_write(PlanCtx c, const uint64_t *blk, uint32_t *ctr, uint32_t *ustart,
-                                                               uint32_t *ub0, uint32_t *ucur, uint32_t *bstart, uint32_t *bb0,
-                                                               uint32_t *bu0, uint32_t *bcur, uint32_t *seg_bin0,
-                                                               uint32_t *mid, uint32_t *big)
+                                                               uint32_t *ub0, uint32_t *ucur, uint32_t *bstart, uint32_t *bu0,
+                                                               uint32_t *bcur, uint32_t *bsh, uint32_t *bfirst,
+                                                               uint32_t *unit_of, uint32_t *mid,
+                                                               uint32_t *big)
 {
     __shared__ uint64_t ws[GP_COUNT_THREADS / 32];
     const uint64_t h0 = c.hist[c.lo];
@@ -172,19 +179,23 @@ __global__ void __launch_bounds__(GP_COUNT_THREADS) k_gp_write(PlanCtx c, const 
             if (s != e) f = plan_flags(c, b, s, e);
         }
         uint64_t tot;
-        const uint64_t x = at + block_scan_excl((f & 1u) | ((uint64_t)((f >> 1) & 1u) << 32), &tot, ws);
+        const uint32_t u = (uint32_t)(at + block_scan_excl(f & 1u, &tot, ws));
         at += tot;
-        const uint32_t u = (uint32_t)x, bin = (uint32_t)(x >> 32);
+        if (b < c.hi) {
+            const uint32_t seg = (uint32_t)(b / NB), rel = ((uint32_t)b & (NB - 1)) - c.seg_lo, sh = c.seg_sh[seg];
+            if ((rel & ((1u << sh) - 1)) == 0) {
+                const uint32_t bin = c.seg_bin0[seg] + (rel >> sh);
+                bstart[bin] = bcur[bin] = (uint32_t)s;
+                bu0[bin] = u;
+                bfirst[bin] = (uint32_t)(b - c.lo);
+                bsh[bin] = sh;
+            }
+            unit_of[b - c.lo] = u + (f & 1u) - 1u;  // (before the first unit: ~0)
+        }
         if (f & 1u) {
             ustart[u] = ucur[u] = (uint32_t)s;
             ub0[u] = (uint32_t)b | (f & 8u ? 0x80000000u : 0u);
         }
-        if (f & 2u) {
-            bstart[bin] = bcur[bin] = (uint32_t)s;
-            bb0[bin] = (uint32_t)b;
-            bu0[bin] = u;
-        }
-        if (f & 4u) seg_bin0[b / NB] = bin;
         if (e - s > (uint64_t)GP_CAP_S) {
             if (e - s <= (uint64_t)GP_CAP_L) mid[atomicAdd(&ctr[GC_MID], 1u)] = u;
             else {
@@ -199,111 +210,62 @@ __global__ void __launch_bounds__(GP_COUNT_THREADS) k_gp_write(PlanCtx c, const 
 
 constexpr int SP_THREADS = 512, SP_ITEMS = 12, SP_TILE = SP_THREADS * SP_ITEMS;
 
-// Tiles of the second pass: every bin's own, from its first tuple.
-__global__ void __launch_bounds__(1024) k_gp_tiles(const uint32_t *bstart, uint32_t *ctr, uint32_t *tile_first, uint32_t *tile_bin)
+// Tiles of the second pass, every bin's own: first tuple, tuples, bin.
+__global__ void __launch_bounds__(1024) k_gp_tiles(const uint32_t *bstart, uint32_t nb, uint32_t *ctr, uint4 *tiles)
 {
     __shared__ uint64_t ws[32];
-    const uint32_t nb = ctr[GC_BINS];
     uint64_t carry = 0;
     for (uint32_t i0 = 0; i0 < nb; i0 += 1024) {
-        const uint32_t i = i0 + threadIdx.x;
-        const uint32_t t = i < nb ? (bstart[i + 1] - bstart[i] + SP_TILE - 1) / SP_TILE : 0;
+        const uint32_t i = i0 + threadIdx.x, s = i < nb ? bstart[i] : 0, e = i < nb ? bstart[i + 1] : 0;
+        const uint32_t t = (e - s + SP_TILE - 1) / SP_TILE;
         uint64_t tot;
         const uint64_t x = carry + block_scan_excl(t, &tot, ws);
-        if (i < nb) {
-            tile_first[i] = (uint32_t)x;
-            for (uint32_t q = 0; q < t; q++) tile_bin[x + q] = i;
-        }
+        for (uint32_t q = 0; q < t; q++) tiles[x + q] = make_uint4(s + q * SP_TILE, min((uint32_t)SP_TILE, e - s - q * SP_TILE), i, 0);
         carry += tot;
     }
     if (threadIdx.x == 0) ctr[GC_TILES] = (uint32_t)carry;
 }
 
-// Digit lookup: a segment's (or a bin's) bucket range in CELLS cells of 2^shift buckets, each with the digits of its first
-// and its last bucket (low and high half); where they differ, a search between them.  One shared-memory read per tuple
-// in nearly all cases: a binary search over the digits' first buckets instead (10 dependent reads) held the passes to
-// 2.6 TB/s with the shared-memory pipe 83 % busy.
-constexpr uint32_t CELLS_1 = 2048, CELLS_2 = 1024;
-
-__host__ __device__ __forceinline__ int cell_shift(uint64_t span, uint32_t cells)
-{
-    int s = 0;
-    while (((span - 1) >> s) >= cells) s++;
-    return s;
-}
-
-__global__ void __launch_bounds__(256) k_gp_cells(const uint32_t *bb0, const uint32_t *seg_bin0, uint32_t b_lo, uint32_t b_hi,
-                                                  int shift, uint32_t *cells)
-{
-    const uint32_t seg = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= CELLS_1) return;
-    const uint32_t d0 = seg_bin0[seg], nd = seg_bin0[seg + 1] - d0;
-    uint32_t v[2];
-    for (int q = 0; q < 2; q++) {
-        const uint64_t x = min((uint64_t)b_hi - 1, b_lo + ((uint64_t)(c + q) << shift) - q);
-        uint32_t a = 0, z = nd - 1;  // the last bin whose first bucket is at or below x
-        while (a < z) {
-            const uint32_t m = (a + z + 1) >> 1;
-            if ((bb0[d0 + m] & (NB - 1)) <= x) a = m; else z = m - 1;
-        }
-        v[q] = a;
-    }
-    cells[(size_t)seg * CELLS_1 + c] = v[0] | (v[1] << 16);
-}
-
-template <class B>
-__device__ __forceinline__ uint32_t cell_digit(const uint32_t *cells, const B *b0, int shift, uint32_t rel, uint32_t b)
-{
-    const uint32_t v = cells[rel >> shift];
-    uint32_t a = v & 0xFFFFu, z = v >> 16;
-    while (a < z) {
-        const uint32_t m = (a + z + 1) >> 1;
-        if (b0[m] <= b) a = m; else z = m - 1;
-    }
-    return a;
-}
-
-template <int DIGITS, class B, uint32_t CELLS> struct SplitSmem {
-    uint64_t key[SP_TILE];   // (the packed reads of k_enum_bins before)
+struct SplitSmem {
+    uint64_t key[SP_TILE];
     uint32_t id[SP_TILE];
-    uint16_t dig[SP_TILE];
-    B b0[DIGITS];            // first bucket of every digit
-    uint32_t hist[DIGITS];   // tuples per digit, then the digit's first place in the tile
-    uint32_t delta[DIGITS];  // global place of a digit's first tuple less its place in the tile
-    uint32_t cells[CELLS];
+    uint16_t dig[SP_TILE];      // a place's digit, times 4
+    uint32_t hist[GP_DIGITS];   // tuples per digit, then the digit's first place in the tile
+    uint32_t delta[GP_DIGITS];  // global place of a digit's first tuple less its place in the tile
     uint32_t ws[SP_THREADS / 32];
 };
-typedef SplitSmem<GP_MAX_BINS, uint32_t, CELLS_1> BinSmem;
-template <int DIGITS> using UnitSmem = SplitSmem<DIGITS, uint16_t, CELLS_2>;
-static_assert(2 * (sizeof(BinSmem) + 1024) <= 228 * 1024 && 2 * (sizeof(UnitSmem<GP_MAX_UNITS>) + 1024) <= 228 * 1024,
-              "two split blocks per SM");
+constexpr uint32_t SP_PACKED = 4096;  // words of packed reads
+struct BinSmem : SplitSmem {
+    uint32_t packed[SP_PACKED];
+};
+struct UnitSmem : SplitSmem {
+    uint16_t cell[GP_DIGITS];   // the bin's buckets in 1024 cells: the digit (times 4) of a cell's first bucket
+    uint16_t b0[GP_DIGITS];     // first bucket of every unit within the bin (bins of more than 1024 buckets)
+};
+constexpr uint32_t SP_CHUNK = 4;  // tiles of the second pass a block takes at a time
+static_assert(2 * (sizeof(UnitSmem) + 1024) <= 228 * 1024 && 2 * (sizeof(BinSmem) + 3 * 1024) <= 228 * 1024, "two split blocks per SM");
+
+__device__ __forceinline__ uint32_t &at_byte(uint32_t *p, uint32_t off) { return *reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(p) + off); }
 
 // Unstable, so there are no ballots and no look-back: ranks by shared-memory atomics, places by one global atomic per
-// digit and tile (the order of a digit's tuples is free), a shared-memory reorder so that a digit's tuples are stored
-// side by side.  rd: digit in (0xFFFF = no tuple).
-template <class Smem, int DIGITS, class LoadId>
-__device__ __forceinline__ void split_tile(Smem &sm, const uint64_t (&key)[SP_ITEMS], uint32_t (&rd)[SP_ITEMS], uint32_t *cur,
-                                           uint32_t nd, LoadId load_id, uint64_t *out_k, uint32_t *out_id, uint32_t n)
+// digit and tile (the order of a digit's tuples is free; its latency passes while the tile is reordered), a
+// shared-memory reorder so that a digit's tuples are stored side by side.  rd: digit times 4 (bits 0-11) and the tuple's rank
+// in it (16-31), or ~0 for none, as the caller's atomics on sm.hist gave them.  Returns the tile's tuples, 0 when one
+// would land past the n tuples (the histogram is not the tuples': the group kernel reports it).
+template <class LoadId>
+__device__ __forceinline__ uint32_t split_order(SplitSmem &sm, const uint32_t (&kl)[SP_ITEMS], const uint32_t (&kh)[SP_ITEMS],
+                                                const uint32_t (&rd)[SP_ITEMS], uint32_t *cur, uint32_t nd, LoadId load_id, uint32_t n)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-    for (int j = 0; j < SP_ITEMS; j++)
-        if (rd[j] != 0xFFFFu) rd[j] |= atomicAdd(&sm.hist[rd[j]], 1u) << 16;
     uint32_t id[SP_ITEMS];
 #pragma unroll
     for (int j = 0; j < SP_ITEMS; j++) id[j] = load_id(j);
     __syncthreads();
-    constexpr int PER = DIGITS / SP_THREADS;
-    uint32_t c[PER], s = 0;
-#pragma unroll
-    for (int q = 0; q < PER; q++) {
-        c[q] = sm.hist[tid * PER + q];
-        s += c[q];
-    }
-    uint32_t g[PER];
-#pragma unroll
-    for (int q = 0; q < PER; q++) g[q] = c[q] && tid * PER + q < nd ? atomicAdd(&cur[tid * PER + q], c[q]) : 0u;
-    uint32_t x = s;
+    static_assert(GP_DIGITS == 2 * SP_THREADS, "two digits per thread");
+    const uint2 c = *reinterpret_cast<const uint2 *>(&sm.hist[2 * tid]);
+    const uint32_t g0 = c.x && 2 * tid < nd ? atomicAdd(&cur[2 * tid], c.x) : 0u;
+    const uint32_t g1 = c.y && 2 * tid + 1 < nd ? atomicAdd(&cur[2 * tid + 1], c.y) : 0u;
+    uint32_t x = c.x + c.y;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(FULLG, x, o);
@@ -311,39 +273,37 @@ __device__ __forceinline__ void split_tile(Smem &sm, const uint64_t (&key)[SP_IT
     }
     if (lane == 31) sm.ws[warp] = x;
     __syncthreads();
-    uint32_t before = x - s, nv = 0;
+    uint32_t before = x - c.x - c.y, nv = 0;
+#pragma unroll
     for (int w = 0; w < SP_THREADS / 32; w++) {
         const uint32_t v = sm.ws[w];
         before += w < warp ? v : 0u;
         nv += v;
     }
-#pragma unroll
-    for (int q = 0; q < PER; q++) {
-        sm.hist[tid * PER + q] = before;
-        sm.delta[tid * PER + q] = g[q] - before;
-        before += c[q];
-    }
+    *reinterpret_cast<uint2 *>(&sm.hist[2 * tid]) = make_uint2(before, before + c.x);
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < SP_ITEMS; j++) {
-        const uint32_t d = rd[j] & 0xFFFFu;
-        if (d != 0xFFFFu) {
-            const uint32_t p = sm.hist[d] + (rd[j] >> 16);
-            sm.key[p] = key[j];
+        if (rd[j] != ~0u) {
+            const uint32_t d = rd[j] & 0xFFFu, p = at_byte(sm.hist, d) + (rd[j] >> 16);
+            sm.key[p] = ((uint64_t)kh[j] << 32) | kl[j];
             sm.id[p] = id[j];
             sm.dig[p] = (uint16_t)d;
         }
     }
-    __syncthreads();
-    for (uint32_t p = tid; p < nv; p += SP_THREADS) {
-        const uint32_t o = p + sm.delta[sm.dig[p]];
-        if (o < n) {  // (a histogram that does not match the tuples is reported by the group kernel)
-            out_k[o] = sm.key[p];
-            out_id[o] = sm.id[p];
-        }
+    *reinterpret_cast<uint2 *>(&sm.delta[2 * tid]) = make_uint2(g0 - before, g1 - before - c.x);
+    return __syncthreads_or((c.x && (uint64_t)g0 + c.x > n) || (c.y && (uint64_t)g1 + c.y > n)) ? 0u : nv;
+}
+
+__device__ __forceinline__ void split_store(SplitSmem &sm, uint32_t nv, uint64_t *out_k, uint32_t *out_id)
+{
+#pragma unroll 4
+    for (uint32_t p = threadIdx.x; p < nv; p += SP_THREADS) {
+        const uint32_t o = p + at_byte(sm.delta, sm.dig[p]);
+        out_k[o] = sm.key[p];
+        out_id[o] = sm.id[p];
     }
-#pragma unroll
-    for (int q = 0; q < PER; q++) sm.hist[tid * PER + q] = 0;  // (read last before the barrier above)
+    *reinterpret_cast<uint2 *>(&sm.hist[2 * threadIdx.x]) = make_uint2(0, 0);
 }
 
 // The tiles of a pass over segments: tile0[q] the segment's first tile, start[q] its first read or tuple, tile_seg the
@@ -358,7 +318,7 @@ __global__ void k_gp_segtiles(const uint32_t *tile0, int nseg, uint32_t *tile_se
     for (uint32_t t = tile0[q] + threadIdx.x; t < tile0[q + 1]; t += blockDim.x) tile_seg[t] = (uint32_t)q;
 }
 
-// First pass, one of two sources: the reads (k_readtile.cuh; the tuples of the buckets [b_lo, b_hi)), or tuples enumerated
+// First pass, one of two sources: the reads (k_readtile.cuh; the tuples of the scan's buckets), or tuples enumerated
 // before (lo = k-mer << 8 | adj, hi = k-mer >> 56; the 3-minimizer variant).
 struct BinCtx {
     ReadTiles t;
@@ -367,176 +327,232 @@ struct BinCtx {
     const uint64_t *lo = nullptr;
     const uint8_t *hi = nullptr;
     const uint32_t *id = nullptr;
-    uint32_t tiles = 0, n = 0, b_lo = 0, b_hi = 0;
-    int bsh = 0, shift = 0;
-    const uint32_t *bb0 = nullptr, *seg_bin0 = nullptr, *cells = nullptr;
+    uint32_t tiles = 0, n = 0;
+    uint64_t k_lo = 0, k_span = 0;  // the scan's k-mers: [k_lo, k_lo + k_span)
+    int bsh = 0;
+    const uint32_t *seg_bin0 = nullptr, *seg_sh = nullptr;
     uint32_t *bcur = nullptr, *err = nullptr;
     SegTiles sg;
     uint64_t *out_k = nullptr;
     uint32_t *out_id = nullptr;
 };
 
-template <bool READS>
-__global__ void __launch_bounds__(SP_THREADS, 2) k_split_bins(BinCtx c)
+__device__ __forceinline__ void bin_tile(const BinCtx &c, uint32_t tile, uint32_t per, uint32_t all, uint32_t &seg, uint32_t &base,
+                                         uint32_t &end)
+{
+    seg = c.sg.tile_seg ? c.sg.tile_seg[tile] : 0u;
+    base = tile * per;
+    end = all;
+    if (c.sg.tile_seg) {
+        base = c.sg.start[seg] + (tile - c.sg.tile0[seg]) * per;
+        end = c.sg.start[seg + 1];
+    }
+    end = min(end, base + per);
+}
+
+// Bound by the instructions of the k-mers (about 90 per position at 38 % issue; two blocks' 64 registers a thread hold 32
+// warps per SM) and the shared-memory reorder; the random stores and the ranks' atomics are about a fifth each.  20M x
+// 150 bp, 2 scans: 35.4 ms for what counting (6.1), enumerating (14.3) and a first split over 13-byte tuples (29.3) took.
+//
+// HI: 2k >= 34 and bins of at least 2^32 k-mers, so a k-mer's bin is a shift of its high word.
+template <bool HI>
+__global__ void __launch_bounds__(SP_THREADS, 2) k_split_reads(BinCtx c)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     BinSmem &sm = *reinterpret_cast<BinSmem *>(smraw);
-    __shared__ uint32_t many[READS ? SP_THREADS : 1];
+    __shared__ uint32_t many[SP_THREADS];
     const int tid = threadIdx.x;
-    const uint64_t lowmask = (1ull << c.bsh) - 1;
-    uint32_t have = ~0u, d0 = 0, nd = 0;  // the segment whose digits are in shared memory
-    for (uint32_t d = tid; d < GP_MAX_BINS; d += SP_THREADS) sm.hist[d] = 0;
+    for (uint32_t d = tid; d < GP_DIGITS; d += SP_THREADS) sm.hist[d] = 0;
+    const uint32_t per = c.t.rpt, rr = tid / c.t.spr, i0 = (tid - rr * c.t.spr) * c.t.P;
+    uint32_t seg, base, end;
+    if (blockIdx.x < c.tiles) {
+        bin_tile(c, blockIdx.x, per, c.n_reads, seg, base, end);
+        rt_pack(c.t, base, end - base, sm.packed);
+    }
     for (uint32_t tile = blockIdx.x; tile < c.tiles; tile += gridDim.x) {
-        const uint32_t seg = c.sg.tile_seg ? c.sg.tile_seg[tile] : 0u;
-        const uint32_t per = READS ? c.t.rpt : (uint32_t)SP_TILE;
-        uint32_t base = tile * per, end = READS ? c.n_reads : c.n;
-        if (c.sg.tile_seg) {
-            base = c.sg.start[seg] + (tile - c.sg.tile0[seg]) * per;
-            end = c.sg.start[seg + 1];
+        const uint32_t d0 = c.seg_bin0[seg], nd = c.seg_bin0[seg + 1] - d0;
+        const int bits = c.bsh + (int)c.seg_sh[seg];  // a k-mer's bits within its bin
+        const uint64_t mask = (1ull << bits) - 1;
+        const uint32_t r = base + rr, L = rr < per && r < end ? c.t.seq_len[r] : 0u;
+        uint32_t id = r;
+        if (c.label && L) {
+            const uint32_t p = c.label[r];
+            id = p == BAD ? r : p;  // findRoot after full compression (metapart.c:543-568)
         }
-        __syncthreads();  // the tile before is stored
-        if (seg != have) {
-            have = seg;
-            d0 = c.seg_bin0[seg];
-            nd = c.seg_bin0[seg + 1] - d0;
-            for (uint32_t d = tid; d < nd; d += SP_THREADS) sm.b0[d] = c.bb0[d0 + d] & (NB - 1);
-            for (uint32_t d = tid; d < CELLS_1; d += SP_THREADS) sm.cells[d] = c.cells[(size_t)seg * CELLS_1 + d];
-        }
-        uint64_t key[SP_ITEMS];
-        uint32_t rd[SP_ITEMS];
-        if constexpr (READS) {
-            uint32_t *packed = reinterpret_cast<uint32_t *>(sm.key);
-            const uint32_t r1 = min(end, base + per);
-            if (c.check_many) many[tid] = 0;
-            rt_pack(c.t, base, r1, packed);
-            __syncthreads();
-#pragma unroll
-            for (int j = 0; j < SP_ITEMS; j++) rd[j] = 0xFFFFu;
-            const uint32_t rr = tid / c.t.spr, i0 = (tid - rr * c.t.spr) * c.t.P, r = base + rr;
-            const uint32_t L = rr < per && r < r1 ? c.t.seq_len[r] : 0u;
-            uint32_t id = r;
-            if (L > (uint32_t)c.t.k && i0 <= L - (uint32_t)c.t.k) {
-                if (c.label) {
-                    const uint32_t p = c.label[r];
-                    id = p == BAD ? r : p;  // findRoot after full compression (metapart.c:543-568)
-                }
-                KmerRoll s;
-                kr_init(s, c.t, packed + rr * rt_stride(c.t), L, i0);
-                const uint32_t m = min(c.t.P, s.last + 1 - i0);
-                uint32_t got = 0;
-#pragma unroll
-                for (int j = 0; j < SP_ITEMS; j++) {
-                    if (j < m) {
-                        uint64_t km;
-                        const bool v = kr_get(s, c.t.k, km);
-                        const uint32_t b = (uint32_t)(km >> c.bsh);
-                        if (v && b >= c.b_lo && b < c.b_hi) {
-                            const uint32_t d = cell_digit(sm.cells, sm.b0, c.shift, b - c.b_lo, b);
-                            key[j] = ((((uint64_t)(b - sm.b0[d]) << c.bsh) | (km & lowmask)) << 6) | kr_adj6(s);
-                            rd[j] = d;
-                            got++;
-                        }
-                        kr_next(s, c.t.k);
+        if (c.check_many) many[tid] = 0;
+        __syncthreads();  // the tile before is stored, this one's reads are packed
+        uint32_t kl[SP_ITEMS], kh[SP_ITEMS], rd[SP_ITEMS];
+        {
+            KmerRoll<HI> s = {};
+            if (L > (uint32_t)c.t.k && i0 <= L - (uint32_t)c.t.k) s.init(c.t, sm.packed + rr * rt_stride(c.t), L, i0);
+            const uint32_t mh = (uint32_t)(mask >> 32), dsh = HI ? bits - 32 : bits;
+            const uint32_t cn[2] = {s.compl_nibbles(s.an[0]), s.compl_nibbles(s.an[1])};
+            const uint32_t cp[2] = {s.compl_nibbles(s.ap[0]), s.compl_nibbles(s.ap[1])};
+            uint32_t got = 0;
+            auto position = [&](auto J) {
+                constexpr int j = decltype(J)::value;
+                const uint64_t f = s.fwd(), q = s.rc();
+                const bool fw = f < q;
+                const uint64_t rel = (fw ? f : q) - c.k_lo;
+                const uint32_t a6 = s.template adj6<j>(fw, cn, cp);
+                rd[j] = ~0u;
+                if (((s.vm >> j) & 1u) && rel < c.k_span) {
+                    const uint32_t d = HI ? (uint32_t)(rel >> 32) >> dsh : (uint32_t)(rel >> dsh);
+                    if constexpr (HI) {
+                        kl[j] = ((uint32_t)rel << 6) | a6;
+                        kh[j] = __funnelshift_l((uint32_t)rel, (uint32_t)(rel >> 32) & mh, 6);
+                    } else {
+                        const uint64_t key = ((rel & mask) << 6) | a6;
+                        kl[j] = (uint32_t)key;
+                        kh[j] = (uint32_t)(key >> 32);
                     }
+                    rd[j] = (d << 2) | (atomicAdd(&sm.hist[d], 1u) << 16);
+                    got++;
                 }
-                // the reference counts a read's k-mers of one scan in 8 bits (enumerateKmers.c:152)
-                if (c.check_many && atomicAdd(&many[rr], got) + got > 255u) atomicOr(c.err, 4u);
-            }
-            split_tile<BinSmem, GP_MAX_BINS>(sm, key, rd, c.bcur + d0, nd, [&](int) { return id; }, c.out_k, c.out_id, c.n);
-        } else {
-            const uint32_t nv = min((uint32_t)SP_TILE, end - base);
-            __syncthreads();
-#pragma unroll
-            for (int j = 0; j < SP_ITEMS; j++) {
-                const uint32_t e = j * SP_THREADS + tid;
-                rd[j] = 0xFFFFu;
-                if (e < nv) {
-                    const uint64_t v = c.lo[base + e], km = (v >> 8) | (c.hi ? (uint64_t)c.hi[base + e] << 56 : 0ull);
-                    const uint32_t b = min(max((uint32_t)(km >> c.bsh), c.b_lo), c.b_hi - 1);
-                    const uint32_t d = cell_digit(sm.cells, sm.b0, c.shift, b - c.b_lo, b);
-                    key[j] = ((((uint64_t)(b - sm.b0[d]) << c.bsh) | (km & lowmask)) << 6) | (v & 63u);
-                    rd[j] = d;
-                }
-            }
-            split_tile<BinSmem, GP_MAX_BINS>(
-                sm, key, rd, c.bcur + d0, nd,
-                [&](int j) { const uint32_t e = j * SP_THREADS + tid; return e < nv ? c.id[base + e] : 0u; }, c.out_k, c.out_id, c.n);
+                s.next();
+            };
+            static_assert(SP_ITEMS == 12, "positions below");
+            position(std::integral_constant<int, 0>{});
+            position(std::integral_constant<int, 1>{});
+            position(std::integral_constant<int, 2>{});
+            position(std::integral_constant<int, 3>{});
+            position(std::integral_constant<int, 4>{});
+            position(std::integral_constant<int, 5>{});
+            position(std::integral_constant<int, 6>{});
+            position(std::integral_constant<int, 7>{});
+            position(std::integral_constant<int, 8>{});
+            position(std::integral_constant<int, 9>{});
+            position(std::integral_constant<int, 10>{});
+            position(std::integral_constant<int, 11>{});
+            // the reference counts a read's k-mers of one scan in 8 bits (enumerateKmers.c:152)
+            if (c.check_many && got && atomicAdd(&many[rr], got) + got > 255u) atomicOr(c.err, 4u);
+        }
+        const uint32_t nv = split_order(sm, kl, kh, rd, c.bcur + d0, nd, [&](int) { return id; }, c.n);
+        split_store(sm, nv, c.out_k, c.out_id);
+        // the next tile's reads while others store (its bytes fetched before the stores instead cost registers that spill: 37.5
+        // against 35.7 ms at 20M x 150 bp, 2 scans)
+        const uint32_t next = tile + gridDim.x;
+        if (next < c.tiles) {
+            bin_tile(c, next, per, c.n_reads, seg, base, end);
+            rt_pack(c.t, base, end - base, sm.packed);
         }
     }
 }
 
-// Second pass: a bin's tuples into its units.  A block takes consecutive tiles, so it sets up a bin's digits once.
-template <int DIGITS, int BLOCKS>
-__global__ void __launch_bounds__(SP_THREADS, BLOCKS) k_split_units(const uint64_t *__restrict__ kk, const uint32_t *__restrict__ id,
-                                                                    uint32_t n, int bsh, const uint32_t *__restrict__ ctr,
-                                                                    const uint32_t *__restrict__ bstart,
-                                                                    const uint32_t *__restrict__ bb0,
-                                                                    const uint32_t *__restrict__ bu0,
-                                                                    const uint32_t *__restrict__ bcur,
-                                                                    const uint32_t *__restrict__ ub0, uint32_t *ucur,
-                                                                    const uint32_t *__restrict__ tile_bin,
-                                                                    const uint32_t *__restrict__ tile_first, uint64_t *out_k,
-                                                                    uint32_t *out_id)
+__global__ void __launch_bounds__(SP_THREADS, 2) k_split_tuples(BinCtx c)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    UnitSmem<DIGITS> &sm = *reinterpret_cast<UnitSmem<DIGITS> *>(smraw);
+    SplitSmem &sm = *reinterpret_cast<SplitSmem *>(smraw);
     const int tid = threadIdx.x;
-    const uint32_t tiles = ctr[GC_TILES], per = (tiles + gridDim.x - 1) / gridDim.x;
-    const uint32_t t0 = blockIdx.x * per, t1 = min(tiles, t0 + per);
-    uint32_t have = ~0u, d0 = 0, nd = 0, bin_start = 0, bin_end = 0, first_tile = 0;
-    int shift = 0;
-    bool whole = false;
-    for (uint32_t d = tid; d < DIGITS; d += SP_THREADS) sm.hist[d] = 0;
-    for (uint32_t tile = t0; tile < t1; tile++) {
-        const uint32_t bin = tile_bin[tile];
+    for (uint32_t d = tid; d < GP_DIGITS; d += SP_THREADS) sm.hist[d] = 0;
+    for (uint32_t tile = blockIdx.x; tile < c.tiles; tile += gridDim.x) {
+        uint32_t seg, base, end;
+        bin_tile(c, tile, SP_TILE, c.n, seg, base, end);
+        const uint32_t d0 = c.seg_bin0[seg], nd = c.seg_bin0[seg + 1] - d0, nv = end - base;
+        const int bits = c.bsh + (int)c.seg_sh[seg];
+        const uint64_t mask = (1ull << bits) - 1;
         __syncthreads();  // the tile before is stored
-        if (bin != have) {
-            have = bin;
-            bin_start = bstart[bin];
-            bin_end = bstart[bin + 1];
-            whole = bcur[bin] == bin_end;  // else the histogram is not the tuples' (the bin's units stay short: k_group)
-            first_tile = tile_first[bin];
-            d0 = bu0[bin];
-            nd = min(bu0[bin + 1] - d0, (uint32_t)DIGITS);
-            const uint32_t first = bb0[bin];
-            for (uint32_t d = tid; d < nd; d += SP_THREADS) sm.b0[d] = (uint16_t)((ub0[d0 + d] & 0x7FFFFFFFu) - first);
-            __syncthreads();
-            const uint32_t span = (uint32_t)sm.b0[nd - 1] + 1;  // buckets from the last unit's first on are its own
-            shift = cell_shift(span, CELLS_2);
-            for (uint32_t c = tid; c < CELLS_2; c += SP_THREADS) {
-                uint32_t v[2];
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    const uint32_t x = ((c + q) << shift) - q;
-                    uint32_t a = 0, z = nd - 1;
-                    while (a < z) {
-                        const uint32_t m = (a + z + 1) >> 1;
-                        if (sm.b0[m] <= x) a = m; else z = m - 1;
-                    }
-                    v[q] = a;
-                }
-                sm.cells[c] = v[0] | (v[1] << 16);
-            }
-            __syncthreads();
-        }
-        if (!whole) continue;
-        const uint32_t base = bin_start + (tile - first_tile) * SP_TILE, nv = min((uint32_t)SP_TILE, bin_end - base);
-        const uint32_t top = (uint32_t)sm.b0[nd - 1];
-        uint64_t key[SP_ITEMS];
-        uint32_t rd[SP_ITEMS];
+        uint32_t kl[SP_ITEMS], kh[SP_ITEMS], rd[SP_ITEMS];
 #pragma unroll
         for (int j = 0; j < SP_ITEMS; j++) {
             const uint32_t e = j * SP_THREADS + tid;
-            key[j] = e < nv ? kk[base + e] : 0ull;
+            rd[j] = ~0u;
+            if (e < nv) {
+                const uint64_t v = c.lo[base + e], km = (v >> 8) | (c.hi ? (uint64_t)c.hi[base + e] << 56 : 0ull);
+                const uint64_t rel = km - c.k_lo;
+                if (rel < c.k_span) {
+                    const uint64_t key = ((rel & mask) << 6) | (v & 63u);
+                    const uint32_t d = (uint32_t)(rel >> bits);
+                    kl[j] = (uint32_t)key;
+                    kh[j] = (uint32_t)(key >> 32);
+                    rd[j] = (d << 2) | (atomicAdd(&sm.hist[d], 1u) << 16);
+                }
+            }
         }
+        const uint32_t got = split_order(
+            sm, kl, kh, rd, c.bcur + d0, nd,
+            [&](int j) { const uint32_t e = j * SP_THREADS + tid; return e < nv ? c.id[base + e] : 0u; }, c.n);
+        split_store(sm, got, c.out_k, c.out_id);
+    }
+}
+
+// Second pass: a bin's tuples into its units.  Blocks take four consecutive tiles at a time, so all of them work in a few
+// neighbouring bins: with long stretches per block instead (a bin or more), 300 bins of 560 units were open at once, L2
+// evicted their half-filled lines, and 2.39 G tuples moved 102 GB through DRAM where they take 57 (26.5 ms; 15.1 now, 3.8
+// TB/s, at 20M x 150 bp, 2 scans).
+__global__ void __launch_bounds__(SP_THREADS, 2) k_split_units(const uint64_t *__restrict__ kk, const uint32_t *__restrict__ id,
+                                                               uint32_t n, int bsh, uint32_t seg_lo, const uint32_t *__restrict__ ctr,
+                                                               const uint32_t *__restrict__ bstart,
+                                                               const uint32_t *__restrict__ bfirst,
+                                                               const uint32_t *__restrict__ bu0,
+                                                               const uint32_t *__restrict__ bcur,
+                                                               const uint32_t *__restrict__ bin_sh,
+                                                               const uint32_t *__restrict__ ub0, uint32_t *ucur,
+                                                               const uint32_t *__restrict__ unit_of, uint32_t nbk,
+                                                               const uint4 *__restrict__ tile_of, uint64_t *out_k,
+                                                               uint32_t *out_id)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    UnitSmem &sm = *reinterpret_cast<UnitSmem *>(smraw);
+    const int tid = threadIdx.x, bits = bsh + 6;
+    const uint32_t tiles = ctr[GC_TILES];
+    uint32_t have = ~0u, d0 = 0, nd = 0;
+    int cs = 0;  // buckets per cell: 2^cs, 0 for bins of at most 1024 buckets
+    bool whole = false;
+    for (uint32_t d = tid; d < GP_DIGITS; d += SP_THREADS) sm.hist[d] = 0;
+    auto tile_at = [&](uint32_t i) { return ((i / SP_CHUNK) * gridDim.x + blockIdx.x) * SP_CHUNK + i % SP_CHUNK; };
+    uint32_t kl[SP_ITEMS], kh[SP_ITEMS];
+    auto load = [&](const uint4 &t) {
+        const uint64_t *kp = kk + t.x + tid;
 #pragma unroll
         for (int j = 0; j < SP_ITEMS; j++) {
-            const uint32_t b = min((uint32_t)(key[j] >> (bsh + 6)), top);
-            rd[j] = j * SP_THREADS + tid < nv ? cell_digit(sm.cells, sm.b0, shift, b, b) : 0xFFFFu;
+            const uint64_t v = j * SP_THREADS + tid < t.y ? kp[j * SP_THREADS] : 0ull;
+            kl[j] = (uint32_t)v;
+            kh[j] = (uint32_t)(v >> 32);
         }
-        split_tile<UnitSmem<DIGITS>, DIGITS>(
-            sm, key, rd, ucur + d0, nd, [&](int j) { const uint32_t e = j * SP_THREADS + tid; return e < nv ? id[base + e] : 0u; },
-            out_k, out_id, n);
+    };
+    uint4 now = make_uint4(0, 0, 0, 0);
+    if (tile_at(0) < tiles) {
+        now = tile_of[tile_at(0)];
+        load(now);
+    }
+    for (uint32_t i = 0; tile_at(i) < tiles; i++) {
+        const uint32_t base = now.x, nv = now.y, bin = now.z;
+        __syncthreads();  // the tile before is stored
+        if (bin != have) {
+            have = bin;
+            whole = bcur[bin] == bstart[bin + 1];  // else the histogram is not the tuples' (the bin's units stay short: k_group)
+            d0 = bu0[bin];
+            nd = min(bu0[bin + 1] - d0, GP_DIGITS);
+            const uint32_t s = bin_sh[bin], b0 = bfirst[bin];
+            cs = s > 10 ? (int)s - 10 : 0;
+            for (uint32_t x = tid; x < GP_DIGITS; x += SP_THREADS) {
+                const uint32_t r = b0 + (x << cs);
+                const uint32_t u = x < (1u << (s - cs)) && r < nbk ? unit_of[r] : d0;
+                sm.cell[x] = (uint16_t)((u + 1 > d0 + 1 ? min(u - d0, nd - 1) : 0u) << 2);
+                if (cs && x < nd) sm.b0[x] = (uint16_t)(((ub0[d0 + x] & (NB - 1)) - seg_lo) & ((1u << s) - 1));
+            }
+            __syncthreads();
+        }
+        uint32_t got = 0;
+        if (whole) {
+            uint32_t rd[SP_ITEMS];
+#pragma unroll
+            for (int j = 0; j < SP_ITEMS; j++) {
+                const uint32_t b = bits >= 32 ? kh[j] >> (bits - 32) : __funnelshift_r(kl[j], kh[j], bits);
+                uint32_t d4 = sm.cell[b >> cs];
+                if (cs)
+                    while (d4 / 4 + 1 < nd && sm.b0[d4 / 4 + 1] <= b) d4 += 4;
+                rd[j] = j * SP_THREADS + tid < nv ? d4 | (atomicAdd(&at_byte(sm.hist, d4), 1u) << 16) : ~0u;
+            }
+            const uint32_t *ip = id + base + tid;
+            got = split_order(sm, kl, kh, rd, ucur + d0, nd, [&](int j) { return j * SP_THREADS + tid < nv ? ip[j * SP_THREADS] : 0u; }, n);
+        }
+        if (tile_at(i + 1) < tiles) {  // the next tile's keys on their way while this one's tuples are stored
+            now = tile_of[tile_at(i + 1)];
+            load(now);
+        }
+        split_store(sm, got, out_k, out_id);
     }
 }
 
@@ -978,9 +994,7 @@ __global__ void k_join_pair(uint32_t *parent, uint32_t a, uint32_t b, uint32_t *
 
 static unsigned blocks_of(uint64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
-static uint32_t bins_bound(uint64_t n, int nseg, int shift) { return (uint32_t)(n >> shift) + 18u * (uint32_t)nseg + 1u; }
-
-// A scan takes the grouped path when its positions fit 32 bits, its read ids 31, and the split's digits suffice.
+// A scan takes the grouped path when its tuple positions fit 32 bits and its read ids 31.
 bool group_fits(uint64_t n, uint64_t n_reads, const SortSegments *segs)
 {
     return n >= 1 && n <= GROUP_MAX_TUPLES && n_reads < GROUP_MAX_READS && (!segs || segs->nseg < 2048);
@@ -992,12 +1006,10 @@ static void group_kernel_attrs()
     int dev = 0;
     cudaGetDevice(&dev);
     std::call_once(once[dev & 63], [] {
-        cudaFuncSetAttribute(k_split_bins<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinSmem));
-        cudaFuncSetAttribute(k_split_bins<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinSmem));
-        cudaFuncSetAttribute(k_split_units<GP_MAX_UNITS, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(UnitSmem<GP_MAX_UNITS>));
-        cudaFuncSetAttribute(k_split_units<GP_MAX_UNITS_L, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(UnitSmem<GP_MAX_UNITS_L>));
+        cudaFuncSetAttribute(k_split_reads<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinSmem));
+        cudaFuncSetAttribute(k_split_reads<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinSmem));
+        cudaFuncSetAttribute(k_split_tuples, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SplitSmem));
+        cudaFuncSetAttribute(k_split_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(UnitSmem));
         cudaFuncSetAttribute(k_group<512, 12, 13>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmemS));
         cudaFuncSetAttribute(k_group<1024, 12, 14>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmemL));
     });
@@ -1008,64 +1020,57 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
     const int nseg = (int)g.seg_tstart.size() - 1;
     const uint32_t nbounds = (uint32_t)g.bounds.size();
     const uint64_t nbk = g.hi - g.lo;
-    uint64_t seg_max = 0;  // a segment's units and bins bound the digits of a pass
-    for (int q = 0; q < nseg; q++) seg_max = std::max<uint64_t>(seg_max, g.seg_tstart[q + 1] - g.seg_tstart[q]);
-    g.unit_shift = GP_UNIT_SHIFT;
-    // units per segment: a start per thread range, per 2^16 buckets, and at most two per 2^unit_shift tuples
-    const uint64_t units_seg = 2 * (seg_max >> g.unit_shift) + nbounds + 20;
-    g.two_level = units_seg > GP_MAX_BINS;
-    // two levels: about as many bins as units per bin
-    int lg = 0;
-    while ((seg_max >> lg) > 1) lg++;
-    g.bin_shift = (g.unit_shift + lg + 1) / 2;
-    while ((seg_max >> g.bin_shift) + 20 > GP_MAX_BINS) g.bin_shift++;
-    g.max_units = 2 * (uint32_t)(g.n >> g.unit_shift) + nbounds + 20u * (uint32_t)nseg + 8;
-    g.max_bins = g.two_level ? bins_bound(g.n, nseg, g.bin_shift) : g.max_units;
-    if (g.two_level) g.max_units += g.max_bins;
-    g.max_tiles = (uint32_t)(g.n / SP_TILE) + g.max_bins + 1;
-    g.cell_shift = cell_shift(nseg > 1 ? (uint64_t)NB : nbk, CELLS_1);
-    g.cells = arena.alloc<uint32_t>((size_t)nseg * CELLS_1);
+    // host side of the plan: every segment's bins and the first tuple of its last range with tuples
+    std::vector<uint32_t> &h = g.h_plan;
+    h.assign(3 * (size_t)nseg + 1, 0);
+    uint32_t *bin0 = h.data(), *sh = bin0 + nseg + 1, *lrs = sh + nseg;
+    for (int q = 0, t = 0; q < nseg; q++) {
+        const uint64_t n = g.seg_tstart[q + 1] - g.seg_tstart[q], span = nseg > 1 ? (uint64_t)NB : nbk;
+        sh[q] = (uint32_t)bin_width(n, span);
+        bin0[q + 1] = bin0[q] + (uint32_t)((span - 1) >> sh[q]) + 1;
+        uint64_t b = g.seg_tstart[q];
+        for (; t < (int)nbounds && g.bounds[t] < g.seg_tstart[q + 1]; t++) b = std::max(b, g.bounds[t]);
+        lrs[q] = (uint32_t)b;
+    }
+    g.bins = bin0[nseg];
+    g.seg_lo = nseg > 1 ? 0u : (uint32_t)g.lo;
+    // units: a start per thread range, segment and bin, and at most two per 2^GP_UNIT_SHIFT tuples
+    g.max_units = 2 * (uint32_t)(g.n >> GP_UNIT_SHIFT) + nbounds + g.bins + 2u * (uint32_t)nseg + 8;
+    g.max_tiles = (uint32_t)(g.n / SP_TILE) + g.bins + 1;
     const uint32_t nblk = blocks_of(nbk, GP_COUNT_BLOCK);
     const size_t brk_words = nbk / 32 + 1;
     uint32_t *brk = arena.alloc<uint32_t>(brk_words + GC_N + (size_t)nseg * QW);
     uint64_t *blk = arena.alloc<uint64_t>(nblk), *d_bounds = arena.alloc<uint64_t>(nbounds);
     g.ustart = arena.alloc<uint32_t>(3 * (size_t)(g.max_units + 1));
-    g.bstart = arena.alloc<uint32_t>(4 * (size_t)(g.max_bins + 1));
-    g.seg_bin0 = arena.alloc<uint32_t>(2 * (size_t)nseg + 1);
-    g.tile_bin = arena.alloc<uint32_t>((size_t)g.max_tiles + g.max_bins);
+    g.bstart = arena.alloc<uint32_t>(5 * (size_t)(g.bins + 1));
+    g.unit_of = arena.alloc<uint32_t>(nbk);
+    g.seg_bin0 = arena.alloc<uint32_t>(h.size());
+    g.tiles = arena.alloc<uint4>(g.max_tiles);
     g.mid = arena.alloc<uint32_t>(2 * (size_t)(g.n / GP_CAP_S + 1));
     g.qlist = arena.alloc<uint32_t>(3 * (size_t)(g.max_units + 1));
-    if (!brk || !blk || !d_bounds || !g.ustart || !g.bstart || !g.seg_bin0 || !g.tile_bin || !g.mid || !g.qlist || !g.cells)
+    if (!brk || !blk || !d_bounds || !g.ustart || !g.bstart || !g.seg_bin0 || !g.tiles || !g.mid || !g.qlist || !g.unit_of)
         return set_error(MP_ENOMEM, "device memory for the scan's plan");
     g.ub0 = g.ustart + g.max_units + 1;
     g.ucur = g.ub0 + g.max_units + 1;
-    g.bb0 = g.bstart + g.max_bins + 1;
-    g.bu0 = g.bb0 + g.max_bins + 1;
-    g.bcur = g.bu0 + g.max_bins + 1;
-    g.lrs = g.seg_bin0 + nseg + 1;
-    g.tile_first = g.tile_bin + g.max_tiles;
+    g.bu0 = g.bstart + g.bins + 1;
+    g.bcur = g.bu0 + g.bins + 1;
+    g.bin_sh = g.bcur + g.bins + 1;
+    g.bfirst = g.bin_sh + g.bins + 1;
+    g.seg_sh = g.seg_bin0 + nseg + 1;
+    g.lrs = g.seg_sh + nseg;
     g.big = g.mid + g.n / GP_CAP_S + 1;
     g.ctr = brk + brk_words;
     g.quirk = g.ctr + GC_N;
-    std::vector<uint32_t> &lrs = g.h_lrs;
-    lrs.assign(nseg, 0);
-    for (int q = 0, t = 0; q < nseg; q++) {  // the last range bound inside the segment's tuples
-        uint64_t b = g.seg_tstart[q];
-        for (; t < (int)nbounds && g.bounds[t] < g.seg_tstart[q + 1]; t++) b = std::max(b, g.bounds[t]);
-        lrs[q] = (uint32_t)b;
-    }
     MP_CUDA(cudaMemsetAsync(brk, 0, (brk_words + GC_N + (size_t)nseg * QW) * 4, st));
     MP_CUDA(cudaMemcpyAsync(d_bounds, g.bounds.data(), nbounds * 8, cudaMemcpyHostToDevice, st));
-    MP_CUDA(cudaMemcpyAsync(g.lrs, lrs.data(), nseg * 4, cudaMemcpyHostToDevice, st));
-    PlanCtx c{g.d_hist, g.lo, g.hi, brk, g.unit_shift, g.bin_shift, g.two_level};
+    MP_CUDA(cudaMemcpyAsync(g.seg_bin0, h.data(), h.size() * 4, cudaMemcpyHostToDevice, st));
+    const PlanCtx c{g.d_hist, g.lo, g.hi, brk, g.seg_sh, g.seg_bin0, g.seg_lo};
     (count_launch(), k_gp_marks<<<blocks_of(nbounds, 64), 64, 0, st>>>(g.d_hist, g.lo, g.hi, d_bounds, (int)nbounds, brk));
     (count_launch(), k_gp_count<<<nblk, GP_COUNT_THREADS, 0, st>>>(c, blk));
-    (count_launch(), k_gp_scan<<<1, 1024, 0, st>>>(blk, nblk, (uint32_t)g.n, nseg, g.ctr, g.ustart, g.bstart, g.bu0, g.seg_bin0));
-    (count_launch(), k_gp_write<<<nblk, GP_COUNT_THREADS, 0, st>>>(c, blk, g.ctr, g.ustart, g.ub0, g.ucur, g.bstart, g.bb0, g.bu0,
-                                                                  g.bcur, g.seg_bin0, g.mid, g.big));
-    (count_launch(), k_gp_cells<<<dim3(CELLS_1 / 256, nseg), 256, 0, st>>>(g.bb0, g.seg_bin0, nseg > 1 ? 0u : (uint32_t)g.lo,
-                                                                          nseg > 1 ? NB : (uint32_t)g.hi, g.cell_shift, g.cells));
-    if (g.two_level) (count_launch(), k_gp_tiles<<<1, 1024, 0, st>>>(g.bstart, g.ctr, g.tile_first, g.tile_bin));
+    (count_launch(), k_gp_scan<<<1, 1024, 0, st>>>(blk, nblk, (uint32_t)g.n, g.bins, g.ctr, g.ustart, g.bstart, g.bu0));
+    (count_launch(), k_gp_write<<<nblk, GP_COUNT_THREADS, 0, st>>>(c, blk, g.ctr, g.ustart, g.ub0, g.ucur, g.bstart, g.bu0, g.bcur,
+                                                                  g.bin_sh, g.bfirst, g.unit_of, g.mid, g.big));
+    (count_launch(), k_gp_tiles<<<1, 1024, 0, st>>>(g.bstart, g.bins, g.ctr, g.tiles));
     MP_CUDA(cudaMemcpyAsync(g.hctr, g.ctr, GC_N * 4, cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaGetLastError());
     return 0;
@@ -1096,18 +1101,18 @@ static int launch_bins(GroupScan &g, BinCtx &c, const std::vector<uint64_t> &seg
         (count_launch(), k_gp_segtiles<<<nseg, 256, 0, st>>>(d, nseg, d + h.size()));
     }
     c.n = (uint32_t)g.n;
-    c.b_lo = nseg > 1 ? 0u : (uint32_t)g.lo;
-    c.b_hi = nseg > 1 ? NB : (uint32_t)g.hi;
     c.bsh = 2 * (g.k - 10);
-    c.shift = g.cell_shift;
-    c.bb0 = g.bb0;
+    c.k_lo = (uint64_t)g.seg_lo << c.bsh;
+    c.k_span = (nseg > 1 ? (uint64_t)NB : g.hi - g.lo) << c.bsh;
     c.seg_bin0 = g.seg_bin0;
-    c.cells = g.cells;
+    c.seg_sh = g.seg_sh;
     c.bcur = g.bcur;
     c.err = g.ctr + GC_ERR;
+    uint32_t least = 16;  // the narrowest bins
+    for (int q = 0; q < nseg; q++) least = std::min(least, g.h_plan[(size_t)nseg + 1 + q]);
+    auto kern = !reads ? k_split_tuples : g.k >= 17 && c.bsh + (int)least >= 32 ? k_split_reads<true> : k_split_reads<false>;
     const unsigned blocks = std::min<unsigned>(c.tiles, 2u * (unsigned)sm_count());
-    if (blocks)
-        (count_launch(), (reads ? k_split_bins<true> : k_split_bins<false>)<<<blocks, SP_THREADS, sizeof(BinSmem), st>>>(c));
+    if (blocks) (count_launch(), kern<<<blocks, SP_THREADS, reads ? sizeof(BinSmem) : sizeof(SplitSmem), st>>>(c));
     MP_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1116,7 +1121,7 @@ int group_bins_reads(GroupScan &g, const uint8_t *fq, const ParsedReads &pr, con
                      const uint32_t *label, uint64_t *k1, uint32_t *id1, DeviceArena &arena, cudaStream_t st)
 {
     BinCtx c;
-    c.t = read_tiles(fq, pr, g.k, pr.max_len, SP_THREADS);
+    c.t = read_tiles(fq, pr, g.k, pr.max_len, SP_THREADS, SP_PACKED);
     c.n_reads = (uint32_t)pr.n_reads;
     c.check_many = pr.max_len > (uint32_t)g.k + 254u;  // a read with 256 positions or more
     c.label = label;
@@ -1139,15 +1144,9 @@ int group_bins_tuples(GroupScan &g, const uint64_t *lo, const uint8_t *hi, const
 
 int group_units(GroupScan &g, const uint64_t *k1, const uint32_t *id1, uint64_t *k2, uint32_t *id2, cudaStream_t st)
 {
-    if (!g.two_level) return 0;
-    const int bsh = 2 * (g.k - 10);
-    const unsigned sms = (unsigned)sm_count();
-    if (g.bin_shift <= 21)
-        (count_launch(), k_split_units<GP_MAX_UNITS, 2><<<std::min(g.max_tiles, 2 * sms), SP_THREADS, sizeof(UnitSmem<GP_MAX_UNITS>), st>>>(
-            k1, id1, (uint32_t)g.n, bsh, g.ctr, g.bstart, g.bb0, g.bu0, g.bcur, g.ub0, g.ucur, g.tile_bin, g.tile_first, k2, id2));
-    else
-        (count_launch(), k_split_units<GP_MAX_UNITS_L, 1><<<std::min(g.max_tiles, sms), SP_THREADS, sizeof(UnitSmem<GP_MAX_UNITS_L>), st>>>(
-            k1, id1, (uint32_t)g.n, bsh, g.ctr, g.bstart, g.bb0, g.bu0, g.bcur, g.ub0, g.ucur, g.tile_bin, g.tile_first, k2, id2));
+    (count_launch(), k_split_units<<<std::min(g.max_tiles, 2u * (unsigned)sm_count()), SP_THREADS, sizeof(UnitSmem), st>>>(
+        k1, id1, (uint32_t)g.n, 2 * (g.k - 10), g.seg_lo, g.ctr, g.bstart, g.bfirst, g.bu0, g.bcur, g.bin_sh, g.ub0,
+        g.ucur, g.unit_of, (uint32_t)(g.hi - g.lo), g.tiles, k2, id2));
     MP_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1156,7 +1155,7 @@ int group_filter(GroupScan &g, const uint64_t *kk, const uint32_t *ids, uint32_t
                  DeviceArena &arena, cudaStream_t st)
 {
     group_kernel_attrs();
-    const uint32_t *fill = g.two_level ? g.ucur : g.bcur;
+    const uint32_t *fill = g.ucur;
     GroupCtx c{kk, ids, g.ustart, g.ub0, fill, g.lrs, nullptr, g.ctr, g.qlist, g.quirk, GC_WORK_S, GC_UNITS, 0, (uint32_t)GP_CAP_S,
                out, parent, filtered};
     const unsigned sms = (unsigned)sm_count();

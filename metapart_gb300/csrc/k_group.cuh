@@ -7,7 +7,7 @@
 namespace mp {
 
 // A scan without the order of its tuples: what the mischief filter and the unions need of the sorted scan is
-// only which tuples share a k-mer, so the tuples are split into units of consecutive m-mer buckets (one or two
+// only which tuples share a k-mer, so the tuples are split into units of consecutive m-mer buckets (two
 // unstable multi-split passes) and grouped by k-mer in shared-memory hash tables.  Results equal filter_scan +
 // union_scan over the sorted scan: the same BAD marks, the same components.
 //
@@ -27,23 +27,24 @@ struct GroupScan {
     std::vector<uint64_t> seg_tstart;  // nseg + 1 tuple offsets ({0, n} for one scan)
 
     // the plan (device), from group_plan
-    bool two_level = false;
-    int unit_shift = 0, bin_shift = 0, cell_shift = 0;
-    uint32_t max_units = 0, max_bins = 0, max_tiles = 0;
+    uint32_t bins = 0, seg_lo = 0, max_units = 0, max_tiles = 0;
     uint32_t *ustart = nullptr, *ub0 = nullptr, *ucur = nullptr;  // units: first tuple, first bucket | range start << 31, fill
-    uint32_t *bstart = nullptr, *bb0 = nullptr, *bu0 = nullptr, *bcur = nullptr;  // bins: first tuple, bucket, unit; fill
-    uint32_t *seg_bin0 = nullptr, *tile_bin = nullptr, *tile_first = nullptr, *cells = nullptr;
+    uint32_t *bstart = nullptr, *bu0 = nullptr, *bcur = nullptr, *bin_sh = nullptr, *bfirst = nullptr;  // bins: first tuple, unit;
+                                                                                  // fill; width; first bucket
+    uint32_t *unit_of = nullptr;  // every bucket's unit
+    uint32_t *seg_bin0 = nullptr, *seg_sh = nullptr;
+    uint4 *tiles = nullptr;       // of the second pass
     uint32_t *mid = nullptr, *big = nullptr;  // units above a small block's and above a large block's capacity
     uint32_t *lrs = nullptr;                  // per segment: first tuple of its last range with tuples
     uint32_t *ctr = nullptr;                  // GC_* counters
     uint32_t *qlist = nullptr;                // grouped stretches of the segments' last ranges
     uint32_t *quirk = nullptr;                // per segment: QW words (see k_gp_quirk)
     uint32_t hctr[16] = {};                   // the counters on the host
-    std::vector<uint32_t> h_lrs, h_tiles;     // sources of uploads still queued
+    std::vector<uint32_t> h_plan, h_tiles;     // sources of uploads still queued
 };
 
 enum GroupCounter : int {
-    GC_UNITS = 0, GC_BINS, GC_TILES, GC_MID, GC_BIG, GC_BIG_TUPLES,  // the plan's counts
+    GC_UNITS = 0, GC_TILES, GC_MID, GC_BIG, GC_BIG_TUPLES,  // the plan's counts
     GC_WORK_S, GC_WORK_L, GC_OUT, GC_QLIST, GC_ERR, GC_N = 16
 };
 
@@ -57,14 +58,13 @@ struct GroupQuirk {
 bool group_fits(uint64_t n, uint64_t n_reads, const SortSegments *segs);
 // Plans g (its inputs set) on the device, its counts copied into g.hctr in stream order.
 int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st);
-// First split pass, into bins (into units when one level does: g.two_level false), of n tuples to (k1, id1): enumerated
-// from the reads (seg_reads: nseg + 1 read offsets; label: the reads' components, null in the first scan; every read at
+// First split pass, into bins, of n tuples to (k1, id1): enumerated from the reads (seg_reads: nseg + 1 read offsets; label: the reads' components, null in the first scan; every read at
 // most 300 positions), or of tuples enumerated before, segment-major.
 int group_bins_reads(GroupScan &g, const uint8_t *fq, const ParsedReads &pr, const std::vector<uint64_t> &seg_reads,
                      const uint32_t *label, uint64_t *k1, uint32_t *id1, DeviceArena &arena, cudaStream_t st);
 int group_bins_tuples(GroupScan &g, const uint64_t *lo, const uint8_t *hi, const uint32_t *id, uint64_t *k1, uint32_t *id1,
                       DeviceArena &arena, cudaStream_t st);
-// Second pass, with two levels: the bins' tuples into units.
+// Second pass: the bins' tuples into units.
 int group_units(GroupScan &g, const uint64_t *k1, const uint32_t *id1, uint64_t *k2, uint32_t *id2, cudaStream_t st);
 // The mischief filter over the split tuples (kk, ids), and every k-mer's reads side by side in out (n ids).
 int group_filter(GroupScan &g, const uint64_t *kk, const uint32_t *ids, uint32_t *out, uint32_t *parent, uint8_t *filtered,

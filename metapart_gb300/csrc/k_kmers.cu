@@ -65,7 +65,7 @@ constexpr int CT_THREADS = 256;
 // m-mer counts of the reads, a tile of reads per block and turn (k_readtile.cuh).  One reduction per k-mer: neighbouring
 // positions almost never share a bucket, so grouping equal buckets first costs more than it saves.  ODD: a byte other
 // than A, C, G, T, N sets DERR_NONACGT.
-template <bool ODD>
+template <bool ODD, bool HI>
 __global__ void __launch_bounds__(CT_THREADS) k_count_tiles(ReadTiles t, uint64_t n_reads, const uint64_t *chunk_rec, int nchunks,
                                                             uint32_t *cc, unsigned long long *glob, uint32_t *err)
 {
@@ -75,23 +75,23 @@ __global__ void __launch_bounds__(CT_THREADS) k_count_tiles(ReadTiles t, uint64_
     const uint64_t tiles = (n_reads + t.rpt - 1) / t.rpt;
     for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const uint64_t r0 = tile * t.rpt, r1 = min(n_reads, r0 + t.rpt);
-        if (rt_pack<ODD>(t, r0, r1, packed)) atomicOr(err, DERR_NONACGT);
+        if (rt_pack<ODD>(t, r0, (uint32_t)(r1 - r0), packed)) atomicOr(err, DERR_NONACGT);
         __syncthreads();
         for (uint32_t x = threadIdx.x; x < (uint32_t)(r1 - r0) * t.spr; x += CT_THREADS) {
             const uint32_t rr = x / t.spr, i0 = (x - rr * t.spr) * t.P, L = t.seq_len[r0 + rr];
             if (L <= (uint32_t)t.k || i0 > L - (uint32_t)t.k) continue;
             uint32_t *ccc = cc ? cc + (size_t)chunk_of(chunk_rec, nchunks, r0 + rr) * NB : nullptr;
-            KmerRoll s;
-            kr_init(s, t, packed + rr * stride, L, i0);
-            const uint32_t m = min(t.P, s.last + 1 - i0);
-            for (uint32_t j = 0; j < m; j++) {
-                uint64_t canon;
-                if (kr_get(s, t.k, canon)) {
-                    const uint32_t b = (uint32_t)(canon >> sh);
+            KmerRoll<HI> s;
+            s.template init<false>(t, packed + rr * stride, L, i0);
+#pragma unroll
+            for (int j = 0; j < RT_P; j++) {
+                if ((s.vm >> j) & 1u) {
+                    const uint64_t f = s.fwd(), r = s.rc();
+                    const uint32_t b = (uint32_t)((f < r ? f : r) >> sh);
                     if (ccc) atomicAdd(&ccc[b], 1u);
                     else atomicAdd(&glob[b], 1ull);
                 }
-                kr_next(s, t.k);
+                s.next();
             }
         }
         __syncthreads();
@@ -378,10 +378,11 @@ void launch_count(const uint8_t *fq, const ParsedReads &pr, int k, int min3, con
         (mp::count_launch(), k_count_min3<<<grid_for(pr.n_reads, 128, 32), 128, 0, st>>>(fq, pr.seq_off, pr.seq_len, 0, pr.n_reads, k,
                                                                           chunk_rec, nchunks, cc, glob, err));
     else if (pr.max_len > (uint32_t)k) {
-        const ReadTiles t = read_tiles(fq, pr, k, std::min<uint32_t>(pr.max_len, (uint32_t)MAX_READ_COUNT), CT_THREADS);
-        (mp::count_launch(), (odd ? k_count_tiles<true> : k_count_tiles<false>)<<<grid_for(pr.n_reads, (int)t.rpt, 16), CT_THREADS,
-                                                                                  t.words() * 4, st>>>(
-            t, pr.n_reads, chunk_rec, nchunks, cc, glob, err));
+        const ReadTiles t = read_tiles(fq, pr, k, std::min<uint32_t>(pr.max_len, (uint32_t)MAX_READ_COUNT), CT_THREADS, 4096);
+        auto kern = odd ? (k >= 17 ? k_count_tiles<true, true> : k_count_tiles<true, false>)
+                        : (k >= 17 ? k_count_tiles<false, true> : k_count_tiles<false, false>);
+        (mp::count_launch(), kern<<<grid_for(pr.n_reads, (int)t.rpt, 16), CT_THREADS, t.words() * 4, st>>>(t, pr.n_reads, chunk_rec,
+                                                                                                     nchunks, cc, glob, err));
     }
     if (cc && glob) (mp::count_launch(), k_sum_chunks<<<NB / 256, 256, 0, st>>>(cc, nchunks, glob));
 }

@@ -926,10 +926,10 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
             k2 = lo;
             id2 = id;
         } else {
-            if (gs.two_level) k2 = j->arena.alloc<uint64_t>(n + 1);
+            k2 = j->arena.alloc<uint64_t>(n + 1);
             id2 = j->arena.alloc<uint32_t>(n + 1);
         }
-        if (!k1 || !id1 || (gs.two_level && !k2) || !id2)
+        if (!k1 || !id1 || !k2 || !id2)
             return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)n);
         rc = min3 ? group_bins_tuples(gs, lo, hi, id, k1, id1, j->arena, j->st)
                   : group_bins_reads(gs, j->d_fq, j->pr, {0, N}, s ? j->d_parent : nullptr, k1, id1, j->arena, j->st);
@@ -940,19 +940,18 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
         if ((rc = group_units(gs, k1, id1, k2, id2, j->st))) return rc;
     }
     SortStats ss;
-    ss.passes = gs.two_level ? 2 : 1;
+    ss.passes = 2;
     ss.pass_ms = j->stage_ms[2] + j->stage_ms[3] - ms0;
-    ss.bytes = n * (uint64_t)(12 + (min3 ? (hi ? 13 : 12) : 0) + (gs.two_level ? 24 : 0));
-    uint32_t *out = gs.two_level ? id1 : id2;
+    ss.bytes = n * (uint64_t)(36 + (min3 ? (hi ? 13 : 12) : 0));
     {
         StageTimer tm(j->st, j->stage_ms, 4);
-        if ((rc = group_filter(gs, gs.two_level ? k2 : k1, gs.two_level ? id2 : id1, out, j->d_parent, j->d_filtered, j->arena, j->st)))
+        if ((rc = group_filter(gs, k2, id2, id1, j->d_parent, j->d_filtered, j->arena, j->st)))
             return rc;
     }
     {
         StageTimer tm(j->st, j->stage_ms, 5);
         std::vector<GroupQuirk> open;
-        if ((rc = group_union(gs, out, j->d_parent, j->d_filtered, N, j->arena, j->st, open))) return rc;
+        if ((rc = group_union(gs, id1, j->d_parent, j->d_filtered, N, j->arena, j->st, open))) return rc;
         for (const GroupQuirk &q : open) {
             uint32_t first = 0;
             if ((rc = scan_first_read(j, gs.k, min3, gs.lo, gs.hi, hist, s > 0, err, &first))) return rc;

@@ -418,10 +418,9 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
             StageTimer tm(st, b->stage_ms, 3);
             if ((rc = group_units(gs, sb.lo[1], sb.id[1], sb.lo[0], sb.id[0], st))) return rc;
         }
-        lo_buf = gs.two_level ? 0 : 1;
         b->sort_pass_ms += b->stage_ms[2] + b->stage_ms[3] - ms0;
-        b->sort_bytes += T_all * (uint64_t)(12 + (gs.two_level ? 24 : 0));
-        b->sort_passes += gs.two_level ? 2 : 1;
+        b->sort_bytes += T_all * 36;
+        b->sort_passes += 2;
         b->sort_tuples += T_all;
     } else {
         // ---- enumeration: every k-mer of every read (one scan per sample), read order

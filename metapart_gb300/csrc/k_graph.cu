@@ -932,8 +932,8 @@ int mate_union(uint32_t *parent, uint64_t n_reads, uint32_t *size, DeviceArena &
                                                                 round, limit));
             (mp::count_launch(), k_pe_bigsmall<<<g, 256, 0, st>>>(parent, size, big, cnts + 4 * r + 2, pra, prb, gmax, gadd));
         }
-        unsigned int h[4 * RB + 4];
-        MP_CUDA(cudaMemcpyAsync(h, cnts, sizeof h, cudaMemcpyDeviceToHost, st));
+        ReadBack<unsigned int> h(arena, 4 * RB + 4);
+        MP_CUDA(cudaMemcpyAsync(h.p, cnts, (4 * RB + 4) * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
         MP_CUDA(cudaStreamSynchronize(st));
         nact = h[4 * (RB - 1) + 1];
         // rounds that reserved nothing leave nothing active: stop counting at the first empty one
@@ -987,9 +987,11 @@ int plan_partitions(const uint32_t *parent, const uint32_t *size, uint64_t n_rea
     (mp::count_launch(), k_root_weight<<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, size, n_reads, w));
     scan_u32_to_u64(w, pre, n_reads + 1, nullptr, tmp, tb, st);
     (mp::count_launch(), k_bounds<<<1, 32, 0, st>>>(pre, n_reads, b));
-    MP_CUDA(cudaMemcpyAsync(bounds_host, b, 17 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    ReadBack<uint64_t> rb(arena, 17);
+    MP_CUDA(cudaMemcpyAsync(rb.p, b, 17 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
     MP_CUDA(cudaGetLastError());
+    std::copy(rb.p, rb.p + 17, bounds_host);
     return 0;
 }
 

@@ -29,6 +29,7 @@ constexpr uint32_t GP_DIGITS = 1024;     // digits of a split pass: bins of a se
 constexpr uint64_t GP_SMALL = 1500000;   // tuples of a segment that fit GP_DIGITS units however they are spread
 constexpr int GP_COUNT_ITEMS = 8, GP_COUNT_THREADS = 256, GP_COUNT_BLOCK = GP_COUNT_ITEMS * GP_COUNT_THREADS;
 constexpr uint32_t GP_NONE = 0x7FFFFFFFu;  // a grouped id that stands for no read
+constexpr size_t PLAN_MAIL = DeviceArena::MAIL - 4096;  // where the plan's counters arrive in the mailbox
 constexpr int QW = 8;  // words per segment: tuples found before the last run, last run's, its read, the run's place
 
 struct PlanCtx {
@@ -1071,8 +1072,24 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
     (count_launch(), k_gp_write<<<nblk, GP_COUNT_THREADS, 0, st>>>(c, blk, g.ctr, g.ustart, g.ub0, g.ucur, g.bstart, g.bu0, g.bcur,
                                                                   g.bin_sh, g.bfirst, g.unit_of, g.mid, g.big));
     (count_launch(), k_gp_tiles<<<1, 1024, 0, st>>>(g.bstart, g.bins, g.ctr, g.tiles));
-    MP_CUDA(cudaMemcpyAsync(g.hctr, g.ctr, GC_N * 4, cudaMemcpyDeviceToHost, st));
+    ReadBack<uint32_t> rb(arena, GC_N, PLAN_MAIL);
+    if (!arena.mail) {
+        g.h_ctr.assign(GC_N, 0);
+        rb.p = g.h_ctr.data();
+    }
+    if (!g.planned) MP_CUDA(cudaEventCreateWithFlags(&g.planned, cudaEventDisableTiming));
+    MP_CUDA(cudaMemcpyAsync(rb.p, g.ctr, GC_N * 4, cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaEventRecord(g.planned, st));
     MP_CUDA(cudaGetLastError());
+    return 0;
+}
+
+// The plan's counters, once they have arrived (the split passes run meanwhile).
+static int group_counts(GroupScan &g, DeviceArena &arena)
+{
+    MP_CUDA(cudaEventSynchronize(g.planned));
+    const uint32_t *p = arena.mail ? reinterpret_cast<const uint32_t *>(arena.mail + PLAN_MAIL) : g.h_ctr.data();
+    std::copy(p, p + GC_N, g.hctr);
     return 0;
 }
 
@@ -1155,6 +1172,7 @@ int group_filter(GroupScan &g, const uint64_t *kk, const uint32_t *ids, uint32_t
                  DeviceArena &arena, cudaStream_t st)
 {
     group_kernel_attrs();
+    if (const int rc = group_counts(g, arena)) return rc;
     const uint32_t *fill = g.ucur;
     GroupCtx c{kk, ids, g.ustart, g.ub0, fill, g.lrs, nullptr, g.ctr, g.qlist, g.quirk, GC_WORK_S, GC_UNITS, 0, (uint32_t)GP_CAP_S,
                out, parent, filtered};
@@ -1239,19 +1257,20 @@ int group_union(GroupScan &g, const uint32_t *out, uint32_t *parent, const uint8
     MP_CUDA(cudaMemsetAsync(err, 0, 4, st));
     (count_launch(), k_gp_union<<<blocks, 256, 0, st>>>(g.ctr, out, parent, filtered, err, arena.lim.union_retries));
     compress_parents(parent, n_reads, st);
-    std::vector<uint32_t> h(GC_N + (size_t)nseg * QW);
-    uint32_t herr = 0;
-    MP_CUDA(cudaMemcpyAsync(h.data(), g.ctr, h.size() * 4, cudaMemcpyDeviceToHost, st));
-    MP_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
+    const size_t words = GC_N + (size_t)nseg * QW;
+    ReadBack<uint32_t> h(arena, words + 1);
+    MP_CUDA(cudaMemcpyAsync(h.p, g.ctr, words * 4, cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaMemcpyAsync(h.p + words, err, 4, cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
     MP_CUDA(cudaGetLastError());
+    const uint32_t herr = h[words];
     if (h[GC_ERR] & 4u)
         return set_error(MP_EUNSUP, "a read has 256 or more k-mers in one scan (the reference counts them in 8 bits, "
                                     "enumerateKmers.c:152)");
     if (h[GC_ERR] & 2u) return set_error(MP_EFMT, "the histogram does not match the scan's tuples");
     if (herr) return set_error(MP_EDEVICE, "union-find retry limit reached (flags 0x%x)", herr);
     for (int q = 0; q < nseg; q++) {
-        const uint32_t *w = h.data() + GC_N + (size_t)q * QW;
+        const uint32_t *w = h.p + GC_N + (size_t)q * QW;
         if (!w[0] && w[1]) open.push_back(GroupQuirk{q, w[2]});
     }
     return 0;

@@ -39,7 +39,13 @@ struct GroupScan {
     uint32_t *ctr = nullptr;                  // GC_* counters
     uint32_t *qlist = nullptr;                // grouped stretches of the segments' last ranges
     uint32_t *quirk = nullptr;                // per segment: QW words (see k_gp_quirk)
-    uint32_t hctr[16] = {};                   // the counters on the host
+    uint32_t hctr[16] = {};                   // the plan's counters on the host, from group_counts on
+    std::vector<uint32_t> h_ctr;              // (where they arrive without a mailbox)
+    cudaEvent_t planned = nullptr;            // after the counters' copy
+    GroupScan() = default;
+    GroupScan(const GroupScan &) = delete;
+    GroupScan &operator=(const GroupScan &) = delete;
+    ~GroupScan() { if (planned) cudaEventDestroy(planned); }
     std::vector<uint32_t> h_plan, h_tiles;     // sources of uploads still queued
 };
 
@@ -56,7 +62,7 @@ struct GroupQuirk {
 };
 
 bool group_fits(uint64_t n, uint64_t n_reads, const SortSegments *segs);
-// Plans g (its inputs set) on the device, its counts copied into g.hctr in stream order.
+// Plans g (its inputs set) on the device; its counts are on their way to the host (group_filter takes them).
 int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st);
 // First split pass, into bins, of n tuples to (k1, id1): enumerated from the reads (seg_reads: nseg + 1 read offsets; label: the reads' components, null in the first scan; every read at
 // most 300 positions), or of tuples enumerated before, segment-major.

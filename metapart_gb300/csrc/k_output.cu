@@ -6,6 +6,8 @@
 // mate 1's root and, when mate 2's root differs, again to mate 2's (:1006-1047).  On the
 // GPU each (file, unit) entry is generated in input order, entries are stably sorted by
 // file, their byte offsets come from one exclusive scan, and a warp copies each record.
+#include <algorithm>
+
 #include "k_output.cuh"
 #include "k_sort.cuh"
 
@@ -174,9 +176,10 @@ int plan_output(const uint8_t *d_fq, const ParsedReads &pr, const uint32_t *d_la
     const unsigned gb = (unsigned)((units + 255) / 256);
     (mp::count_launch(), k_out_dest<<<gb, 256, 0, st>>>(c, nent, f1, f2));
     scan_u32_to_u64(nent, eoff, units, ntot, tmp, tb, st);
-    uint64_t n = 0;
-    MP_CUDA(cudaMemcpyAsync(&n, ntot, sizeof n, cudaMemcpyDeviceToHost, st));
+    ReadBack<uint64_t> rb(arena, nf + 1);
+    MP_CUDA(cudaMemcpyAsync(rb.p, ntot, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
+    const uint64_t n = rb[0];
     SortBufs sb;
     for (int i = 0; i < 2; i++) {
         sb.lo[i] = arena.alloc<uint64_t>(n + 1);
@@ -196,11 +199,12 @@ int plan_output(const uint8_t *d_fq, const ParsedReads &pr, const uint32_t *d_la
     (mp::count_launch(), k_out_len<<<ge, 256, 0, st>>>(c, sb.id[sb.cur], n, len, sb.lo[sb.cur], fbytes));
     scan_u64(len, plan->off, n, ntot, tmp2, tb2, st);
     MP_CUDA(cudaMemcpyAsync(plan->val, sb.id[sb.cur], n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
-    uint64_t total = 0;
-    MP_CUDA(cudaMemcpyAsync(&total, ntot, sizeof total, cudaMemcpyDeviceToHost, st));
-    MP_CUDA(cudaMemcpyAsync(file_sizes.data(), fbytes, nf * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaMemcpyAsync(rb.p, ntot, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaMemcpyAsync(rb.p + 1, fbytes, nf * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
     MP_CUDA(cudaGetLastError());
+    const uint64_t total = rb[0];
+    std::copy(rb.p + 1, rb.p + 1 + nf, file_sizes.begin());
     plan->n = n;
     plan->total = total;
     plan->rec_start = pr.rec_start;
@@ -322,9 +326,10 @@ int plan_output_batch(const ParsedReads &pr, const uint32_t *d_label, int interl
     const unsigned gb = (unsigned)((units + 255) / 256);
     if (units) (mp::count_launch(), k_outb_dest<<<gb, 256, 0, st>>>(bc, nent, f1, f2));
     scan_u32_to_u64(nent, eoff, units, ntot, tmp, tb, st);
-    uint64_t n = 0;
-    MP_CUDA(cudaMemcpyAsync(&n, ntot, sizeof n, cudaMemcpyDeviceToHost, st));
+    ReadBack<uint64_t> rb(arena, nf + 1);
+    MP_CUDA(cudaMemcpyAsync(rb.p, ntot, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
+    const uint64_t n = rb[0];
     SortBufs sb;
     for (int i = 0; i < 2; i++) {
         sb.lo[i] = arena.alloc<uint64_t>(n + 1);
@@ -344,11 +349,12 @@ int plan_output_batch(const ParsedReads &pr, const uint32_t *d_label, int interl
     if (n) (mp::count_launch(), k_out_len<<<ge, 256, 0, st>>>(c, sb.id[sb.cur], n, len, sb.lo[sb.cur], fbytes));
     scan_u64(len, plan->off, n, ntot, tmp2, tb2, st);
     if (n) MP_CUDA(cudaMemcpyAsync(plan->val, sb.id[sb.cur], n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
-    uint64_t total = 0;
-    MP_CUDA(cudaMemcpyAsync(&total, ntot, sizeof total, cudaMemcpyDeviceToHost, st));
-    MP_CUDA(cudaMemcpyAsync(file_sizes.data(), fbytes, nf * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaMemcpyAsync(rb.p, ntot, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaMemcpyAsync(rb.p + 1, fbytes, nf * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
     MP_CUDA(cudaGetLastError());
+    const uint64_t total = rb[0];
+    std::copy(rb.p + 1, rb.p + 1 + nf, file_sizes.begin());
     plan->n = n;
     plan->total = total;
     plan->rec_start = pr.rec_start;

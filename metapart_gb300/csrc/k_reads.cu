@@ -4,6 +4,7 @@
 // quality as long as the sequence -- the walk getNextRead does (genHistograms.c:60-80,
 // metapart.c:296-369).  The parser finds every newline with coalesced 16-byte loads,
 // compacts their positions in order, and derives the record table from every fourth one.
+#include <algorithm>
 #include <cstdio>
 
 #include "k_reads.cuh"
@@ -263,9 +264,10 @@ int parse_fastq_range(const uint8_t *d_base, uint64_t begin, uint64_t end, Parse
     if (!seg_counts || !seg_off || !total || !tmp) return set_error(MP_ENOMEM, "device memory for the FASTQ parse");
     (mp::count_launch(), k_nl_count<<<(unsigned)segs, NL_THREADS, 0, st>>>(d_buf, na, skip, seg_counts));
     scan_u32_to_u64(seg_counts, seg_off, segs, total, tmp, tb, st);
-    uint64_t n_nl = 0;
-    MP_CUDA(cudaMemcpyAsync(&n_nl, total, sizeof n_nl, cudaMemcpyDeviceToHost, st));
+    ReadBack<uint64_t> rb(arena, 4);
+    MP_CUDA(cudaMemcpyAsync(&rb[0], total, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
+    const uint64_t n_nl = rb[0];
     if (n_nl == 0 || n_nl % 4) return set_error(MP_EFMT, "FASTQ line count %llu is not a multiple of 4", (unsigned long long)n_nl);
     uint64_t *nl = arena.alloc<uint64_t>(n_nl);
     if (!nl) return set_error(MP_ENOMEM, "device memory for newline positions");
@@ -280,13 +282,13 @@ int parse_fastq_range(const uint8_t *d_base, uint64_t begin, uint64_t end, Parse
     MP_CUDA(cudaMemsetAsync(bad, 0xFF, sizeof *bad, st));
     MP_CUDA(cudaMemsetAsync(bad + 1, 0, sizeof *bad, st));
     (mp::count_launch(), k_records<<<(unsigned)((n_rec + 255) / 256), 256, 0, st>>>(nl, n_rec, pr->rec_start, pr->seq_off, pr->seq_len, bad));
-    unsigned long long hb[2] = {0, 0};
-    uint64_t last_end = 0;
-    MP_CUDA(cudaMemcpyAsync(hb, bad, sizeof hb, cudaMemcpyDeviceToHost, st));
-    MP_CUDA(cudaMemcpyAsync(&last_end, pr->rec_start + n_rec, sizeof last_end, cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaMemcpyAsync(&rb[1], bad, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaMemcpyAsync(&rb[3], pr->rec_start + n_rec, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
+    const uint64_t hb[2] = {rb[1], rb[2]}, last_end = rb[3];
     MP_CUDA(cudaGetLastError());
-    if (hb[0] != ~0ull) return set_error(MP_EFMT, "FASTQ record %llu: quality length differs from the sequence length", hb[0]);
+    if (hb[0] != ~0ull) return set_error(MP_EFMT, "FASTQ record %llu: quality length differs from the sequence length",
+                                          (unsigned long long)hb[0]);
     pr->max_len = (uint32_t)hb[1];
     if (last_end != n) return set_error(MP_EFMT, "FASTQ input does not end with a complete record");
     arena.release_scratch();
@@ -321,8 +323,10 @@ int records_at_offsets(const ParsedReads *pr, const uint64_t *h_offsets, int nq,
     if (!dq || !dr) return set_error(MP_ENOMEM, "device memory");
     MP_CUDA(cudaMemcpyAsync(dq, h_offsets, nq * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     (mp::count_launch(), k_record_of_offset<<<(nq + 127) / 128, 128, 0, st>>>(pr->rec_start, pr->n_reads, dq, nq, dr));
-    MP_CUDA(cudaMemcpyAsync(h_rec, dr, nq * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    ReadBack<uint64_t> rb(arena, nq);
+    MP_CUDA(cudaMemcpyAsync(rb.p, dr, nq * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
+    std::copy(rb.p, rb.p + nq, h_rec);
     arena.release_scratch();
     for (int i = 0; i < nq; i++)
         if (h_rec[i] == ~0ull)

@@ -10,18 +10,28 @@ namespace mp {
 // Stream-ordered device allocations of one job.  Scratch allocations live until
 // release_scratch(); persistent ones until release_all().  Sizes are charged
 // against the context's HBM budget, which jobs running on other host threads share.
+//
+// Allocations of up to SLAB_PIECE bytes are cut from two slabs of SLAB bytes (one each for scratch and persistent ones,
+// reused in stream order, given back by release_all): a small job makes 140 allocations of which all but a few are
+// small, at 1-2 us each to take and to free.
 struct DeviceArena {
+    static constexpr size_t SLAB = 1u << 20, SLAB_PIECE = 64u << 10;
+    struct Slab {
+        char *p = nullptr;
+        size_t at = 0;
+    };
     cudaStream_t st = nullptr;
     std::vector<std::pair<void *, size_t>> persistent, scratch;
+    Slab slab[2];  // scratch, persistent
     std::atomic<uint64_t> *budget_used = nullptr;  // shared with the context
     uint64_t budget_limit = ~0ull;
     uint64_t peak = 0, live = 0;
     WaitLimits lim;  // the bounded waits of the kernels this arena's work launches
+    unsigned char *mail = nullptr;  // MAIL pinned bytes of the arena's owner, for read-backs (nullable)
+    static constexpr size_t MAIL = 64u << 10;
 
-    void *raw(size_t bytes, bool keep)
+    void *exact(size_t bytes, std::vector<std::pair<void *, size_t>> &v)
     {
-        bytes = (bytes + 255) & ~(size_t)255;
-        if (bytes == 0) bytes = 256;
         if (budget_used) {  // reserve first, so concurrent jobs never overshoot the budget together
             uint64_t cur = budget_used->load();
             do {
@@ -34,15 +44,34 @@ struct DeviceArena {
             if (budget_used) budget_used->fetch_sub(bytes);
             return nullptr;
         }
-        (keep ? persistent : scratch).push_back({p, bytes});
+        v.push_back({p, bytes});
         live += bytes;
         if (live > peak) peak = live;
         return p;
+    }
+    void *raw(size_t bytes, bool keep)
+    {
+        bytes = (bytes + 255) & ~(size_t)255;
+        if (bytes == 0) bytes = 256;
+        if (bytes <= SLAB_PIECE) {
+            Slab &s = slab[keep];
+            if (!s.p) {
+                s.p = (char *)exact(SLAB, persistent);  // (both slabs stay until release_all)
+                s.at = 0;
+            }
+            if (s.p && s.at + bytes <= SLAB) {
+                void *p = s.p + s.at;
+                s.at += bytes;
+                return p;
+            }
+        }
+        return exact(bytes, keep ? persistent : scratch);
     }
     template <typename T> T *alloc(size_t n) { return (T *)raw(n * sizeof(T), false); }
     template <typename T> T *alloc_persistent(size_t n) { return (T *)raw(n * sizeof(T), true); }
     void free_one(std::vector<std::pair<void *, size_t>> &v, void *p)
     {
+        if (p == slab[0].p || p == slab[1].p) return;  // a slab's first piece
         for (size_t i = 0; i < v.size(); i++)
             if (v[i].first == p) {
                 cudaFreeAsync(p, st);
@@ -54,25 +83,46 @@ struct DeviceArena {
     }
     void free_persistent(void *p) { if (p) free_one(persistent, p); }
     void free_scratch(void *p) { if (p) free_one(scratch, p); }
-    void release_scratch()
+    void drop(std::vector<std::pair<void *, size_t>> &v)
     {
-        for (auto &x : scratch) {
+        for (auto &x : v) {
             cudaFreeAsync(x.first, st);
             if (budget_used) budget_used->fetch_sub(x.second);
             live -= x.second;
         }
-        scratch.clear();
+        v.clear();
+    }
+    void release_scratch()
+    {
+        drop(scratch);
+        slab[0].at = 0;
     }
     void release_all()
     {
-        release_scratch();
-        for (auto &x : persistent) {
-            cudaFreeAsync(x.first, st);
-            if (budget_used) budget_used->fetch_sub(x.second);
-            live -= x.second;
-        }
-        persistent.clear();
+        drop(scratch);
+        drop(persistent);
+        slab[0] = slab[1] = Slab{};
     }
+};
+
+// n values read back from the device: in the arena owner's pinned mailbox (from byte `at` on) where there is one with room
+// for them, so that the copy waits for nothing but its stream, else in memory of their own.  Valid after the stream is
+// waited for, until the next read-back at the same place.
+template <typename T> struct ReadBack {
+    std::vector<T> own;
+    T *p;
+    ReadBack(DeviceArena &a, size_t n, size_t at = 0)
+    {
+        if (a.mail && at + n * sizeof(T) <= DeviceArena::MAIL) {
+            p = reinterpret_cast<T *>(a.mail + at);
+        } else {
+            own.resize(n);
+            p = own.data();
+        }
+    }
+    T &operator[](size_t i) { return p[i]; }
+    ReadBack(const ReadBack &) = delete;
+    ReadBack &operator=(const ReadBack &) = delete;
 };
 
 // CUDA events owned by a scope: destroyed on every return path.

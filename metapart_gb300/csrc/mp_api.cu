@@ -113,7 +113,8 @@ struct mp_job {
     bool output_ready = false;  // out_plan holds the partition files' layout
     OutputPlan out_plan;
     std::string dump_dir;
-    double stage_ms[8] = {0};
+    StageClock clk;
+    std::vector<uint64_t> cr_starts, cr_rec;  // the last chunk starts whose records were looked up in the job's reads
     SortStats sort_stats;
     int sort_passes_total = 0;
     double sort_ms_total = 0;
@@ -267,6 +268,15 @@ int range_bounds(const uint64_t *hist, const uint64_t *ltr, int T, uint64_t scan
     return 0;
 }
 
+// Makes the pages of a caller's array present before the GPU copies into it: a page first touched by the copy costs about
+// 20 us, by the host 1.
+void touch_pages(void *p, size_t bytes)
+{
+    volatile char *c = static_cast<volatile char *>(p);
+    for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
+    if (bytes) c[bytes - 1] = 0;
+}
+
 int chunk_records(mp_job *j, const uint64_t *chunk_starts, int nchunks, std::vector<uint64_t> &rec)
 {
     rec.assign(nchunks + 1, 0);
@@ -274,7 +284,16 @@ int chunk_records(mp_job *j, const uint64_t *chunk_starts, int nchunks, std::vec
         if (chunk_starts[c + 1] < chunk_starts[c]) return set_error(MP_EFMT, "chunk offsets are not ascending");
     if (chunk_starts[0] != 0 || chunk_starts[nchunks] != j->fq_bytes)
         return set_error(MP_EFMT, "chunks do not cover the input");
-    return records_at_offsets(&j->pr, chunk_starts, nchunks + 1, rec.data(), j->arena, j->st);
+    if ((int)j->cr_starts.size() == nchunks + 1 && std::equal(chunk_starts, chunk_starts + nchunks + 1, j->cr_starts.begin())) {
+        rec = j->cr_rec;  // looked up in these reads before (cleared with them)
+        return 0;
+    }
+    const int rc = records_at_offsets(&j->pr, chunk_starts, nchunks + 1, rec.data(), j->arena, j->st);
+    if (!rc) {
+        j->cr_starts.assign(chunk_starts, chunk_starts + nchunks + 1);
+        j->cr_rec = rec;
+    }
+    return rc;
 }
 
 }  // namespace
@@ -323,6 +342,10 @@ int mp_job_create(mp_ctx *ctx, mp_job **out)
         return set_error(MP_ECUDA, "cannot create a stream");
     }
     j->arena.st = j->st;
+    if (cudaHostAlloc((void **)&j->arena.mail, DeviceArena::MAIL, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        j->arena.mail = nullptr;
+    }
     j->arena.budget_used = &ctx->used;
     j->arena.budget_limit = ctx->budget;
     const char *ck = getenv("MP_CHECK");
@@ -339,6 +362,7 @@ void mp_job_destroy(mp_job *job)
     cudaStreamSynchronize(job->st);
     cudaStreamDestroy(job->st);
     if (job->copy_st) cudaStreamDestroy(job->copy_st);
+    if (job->arena.mail) cudaFreeHost(job->arena.mail);
     delete job;
 }
 
@@ -349,9 +373,10 @@ static int load_common(mp_job *j, uint64_t nbytes, const uint64_t *file_sizes, i
     if (tot != nbytes) return set_error(MP_EARG, "file sizes do not add up to the input size");
     j->fq_bytes = nbytes;
     j->interleaved = interleaved;
-    j->stage_ms[0] = 0;
+    j->cr_starts.clear();
+    j->clk.clear(0);
     {
-        StageTimer tm(j->st, j->stage_ms, 0);
+        StageTimer tm(j->clk, j->st, 0);
         int rc = parse_fastq(j->d_fq, nbytes, &j->pr, j->arena, j->st);
         if (rc) return rc;
     }
@@ -418,6 +443,7 @@ int mp_job_reset(mp_job *j)
     j->d_fq = nullptr;
     j->fq_bytes = 0;
     j->pr = ParsedReads{};
+    j->cr_starts.clear();
     j->d_parent = j->d_size = nullptr;
     j->d_filtered = nullptr;
     j->d_out = nullptr;
@@ -444,36 +470,40 @@ int mp_job_count(mp_job *j, int k, int min3, const uint64_t *chunk_starts, int n
         j->kc_pieces = 0;
         return set_error(MP_EUNSUP, "a read is longer than %d bases", MAX_READ_COUNT);
     }
-    j->stage_ms[1] = 0;
+    j->clk.clear(1);
     uint64_t *d_rec = j->arena.alloc<uint64_t>(nchunks + 1);
-    unsigned long long *glob = j->arena.alloc<unsigned long long>(NB);
+    unsigned long long *glob = j->arena.alloc<unsigned long long>(NB + 1);
+    uint64_t *prefix = j->arena.alloc<uint64_t>(NB + 1);
+    const size_t tb = scan_tmp_bytes(NB + 1);
+    void *tmp = j->arena.alloc<uint8_t>(tb);
     uint32_t *cc = chunk_counts_out ? j->arena.alloc<uint32_t>((size_t)nchunks * NB) : nullptr;
     uint32_t *err = j->arena.alloc<uint32_t>(1);
-    if (!d_rec || !glob || !err || (chunk_counts_out && !cc)) return set_error(MP_ENOMEM, "device memory for counting");
+    if (!d_rec || !glob || !prefix || !tmp || !err || (chunk_counts_out && !cc)) return set_error(MP_ENOMEM, "device memory for counting");
     MP_CUDA(cudaMemcpyAsync(d_rec, rec.data(), (nchunks + 1) * 8, cudaMemcpyHostToDevice, j->st));
-    MP_CUDA(cudaMemsetAsync(glob, 0, NB * 8, j->st));
+    MP_CUDA(cudaMemsetAsync(glob, 0, (NB + 1) * 8, j->st));
     MP_CUDA(cudaMemsetAsync(err, 0, 4, j->st));
     if (cc) MP_CUDA(cudaMemsetAsync(cc, 0, (size_t)nchunks * NB * 4, j->st));
     {
-        StageTimer tm(j->st, j->stage_ms, 1);
+        StageTimer tm(j->clk, j->st, 1);
         launch_count(j->d_fq, j->pr, k, min3, d_rec, nchunks, cc, glob, err, j->st, j->store == STORE_PACKED);
         j->kc_pieces = j->store != STORE_FASTQ && !min3 ? 1 : 0;
     }
-    std::vector<unsigned long long> g(NB);
-    uint32_t herr = 0;
-    MP_CUDA(cudaMemcpyAsync(g.data(), glob, NB * 8, cudaMemcpyDeviceToHost, j->st));
-    MP_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, j->st));
+    // the prefix straight into the caller's array (on the host, two 8 MB arrays were first touched and walked: 1 ms)
+    scan_u64((const uint64_t *)glob, prefix, NB + 1, nullptr, tmp, tb, j->st);
+    ReadBack<uint32_t> rb(j->arena, 1);
+    MP_CUDA(cudaMemcpyAsync(rb.p, err, 4, cudaMemcpyDeviceToHost, j->st));
+    touch_pages(hist_out, (NB + 1) * 8);
+    MP_CUDA(cudaMemcpyAsync(hist_out, prefix, (NB + 1) * 8, cudaMemcpyDeviceToHost, j->st));
     if (cc) MP_CUDA(cudaMemcpyAsync(chunk_counts_out, cc, (size_t)nchunks * NB * 4, cudaMemcpyDeviceToHost, j->st));
     MP_CUDA(cudaStreamSynchronize(j->st));
     MP_CUDA(cudaGetLastError());
+    const uint32_t herr = rb[0];
     j->arena.release_scratch();
     if (herr & DERR_LONG_READ) {
         j->kc_pieces = 0;
         return set_error(MP_EUNSUP, "a read is longer than %d bases", MAX_READ_COUNT);
     }
     if (herr & DERR_NONACGT) j->kc_pieces = 0;  // a byte that packed reads cannot hold
-    hist_out[0] = 0;
-    for (uint32_t b = 1; b <= NB; b++) hist_out[b] = hist_out[b - 1] + g[b - 1];
     if (chunk_reads_out)
         for (int c = 0; c < nchunks; c++) chunk_reads_out[c] = rec[c + 1] - rec[c];
     return 0;
@@ -481,7 +511,10 @@ int mp_job_count(mp_job *j, int k, int min3, const uint64_t *chunk_starts, int n
 
 namespace {
 
-constexpr int LC_SEGMENTS = 8;  // upload segments of mp_job_load_count
+// Upload segments of mp_job_load_count: a segment costs two waits and a dozen launches (about 100 us), the link moves 20 MB
+// in that time.  Inputs under 1 MB go up at once.
+constexpr int LC_SEGMENTS = 8;
+constexpr uint64_t LC_SEGMENT_BYTES = 24ull << 20, LC_LEAST_BYTES = 1000000;
 
 // The pipelined body of mp_job_load_count: segment i's bytes go up on the copy stream while the job
 // stream parses and counts segment i - 1.  Each segment holds whole chunks, so it starts on a record
@@ -525,11 +558,13 @@ int load_count_pipelined(mp_job *j, const char *bytes, uint64_t nbytes, const ui
     if (tot != nbytes) return MP_EARG;
     j->fq_bytes = nbytes;
     j->interleaved = interleaved;
-    j->stage_ms[0] = j->stage_ms[1] = 0;
-    unsigned long long *glob = j->arena.alloc_persistent<unsigned long long>(NB);
+    j->cr_starts.clear();
+    j->clk.clear(0);
+    j->clk.clear(1);
+    unsigned long long *glob = j->arena.alloc_persistent<unsigned long long>(NB + 1);
     uint32_t *err = j->arena.alloc_persistent<uint32_t>(1);
     if (!glob || !err) return MP_ENOMEM;
-    MP_CUDA(cudaMemsetAsync(glob, 0, NB * 8, j->st));
+    MP_CUDA(cudaMemsetAsync(glob, 0, (NB + 1) * 8, j->st));
     MP_CUDA(cudaMemsetAsync(err, 0, 4, j->st));
     j->kc_pieces = 0;
     std::vector<ParsedReads> prs(S);
@@ -537,20 +572,20 @@ int load_count_pipelined(mp_job *j, const char *bytes, uint64_t nbytes, const ui
     for (int i = 0; i < S; i++) {
         MP_CUDA(cudaStreamWaitEvent(j->st, ev[i], 0));
         {
-            StageTimer tm(j->st, j->stage_ms, 0);
+            StageTimer tm(j->clk, j->st, 0);
             if (parse_fastq_range(j->d_fq, seg[i], seg[i + 1], &prs[i], j->arena, j->st)) return MP_EFMT;
         }
         R[i + 1] = R[i] + prs[i].n_reads;
         j->pr.max_len = std::max(j->pr.max_len, prs[i].max_len);
         if (prs[i].max_len > (uint32_t)MAX_READ_COUNT) return MP_EUNSUP;
-        StageTimer tm(j->st, j->stage_ms, 1);
+        StageTimer tm(j->clk, j->st, 1);
         launch_count(j->d_fq + seg[i], prs[i], k, 0, nullptr, 0, nullptr, glob, err, j->st, j->store == STORE_PACKED);
     }
     j->kc_pieces = S;
     const uint64_t N = R[S];
     if (N >= UMAX32 || (interleaved && (N & 1))) return MP_EFMT;
     {
-        StageTimer tm(j->st, j->stage_ms, 0);
+        StageTimer tm(j->clk, j->st, 0);
         j->pr.n_reads = N;
         j->pr.rec_start = j->arena.alloc_persistent<uint64_t>(N + 1);
         j->pr.seq_off = j->arena.alloc_persistent<uint64_t>(N + 1);
@@ -573,19 +608,23 @@ int load_count_pipelined(mp_job *j, const char *bytes, uint64_t nbytes, const ui
     }
     std::vector<uint64_t> rec;
     if (chunk_records(j, chunk_starts, nchunks, rec)) return MP_EFMT;
-    std::vector<unsigned long long> g(NB);
-    uint32_t herr = 0;
-    MP_CUDA(cudaMemcpyAsync(g.data(), glob, NB * 8, cudaMemcpyDeviceToHost, j->st));
-    MP_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, j->st));
+    uint64_t *prefix = j->arena.alloc<uint64_t>(NB + 1);
+    const size_t tb = scan_tmp_bytes(NB + 1);
+    void *tmp = j->arena.alloc<uint8_t>(tb);
+    if (!prefix || !tmp) return MP_ENOMEM;
+    scan_u64((const uint64_t *)glob, prefix, NB + 1, nullptr, tmp, tb, j->st);
+    ReadBack<uint32_t> rb(j->arena, 1);
+    MP_CUDA(cudaMemcpyAsync(rb.p, err, 4, cudaMemcpyDeviceToHost, j->st));
+    touch_pages(hist_out, (NB + 1) * 8);
+    MP_CUDA(cudaMemcpyAsync(hist_out, prefix, (NB + 1) * 8, cudaMemcpyDeviceToHost, j->st));
     MP_CUDA(cudaStreamSynchronize(j->st));
     MP_CUDA(cudaGetLastError());
+    const uint32_t herr = rb[0];
     j->arena.free_persistent(glob);
     j->arena.free_persistent(err);
     j->arena.release_scratch();
     if (herr & DERR_NONACGT) j->kc_pieces = 0;  // a byte that packed reads cannot hold
     if (herr & ~DERR_NONACGT) return MP_EUNSUP;
-    hist_out[0] = 0;
-    for (uint32_t b = 1; b <= NB; b++) hist_out[b] = hist_out[b - 1] + g[b - 1];
     if (chunk_reads_out)
         for (int c = 0; c < nchunks; c++) chunk_reads_out[c] = rec[c + 1] - rec[c];
     return 0;
@@ -613,10 +652,11 @@ int mp_job_load_count(mp_job *j, const char *bytes, uint64_t nbytes, const uint6
     bool ok = pinned && !min3 && j->store != STORE_FASTQ && nchunks >= 2 && chunk_starts[0] == 0 &&
               chunk_starts[nchunks] == nbytes;
     for (int c = 0; ok && c < nchunks; c++) ok = chunk_starts[c] <= chunk_starts[c + 1];
-    if (!ok) return one_by_one();
+    if (!ok || nbytes < LC_LEAST_BYTES) return one_by_one();
+    const uint64_t parts = std::min<uint64_t>(LC_SEGMENTS, std::max<uint64_t>(2, nbytes / LC_SEGMENT_BYTES));
     std::vector<uint64_t> seg = {0};
-    for (int c = 1; c < nchunks; c++)
-        if (chunk_starts[c] > seg.back() && chunk_starts[c] >= (uint64_t)((double)nbytes * seg.size() / LC_SEGMENTS))
+    for (int c = 1; c < nchunks && seg.size() < parts; c++)
+        if (chunk_starts[c] > seg.back() && chunk_starts[c] >= (uint64_t)((double)nbytes * seg.size() / (double)parts))
             seg.push_back(chunk_starts[c]);
     seg.push_back(nbytes);
     if (seg.size() < 3) return one_by_one();
@@ -745,7 +785,7 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
         SortBufs sb = sb0;
         uint64_t n = 0;
         {
-            StageTimer tm(j->st, j->stage_ms, 2);
+            StageTimer tm(j->clk, j->st, 2);
             launch_enum_count(j->d_fq, j->pr, k, 0, (uint32_t)b0, (uint32_t)b1, cnt, err, j->st);
             MP_CUDA(cudaMemsetAsync(cnt + N, 0, 4, j->st));
             scan_u32_to_u64(cnt, off, N + 1, ntot, tmp, tb, j->st);
@@ -763,7 +803,7 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
         if (herr) return set_error(MP_EDEVICE, "enumeration flags 0x%x", herr);
         int lo_buf = 0, hi_buf = 0;
         {
-            StageTimer tm(j->st, j->stage_ms, 3);
+            StageTimer tm(j->clk, j->st, 3);
             SortStats ss;
             int r = bucket_sort(sb, n, has_hi, k, d_hist, b0, b1, j->arena, j->st, &ss, &lo_buf, &hi_buf);
             if (r) return r;
@@ -792,7 +832,7 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
         for (int t = 1; t <= T; t++)
             if (rb[t] > p0 && rb[t] <= p1) ends.push_back(rb[t] - p0);
         {
-            StageTimer tm(j->st, j->stage_ms, 4);
+            StageTimer tm(j->clk, j->st, 4);
             if ((rc = filter_scan(tp, ends, j->d_parent, j->d_filtered, j->arena, j->st, !j->dump_dir.empty()))) return rc;
         }
         zs[i] = tp.z;
@@ -850,7 +890,7 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
         std::vector<uint8_t> part_seen(which.size()), has_valid;
         for (size_t q = 0; q < which.size(); q++) part_seen[q] = seen[which[q]];
         {
-            StageTimer tm(j->st, j->stage_ms, 5);
+            StageTimer tm(j->clk, j->st, 5);
             if ((rc = union_piece(tp, bounds, part_seen, last_kmer, first_id, first_parent != BAD, j->d_parent,
                                   j->d_filtered, j->arena, j->st, has_valid, anchor)))
                 return rc;
@@ -858,7 +898,7 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
         for (size_t q = 0; q < which.size(); q++) seen[which[q]] |= has_valid[q];
     }
     {
-        StageTimer tm(j->st, j->stage_ms, 5);
+        StageTimer tm(j->clk, j->st, 5);
         if (have_first && first_parent == BAD) hook_bad_anchor(j->d_parent, first_id, anchor, anchor + 1, j->st);
         compress_parents(j->d_parent, N, j->st);
         MP_CUDA(cudaMemcpyAsync(&j->hooked_bad, anchor + 1, 4, cudaMemcpyDeviceToHost, j->st));
@@ -916,11 +956,10 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
 {
     const uint64_t N = j->pr.n_reads, n = gs.n;
     int rc = 0;
-    const double ms0 = j->stage_ms[2] + j->stage_ms[3];
     uint64_t *k1 = j->arena.alloc<uint64_t>(n + 1), *k2 = nullptr;
     uint32_t *id1 = j->arena.alloc<uint32_t>(n + 1), *id2 = nullptr;
     {
-        StageTimer tm(j->st, j->stage_ms, min3 ? 3 : 2);
+        StageTimer tm(j->clk, j->st, min3 ? 3 : 2, SPLIT_SLOT);
         if ((rc = group_plan(gs, j->arena, j->st))) return rc;
         if (min3) {
             k2 = lo;
@@ -936,20 +975,19 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
         if (rc) return rc;
     }
     {
-        StageTimer tm(j->st, j->stage_ms, 3);
+        StageTimer tm(j->clk, j->st, 3, SPLIT_SLOT);
         if ((rc = group_units(gs, k1, id1, k2, id2, j->st))) return rc;
     }
     SortStats ss;
     ss.passes = 2;
-    ss.pass_ms = j->stage_ms[2] + j->stage_ms[3] - ms0;
     ss.bytes = n * (uint64_t)(36 + (min3 ? (hi ? 13 : 12) : 0));
     {
-        StageTimer tm(j->st, j->stage_ms, 4);
+        StageTimer tm(j->clk, j->st, 4);
         if ((rc = group_filter(gs, k2, id2, id1, j->d_parent, j->d_filtered, j->arena, j->st)))
             return rc;
     }
     {
-        StageTimer tm(j->st, j->stage_ms, 5);
+        StageTimer tm(j->clk, j->st, 5);
         std::vector<GroupQuirk> open;
         if ((rc = group_union(gs, id1, j->d_parent, j->d_filtered, N, j->arena, j->st, open))) return rc;
         for (const GroupQuirk &q : open) {
@@ -995,7 +1033,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
     j->chunk_rec = rec;
     j->partitioned = false;
     j->output_ready = false;
-    for (int s = 2; s < 8; s++) j->stage_ms[s] = 0;
+    for (int s = 2; s <= SPLIT_SLOT; s++) j->clk.clear(s);
     j->sort_passes_total = 0;
     j->sort_ms_total = 0;
     j->sort_bytes_total = 0;
@@ -1041,7 +1079,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         d_b = j->arena.alloc_persistent<uint32_t>(S + 1);
         if (!cnt_all || !d_b) return set_error(MP_ENOMEM, "device memory for enumeration counts");
         std::vector<uint32_t> hb(scanR.begin(), scanR.end());
-        StageTimer tm(j->st, j->stage_ms, 2);
+        StageTimer tm(j->clk, j->st, 2);
         MP_CUDA(cudaMemcpyAsync(d_b, hb.data(), (S + 1) * 4, cudaMemcpyHostToDevice, j->st));
         if (launch_enum_count_scans(j->d_fq, j->pr, k, d_b, S, cnt_all, N + 1, err, j->st))
             return set_error(MP_EARG, "enumeration count over %d scans", S);
@@ -1113,7 +1151,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         int lo_buf = 0, hi_buf = 0;
         uint64_t n = 0;
         {
-            StageTimer tm(j->st, j->stage_ms, 2);
+            StageTimer tm(j->clk, j->st, 2);
             if (!cnt_all) {
                 launch_enum_count(j->d_fq, j->pr, k, p->min3, (uint32_t)lo, (uint32_t)hi, cnt, err, j->st);
                 MP_CUDA(cudaMemsetAsync(cnt + N, 0, 4, j->st));
@@ -1157,7 +1195,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         snprintf(name, sizeof name, "scan%d_enum.bin", s);
         if ((rc = dump_tuples(j, name, sb.lo[0], sb.hi[0], sb.id[0], n))) return rc;
         {
-            StageTimer tm(j->st, j->stage_ms, 3);
+            StageTimer tm(j->clk, j->st, 3);
             SortStats ss;
             if ((rc = bucket_sort(sb, n, has_hi, k, d_hist, lo, hi, j->arena, j->st, &ss, &lo_buf, &hi_buf))) return rc;
             add_sort_stats(j, ss, n);
@@ -1171,7 +1209,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         snprintf(name, sizeof name, "scan%d_sorted.bin", s);
         if ((rc = dump_tuples(j, name, tp.lo, tp.hi, tp.id, n))) return rc;
         {
-            StageTimer tm(j->st, j->stage_ms, 4);
+            StageTimer tm(j->clk, j->st, 4);
             if ((rc = filter_scan(tp, rb, j->d_parent, j->d_filtered, j->arena, j->st, !j->dump_dir.empty()))) return rc;
         }
         snprintf(name, sizeof name, "scan%d_filtered.bin", s);
@@ -1185,7 +1223,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             if (rc) return rc;
         }
         {
-            StageTimer tm(j->st, j->stage_ms, 5);
+            StageTimer tm(j->clk, j->st, 5);
             if ((rc = union_scan(tp, rb, j->d_parent, j->d_filtered, N, j->arena, j->st, j->hooked_bad, &j->hooked_bad)))
                 return rc;
         }
@@ -1198,7 +1236,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
     j->arena.free_persistent(d_hist);
     j->kc_pieces = 0;
     {
-        StageTimer tm(j->st, j->stage_ms, 6);
+        StageTimer tm(j->clk, j->st, 6);
         if (!j->dump_dir.empty()) {
             MP_CUDA(cudaMemsetAsync(j->d_size, 0, N * 4, j->st));
             (mp::count_launch(), k_sizes_raw<<<gN, 256, 0, j->st>>>(j->d_parent, N, j->d_size));
@@ -1239,8 +1277,8 @@ namespace {
 int plan_job_output(mp_job *j)
 {
     if (j->output_ready) return 0;
-    StageTimer tm(j->st, j->stage_ms, 7);
-    j->stage_ms[7] = 0;
+    j->clk.clear(7);
+    StageTimer tm(j->clk, j->st, 7);
     int rc = plan_output(j->d_fq, j->pr, j->d_parent, j->bounds, j->chunk_rec.data(), j->nchunks, j->T, j->interleaved,
                          &j->out_plan, j->out_sizes, j->arena, j->st);
     j->arena.release_scratch();
@@ -1254,7 +1292,7 @@ int plan_job_output(mp_job *j)
 int materialize_output(mp_job *j)
 {
     if (j->d_out) return 0;
-    StageTimer tm(j->st, j->stage_ms, 7);
+    StageTimer tm(j->clk, j->st, 7);
     j->d_out = j->arena.alloc_persistent<uint8_t>(j->out_total + 16);
     if (!j->d_out) return set_error(MP_ENOMEM, "device memory for the output bytes");
     return copy_output(j->out_plan, j->d_fq, j->d_out, j->st);
@@ -1265,9 +1303,11 @@ int materialize_output(mp_job *j)
 // small writes use the host link worse than the copy engine).
 int materialize_and_download(mp_job *j, uint8_t *out)
 {
-    constexpr int K = 8;
+    constexpr int KM = 8;
+    constexpr uint64_t BATCH_BYTES = 16ull << 20;  // (a batch costs about 15 us beside its copy: 3 MB of the link)
     const OutputPlan &pl = j->out_plan;
-    if (pl.n < (uint64_t)K * 1024 || pl.total == 0) {
+    const int K = (int)std::min<uint64_t>(KM, pl.total / BATCH_BYTES);
+    if (pl.n < (uint64_t)KM * 1024 || K < 2) {
         int rc = materialize_output(j);
         if (rc) return rc;
         MP_CUDA(cudaMemcpyAsync(out, j->d_out, j->out_total, cudaMemcpyDeviceToHost, j->st));
@@ -1278,18 +1318,19 @@ int materialize_and_download(mp_job *j, uint8_t *out)
         j->copy_st = nullptr;
         return set_error(MP_ECUDA, "cannot create a stream");
     }
-    uint64_t e[K + 1], o[K + 1];
-    for (int b = 0; b <= K; b++) e[b] = pl.n * (uint64_t)b / K;
+    uint64_t e[KM + 1];
+    ReadBack<uint64_t> o(j->arena, KM + 1);
+    for (int b = 0; b <= K; b++) e[b] = pl.n * (uint64_t)b / (uint64_t)K;
     for (int b = 0; b < K; b++) MP_CUDA(cudaMemcpyAsync(&o[b], pl.off + e[b], 8, cudaMemcpyDeviceToHost, j->st));
-    o[K] = pl.total;
     j->d_out = j->arena.alloc_persistent<uint8_t>(pl.total + 16);
     if (!j->d_out) return set_error(MP_ENOMEM, "device memory for the output bytes");
     MP_CUDA(cudaStreamSynchronize(j->st));
-    cudaEvent_t ev[K];
+    o[K] = pl.total;
+    cudaEvent_t ev[KM];
     for (auto &x : ev) cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
     int rc = 0;
     {
-        StageTimer tm(j->st, j->stage_ms, 7);
+        StageTimer tm(j->clk, j->st, 7);
         for (int b = 0; b < K && !rc; b++) {
             rc = copy_output_range(pl, e[b], e[b + 1], j->d_fq, j->d_out, j->st);
             cudaEventRecord(ev[b], j->st);
@@ -1417,10 +1458,20 @@ int mp_job_set_dump_dir(mp_job *j, const char *dir)
     return 0;
 }
 
+// (the clock of a const job: reading the times settles what is pending)
+static const double *stage_times(const mp_job *j)
+{
+    StageClock &c = const_cast<mp_job *>(j)->clk;
+    if (!c.pending.empty()) cudaSetDevice(j->ctx->device);
+    c.resolve();
+    return c.ms;
+}
+
 int mp_job_stage_ms(const mp_job *j, double *ms, int n)
 {
     if (!j || !ms) return set_error(MP_EARG, "null argument");
-    for (int i = 0; i < n && i < 8; i++) ms[i] = j->stage_ms[i];
+    const double *t = stage_times(j);
+    for (int i = 0; i < n && i < 8; i++) ms[i] = t[i];
     return 0;
 }
 
@@ -1429,7 +1480,7 @@ int mp_job_sort_stats(const mp_job *j, uint64_t *tuples, int *passes, double *pa
     if (!j) return set_error(MP_EARG, "null job");
     if (tuples) *tuples = j->sort_tuples_total;
     if (passes) *passes = j->sort_passes_total;
-    if (pass_ms) *pass_ms = j->sort_ms_total;
+    if (pass_ms) *pass_ms = j->sort_ms_total + stage_times(j)[SPLIT_SLOT];
     if (bytes) *bytes = j->sort_bytes_total;
     return 0;
 }
@@ -1443,7 +1494,7 @@ int mp_job_sort_split(const mp_job *j, double *pass_ms, double *unit_ms, double 
         for (int q = 0; q < 3; q++) unit_counters[1 + q] = j->phase_total[q];
         for (int q = 0; q < 7; q++) unit_counters[4 + q] = j->pass_cycles_total[q];
     }
-    if (pass_ms) *pass_ms = j->sort_ms_total;
+    if (pass_ms) *pass_ms = j->sort_ms_total + stage_times(j)[SPLIT_SLOT];
     if (unit_ms) *unit_ms = j->seg_ms_total;
     if (big_ms) *big_ms = j->big_ms_total;
     if (units) *units = j->units_total;

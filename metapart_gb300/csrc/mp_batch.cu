@@ -118,7 +118,7 @@ struct mp_batch {
     cudaStream_t st = nullptr, copy_st = nullptr, dl_st = nullptr;  // kernels, uploads, downloads
     DeviceArena arena;  // a group's stage state, released once the group's kernels are queued
     DeviceArena io;     // the groups' FASTQ and partition-file bytes: freed once their copies are done
-    double stage_ms[8] = {0};
+    StageClock clk;
     int groups = 0;
     double sort_pass_ms = 0;
     uint64_t sort_bytes = 0, sort_tuples = 0;
@@ -274,7 +274,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
         const uint64_t b0 = g[qa].byte0, b1 = g[qb - 1].byte0 + smp[g[qb - 1].idx].nbytes;
         MP_CUDA(cudaStreamWaitEvent(st, ev[u], 0));
         {
-            StageTimer tm(st, b->stage_ms, 0);
+            StageTimer tm(b->clk, st, 0);
             rc = parse_fastq_range(d_fq, b0, b1, &prs[u], A, st);
         }
         if (rc) {  // name the sample: parse the segment's samples one by one until one fails
@@ -315,7 +315,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
         }
         if (rc) return rc;
         RU[u + 1] = R[qb];
-        StageTimer tm(st, b->stage_ms, 1);
+        StageTimer tm(b->clk, st, 1);
         if (prs[u].max_len > (uint32_t)MAX_READ_COUNT && prs[u].max_len > (uint32_t)k)
             return set_error(MP_EUNSUP, "a read is longer than %d bases", MAX_READ_COUNT);
         max_len = std::max(max_len, prs[u].max_len);
@@ -330,7 +330,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     // ---- one read table for the group, global read ids
     ParsedReads pr;
     {
-        StageTimer tm(st, b->stage_ms, 0);
+        StageTimer tm(b->clk, st, 0);
         pr.n_reads = N;
         pr.max_len = max_len;
         pr.rec_start = A.alloc_persistent<uint64_t>(N + 1);
@@ -362,7 +362,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     std::vector<int> hstat(nseg);
     uint32_t herr = 0;
     {
-        StageTimer tm(st, b->stage_ms, 1);
+        StageTimer tm(b->clk, st, 1);
         scan_u32_to_u64(cc, shist, (size_t)nseg * NB, shist + (size_t)nseg * NB, tmph, tbh, st);
         MP_CUDA(cudaMemcpyAsync(dT, hT.data(), nseg * 4, cudaMemcpyHostToDevice, st));
         MP_CUDA(cudaMemcpyAsync(drb0, hrb0.data(), (nseg + 1) * 4, cudaMemcpyHostToDevice, st));
@@ -396,7 +396,6 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     int lo_buf = 0, hi_buf = 0;
     if (grouped) {
         // ---- enumeration into bins and units of every sample's buckets
-        const double ms0 = b->stage_ms[2] + b->stage_ms[3];
         gs.k = k;
         gs.n = T_all;
         gs.d_hist = shist;
@@ -410,22 +409,21 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
             if (!sb.lo[x] || !sb.id[x]) return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)T_all);
         }
         {
-            StageTimer tm(st, b->stage_ms, 2);
+            StageTimer tm(b->clk, st, 2, SPLIT_SLOT);
             if ((rc = group_plan(gs, A, st))) return rc;
             if ((rc = group_bins_reads(gs, d_fq, pr, R, nullptr, sb.lo[1], sb.id[1], A, st))) return rc;
         }
         {
-            StageTimer tm(st, b->stage_ms, 3);
+            StageTimer tm(b->clk, st, 3, SPLIT_SLOT);
             if ((rc = group_units(gs, sb.lo[1], sb.id[1], sb.lo[0], sb.id[0], st))) return rc;
         }
-        b->sort_pass_ms += b->stage_ms[2] + b->stage_ms[3] - ms0;
         b->sort_bytes += T_all * 36;
         b->sort_passes += 2;
         b->sort_tuples += T_all;
     } else {
         // ---- enumeration: every k-mer of every read (one scan per sample), read order
         {
-            StageTimer tm(st, b->stage_ms, 2);
+            StageTimer tm(b->clk, st, 2);
             uint32_t *cnt = A.alloc<uint32_t>(N + 1);
             uint64_t *off = A.alloc<uint64_t>(N + 2), *ntot = A.alloc<uint64_t>(1);
             const size_t tb = scan_tmp_bytes(N + 1);
@@ -456,7 +454,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
             A.release_scratch();
         }
         // ---- sort: every sample's tuples by (k-mer, adjacency), within the sample's range
-        StageTimer tm(st, b->stage_ms, 3);
+        StageTimer tm(b->clk, st, 3);
         SortStats ss;
         if ((rc = bucket_sort(sb, T_all, has_hi, k, shist, 0, (uint64_t)nseg * NB, A, st, &ss, &lo_buf, &hi_buf, &segs)))
             return rc;
@@ -483,10 +481,10 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     MP_CUDA(cudaMemsetAsync(filtered, 0, N + 1, st));
     if (grouped) {
         {
-            StageTimer tm(st, b->stage_ms, 4);
+            StageTimer tm(b->clk, st, 4);
             if ((rc = group_filter(gs, tp.lo, tp.id, sb.id[lo_buf ^ 1], parent, filtered, A, st))) return rc;
         }
-        StageTimer tm(st, b->stage_ms, 5);
+        StageTimer tm(b->clk, st, 5);
         std::vector<GroupQuirk> open;
         if ((rc = group_union(gs, sb.id[lo_buf ^ 1], parent, filtered, N, A, st, open))) return rc;
         for (const GroupQuirk &q : open) {
@@ -498,13 +496,13 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
         A.free_persistent(sb.id[lo_buf ^ 1]);
     } else {
         {
-            StageTimer tm(st, b->stage_ms, 4);
+            StageTimer tm(b->clk, st, 4);
             if ((rc = filter_scan(tp, rb, parent, filtered, A, st, false, true))) return rc;
         }
         std::vector<uint32_t> rseg(Rn);
         for (int q = 0; q < nseg; q++)
             for (uint32_t t = hrb0[q]; t < hrb0[q + 1]; t++) rseg[t] = (uint32_t)q;
-        StageTimer tm(st, b->stage_ms, 5);
+        StageTimer tm(b->clk, st, 5);
         if ((rc = union_segments(tp, rb, rseg, segs.tstart, parent, filtered, N, A, st))) return rc;
     }
     A.release_scratch();
@@ -515,7 +513,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     // ---- mate union and every sample's partitions
     std::vector<uint64_t> bounds((size_t)nseg * 17);
     {
-        StageTimer tm(st, b->stage_ms, 6);
+        StageTimer tm(b->clk, st, 6);
         int rounds = 0;
         if ((rc = mate_union(parent, N, size, A, st, &rounds))) return rc;
         if ((rc = plan_partitions_segments(parent, size, N, R, bounds.data(), A, st))) return rc;
@@ -532,7 +530,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
         Ts[q] = smp[g[q].idx].num_threads;
     }
     {
-        StageTimer tm(st, b->stage_ms, 7);
+        StageTimer tm(b->clk, st, 7);
         if ((rc = plan_output_batch(pr, parent, il, R, bounds, crec, Ts, &plan, fsz, file0, A, st))) return rc;
         A.release_scratch();
     }
@@ -570,7 +568,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     pending.out = d_out;
     {
         constexpr int KB = 8;
-        StageTimer tm(st, b->stage_ms, 7);
+        StageTimer tm(b->clk, st, 7);
         uint64_t e[KB + 1], o[KB + 1];
         for (int x = 0; x <= KB; x++) e[x] = plan.n * (uint64_t)x / KB;
         for (int x = 0; x < KB; x++)
@@ -621,6 +619,10 @@ int mp_batch_create(mp_ctx *ctx, mp_batch **out)
     }
     b->arena.st = b->st;
     b->io.st = b->st;
+    if (cudaHostAlloc((void **)&b->arena.mail, DeviceArena::MAIL, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        b->arena.mail = nullptr;
+    }
     ctx_budget(ctx, &b->arena.budget_used, &b->arena.budget_limit);
     ctx_budget(ctx, &b->io.budget_used, &b->io.budget_limit);
     *out = b;
@@ -639,6 +641,7 @@ void mp_batch_destroy(mp_batch *b)
     cudaStreamDestroy(b->st);
     cudaStreamDestroy(b->copy_st);
     cudaStreamDestroy(b->dl_st);
+    if (b->arena.mail) cudaFreeHost(b->arena.mail);
     delete b;
 }
 
@@ -653,7 +656,7 @@ int mp_batch_run(mp_batch *b, const mp_batch_params *p, int nsamples, const mp_b
         results[q].status = MP_EARG;
         snprintf(results[q].error, sizeof results[q].error, "not run");
     }
-    for (auto &v : b->stage_ms) v = 0;
+    for (int s = 0; s <= SPLIT_SLOT; s++) b->clk.clear(s);
     b->groups = 0;
     b->sort_pass_ms = 0;
     b->sort_bytes = b->sort_tuples = 0;
@@ -736,10 +739,20 @@ int mp_batch_run(mp_batch *b, const mp_batch_params *p, int nsamples, const mp_b
     return rc;
 }
 
+// (the clock of a const batch: reading the times settles what is pending)
+static const double *batch_times(const mp_batch *b)
+{
+    StageClock &c = const_cast<mp_batch *>(b)->clk;
+    if (!c.pending.empty()) cudaSetDevice(b->device);
+    c.resolve();
+    return c.ms;
+}
+
 int mp_batch_stage_ms(const mp_batch *b, double *ms, int n)
 {
     if (!b || !ms) return set_error(MP_EARG, "null argument");
-    for (int i = 0; i < n && i < 8; i++) ms[i] = b->stage_ms[i];
+    const double *t = batch_times(b);
+    for (int i = 0; i < n && i < 8; i++) ms[i] = t[i];
     return 0;
 }
 
@@ -760,7 +773,7 @@ int mp_batch_sort_stats(const mp_batch *b, uint64_t *tuples, int *passes, double
     if (!b) return set_error(MP_EARG, "null batch");
     if (tuples) *tuples = b->sort_tuples;
     if (passes) *passes = b->sort_passes;
-    if (pass_ms) *pass_ms = b->sort_pass_ms;
+    if (pass_ms) *pass_ms = b->sort_pass_ms + batch_times(b)[SPLIT_SLOT];
     if (bytes) *bytes = b->sort_bytes;
     return 0;
 }

@@ -1,6 +1,9 @@
 // Host-side pieces shared by the job driver (mp_api.cu) and the batch driver (mp_batch.cu).
 #pragma once
 #include <nvtx3/nvToolsExt.h>
+
+#include <vector>
+
 #include "k_reads.cuh"
 
 namespace mp {
@@ -15,33 +18,87 @@ void ctx_budget(mp_ctx *ctx, std::atomic<uint64_t> **used, uint64_t *limit);
 // parent[x] = x for every read.
 void launch_init_parent(uint32_t *parent, uint64_t n, cudaStream_t st);
 
-// Device time of the work queued on a stream while the timer lives, added to *slot (ms).
 // The stages of a job or batch, in the order of their time slots (mp_job_stage_ms, mp_batch_stage_ms).
 constexpr const char *STAGE_NAMES[8] = {"parse", "count", "enumerate", "sort", "filter", "union_find",
                                         "mate_union_plan", "output"};
+constexpr int SPLIT_SLOT = 8;  // the split passes of grouped scans, apart
 
-// A stage's device time (CUDA events on its stream, added to its slot) and an NVTX range of the stage's
-// name for a profiler's timeline (a no-op without one attached).
+// Device time per stage in ms, from event pairs that are read when the times are asked for: a stage's end is not waited
+// for (eight waits per job, 10-20 us each, kept the host from queueing ahead).
+struct StageClock {
+    struct Pending {
+        cudaEvent_t a, b;
+        int slot[2];
+    };
+    double ms[9] = {0};
+    std::vector<Pending> pending;
+    std::vector<cudaEvent_t> pool;
+
+    cudaEvent_t take()
+    {
+        cudaEvent_t e = nullptr;
+        if (!pool.empty()) {
+            e = pool.back();
+            pool.pop_back();
+        } else {
+            cudaEventCreate(&e);
+        }
+        return e;
+    }
+    void clear(int slot)
+    {
+        ms[slot] = 0;
+        for (size_t i = 0; i < pending.size();) {
+            Pending &p = pending[i];
+            for (int &s : p.slot)
+                if (s == slot) s = -1;
+            if (p.slot[0] < 0 && p.slot[1] < 0) {
+                pool.push_back(p.a);
+                pool.push_back(p.b);
+                pending.erase(pending.begin() + (long)i);
+            } else {
+                i++;
+            }
+        }
+    }
+    void resolve()
+    {
+        for (Pending &p : pending) {
+            float x = 0;
+            cudaEventSynchronize(p.b);
+            if (cudaEventElapsedTime(&x, p.a, p.b) != cudaSuccess) cudaGetLastError();
+            for (int s : p.slot)
+                if (s >= 0) ms[s] += x;
+            pool.push_back(p.a);
+            pool.push_back(p.b);
+        }
+        pending.clear();
+    }
+    ~StageClock()
+    {
+        for (Pending &p : pending) {
+            cudaEventDestroy(p.a);
+            cudaEventDestroy(p.b);
+        }
+        for (auto e : pool) cudaEventDestroy(e);
+    }
+};
+
+// The device time of the work queued on a stream while the timer lives, for a stage's slot (and another's), and an NVTX
+// range of the stage's name for a profiler's timeline (a no-op without one attached).
 struct StageTimer {
-    cudaEvent_t a, b;
+    StageClock &c;
+    StageClock::Pending p;
     cudaStream_t st;
-    double *acc;
-    StageTimer(cudaStream_t s, double *slots, int stage) : st(s), acc(slots + stage)
+    StageTimer(StageClock &clk, cudaStream_t s, int stage, int also = -1) : c(clk), p{clk.take(), clk.take(), {stage, also}}, st(s)
     {
         nvtxRangePushA(STAGE_NAMES[stage]);
-        cudaEventCreate(&a);
-        cudaEventCreate(&b);
-        cudaEventRecord(a, st);
+        cudaEventRecord(p.a, st);
     }
     ~StageTimer()
     {
-        cudaEventRecord(b, st);
-        cudaEventSynchronize(b);
-        float ms = 0;
-        cudaEventElapsedTime(&ms, a, b);
-        *acc += ms;
-        cudaEventDestroy(a);
-        cudaEventDestroy(b);
+        cudaEventRecord(p.b, st);
+        c.pending.push_back(p);
         nvtxRangePop();
     }
     StageTimer(const StageTimer &) = delete;

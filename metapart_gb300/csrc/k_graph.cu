@@ -5,7 +5,10 @@
 // 0xBADBADBAD (metapart.c:2330-2340).  Components hook the smaller root under the larger
 // one, so every component's root is its largest read id (metapart.c:2683-2716,
 // unionfind.h:58-66) regardless of the order unions run in.
+#include <cooperative_groups.h>
+
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "k_graph.cuh"
@@ -711,6 +714,269 @@ __global__ void k_pe_bigsmall(uint32_t *parent, uint32_t *size, const uint32_t *
         pe_bigsmall_one(parent, size, list[t], pra, prb, gmax, gadd);
 }
 
+// All remaining rounds in one cluster of blocks: the steps of a round are parted by cluster barriers (hardware, about a
+// microsecond) instead of launches, and a pair's state stays in its block's shared memory.  Three launches and the gaps
+// between them took 14-21 us a round for 24,000 to 75,000 pairs.  Parents and sizes change under the kernel and are read
+// from L2.
+//
+// Waiting pairs sleep.  Scattered loads and atomics of 16 SMs bound a round in which every pair finds its roots and
+// reserves them again (9 us for 24,000 pairs, nearly all of them behind the few hundred pairs of one component).  Here a
+// reservation holds until its pair is done: hold[x] is the first live pair of small root x, which alone may merge x, so
+// pairs on x have nothing to look at before that pair's bit in the bitmap of done pairs is set.  The pairs of both roots
+// of a merge then wake together and reserve the new one.
+//
+// A single is a root of one read (or of one BAD read): its own pair is the only one that touches it, so a pair of a
+// single and a small component X merges whatever X's size, and matters to X's other pairs only through X's size.  All
+// pairs of X and singles that come before hold[X] therefore commit in one round, as if in order; they reserve nothing
+// (first[X] keeps the pair hold[X] back for that round).  One a round they were half of 1M reads' 152 rounds.
+//
+// What is left of a round is four dependent trips to L2 and three barriers, 7 us.  Mate union of 1M reads 3.1 -> 1.2 ms, of
+// 100k 1.08 -> 0.54 ms.
+constexpr int PEC_THREADS = 1024, PEC_ITEMS = 8, PEC_PAIRS = PEC_THREADS * PEC_ITEMS, PEC_BLOCKS = 16;
+constexpr uint32_t PEC_NONE = 0xFFFFFFFFu;
+constexpr unsigned PEC_COMMITTED = 1u << 20;  // above any count of pairs
+
+// Earlier pairs have larger keys; the low half is the pair's place in the list.
+__device__ __forceinline__ unsigned long long pe_hold_key(uint32_t j, uint32_t t)
+{
+    return ((unsigned long long)(0xFFFFFFFFu - j) << 32) | t;
+}
+
+// an item's flags
+constexpr unsigned PE_LIVE = 1, PE_AWAKE = 2, PE_SA = 4, PE_SB = 8, PE_OA = 16, PE_OB = 32, PE_GROUP = 64;
+
+// Key for a small root: over none, an earlier key or that of a pair that is done (the done ones before this round).
+__device__ __forceinline__ void pe_hold(unsigned long long *hold, unsigned long long key, const uint32_t *done)
+{
+    unsigned long long v = __ldcg(hold);
+    if (v && (done[(uint32_t)v >> 5] >> ((uint32_t)v & 31) & 1u)) {
+        const unsigned long long u = atomicCAS(hold, v, key);
+        if (u == v) return;
+        v = u;  // of this round
+    }
+    if (v < key) atomicMax(hold, key);
+}
+
+struct PeState {
+    uint32_t pj[PEC_PAIRS];                // the pair
+    uint32_t xa[PEC_PAIRS], xb[PEC_PAIRS]; // its ends' roots when it was last awake
+    uint32_t ha[PEC_PAIRS], hb[PEC_PAIRS]; // the pairs (places in the list) it sleeps behind
+    uint32_t done[PEC_BLOCKS * PEC_PAIRS / 32];
+    uint16_t awake[PEC_PAIRS];             // this round's items
+    uint8_t fl[PEC_PAIRS];
+    unsigned nawake, live;
+    unsigned state[3], groups[3]; // the cluster's, by round modulo 3 (every block's copy): live pairs | blocks that committed
+};
+
+// The cluster's barrier.  One warp's release covers the block's writes (the block barrier orders them before it): a
+// release by every thread costs a fence per warp, which was most of a short round.
+__device__ __forceinline__ void pe_sync()
+{
+    __syncthreads();
+    if (threadIdx.x < 32)
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    else
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+struct PeCluster {
+    uint32_t *parent, *size;
+    const uint32_t *act;
+    uint32_t nact;
+    unsigned long long *hold, *first, *gmax, *gadd;
+    uint32_t *done;                           // a bit per place in act, clear
+    uint32_t round, limit, batch, max_round;  // rounds so far; ends are looked for as in batches of this many launched rounds
+    unsigned int *out;                        // [0] the last round, [1] pairs left when max_round came first
+};
+
+__global__ void __launch_bounds__(PEC_THREADS, 1) k_pe_cluster(PeCluster c)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ __align__(16) unsigned char pe_smem[];
+    PeState &s = *reinterpret_cast<PeState *>(pe_smem);
+    const uint32_t nb = gridDim.x, me = blockIdx.x, nact = c.nact;
+    const uint32_t mine = nact > me ? (nact - me + nb - 1) / nb : 0;  // item l is act[l nb + me]
+    const int lane = threadIdx.x & 31;
+    const bool lead = threadIdx.x == 0, first = lead && me == 0;
+    if (threadIdx.x < 3) s.state[threadIdx.x] = s.groups[threadIdx.x] = 0;
+    if (lead) {
+        s.nawake = mine;
+        s.live = mine;
+    }
+    for (uint32_t l = threadIdx.x; l < mine; l += PEC_THREADS) {
+        const uint32_t j = c.act[(uint64_t)l * nb + me];
+        s.pj[l] = j;
+        s.xa[l] = 2 * j;
+        s.xb[l] = 2 * j + 1;
+        s.ha[l] = s.hb[l] = PEC_NONE;
+        s.fl[l] = PE_LIVE | PE_AWAKE;
+        s.awake[l] = (uint16_t)l;
+    }
+    for (uint32_t w = threadIdx.x; w < (nact + 31) / 32; w += PEC_THREADS) s.done[w] = 0;
+    pe_sync();
+    uint32_t round = c.round;
+    bool over = false;
+    for (;;) {
+        const int slot = round % 3;
+        round++;
+        const uint32_t nawake = s.nawake;
+        // roots, and reservations; a pair of one component, or of two above the limit, is done
+        for (uint32_t i = threadIdx.x; i < nawake; i += PEC_THREADS) {
+            const uint32_t l = s.awake[i], j = s.pj[l];
+            uint32_t xa = s.xa[l], xb = s.xb[l], za = 0, zb = 0;
+            for (uint32_t it = 0; it < UF_CAP; it++) {
+                const uint32_t pa = __ldcg(c.parent + xa), pb = __ldcg(c.parent + xb);
+                za = __ldcg(c.size + xa);
+                zb = __ldcg(c.size + xb);
+                const bool end = pa == pb || (pa == xa && pb == xb);
+                xa = pa;
+                xb = pb;
+                if (end) break;
+            }
+            const bool sa = za <= c.limit, sb = zb <= c.limit;
+            if (xa == xb || !(sa || sb)) {
+                const uint32_t t = l * nb + me;
+                s.fl[l] = 0;
+                atomicSub(&s.live, 1u);
+                atomicOr(c.done + (t >> 5), 1u << (t & 31));
+                continue;
+            }
+            s.xa[l] = xa;
+            s.xb[l] = xb;
+            const bool oa = za <= 1 && zb > 1 && sb, ob = zb <= 1 && za > 1 && sa;
+            s.fl[l] = (uint8_t)(PE_LIVE | PE_AWAKE | (sa ? PE_SA : 0) | (sb ? PE_SB : 0) | (oa ? PE_OA : 0) | (ob ? PE_OB : 0));
+            if (oa || ob) {
+                atomicMax(&c.first[oa ? xb : xa], resv_key(round, j));
+            } else {
+                const unsigned long long key = pe_hold_key(j, l * nb + me);
+                if (sa) pe_hold(&c.hold[xa], key, s.done);
+                if (sb) pe_hold(&c.hold[xb], key, s.done);
+            }
+        }
+        pe_sync();
+        // a pair commits when it holds its small roots, or, with a single, comes before the pair that holds the other root;
+        // two small roots merge at once, a single or a small root beside a large one with the others of that root
+        bool any_group = false, any_commit = false;
+        for (uint32_t i = threadIdx.x; i < nawake; i += PEC_THREADS) {
+            const uint32_t l = s.awake[i], t = l * nb + me;
+            const unsigned f = s.fl[l];
+            if (!(f & PE_LIVE)) continue;
+            const uint32_t j = s.pj[l], xa = s.xa[l], xb = s.xb[l];
+            const unsigned long long key = pe_hold_key(j, t), stamp = resv_key(round, j);
+            const unsigned long long va = __ldcg(&c.hold[xa]), vb = __ldcg(&c.hold[xb]);
+            const unsigned long long wa = __ldcg(&c.first[xa]), wb = __ldcg(&c.first[xb]);
+            const uint32_t za = __ldcg(c.size + xa), zb = __ldcg(c.size + xb);  // (of a small root held here, as they were)
+            uint32_t ha = PEC_NONE, hb = PEC_NONE;
+            bool ok = true;
+            if (f & (PE_OA | PE_OB)) {
+                unsigned long long v = f & PE_OA ? vb : va;
+                if (v && (s.done[(uint32_t)v >> 5] >> ((uint32_t)v & 31) & 1u)) v = 0;
+                if (v > key) ha = (uint32_t)v;
+                ok = v < key;
+            } else {
+                if (f & PE_SA) {
+                    if (va != key) ha = (uint32_t)va;
+                    ok = va == key && wa < stamp;
+                }
+                if (f & PE_SB) {
+                    if (vb != key) hb = (uint32_t)vb;
+                    ok = ok && vb == key && wb < stamp;
+                }
+            }
+            if (!ok) {
+                s.ha[l] = ha;
+                s.hb[l] = hb;
+                if (ha != PEC_NONE || hb != PEC_NONE) s.fl[l] = (uint8_t)(f & ~PE_AWAKE);
+                continue;
+            }
+            any_commit = true;
+            atomicSub(&s.live, 1u);
+            atomicOr(c.done + (t >> 5), 1u << (t & 31));
+            if ((f & (PE_SA | PE_SB)) == (PE_SA | PE_SB) && !(f & (PE_OA | PE_OB))) {
+                const uint32_t hi = max(xa, xb), lo = min(xa, xb);
+                c.parent[lo] = hi;
+                c.size[hi] = za + zb;
+                c.size[lo] = 0;
+                s.fl[l] = 0;
+            } else {
+                const bool a = (f & PE_SA) && !(f & PE_OB);  // a is the end that joins
+                const uint32_t g = a ? xb : xa, x = a ? xa : xb;
+                atomicMax(&c.gmax[g], ((unsigned long long)round << 32) | x);
+                atomicAdd(&c.gadd[g], (unsigned long long)(a ? za : zb));
+                s.xa[l] = g;
+                s.xb[l] = x;
+                s.fl[l] = PE_GROUP;
+                any_group = true;
+            }
+        }
+        any_group = __syncthreads_or(any_group);
+        any_commit = __syncthreads_or(any_commit);
+        if (threadIdx.x < nb) {
+            PeState &o = *cl.map_shared_rank(&s, threadIdx.x);
+            atomicAdd(&o.state[slot], s.live + (any_commit ? PEC_COMMITTED : 0u));
+            if (any_group) atomicAdd(&o.groups[slot], 1u);
+        }
+        if (lead) {
+            s.state[(slot + 1) % 3] = s.groups[(slot + 1) % 3] = 0;
+            s.nawake = 0;
+        }
+        pe_sync();
+        const unsigned left = s.state[slot] % PEC_COMMITTED;
+        const bool last = (round - c.round) % c.batch == 0;
+        if (left == 0 || (last && round + c.batch > c.max_round)) {
+            // (a round that committed pairs is followed by the one that finds none left, unless a batch ends with it)
+            if (first) {
+                c.out[0] = round + (left == 0 && s.state[slot] >= PEC_COMMITTED && !last);
+                c.out[1] = left;
+            }
+            over = true;
+        }
+        if (s.groups[slot]) {
+            for (uint32_t i = threadIdx.x; i < nawake; i += PEC_THREADS) {
+                const uint32_t l = s.awake[i];
+                if (!(s.fl[l] & PE_GROUP)) continue;
+                s.fl[l] = 0;
+                const uint32_t g = s.xa[l], x = s.xb[l];
+                const uint32_t mx = (uint32_t)(__ldcg(&c.gmax[g]) & 0xFFFFFFFFu), R = max(mx, g);
+                if (x != mx) {
+                    c.parent[x] = R;
+                    c.size[x] = 0;
+                    continue;
+                }
+                // the group's one writer; a small root's first pair holds the new one as well
+                const uint32_t tot = __ldcg(&c.size[g]) + (uint32_t)__ldcg(&c.gadd[g]);
+                if (R != g) c.hold[R] = __ldcg(&c.hold[g]);
+                c.parent[R != g ? g : x] = R;
+                c.size[R != g ? g : x] = 0;
+                c.size[R] = tot;
+                c.gadd[g] = 0;
+            }
+        }
+        if (over) break;
+        // who is awake in the next round
+        for (uint32_t w = threadIdx.x; w < (nact + 31) / 32; w += PEC_THREADS) s.done[w] = __ldcg(c.done + w);
+        __syncthreads();
+        for (uint32_t l0 = threadIdx.x & ~31u; l0 < mine; l0 += PEC_THREADS) {
+            const uint32_t l = l0 + lane;
+            const unsigned f = l < mine ? s.fl[l] : 0u;
+            bool up = (f & PE_LIVE) && (f & PE_AWAKE);
+            if ((f & PE_LIVE) && !up) {
+                const uint32_t ha = s.ha[l], hb = s.hb[l];
+                up = (ha != PEC_NONE && (s.done[ha >> 5] >> (ha & 31) & 1u)) || (hb != PEC_NONE && (s.done[hb >> 5] >> (hb & 31) & 1u));
+            }
+            const uint32_t m = __ballot_sync(FULLW, up);
+            uint32_t base = 0;
+            if (lane == 0 && m) base = atomicAdd(&s.nawake, (unsigned)__popc(m));
+            base = __shfl_sync(FULLW, base, 0);
+            if (up) s.awake[base + __popc(m & ((1u << lane) - 1))] = (uint16_t)l;
+        }
+        pe_sync();
+    }
+    pe_sync();  // no block leaves while another reads the first one's counters
+}
+
 // --------------------------------------------------------------- host side
 
 static unsigned blocks_for(uint64_t n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -891,6 +1157,33 @@ int mate_union_and_plan(uint32_t *parent, uint64_t n_reads, uint32_t *size, uint
     return rc ? rc : plan_partitions(parent, size, n_reads, bounds_out, arena, st);
 }
 
+// Blocks of the mate union's cluster: 16 where the device takes a cluster of that size, else 8 (portable).
+static int pe_cluster_blocks()
+{
+    static int blocks[64];  // (a property of the device)
+    static std::once_flag once[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::call_once(once[dev & 63], [dev] {
+        cudaFuncSetAttribute(k_pe_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PeState));
+        cudaFuncSetAttribute(k_pe_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim = {PEC_BLOCKS, 1, 1};
+        cfg.gridDim = dim3(PEC_BLOCKS);
+        cfg.blockDim = dim3(PEC_THREADS);
+        cfg.dynamicSmemBytes = sizeof(PeState);
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        const bool ok = cudaOccupancyMaxActiveClusters(&n, k_pe_cluster, &cfg) == cudaSuccess && n > 0;
+        cudaGetLastError();
+        blocks[dev & 63] = ok ? PEC_BLOCKS : 8;
+    });
+    return blocks[dev & 63];
+}
+
 int mate_union(uint32_t *parent, uint64_t n_reads, uint32_t *size, DeviceArena &arena, cudaStream_t st, int *rounds_out)
 {
     const uint32_t limit = 1000;
@@ -902,20 +1195,51 @@ int mate_union(uint32_t *parent, uint64_t n_reads, uint32_t *size, DeviceArena &
     uint32_t *big = arena.alloc<uint32_t>(npairs + 1);
     uint32_t *psa = arena.alloc<uint32_t>(npairs + 1), *psb = arena.alloc<uint32_t>(npairs + 1);
     unsigned long long *resv = arena.alloc<unsigned long long>(n_reads);
+    unsigned long long *hold = arena.alloc<unsigned long long>(n_reads), *first = arena.alloc<unsigned long long>(n_reads);
+    uint32_t *done = arena.alloc<uint32_t>(PEC_BLOCKS * PEC_PAIRS / 32);
     unsigned long long *gmax = arena.alloc<unsigned long long>(n_reads);
     unsigned long long *gadd = arena.alloc<unsigned long long>(n_reads);
     constexpr int RB = 8;  // rounds launched between host synchronisations
     // per round r of a batch: [4r] reserved pairs, [4r+1] pairs left for the next round, [4r+2] big-small merges;
     // [4 RB + 1] the batch's first active count
     unsigned int *cnts = arena.alloc<unsigned int>(4 * RB + 4);
-    if (!act || !act2 || !pra || !prb || !big || !psa || !psb || !resv || !gmax || !gadd || !cnts)
+    if (!act || !act2 || !pra || !prb || !big || !psa || !psb || !resv || !hold || !first || !done || !gmax || !gadd || !cnts)
         return set_error(MP_ENOMEM, "device memory for the mate union");
     MP_CUDA(cudaMemsetAsync(resv, 0, n_reads * sizeof(unsigned long long), st));
+    MP_CUDA(cudaMemsetAsync(hold, 0, n_reads * sizeof(unsigned long long), st));
+    MP_CUDA(cudaMemsetAsync(first, 0, n_reads * sizeof(unsigned long long), st));
+    MP_CUDA(cudaMemsetAsync(done, 0, PEC_BLOCKS * PEC_PAIRS / 8, st));
     MP_CUDA(cudaMemsetAsync(gmax, 0, n_reads * sizeof(unsigned long long), st));
     MP_CUDA(cudaMemsetAsync(gadd, 0, n_reads * sizeof(unsigned long long), st));
     (mp::count_launch(), k_pe_prepare<<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads, act, npairs));
     uint32_t nact = (uint32_t)npairs, round = 0;
+    const uint32_t most_blocks = (uint32_t)pe_cluster_blocks();
     while (nact > 0) {
+        if (round + RB <= arena.lim.mate_rounds && nact <= most_blocks * (round ? PEC_PAIRS : PEC_THREADS + PEC_THREADS / 2)) {
+            // the rest (not many fresh pairs: all of them are awake in the first round, 66 us for 50,000 on 16 SMs where a
+            // launched one takes 16) in one cluster, of as few blocks as give each thread a pair (cheaper barriers)
+            uint32_t cluster = 1;
+            while (cluster < most_blocks && cluster * PEC_THREADS < nact) cluster *= 2;
+            PeCluster c{parent, size, act, nact, hold, first, gmax, gadd, done, round, limit, (uint32_t)RB, arena.lim.mate_rounds, cnts};
+            cudaLaunchConfig_t cfg{};
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim = {cluster, 1, 1};
+            cfg.gridDim = dim3(cluster);
+            cfg.blockDim = dim3(PEC_THREADS);
+            cfg.dynamicSmemBytes = sizeof(PeState);
+            cfg.stream = st;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            mp::count_launch();
+            MP_CUDA(cudaLaunchKernelEx(&cfg, k_pe_cluster, c));
+            ReadBack<unsigned int> h(arena, 2);
+            MP_CUDA(cudaMemcpyAsync(h.p, cnts, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+            MP_CUDA(cudaStreamSynchronize(st));
+            round = h[0];
+            if (h[1]) return set_error(MP_EDEVICE, "mate union did not converge within %u rounds", arena.lim.mate_rounds);
+            break;
+        }
         if (round + RB > arena.lim.mate_rounds)
             return set_error(MP_EDEVICE, "mate union did not converge within %u rounds", arena.lim.mate_rounds);
         // counts only shrink, so nact bounds every list of the batch

@@ -27,7 +27,7 @@ constexpr int GP_CAP_S = 6128;           // most tuples of a unit for the 512-th
 constexpr int GP_CAP_L = 12288;          // and for the 1024-thread blocks; a larger bucket takes the device-wide sort
 constexpr uint32_t GP_DIGITS = 1024;     // digits of a split pass: bins of a segment, units of a bin
 constexpr uint64_t GP_SMALL = 1500000;   // tuples of a segment that fit GP_DIGITS units however they are spread
-constexpr int GP_COUNT_ITEMS = 8, GP_COUNT_THREADS = 256, GP_COUNT_BLOCK = GP_COUNT_ITEMS * GP_COUNT_THREADS;
+constexpr int GP_COUNT_BLOCK = 512;      // buckets per block of the planning kernels, one per thread
 constexpr uint32_t GP_NONE = 0x7FFFFFFFu;  // a grouped id that stands for no read
 constexpr size_t PLAN_MAIL = DeviceArena::MAIL - 4096;  // where the plan's counters arrive in the mailbox
 constexpr int QW = 8;  // words per segment: tuples found before the last run, last run's, its read, the run's place
@@ -123,20 +123,16 @@ __device__ __forceinline__ uint64_t block_scan_excl(uint64_t v, uint64_t *total,
 }
 
 // Units starting in each block of GP_COUNT_BLOCK buckets.
-__global__ void __launch_bounds__(GP_COUNT_THREADS) k_gp_count(PlanCtx c, uint64_t *blk)
+__global__ void __launch_bounds__(GP_COUNT_BLOCK) k_gp_count(PlanCtx c, uint64_t *blk)
 {
-    __shared__ uint64_t ws[GP_COUNT_THREADS / 32];
-    uint64_t v = 0;
-    const uint64_t h0 = c.hist[c.lo];
-    for (int i = 0; i < GP_COUNT_ITEMS; i++) {
-        const uint64_t b = c.lo + (uint64_t)blockIdx.x * GP_COUNT_BLOCK + (uint64_t)i * GP_COUNT_THREADS + threadIdx.x;
-        if (b >= c.hi) break;
-        const uint64_t s = c.hist[b], e = c.hist[b + 1];
-        if (s != e) v += plan_flags(c, b, s - h0, e - h0) & 1u;
+    const uint64_t b = c.lo + (uint64_t)blockIdx.x * GP_COUNT_BLOCK + threadIdx.x;
+    bool f = false;
+    if (b < c.hi) {
+        const uint64_t h0 = c.hist[c.lo], s = c.hist[b], e = c.hist[b + 1];
+        f = s != e && (plan_flags(c, b, s - h0, e - h0) & 1u);
     }
-    uint64_t tot;
-    block_scan_excl(v, &tot, ws);
-    if (threadIdx.x == 0) blk[blockIdx.x] = tot;
+    const int n = __syncthreads_count(f);
+    if (threadIdx.x == 0) blk[blockIdx.x] = (uint64_t)n;
 }
 
 // Exclusive scan of the blocks' counts by one block; the sentinels past the last unit and bin.
@@ -161,48 +157,48 @@ __global__ void __launch_bounds__(1024) k_gp_scan(uint64_t *blk, uint32_t nblk, 
 }
 
 // The unit and bin arrays.  A bucket above GP_CAP_S tuples is a unit of its own (plan_flags), so its size is known here.
-__global__ void __launch_bounds__(GP_COUNT_THREADS) k_gp_write(PlanCtx c, const uint64_t *blk, uint32_t *ctr, uint32_t *ustart,
-                                                               uint32_t *ub0, uint32_t *ucur, uint32_t *bstart, uint32_t *bu0,
-                                                               uint32_t *bcur, uint32_t *bsh, uint32_t *bfirst,
-                                                               uint32_t *unit_of, uint32_t *mid,
-                                                               uint32_t *big)
+// One bucket per thread and one block scan: with eight buckets per thread in turn (eight scans) this and k_gp_count took
+// 36 and 31 us for a scan of all buckets.
+__global__ void __launch_bounds__(GP_COUNT_BLOCK) k_gp_write(PlanCtx c, const uint64_t *blk, uint32_t *ctr, uint32_t *ustart,
+                                                             uint32_t *ub0, uint32_t *ucur, uint32_t *bstart, uint32_t *bu0,
+                                                             uint32_t *bcur, uint32_t *bsh, uint32_t *bfirst, uint32_t *unit_of,
+                                                             uint32_t *mid, uint32_t *big)
 {
-    __shared__ uint64_t ws[GP_COUNT_THREADS / 32];
-    const uint64_t h0 = c.hist[c.lo];
-    uint64_t at = blk[blockIdx.x];
-    for (int i = 0; i < GP_COUNT_ITEMS; i++) {
-        const uint64_t b = c.lo + (uint64_t)blockIdx.x * GP_COUNT_BLOCK + (uint64_t)i * GP_COUNT_THREADS + threadIdx.x;
-        uint64_t s = 0, e = 0;
-        uint32_t f = 0;
-        if (b < c.hi) {
-            s = c.hist[b] - h0;
-            e = c.hist[b + 1] - h0;
-            if (s != e) f = plan_flags(c, b, s, e);
-        }
-        uint64_t tot;
-        const uint32_t u = (uint32_t)(at + block_scan_excl(f & 1u, &tot, ws));
-        at += tot;
-        if (b < c.hi) {
-            const uint32_t seg = (uint32_t)(b / NB), rel = ((uint32_t)b & (NB - 1)) - c.seg_lo, sh = c.seg_sh[seg];
-            if ((rel & ((1u << sh) - 1)) == 0) {
-                const uint32_t bin = c.seg_bin0[seg] + (rel >> sh);
-                bstart[bin] = bcur[bin] = (uint32_t)s;
-                bu0[bin] = u;
-                bfirst[bin] = (uint32_t)(b - c.lo);
-                bsh[bin] = sh;
-            }
-            unit_of[b - c.lo] = u + (f & 1u) - 1u;  // (before the first unit: ~0)
-        }
-        if (f & 1u) {
-            ustart[u] = ucur[u] = (uint32_t)s;
-            ub0[u] = (uint32_t)b | (f & 8u ? 0x80000000u : 0u);
-        }
-        if (e - s > (uint64_t)GP_CAP_S) {
-            if (e - s <= (uint64_t)GP_CAP_L) mid[atomicAdd(&ctr[GC_MID], 1u)] = u;
-            else {
-                big[atomicAdd(&ctr[GC_BIG], 1u)] = u;
-                atomicAdd(&ctr[GC_BIG_TUPLES], (uint32_t)(e - s));
-            }
+    __shared__ uint32_t ws[GP_COUNT_BLOCK / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t b = c.lo + (uint64_t)blockIdx.x * GP_COUNT_BLOCK + threadIdx.x;
+    uint64_t s = 0, e = 0;
+    uint32_t f = 0;
+    if (b < c.hi) {
+        const uint64_t h0 = c.hist[c.lo];
+        s = c.hist[b] - h0;
+        e = c.hist[b + 1] - h0;
+        if (s != e) f = plan_flags(c, b, s, e);
+    }
+    const uint32_t m = __ballot_sync(FULLG, f & 1u);
+    if (lane == 0) ws[warp] = (uint32_t)__popc(m);
+    __syncthreads();
+    if (b >= c.hi) return;
+    uint32_t u = (uint32_t)blk[blockIdx.x] + (uint32_t)__popc(m & ((1u << lane) - 1));  // units that start before b
+    for (int w = 0; w < warp; w++) u += ws[w];
+    const uint32_t seg = (uint32_t)(b / NB), rel = ((uint32_t)b & (NB - 1)) - c.seg_lo, sh = c.seg_sh[seg];
+    if ((rel & ((1u << sh) - 1)) == 0) {
+        const uint32_t bin = c.seg_bin0[seg] + (rel >> sh);
+        bstart[bin] = bcur[bin] = (uint32_t)s;
+        bu0[bin] = u;
+        bfirst[bin] = (uint32_t)(b - c.lo);
+        bsh[bin] = sh;
+    }
+    unit_of[b - c.lo] = u + (f & 1u) - 1u;  // (before the first unit: ~0)
+    if (f & 1u) {
+        ustart[u] = ucur[u] = (uint32_t)s;
+        ub0[u] = (uint32_t)b | (f & 8u ? 0x80000000u : 0u);
+    }
+    if (e - s > (uint64_t)GP_CAP_S) {
+        if (e - s <= (uint64_t)GP_CAP_L) mid[atomicAdd(&ctr[GC_MID], 1u)] = u;
+        else {
+            big[atomicAdd(&ctr[GC_BIG], 1u)] = u;
+            atomicAdd(&ctr[GC_BIG_TUPLES], (uint32_t)(e - s));
         }
     }
 }
@@ -1067,9 +1063,9 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
     MP_CUDA(cudaMemcpyAsync(g.seg_bin0, h.data(), h.size() * 4, cudaMemcpyHostToDevice, st));
     const PlanCtx c{g.d_hist, g.lo, g.hi, brk, g.seg_sh, g.seg_bin0, g.seg_lo};
     (count_launch(), k_gp_marks<<<blocks_of(nbounds, 64), 64, 0, st>>>(g.d_hist, g.lo, g.hi, d_bounds, (int)nbounds, brk));
-    (count_launch(), k_gp_count<<<nblk, GP_COUNT_THREADS, 0, st>>>(c, blk));
+    (count_launch(), k_gp_count<<<nblk, GP_COUNT_BLOCK, 0, st>>>(c, blk));
     (count_launch(), k_gp_scan<<<1, 1024, 0, st>>>(blk, nblk, (uint32_t)g.n, g.bins, g.ctr, g.ustart, g.bstart, g.bu0));
-    (count_launch(), k_gp_write<<<nblk, GP_COUNT_THREADS, 0, st>>>(c, blk, g.ctr, g.ustart, g.ub0, g.ucur, g.bstart, g.bu0, g.bcur,
+    (count_launch(), k_gp_write<<<nblk, GP_COUNT_BLOCK, 0, st>>>(c, blk, g.ctr, g.ustart, g.ub0, g.ucur, g.bstart, g.bu0, g.bcur,
                                                                   g.bin_sh, g.bfirst, g.unit_of, g.mid, g.big));
     (count_launch(), k_gp_tiles<<<1, 1024, 0, st>>>(g.bstart, g.bins, g.ctr, g.tiles));
     ReadBack<uint32_t> rb(arena, GC_N, PLAN_MAIL);

@@ -4,12 +4,11 @@
 // component root falls in the partition's read-id range, written by thread tid (the
 // thread owning the record's chunk).  An interleaved pair is written to the partition of
 // mate 1's root and, when mate 2's root differs, again to mate 2's (:1006-1047).  On the
-// GPU each (file, unit) entry is generated in input order, entries are stably sorted by
-// file, their byte offsets come from one exclusive scan, and a warp copies each record.
+// GPU the entries take their places by one stable partition into the 16 parts (OutBlock), and a warp
+// copies each record.
 #include <algorithm>
 
 #include "k_output.cuh"
-#include "k_sort.cuh"
 
 namespace mp {
 
@@ -22,83 +21,221 @@ __device__ __forceinline__ uint32_t part_of(const uint64_t *bounds, uint32_t roo
 
 struct OutCtx {
     const uint64_t *rec_start;
-    const uint32_t *label;
-    const uint64_t *bounds;    // 17
-    const uint64_t *chunk_rec; // nchunks + 1
-    int nchunks, T, per_thread, interleaved;
-    uint64_t units;
+    int interleaved;
 };
 
-__device__ __forceinline__ uint32_t tid_of(const OutCtx &c, uint64_t rec)
+// The plan's input: samples one after another in the reads (one for a job); sample q's files are the global files
+// file0[q] + part * T[q] + tid, its blocks (of OP_UNITS units, a unit being a read or an interleaved pair) blk0[q] on.
+struct OutPlanCtx {
+    const uint64_t *rec_start;
+    const uint32_t *label;
+    const uint64_t *srec;       // nseg + 1 read offsets
+    const uint64_t *bounds;     // nseg x 17, each sample's own read ids
+    const uint64_t *chunk_rec;  // every sample's nchunks + 1 chunk record starts (its own read ids), one after another
+    const uint32_t *chunk0;     // nseg + 1: where each sample's chunk records start in chunk_rec
+    const uint32_t *T, *per_thread, *file0, *blk0;  // per sample (blk0: nseg + 1)
+    int nseg, interleaved;
+};
+
+constexpr int OP_THREADS = 256, OP_ROUNDS = 4, OP_UNITS = OP_THREADS * OP_ROUNDS;
+
+// The file order is part, then thread, then input order, and a record's thread never falls as the records go on (threads
+// own consecutive chunks): the entries of a file are the part's entries in input order, cut at the threads' first
+// records.  So the layout is one stable partition into 16 parts: the blocks' entries and bytes per part, scanned in (part,
+// block) order, and then every entry's place.  (Sorted by file with the radix sort: 10 launches and a host wait more.)
+struct OutBlock {
+    uint64_t len[OP_ROUNDS];             // bytes of this lane's unit of every round
+    uint32_t p0[OP_ROUNDS], p1[OP_ROUNDS];  // its parts: one (p1 = 16) or, mates in two components, two
+    uint32_t seg, blk, nblk;             // the block's sample, its number in the sample and the sample's blocks
+    uint64_t u0;                         // lane's first unit (round r: u0 + 32 r) in all reads' units
+};
+
+__device__ __forceinline__ uint32_t tid_of(const OutPlanCtx &c, uint32_t q, uint64_t lr)
 {
-    int lo = 0, hi = c.nchunks - 1;
+    const uint64_t *cr = c.chunk_rec + c.chunk0[q];
+    int lo = 0, hi = (int)(c.chunk0[q + 1] - c.chunk0[q]) - 2;  // the sample's chunk holding lr
     while (lo < hi) {
-        int m = (lo + hi + 1) >> 1;
-        if (c.chunk_rec[m] <= rec) lo = m; else hi = m - 1;
+        const int m = (lo + hi + 1) >> 1;
+        if (cr[m] <= lr) lo = m; else hi = m - 1;
     }
-    return (uint32_t)(lo / c.per_thread);
+    return (uint32_t)lo / c.per_thread[q];
 }
 
-// entries per unit (1 or 2) and the file of each
-__global__ void k_out_dest(OutCtx c, uint32_t *nent, uint32_t *f1, uint32_t *f2)
+__device__ __forceinline__ void out_block(const OutPlanCtx &c, OutBlock &o)
 {
-    const uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= c.units) return;
-    const uint64_t r = c.interleaved ? 2 * u : u;
-    const uint32_t t = tid_of(c, r);
-    const uint32_t pu = c.label[r];
-    f1[u] = part_of(c.bounds, pu) * c.T + t;
-    uint32_t ne = 1;
-    if (c.interleaved) {
-        const uint32_t pv = c.label[r + 1];
-        if (pu != pv) {
-            f2[u] = part_of(c.bounds, pv) * c.T + t;
-            ne = 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int lo = 0, hi = c.nseg - 1;  // the last sample whose blocks start at or below this one
+    while (lo < hi) {
+        const int m = (lo + hi + 1) >> 1;
+        if (c.blk0[m] <= blockIdx.x) lo = m; else hi = m - 1;
+    }
+    o.seg = (uint32_t)lo;
+    o.blk = blockIdx.x - c.blk0[lo];
+    o.nblk = c.blk0[lo + 1] - c.blk0[lo];
+    const int il = c.interleaved ? 1 : 0;
+    const uint64_t R = c.srec[lo], units = (c.srec[lo + 1] - R) >> il, first = (uint64_t)o.blk * OP_UNITS + warp * (32 * OP_ROUNDS) + lane;
+    const uint64_t *b = c.bounds + (uint64_t)lo * 17;
+    o.u0 = (R >> il) + first;
+#pragma unroll
+    for (int r = 0; r < OP_ROUNDS; r++) {
+        o.len[r] = 0;
+        o.p0[r] = o.p1[r] = 16;
+        if (first + 32 * r >= units) continue;
+        const uint64_t u = R + ((first + 32 * r) << il);
+        o.len[r] = c.rec_start[u + 1 + il] - c.rec_start[u];
+        const uint32_t pu = c.label[u];
+        o.p0[r] = part_of(b, (uint32_t)(pu - R));
+        if (il) {
+            const uint32_t pv = c.label[u + 1];
+            if (pu != pv) o.p1[r] = part_of(b, (uint32_t)(pv - R));
         }
     }
-    nent[u] = ne;
 }
 
-__global__ void k_out_entries(OutCtx c, const uint32_t *f1, const uint32_t *f2, const uint32_t *nent,
-                              const uint64_t *eoff, uint64_t *key, uint32_t *val)
+// Sums over the lanes up to and including this one.
+__device__ __forceinline__ uint64_t lanes_scan(uint64_t x, bool small)
 {
-    const uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= c.units) return;
-    const uint64_t o = eoff[u];
-    key[o] = f1[u];
-    val[o] = (uint32_t)u;
-    if (nent[u] == 2) {
-        key[o + 1] = f2[u];
-        val[o + 1] = (uint32_t)u;
-    }
-}
-
-// Entry lengths; file sizes by one atomic per file and warp (entries are sorted by file, so a
-// warp's lanes of one file are contiguous: the last lane adds its segment of an inclusive scan).
-__global__ void k_out_len(OutCtx c, const uint32_t *val, uint64_t n, uint64_t *len, const uint64_t *key,
-                          unsigned long long *file_bytes)
-{
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    const bool v = i < n;
-    uint64_t l = 0, f = ~0ull;
-    if (v) {
-        const uint64_t u = val[i];
-        const uint64_t r0 = c.interleaved ? 2 * u : u, r1 = c.interleaved ? 2 * u + 2 : u + 1;
-        l = c.rec_start[r1] - c.rec_start[r0];
-        len[i] = l;
-        f = key[i];
+    if (small) {
+        uint32_t v = (uint32_t)x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+            if (lane >= o) v += y;
+        }
+        return v;
     }
-    uint64_t incl = l;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint64_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += y;
+        const uint64_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
     }
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, f);
-    const int first = __ffs(peers) - 1, last = 31 - __clz(peers);
-    const uint64_t before = __shfl_sync(0xFFFFFFFFu, incl, first > 0 ? first - 1 : 0);
-    if (v && lane == last) atomicAdd(&file_bytes[f], (unsigned long long)(incl - (first > 0 ? before : 0)));
+    return x;
+}
+
+// Walks a warp's units part by part: f(round, part, lane's entries, entries before the lane, bytes before it, the warp's
+// entries and bytes) with the counts of one round.
+template <class F> __device__ __forceinline__ void out_walk(const OutBlock &o, F f)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int r = 0; r < OP_ROUNDS; r++) {
+        const bool small = !__any_sync(0xFFFFFFFFu, o.len[r] >= (1ull << 25));
+        const bool two = __any_sync(0xFFFFFFFFu, o.p1[r] < 16);
+        uint32_t left = __reduce_or_sync(0xFFFFFFFFu, (1u << o.p0[r]) | (1u << o.p1[r])) & 0xFFFFu;
+        while (left) {
+            const uint32_t p = __ffs(left) - 1;
+            left &= left - 1;
+            const uint32_t n = (o.p0[r] == p ? 1u : 0u) + (o.p1[r] == p ? 1u : 0u);
+            const uint64_t b = lanes_scan(n * o.len[r], small);
+            uint32_t e;
+            if (two) {
+                e = (uint32_t)lanes_scan(n, true);
+            } else {
+                e = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, n) & ((2u << lane) - 1));
+            }
+            f(r, p, n, e - n, b - n * o.len[r], __shfl_sync(0xFFFFFFFFu, e, 31), __shfl_sync(0xFFFFFFFFu, b, 31));
+        }
+    }
+}
+
+// Entries and bytes of every (part, block), and the files' sizes.
+__global__ void __launch_bounds__(OP_THREADS) k_out_count(OutPlanCtx c, uint32_t *cnt, uint64_t *bytes, unsigned long long *file_bytes)
+{
+    __shared__ uint32_t se[OP_THREADS / 32][16];
+    __shared__ uint64_t sb[OP_THREADS / 32][16];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < (OP_THREADS / 32) * 16; i += OP_THREADS) {
+        (&se[0][0])[i] = 0;
+        (&sb[0][0])[i] = 0;
+    }
+    __syncthreads();
+    OutBlock o;
+    out_block(c, o);
+    const uint64_t units = (c.srec[o.seg + 1] - c.srec[o.seg]) >> (c.interleaved ? 1 : 0), b0 = (uint64_t)o.blk * OP_UNITS;
+    const uint32_t T = c.T[o.seg];
+    const uint32_t ta = tid_of(c, o.seg, b0 << c.interleaved), tz = tid_of(c, o.seg, (min(units, b0 + OP_UNITS) - 1) << c.interleaved);
+    out_walk(o, [&](int, uint32_t p, uint32_t, uint32_t, uint64_t, uint32_t e, uint64_t b) {
+        if (lane == 0) {
+            se[warp][p] += e;
+            sb[warp][p] += b;
+        }
+    });
+    if (ta != tz) {  // a thread's first record lies in the block: its files' bytes unit by unit
+#pragma unroll
+        for (int r = 0; r < OP_ROUNDS; r++) {
+            if (o.p0[r] == 16) continue;
+            const uint32_t f = c.file0[o.seg] + tid_of(c, o.seg, (o.u0 + 32 * r - (c.srec[o.seg] >> c.interleaved)) << c.interleaved);
+            atomicAdd(&file_bytes[f + o.p0[r] * T], (unsigned long long)o.len[r]);
+            if (o.p1[r] < 16) atomicAdd(&file_bytes[f + o.p1[r] * T], (unsigned long long)o.len[r]);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 16) {
+        const uint32_t p = threadIdx.x;
+        uint32_t e = 0;
+        uint64_t b = 0;
+        for (int w = 0; w < OP_THREADS / 32; w++) {
+            e += se[w][p];
+            b += sb[w][p];
+        }
+        const size_t cell = 16 * (size_t)c.blk0[o.seg] + (size_t)p * o.nblk + o.blk;
+        cnt[cell] = e;
+        bytes[cell] = b;
+        if (ta == tz && b) atomicAdd(&file_bytes[c.file0[o.seg] + p * T + ta], (unsigned long long)b);
+    }
+}
+
+// Every entry's unit and byte offset at its place.
+__global__ void __launch_bounds__(OP_THREADS) k_out_place(OutPlanCtx c, const uint64_t *cell_e, const uint64_t *cell_b, uint32_t *val,
+                                                          uint64_t *off)
+{
+    __shared__ uint32_t se[OP_THREADS / 32][16];
+    __shared__ uint64_t sb[OP_THREADS / 32][16], be[16];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < (OP_THREADS / 32) * 16; i += OP_THREADS) {
+        (&se[0][0])[i] = 0;
+        (&sb[0][0])[i] = 0;
+    }
+    __syncthreads();
+    OutBlock o;
+    out_block(c, o);
+    out_walk(o, [&](int, uint32_t p, uint32_t, uint32_t, uint64_t, uint32_t e, uint64_t b) {
+        if (lane == 0) {
+            se[warp][p] += e;
+            sb[warp][p] += b;
+        }
+    });
+    __syncthreads();
+    if (threadIdx.x < 16) {  // the warps' first places
+        const uint32_t p = threadIdx.x;
+        const size_t cell = 16 * (size_t)c.blk0[o.seg] + (size_t)p * o.nblk + o.blk;
+        uint32_t e = 0;
+        uint64_t b = cell_b[cell];
+        be[p] = cell_e[cell];
+        for (int w = 0; w < OP_THREADS / 32; w++) {
+            const uint32_t x = se[w][p];
+            const uint64_t y = sb[w][p];
+            se[w][p] = e;
+            sb[w][p] = b;
+            e += x;
+            b += y;
+        }
+    }
+    __syncthreads();
+    out_walk(o, [&](int r, uint32_t p, uint32_t n, uint32_t e, uint64_t b, uint32_t we, uint64_t wb) {
+        const uint64_t ew = be[p] + se[warp][p], bw = sb[warp][p];
+        for (uint32_t q = 0; q < n; q++) {
+            val[ew + e + q] = (uint32_t)(o.u0 + 32 * r);
+            off[ew + e + q] = bw + b + q * o.len[r];
+        }
+        __syncwarp();
+        if (lane == 0) {
+            se[warp][p] += we;
+            sb[warp][p] += wb;
+        }
+        __syncwarp();
+    });
 }
 
 // One record (l bytes at fq + s) to out + o by a warp.
@@ -148,120 +285,10 @@ int plan_output(const uint8_t *d_fq, const ParsedReads &pr, const uint32_t *d_la
                 std::vector<uint64_t> &file_sizes, DeviceArena &arena, cudaStream_t st)
 {
     (void)d_fq;
-    const uint64_t units = interleaved ? pr.n_reads / 2 : pr.n_reads;
-    const int nf = 16 * T;
-    file_sizes.assign(nf, 0);
-    OutCtx c;
-    c.rec_start = pr.rec_start;
-    c.label = d_label;
-    c.nchunks = nchunks;
-    c.T = T;
-    c.per_thread = nchunks / T;
-    c.interleaved = interleaved;
-    c.units = units;
-    uint64_t *bounds = arena.alloc<uint64_t>(17), *chunk_rec = arena.alloc<uint64_t>(nchunks + 1);
-    uint32_t *nent = arena.alloc<uint32_t>(units + 1), *f1 = arena.alloc<uint32_t>(units + 1),
-             *f2 = arena.alloc<uint32_t>(units + 1);
-    uint64_t *eoff = arena.alloc<uint64_t>(units + 1), *ntot = arena.alloc<uint64_t>(1);
-    unsigned long long *fbytes = arena.alloc<unsigned long long>(nf);
-    size_t tb = scan_tmp_bytes(2 * units + 2);
-    void *tmp = arena.alloc<uint8_t>(tb);
-    if (!bounds || !chunk_rec || !nent || !f1 || !f2 || !eoff || !ntot || !fbytes || !tmp)
-        return set_error(MP_ENOMEM, "device memory for the output gather");
-    MP_CUDA(cudaMemcpyAsync(bounds, bounds_host, 17 * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    MP_CUDA(cudaMemcpyAsync(chunk_rec, chunk_rec_host, (nchunks + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    MP_CUDA(cudaMemsetAsync(fbytes, 0, nf * sizeof(unsigned long long), st));
-    c.bounds = bounds;
-    c.chunk_rec = chunk_rec;
-    const unsigned gb = (unsigned)((units + 255) / 256);
-    (mp::count_launch(), k_out_dest<<<gb, 256, 0, st>>>(c, nent, f1, f2));
-    scan_u32_to_u64(nent, eoff, units, ntot, tmp, tb, st);
-    ReadBack<uint64_t> rb(arena, nf + 1);
-    MP_CUDA(cudaMemcpyAsync(rb.p, ntot, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    MP_CUDA(cudaStreamSynchronize(st));
-    const uint64_t n = rb[0];
-    SortBufs sb;
-    for (int i = 0; i < 2; i++) {
-        sb.lo[i] = arena.alloc<uint64_t>(n + 1);
-        sb.id[i] = arena.alloc<uint32_t>(n + 1);
-        if (!sb.lo[i] || !sb.id[i]) return set_error(MP_ENOMEM, "device memory for the output entries");
-    }
-    (mp::count_launch(), k_out_entries<<<gb, 256, 0, st>>>(c, f1, f2, nent, eoff, sb.lo[0], sb.id[0]));
-    int rc = radix_sort(sb, n, false, arena, st, nullptr);
-    if (rc) return rc;
-    uint64_t *len = arena.alloc<uint64_t>(n + 1);
-    plan->val = arena.alloc_persistent<uint32_t>(n + 1);
-    plan->off = arena.alloc_persistent<uint64_t>(n + 1);
-    size_t tb2 = scan_tmp_bytes(n + 1);
-    void *tmp2 = arena.alloc<uint8_t>(tb2);
-    if (!len || !plan->val || !plan->off || !tmp2) return set_error(MP_ENOMEM, "device memory for the output offsets");
-    const unsigned ge = (unsigned)((n + 255) / 256);
-    (mp::count_launch(), k_out_len<<<ge, 256, 0, st>>>(c, sb.id[sb.cur], n, len, sb.lo[sb.cur], fbytes));
-    scan_u64(len, plan->off, n, ntot, tmp2, tb2, st);
-    MP_CUDA(cudaMemcpyAsync(plan->val, sb.id[sb.cur], n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
-    MP_CUDA(cudaMemcpyAsync(rb.p, ntot, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    MP_CUDA(cudaMemcpyAsync(rb.p + 1, fbytes, nf * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    MP_CUDA(cudaStreamSynchronize(st));
-    MP_CUDA(cudaGetLastError());
-    const uint64_t total = rb[0];
-    std::copy(rb.p + 1, rb.p + 1 + nf, file_sizes.begin());
-    plan->n = n;
-    plan->total = total;
-    plan->rec_start = pr.rec_start;
-    plan->interleaved = interleaved;
-    return 0;
-}
-
-// ------------------------------------------------------ batches of samples
-
-// Samples one after another in the read ids; sample q's files are the global files file0[q] + j.
-struct BatchOutCtx {
-    const uint32_t *label;
-    const uint64_t *srec;       // nseg + 1 read offsets
-    const uint64_t *bounds;     // nseg x 17, each sample's own read ids
-    const uint64_t *chunk_rec;  // every sample's nchunks + 1 chunk record starts (its own read ids), one after another
-    const uint32_t *chunk0;     // nseg + 1: where each sample's chunk records start in chunk_rec
-    const uint32_t *T, *per_thread, *file0;  // per sample
-    int nseg, interleaved;
-    uint64_t units;
-};
-
-__device__ __forceinline__ uint32_t seg_of(const uint64_t *srec, int nseg, uint64_t r)
-{
-    int lo = 0, hi = nseg - 1;  // the last sample starting at or below r
-    while (lo < hi) {
-        const int m = (lo + hi + 1) >> 1;
-        if (srec[m] <= r) lo = m; else hi = m - 1;
-    }
-    return (uint32_t)lo;
-}
-
-__global__ void k_outb_dest(BatchOutCtx c, uint32_t *nent, uint32_t *f1, uint32_t *f2)
-{
-    const uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= c.units) return;
-    const uint64_t r = c.interleaved ? 2 * u : u;
-    const uint32_t q = seg_of(c.srec, c.nseg, r);
-    const uint64_t R = c.srec[q], lr = r - R;
-    const uint64_t *cr = c.chunk_rec + c.chunk0[q];
-    int lo = 0, hi = (int)(c.chunk0[q + 1] - c.chunk0[q]) - 2;  // the sample's chunk holding lr
-    while (lo < hi) {
-        const int m = (lo + hi + 1) >> 1;
-        if (cr[m] <= lr) lo = m; else hi = m - 1;
-    }
-    const uint32_t t = (uint32_t)lo / c.per_thread[q], T = c.T[q];
-    const uint64_t *b = c.bounds + (uint64_t)q * 17;
-    const uint32_t pu = c.label[r];
-    f1[u] = c.file0[q] + part_of(b, (uint32_t)(pu - R)) * T + t;
-    uint32_t ne = 1;
-    if (c.interleaved) {
-        const uint32_t pv = c.label[r + 1];
-        if (pu != pv) {
-            f2[u] = c.file0[q] + part_of(b, (uint32_t)(pv - R)) * T + t;
-            ne = 2;
-        }
-    }
-    nent[u] = ne;
+    std::vector<uint64_t> file0;
+    return plan_output_batch(pr, d_label, interleaved, {0, pr.n_reads}, std::vector<uint64_t>(bounds_host, bounds_host + 17),
+                             {std::vector<uint64_t>(chunk_rec_host, chunk_rec_host + nchunks + 1)}, {T}, plan, file_sizes, file0,
+                             arena, st);
 }
 
 int plan_output_batch(const ParsedReads &pr, const uint32_t *d_label, int interleaved, const std::vector<uint64_t> &seg_reads,
@@ -270,93 +297,73 @@ int plan_output_batch(const ParsedReads &pr, const uint32_t *d_label, int interl
                       std::vector<uint64_t> &file0, DeviceArena &arena, cudaStream_t st)
 {
     const int nseg = (int)seg_reads.size() - 1;
-    const uint64_t units = interleaved ? pr.n_reads / 2 : pr.n_reads;
-    std::vector<uint32_t> c0(nseg + 1, 0), hT(nseg), hpt(nseg), hf0(nseg);
-    std::vector<uint64_t> crec;
+    // 64-bit words, then 32-bit ones, in one upload: read offsets, bounds, chunk records; chunk0, blk0, T, per_thread, file0
+    std::vector<uint64_t> w(seg_reads.begin(), seg_reads.end());
+    w.insert(w.end(), bounds_host.begin(), bounds_host.end());
+    const size_t at_cr = w.size();
+    std::vector<uint32_t> v(5 * (size_t)nseg + 2);
+    uint32_t *c0 = v.data(), *blk0 = c0 + nseg + 1, *hT = blk0 + nseg + 1, *hpt = hT + nseg, *hf0 = hpt + nseg;
     file0.assign(nseg + 1, 0);
+    uint64_t blocks = 0, ncr = 0;
     for (int q = 0; q < nseg; q++) {
         const int nch = (int)chunk_rec_host[q].size() - 1;
         if (nch < 1 || T[q] < 1 || nch % T[q]) return set_error(MP_EARG, "sample %d: numThreads must divide its chunks", q);
-        c0[q] = (uint32_t)crec.size();
-        crec.insert(crec.end(), chunk_rec_host[q].begin(), chunk_rec_host[q].end());
+        c0[q] = (uint32_t)ncr;
+        ncr += chunk_rec_host[q].size();
+        w.insert(w.end(), chunk_rec_host[q].begin(), chunk_rec_host[q].end());
+        blk0[q] = (uint32_t)blocks;
+        blocks += ((seg_reads[q + 1] - seg_reads[q]) / (interleaved ? 2 : 1) + OP_UNITS - 1) / OP_UNITS;
         hT[q] = (uint32_t)T[q];
         hpt[q] = (uint32_t)(nch / T[q]);
         hf0[q] = (uint32_t)file0[q];
         file0[q + 1] = file0[q] + 16ull * (uint64_t)T[q];
     }
-    c0[nseg] = (uint32_t)crec.size();
-    const uint64_t nf = file0[nseg];
+    c0[nseg] = (uint32_t)ncr;
+    blk0[nseg] = (uint32_t)blocks;
+    const uint64_t nf = file0[nseg], cells = 16 * blocks, units = seg_reads[nseg] / (interleaved ? 2 : 1);
     file_sizes.assign(nf, 0);
-    uint64_t *srec = arena.alloc<uint64_t>(nseg + 1), *bnd = arena.alloc<uint64_t>((size_t)nseg * 17);
-    uint64_t *dcr = arena.alloc<uint64_t>(crec.size());
-    uint32_t *dc0 = arena.alloc<uint32_t>(nseg + 1), *dT = arena.alloc<uint32_t>(nseg), *dpt = arena.alloc<uint32_t>(nseg),
-             *df0 = arena.alloc<uint32_t>(nseg);
-    uint32_t *nent = arena.alloc<uint32_t>(units + 1), *f1 = arena.alloc<uint32_t>(units + 1),
-             *f2 = arena.alloc<uint32_t>(units + 1);
-    uint64_t *eoff = arena.alloc<uint64_t>(units + 1), *ntot = arena.alloc<uint64_t>(1);
-    unsigned long long *fbytes = arena.alloc<unsigned long long>(nf);
-    size_t tb = scan_tmp_bytes(2 * units + 2);
+    const size_t n64 = w.size();
+    w.resize(n64 + (v.size() + 1) / 2);
+    std::copy(v.begin(), v.end(), reinterpret_cast<uint32_t *>(w.data() + n64));
+    uint64_t *dw = arena.alloc<uint64_t>(w.size());
+    uint32_t *cnt = arena.alloc<uint32_t>(cells + 1);
+    uint64_t *bytes = arena.alloc<uint64_t>(cells + 1), *cell_e = arena.alloc<uint64_t>(cells + 1), *cell_b = arena.alloc<uint64_t>(cells + 1);
+    unsigned long long *tail = arena.alloc<unsigned long long>(nf + 2);  // total entries and bytes, then the file sizes
+    const size_t tb = scan_tmp_bytes(cells + 1);
     void *tmp = arena.alloc<uint8_t>(tb);
-    if (!srec || !bnd || !dcr || !dc0 || !dT || !dpt || !df0 || !nent || !f1 || !f2 || !eoff || !ntot || !fbytes || !tmp)
-        return set_error(MP_ENOMEM, "device memory for the output gather");
-    MP_CUDA(cudaMemcpyAsync(srec, seg_reads.data(), (nseg + 1) * 8, cudaMemcpyHostToDevice, st));
-    MP_CUDA(cudaMemcpyAsync(bnd, bounds_host.data(), (size_t)nseg * 17 * 8, cudaMemcpyHostToDevice, st));
-    MP_CUDA(cudaMemcpyAsync(dcr, crec.data(), crec.size() * 8, cudaMemcpyHostToDevice, st));
-    MP_CUDA(cudaMemcpyAsync(dc0, c0.data(), (nseg + 1) * 4, cudaMemcpyHostToDevice, st));
-    MP_CUDA(cudaMemcpyAsync(dT, hT.data(), nseg * 4, cudaMemcpyHostToDevice, st));
-    MP_CUDA(cudaMemcpyAsync(dpt, hpt.data(), nseg * 4, cudaMemcpyHostToDevice, st));
-    MP_CUDA(cudaMemcpyAsync(df0, hf0.data(), nseg * 4, cudaMemcpyHostToDevice, st));
-    MP_CUDA(cudaMemsetAsync(fbytes, 0, nf * sizeof(unsigned long long), st));
-    BatchOutCtx bc;
-    bc.label = d_label;
-    bc.srec = srec;
-    bc.bounds = bnd;
-    bc.chunk_rec = dcr;
-    bc.chunk0 = dc0;
-    bc.T = dT;
-    bc.per_thread = dpt;
-    bc.file0 = df0;
-    bc.nseg = nseg;
-    bc.interleaved = interleaved;
-    bc.units = units;
-    OutCtx c{};
+    const uint64_t most = units * (interleaved ? 2 : 1);  // entries at most
+    plan->val = arena.alloc_persistent<uint32_t>(most + 1);
+    plan->off = arena.alloc_persistent<uint64_t>(most + 1);
+    if (!dw || !cnt || !bytes || !cell_e || !cell_b || !tail || !tmp || !plan->val || !plan->off)
+        return set_error(MP_ENOMEM, "device memory for the output plan");
+    MP_CUDA(cudaMemcpyAsync(dw, w.data(), w.size() * 8, cudaMemcpyHostToDevice, st));
+    MP_CUDA(cudaMemsetAsync(tail, 0, (nf + 2) * sizeof(unsigned long long), st));
+    OutPlanCtx c;
     c.rec_start = pr.rec_start;
-    c.interleaved = interleaved;
-    c.units = units;
-    const unsigned gb = (unsigned)((units + 255) / 256);
-    if (units) (mp::count_launch(), k_outb_dest<<<gb, 256, 0, st>>>(bc, nent, f1, f2));
-    scan_u32_to_u64(nent, eoff, units, ntot, tmp, tb, st);
-    ReadBack<uint64_t> rb(arena, nf + 1);
-    MP_CUDA(cudaMemcpyAsync(rb.p, ntot, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    MP_CUDA(cudaStreamSynchronize(st));
-    const uint64_t n = rb[0];
-    SortBufs sb;
-    for (int i = 0; i < 2; i++) {
-        sb.lo[i] = arena.alloc<uint64_t>(n + 1);
-        sb.id[i] = arena.alloc<uint32_t>(n + 1);
-        if (!sb.lo[i] || !sb.id[i]) return set_error(MP_ENOMEM, "device memory for the output entries");
+    c.label = d_label;
+    c.srec = dw;
+    c.bounds = dw + nseg + 1;
+    c.chunk_rec = dw + at_cr;
+    c.chunk0 = reinterpret_cast<uint32_t *>(dw + n64);
+    c.blk0 = c.chunk0 + nseg + 1;
+    c.T = c.blk0 + nseg + 1;
+    c.per_thread = c.T + nseg;
+    c.file0 = c.per_thread + nseg;
+    c.nseg = nseg;
+    c.interleaved = interleaved ? 1 : 0;
+    if (blocks) {
+        (mp::count_launch(), k_out_count<<<(unsigned)blocks, OP_THREADS, 0, st>>>(c, cnt, bytes, tail + 2));
+        scan_u32_to_u64(cnt, cell_e, cells, (uint64_t *)tail, tmp, tb, st);
+        scan_u64(bytes, cell_b, cells, (uint64_t *)tail + 1, tmp, tb, st);
+        (mp::count_launch(), k_out_place<<<(unsigned)blocks, OP_THREADS, 0, st>>>(c, cell_e, cell_b, plan->val, plan->off));
     }
-    if (units) (mp::count_launch(), k_out_entries<<<gb, 256, 0, st>>>(c, f1, f2, nent, eoff, sb.lo[0], sb.id[0]));
-    int rc = radix_sort(sb, n, false, arena, st, nullptr);
-    if (rc) return rc;
-    uint64_t *len = arena.alloc<uint64_t>(n + 1);
-    plan->val = arena.alloc_persistent<uint32_t>(n + 1);
-    plan->off = arena.alloc_persistent<uint64_t>(n + 1);
-    size_t tb2 = scan_tmp_bytes(n + 1);
-    void *tmp2 = arena.alloc<uint8_t>(tb2);
-    if (!len || !plan->val || !plan->off || !tmp2) return set_error(MP_ENOMEM, "device memory for the output offsets");
-    const unsigned ge = (unsigned)((n + 255) / 256);
-    if (n) (mp::count_launch(), k_out_len<<<ge, 256, 0, st>>>(c, sb.id[sb.cur], n, len, sb.lo[sb.cur], fbytes));
-    scan_u64(len, plan->off, n, ntot, tmp2, tb2, st);
-    if (n) MP_CUDA(cudaMemcpyAsync(plan->val, sb.id[sb.cur], n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
-    MP_CUDA(cudaMemcpyAsync(rb.p, ntot, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    MP_CUDA(cudaMemcpyAsync(rb.p + 1, fbytes, nf * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    ReadBack<uint64_t> rb(arena, nf + 2);
+    MP_CUDA(cudaMemcpyAsync(rb.p, tail, (nf + 2) * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
     MP_CUDA(cudaGetLastError());
-    const uint64_t total = rb[0];
-    std::copy(rb.p + 1, rb.p + 1 + nf, file_sizes.begin());
-    plan->n = n;
-    plan->total = total;
+    std::copy(rb.p + 2, rb.p + 2 + nf, file_sizes.begin());
+    plan->n = rb[0];
+    plan->total = rb[1];
     plan->rec_start = pr.rec_start;
     plan->interleaved = interleaved;
     return 0;

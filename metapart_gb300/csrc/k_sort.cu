@@ -359,10 +359,24 @@ int count_unsorted(const uint64_t *lo, const uint8_t *hi, uint64_t n, unsigned l
     return 0;
 }
 
-int radix_sort(SortBufs &b, uint64_t n, bool has_hi, DeviceArena &arena, cudaStream_t st, SortStats *stats)
+static int copy_tuples(const SortInput &in, SortBufs &b, int to, uint64_t n, cudaStream_t st)
+{
+    b.cur = to;
+    if (!n) return 0;
+    MP_CUDA(cudaMemcpyAsync(b.lo[to], in.lo, n * 8, cudaMemcpyDeviceToDevice, st));
+    MP_CUDA(cudaMemcpyAsync(b.id[to], in.id, n * 4, cudaMemcpyDeviceToDevice, st));
+    if (in.hi) MP_CUDA(cudaMemcpyAsync(b.hi[to], in.hi, n, cudaMemcpyDeviceToDevice, st));
+    return 0;
+}
+
+int radix_sort(SortBufs &b, uint64_t n, bool has_hi, DeviceArena &arena, cudaStream_t st, SortStats *stats, const SortInput *from)
 {
     if (stats) *stats = SortStats{};
-    if (n <= 1) return 0;
+    const SortInput in = from ? *from : SortInput{b.lo[b.cur], has_hi ? b.hi[b.cur] : nullptr, b.id[b.cur]};
+    if (n <= 1) {
+        if (from) return copy_tuples(in, b, 0, n, st);
+        return 0;
+    }
     unsigned long long *ghist = arena.alloc<unsigned long long>(9 * 256);
     uint64_t *dbase = arena.alloc<uint64_t>(9 * 256);
     uint32_t *ctr = arena.alloc<uint32_t>(16);
@@ -377,7 +391,7 @@ int radix_sort(SortBufs &b, uint64_t n, bool has_hi, DeviceArena &arena, cudaStr
     Events ht(2);
     cudaEvent_t e0 = ht[0], e1 = ht[1];
     cudaEventRecord(e0, st);
-    (mp::count_launch(), k_hist_upfront<<<8 * sm_count(), 256, 0, st>>>(b.lo[b.cur], has_hi ? b.hi[b.cur] : nullptr, n, ghist));
+    (mp::count_launch(), k_hist_upfront<<<8 * sm_count(), 256, 0, st>>>(in.lo, in.hi, n, ghist));
     cudaEventRecord(e1, st);
     std::vector<unsigned long long> h(9 * 256);
     MP_CUDA(cudaMemcpyAsync(h.data(), ghist, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
@@ -401,19 +415,26 @@ int radix_sort(SortBufs &b, uint64_t n, bool has_hi, DeviceArena &arena, cudaStr
     MP_CUDA(cudaMemcpyAsync(dbase, base.data(), base.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     sort_kernel_attrs();
     const uint32_t pf = onesweep_prefetch_tiles();
+    if (from) {  // the last pass ends in buffer 0
+        b.cur = (int)(passes.size() & 1);
+        if (passes.empty()) {
+            const int rc = copy_tuples(in, b, 0, n, st);
+            if (rc) return rc;
+        }
+    }
     Events ev(passes.size() + 1);
     cudaEventRecord(ev[0], st);
     for (size_t pi = 0; pi < passes.size(); pi++) {
         const int dgt = passes[pi];
         const int src = b.cur, dst = b.cur ^ 1;
-        const uint8_t *ih = has_hi ? b.hi[src] : nullptr;
+        const SortInput s = pi ? SortInput{b.lo[src], has_hi ? b.hi[src] : nullptr, b.id[src]} : in;
         uint8_t *oh = has_hi ? b.hi[dst] : nullptr;
         if (dgt < 8)
-            (mp::count_launch(), k_onesweep<0><<<(unsigned)tiles, ST, sizeof(SortSmem), st>>>(b.lo[src], ih, b.id[src], b.lo[dst], oh,
+            (mp::count_launch(), k_onesweep<0><<<(unsigned)tiles, ST, sizeof(SortSmem), st>>>(s.lo, s.hi, s.id, b.lo[dst], oh,
                                                                          b.id[dst], n, 8 * dgt, 8, dbase + dgt * 256, nullptr, status,
                                                                          ctr + pi, (uint32_t)(pi + 1), err, pf, nullptr, Segs{}, arena.lim.lookback_spins));
         else
-            (mp::count_launch(), k_onesweep<1><<<(unsigned)tiles, ST, sizeof(SortSmem), st>>>(b.lo[src], ih, b.id[src], b.lo[dst], oh,
+            (mp::count_launch(), k_onesweep<1><<<(unsigned)tiles, ST, sizeof(SortSmem), st>>>(s.lo, s.hi, s.id, b.lo[dst], oh,
                                                                          b.id[dst], n, 0, 8, dbase + dgt * 256, nullptr, status,
                                                                          ctr + pi, (uint32_t)(pi + 1), err, pf, nullptr, Segs{}, arena.lim.lookback_spins));
         cudaEventRecord(ev[pi + 1], st);
@@ -948,25 +969,70 @@ static uint32_t onesweep_prefetch_tiles()
     return (uint32_t)w * (uint32_t)sm_count();
 }
 
-static void sort_kernel_attrs()
+
+// The listed units (start, tuples, first bucket), from buffer in to buffer out.
+template <int THREADS, int CAP, typename Smem>
+static int sort_listed_units(const std::vector<uint64_t> &us, const std::vector<uint32_t> &uc, const std::vector<uint32_t> &ub,
+                             const SortBufs &b, int in, int out, bool has_hi, int bsh, int lowbits, int unit_bits,
+                             unsigned long long *trace, DeviceArena &arena, cudaStream_t st)
 {
-    static std::once_flag once[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::call_once(once[dev & 63], [] {
-        cudaFuncSetAttribute(k_onesweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-        cudaFuncSetAttribute(k_onesweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-        cudaFuncSetAttribute(k_onesweep<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-        cudaFuncSetAttribute(k_onesweep<2, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-        cudaFuncSetAttribute(k_onesweep<2, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-        cudaFuncSetAttribute(k_onesweep<2, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-        cudaFuncSetAttribute(k_onesweep<2, 8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-        cudaFuncSetAttribute(k_onesweep<2, 7, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-        cudaFuncSetAttribute(k_onesweep<2, 6, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-        cudaFuncSetAttribute(k_onesweep<2, 5, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
-        cudaFuncSetAttribute(k_segsort<1024, SS_CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SegSmemL));
-        cudaFuncSetAttribute(k_segsort<512, SS_SMALL_CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SegSmemS));
-    });
+    const uint64_t nu = us.size();
+    uint64_t *d_us = arena.alloc<uint64_t>(nu);
+    uint32_t *d_uc = arena.alloc<uint32_t>(nu), *d_ub = arena.alloc<uint32_t>(nu);
+    if (!d_us || !d_uc || !d_ub) return set_error(MP_ENOMEM, "device memory for sort units");
+    MP_CUDA(cudaMemcpyAsync(d_us, us.data(), nu * 8, cudaMemcpyHostToDevice, st));
+    MP_CUDA(cudaMemcpyAsync(d_uc, uc.data(), nu * 4, cudaMemcpyHostToDevice, st));
+    MP_CUDA(cudaMemcpyAsync(d_ub, ub.data(), nu * 4, cudaMemcpyHostToDevice, st));
+    (mp::count_launch(), k_segsort<THREADS, CAP><<<(unsigned)std::min<uint64_t>(nu, 1024ull / THREADS * (uint64_t)sm_count()),
+                                                   THREADS, sizeof(Smem), st>>>(
+        d_us, d_uc, d_ub, (uint32_t)nu, b.lo[in], has_hi ? b.hi[in] : nullptr, b.id[in], b.lo[out], b.id[out], bsh, lowbits,
+        unit_bits, trace));
+    return 0;
+}
+
+// The oversized buckets (start, tuples, bucket; ascending): gathered, sorted together by the device-wide sort, put back.
+static int sort_big_buckets(const std::vector<uint64_t> &bs, const std::vector<uint32_t> &bc, const std::vector<uint32_t> &bb,
+                            const SortBufs &b, int in, int out, int lowbits, DeviceArena &arena, cudaStream_t st, uint64_t *nbig)
+{
+    const size_t nb = bs.size();
+    std::vector<uint64_t> bo(nb);
+    uint64_t *d_bs = arena.alloc<uint64_t>(nb), *d_bo = arena.alloc<uint64_t>(nb + 1);
+    uint32_t *d_bc = arena.alloc<uint32_t>(nb), *d_bb = arena.alloc<uint32_t>(nb);
+    if (!d_bs || !d_bo || !d_bc || !d_bb) return set_error(MP_ENOMEM, "device memory for oversized buckets");
+    MP_CUDA(cudaMemcpyAsync(d_bs, bs.data(), nb * 8, cudaMemcpyHostToDevice, st));
+    MP_CUDA(cudaMemcpyAsync(d_bc, bc.data(), nb * 4, cudaMemcpyHostToDevice, st));
+    MP_CUDA(cudaMemcpyAsync(d_bb, bb.data(), nb * 4, cudaMemcpyHostToDevice, st));
+    // batches of oversized buckets whose index fits above the low key bits
+    const size_t per_batch = lowbits >= 44 ? ((size_t)1 << (64 - lowbits)) : ((size_t)1 << 20);
+    uint64_t maxbatch = 0;
+    *nbig = 0;
+    for (size_t b0 = 0; b0 < nb; b0 += per_batch) {
+        uint64_t t = 0;
+        for (size_t q = b0; q < nb && q < b0 + per_batch; q++) t += bc[q];
+        if (t > maxbatch) maxbatch = t;
+        *nbig += t;
+    }
+    SortBufs t;
+    for (int q = 0; q < 2; q++) {
+        t.lo[q] = arena.alloc<uint64_t>(maxbatch + 1);
+        t.id[q] = arena.alloc<uint32_t>(maxbatch + 1);
+        if (!t.lo[q] || !t.id[q]) return set_error(MP_ENOMEM, "device memory for oversized buckets");
+    }
+    for (size_t b0 = 0; b0 < nb; b0 += per_batch) {
+        const size_t b1 = std::min<size_t>(nb, b0 + per_batch);
+        uint64_t acc = 0;
+        for (size_t q = b0; q < b1; q++) { bo[q] = acc; acc += bc[q]; }
+        MP_CUDA(cudaMemcpyAsync(d_bo + b0, bo.data() + b0, (b1 - b0) * 8, cudaMemcpyHostToDevice, st));
+        t.cur = 0;
+        (mp::count_launch(), k_big_gather<<<(unsigned)(b1 - b0), 256, 0, st>>>(d_bs + b0, d_bc + b0, d_bo + b0, b.lo[in],
+                                                                              b.id[in], t.lo[0], t.id[0], lowbits));
+        int rc = radix_sort(t, acc, false, arena, st, nullptr);
+        if (rc) return rc;
+        (mp::count_launch(), k_big_scatter<<<(unsigned)(b1 - b0), 256, 0, st>>>(d_bs + b0, d_bc + b0, d_bb + b0, d_bo + b0,
+                                                                               t.lo[t.cur], t.id[t.cur], b.lo[out],
+                                                                               b.id[out], lowbits));
+    }
+    return 0;
 }
 
 int bucket_sort(SortBufs &b, uint64_t n, bool has_hi, int k, const uint64_t *d_hist, uint64_t scan_lo, uint64_t scan_hi,
@@ -1136,10 +1202,12 @@ int bucket_sort(SortBufs &b, uint64_t n, bool has_hi, int k, const uint64_t *d_h
             lowbits, tune.unit_bits, trace));
     // buckets above a small unit: up to SS_CAP tuples each is a unit of its own for the 1024-thread blocks,
     // the rest take the device-wide sort
-    std::vector<uint32_t> bc;
+    std::vector<uint64_t> hs;
+    std::vector<uint32_t> bc, hk;
     if (nb) {
-        std::vector<uint64_t> hs(nb);
-        std::vector<uint32_t> hc(nb), hk(nb);
+        std::vector<uint32_t> hc(nb);
+        hs.resize(nb);
+        hk.resize(nb);
         MP_CUDA(cudaMemcpyAsync(hs.data(), d_bs, nb * 8, cudaMemcpyDeviceToHost, st));
         MP_CUDA(cudaMemcpyAsync(hc.data(), d_bc, nb * 4, cudaMemcpyDeviceToHost, st));
         MP_CUDA(cudaMemcpyAsync(hk.data(), d_bb, nb * 4, cudaMemcpyDeviceToHost, st));
@@ -1160,60 +1228,18 @@ int bucket_sort(SortBufs &b, uint64_t n, bool has_hi, int k, const uint64_t *d_h
         nm = ms.size();
         nb = gs.size();
         if (nm) {
-            uint64_t *d_ms = arena.alloc<uint64_t>(nm);
-            uint32_t *d_mc = arena.alloc<uint32_t>(nm), *d_mk = arena.alloc<uint32_t>(nm);
-            if (!d_ms || !d_mc || !d_mk) return set_error(MP_ENOMEM, "device memory for sort units");
-            MP_CUDA(cudaMemcpyAsync(d_ms, ms.data(), nm * 8, cudaMemcpyHostToDevice, st));
-            MP_CUDA(cudaMemcpyAsync(d_mc, mc.data(), nm * 4, cudaMemcpyHostToDevice, st));
-            MP_CUDA(cudaMemcpyAsync(d_mk, mk.data(), nm * 4, cudaMemcpyHostToDevice, st));
-            (mp::count_launch(), k_segsort<1024, SS_CAP><<<(unsigned)std::min<uint64_t>(nm, (uint64_t)sm_count()), 1024,
-                                                          sizeof(SegSmemL), st>>>(
-                d_ms, d_mc, d_mk, (uint32_t)nm, b.lo[in], has_hi ? b.hi[in] : nullptr, b.id[in], b.lo[out], b.id[out], bsh,
-                lowbits, tune.unit_bits, trace));
+            const int rc = sort_listed_units<1024, SS_CAP, SegSmemL>(ms, mc, mk, b, in, out, has_hi, bsh, lowbits, tune.unit_bits,
+                                                                     trace, arena, st);
+            if (rc) return rc;
         }
-        if (nb) {  // the oversized buckets, in order, at the front of the lists
-            MP_CUDA(cudaMemcpyAsync(d_bs, gs.data(), nb * 8, cudaMemcpyHostToDevice, st));
-            MP_CUDA(cudaMemcpyAsync(d_bc, bc.data(), nb * 4, cudaMemcpyHostToDevice, st));
-            MP_CUDA(cudaMemcpyAsync(d_bb, gk.data(), nb * 4, cudaMemcpyHostToDevice, st));
-            MP_CUDA(cudaStreamSynchronize(st));  // gs, bc and gk are host vectors of this block
-        }
+        hs.swap(gs);
+        hk.swap(gk);
     }
     cudaEventRecord(ev[2], st);
     uint64_t nbig = 0;
     if (nb) {
-        std::vector<uint64_t> bo(nb);
-        uint64_t *d_bo = arena.alloc<uint64_t>(nb + 1);
-        if (!d_bo) return set_error(MP_ENOMEM, "device memory for oversized buckets");
-        // batches of oversized buckets whose index fits above the low key bits
-        const size_t per_batch = lowbits >= 44 ? ((size_t)1 << (64 - lowbits)) : ((size_t)1 << 20);
-        uint64_t maxbatch = 0;
-        for (size_t b0 = 0; b0 < nb; b0 += per_batch) {
-            uint64_t t = 0;
-            for (size_t q = b0; q < nb && q < b0 + per_batch; q++) t += bc[q];
-            if (t > maxbatch) maxbatch = t;
-            nbig += t;
-        }
-        SortBufs t;
-        for (int q = 0; q < 2; q++) {
-            t.lo[q] = arena.alloc<uint64_t>(maxbatch + 1);
-            t.id[q] = arena.alloc<uint32_t>(maxbatch + 1);
-            if (!t.lo[q] || !t.id[q]) return set_error(MP_ENOMEM, "device memory for oversized buckets");
-        }
-        for (size_t b0 = 0; b0 < nb; b0 += per_batch) {
-            const size_t b1 = std::min<size_t>(nb, b0 + per_batch);
-            uint64_t acc = 0;
-            for (size_t q = b0; q < b1; q++) { bo[q] = acc; acc += bc[q]; }
-            MP_CUDA(cudaMemcpyAsync(d_bo + b0, bo.data() + b0, (b1 - b0) * 8, cudaMemcpyHostToDevice, st));
-            t.cur = 0;
-            (mp::count_launch(), k_big_gather<<<(unsigned)(b1 - b0), 256, 0, st>>>(d_bs + b0, d_bc + b0, d_bo + b0, b.lo[in],
-                                                                                  b.id[in], t.lo[0], t.id[0], lowbits));
-            SortStats bst;
-            int rc = radix_sort(t, acc, false, arena, st, &bst);
-            if (rc) return rc;
-            (mp::count_launch(), k_big_scatter<<<(unsigned)(b1 - b0), 256, 0, st>>>(d_bs + b0, d_bc + b0, d_bb + b0, d_bo + b0,
-                                                                                   t.lo[t.cur], t.id[t.cur], b.lo[out],
-                                                                                   b.id[out], lowbits));
-        }
+        const int rc = sort_big_buckets(hs, bc, hk, b, in, out, lowbits, arena, st, &nbig);
+        if (rc) return rc;
     }
     cudaEventRecord(ev[3], st);
     unsigned long long ht[16] = {};
@@ -1245,6 +1271,406 @@ int bucket_sort(SortBufs &b, uint64_t n, bool has_hi, int k, const uint64_t *d_h
     *out_lo_buf = out;  // lo and id end in the other buffer; hi (constant within a bucket) stays in `in`
     *out_hi_buf = in;
     b.cur = out;
+    return 0;
+}
+
+// ---------------------------------------------------------------------------
+// Sort by units (mp_sort_tuples): two stable digit passes over a 16-bit window of the key below its highest varying bit,
+// then every unit of consecutive buckets in shared memory by rank.
+//
+// A digit pass moves 25 bytes a tuple each way and takes 0.27 ms for 24 million tuples of 13 bytes (the ranking and the
+// look-back, not the bytes, bound it), and a 70-bit key needs nine.  After two, the tuples lie in buckets of a few hundred,
+// and the rest is one read and one write: a unit's tuples are dropped into 4,096 bins by the next bits of the key, in any
+// order, and a tuple's place is its bin's start plus the tuples of the bin that come before it by (key, place in the
+// input order) -- a handful of comparisons, so no further pass is made and ties keep their order.
+// 24 million tuples: nine passes 3.1 ms, two passes (0.47) and units (0.35) 1.14 ms.
+
+constexpr int UW_BITS = 16;                    // the window: two digits of eight bits
+constexpr uint32_t UW_BUCKETS = 1u << UW_BITS;
+constexpr uint32_t UNIT_QUANTUM = 4096;        // a unit starts at the first bucket at or after each multiple
+constexpr uint32_t UNIT_LONE = SS_SMALL_CAP - UNIT_QUANTUM;  // a larger bucket starts a unit, so only its own can outgrow a block
+constexpr int UR_THREADS = 512, UR_BINBITS = 12, UR_BINS = 1 << UR_BINBITS;
+constexpr uint32_t UR_MOST = 384;              // tuples of a bin ranked by comparison; units with more take digit passes
+
+struct KeyBits {  // of all keys: the bits set in some, the bits clear in some
+    unsigned long long lo1, lo0, hi1, hi0;
+};
+
+// The window's first k-mer bit; t: the highest varying bit of the key (hi << 64 | lo), -1 none.
+__host__ __device__ __forceinline__ int window_shift(int t) { return t - 8 + 1 > UW_BITS ? t - 8 + 1 - UW_BITS : 0; }
+
+__device__ __forceinline__ int top_varying(const KeyBits &k)
+{
+    const unsigned long long vh = k.hi1 & k.hi0 & 0xFF, vl = k.lo1 & k.lo0;
+    return vh ? 127 - __clzll((long long)vh) : vl ? 63 - __clzll((long long)vl) : -1;
+}
+
+__global__ void __launch_bounds__(256) k_key_bits(const uint64_t *__restrict__ lo, const uint8_t *__restrict__ hi, uint64_t n,
+                                                  KeyBits *out)
+{
+    unsigned long long a = 0, b = 0, c = 0, d = 0;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const unsigned long long k = lo[i], h = hi ? hi[i] : 0u;
+        a |= k;
+        b |= ~k;
+        c |= h;
+        d |= ~h;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        a |= __shfl_xor_sync(FULLM, a, o);
+        b |= __shfl_xor_sync(FULLM, b, o);
+        c |= __shfl_xor_sync(FULLM, c, o);
+        d |= __shfl_xor_sync(FULLM, d, o);
+    }
+    __shared__ unsigned long long r[4][8];
+    if ((threadIdx.x & 31) == 0) {
+        const int w = threadIdx.x >> 5;
+        r[0][w] = a, r[1][w] = b, r[2][w] = c, r[3][w] = d;
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        unsigned long long v = 0;
+        for (int w = 0; w < 8; w++) v |= r[threadIdx.x][w];
+        unsigned long long *o = &out->lo1 + threadIdx.x;
+        if (v & ~*(volatile unsigned long long *)o) atomicOr(o, v);
+    }
+}
+
+// Counts of the window's two digits.
+__global__ void __launch_bounds__(256) k_window_hist(const uint64_t *__restrict__ lo, const uint8_t *__restrict__ hi, uint64_t n,
+                                                     const KeyBits *bits, unsigned int *cnt)
+{
+    __shared__ uint32_t h[512];
+    h[threadIdx.x] = h[threadIdx.x + 256] = 0;
+    const int t = top_varying(*bits), bsh = window_shift(t);
+    __syncthreads();
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const uint64_t k = lo[i];
+        const uint32_t x = hi ? (uint32_t)hi[i] : 0u;
+        atomicAdd(&h[digit_of<2>(k, x, bsh)], 1u);
+        atomicAdd(&h[256 + digit_of<2>(k, x, bsh + 8)], 1u);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 512; i += 256)
+        if (h[i]) atomicAdd(&cnt[i], h[i]);
+}
+
+// Block p: the digit offsets of pass p and how many of its digits occur.
+__global__ void __launch_bounds__(256) k_window_digits(const unsigned int *cnt, uint64_t *dbase, unsigned int *occur)
+{
+    __shared__ uint32_t ws[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = blockIdx.x;
+    const uint32_t c = cnt[p * 256 + threadIdx.x];
+    uint32_t x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULLM, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) ws[warp] = x;
+    const int nz = __syncthreads_count(c != 0);
+    uint32_t before = 0;
+    for (int w = 0; w < warp; w++) before += ws[w];
+    dbase[p * 256 + threadIdx.x] = before + x - c;
+    if (threadIdx.x == 0) occur[p] = (unsigned)nz;
+}
+
+__device__ __forceinline__ uint32_t window_bucket(const uint64_t *lo, const uint8_t *hi, uint64_t i, int bsh)
+{
+    return (uint32_t)((((lo[i] >> 8) | ((uint64_t)(hi ? hi[i] : 0) << 56)) >> bsh) & (UW_BUCKETS - 1));
+}
+
+// First tuple and end of every bucket that occurs (end 0: it does not).
+__global__ void __launch_bounds__(256) k_bucket_bounds(const uint64_t *__restrict__ lo, const uint8_t *__restrict__ hi, uint64_t n,
+                                                       int bsh, uint32_t *first, uint32_t *end)
+{
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const uint32_t b = window_bucket(lo, hi, i, bsh), p = i ? window_bucket(lo, hi, i - 1, bsh) : UW_BUCKETS;
+        if (b != p) {
+            first[b] = (uint32_t)i;
+            if (i) end[p] = (uint32_t)i;
+        }
+        if (i + 1 == n) end[b] = (uint32_t)n;
+    }
+}
+
+// Whether bucket b starts a unit: the first to start in a quantum, a large one, or the first of a block of 2^r buckets
+// (a unit's keys, relative to its first bucket, fit 64 bits).
+__global__ void __launch_bounds__(256) k_unit_flags(const uint64_t *__restrict__ lo, const uint8_t *__restrict__ hi, int bsh, int r,
+                                                    const uint32_t *first, const uint32_t *end, uint32_t *flag)
+{
+    const uint32_t b = blockIdx.x * 256 + threadIdx.x, e = end[b];
+    uint32_t f = 0;
+    if (e) {
+        const uint32_t s = first[b];
+        f = s == 0 || e - s > UNIT_LONE;
+        if (!f) {
+            const uint32_t p = window_bucket(lo, hi, s - 1, bsh);
+            f = first[p] / UNIT_QUANTUM != s / UNIT_QUANTUM || (p >> r) != (b >> r);
+        }
+    }
+    flag[b] = f;
+}
+
+__global__ void __launch_bounds__(256) k_unit_starts(const uint32_t *flag, const uint64_t *off, const uint32_t *first, uint32_t *ustart)
+{
+    const uint32_t b = blockIdx.x * 256 + threadIdx.x;
+    if (flag[b]) ustart[off[b]] = first[b];
+}
+
+struct UnitRankSmem {
+    uint64_t key[SS_SMALL_CAP];  // in bin order
+    uint32_t id[SS_SMALL_CAP];
+    uint32_t bin[UR_BINS + 4];   // counts, then starts
+    uint16_t at[SS_SMALL_CAP];   // place in the input order
+    uint32_t wsum[UR_THREADS / 32];
+};
+static_assert(2 * (sizeof(UnitRankSmem) + 1024) <= 228 * 1024, "two blocks per SM");
+static_assert(UR_BINS == UR_THREADS * 8, "a thread scans eight bins");
+
+struct UnitRank {
+    const uint64_t *lo_in;
+    const uint8_t *hi_in;
+    const uint32_t *id_in;
+    uint64_t *lo_out;
+    uint32_t *id_out;
+    const uint32_t *ustart;
+    const uint64_t *nunits;
+    uint64_t n;
+    int bsh;
+    unsigned int *nlist;  // units left to the digit passes: start, tuples, first bucket
+    uint32_t *list;
+};
+
+// Bound by the ranking's shared-memory reads (about ten a tuple) and by latency: two blocks an SM, twelve loads in flight
+// a thread, the next unit's tuples prefetched into L2.
+__global__ void __launch_bounds__(UR_THREADS, 2) k_unit_rank(UnitRank c)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    UnitRankSmem &sm = *reinterpret_cast<UnitRankSmem *>(smraw);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lowbits = c.bsh + 8;
+    const uint32_t nu = (uint32_t)*c.nunits;
+    for (uint32_t u = blockIdx.x; u < nu; u += gridDim.x) {
+        const uint64_t start = c.ustart[u], end = u + 1 < nu ? (uint64_t)c.ustart[u + 1] : c.n;
+        const uint32_t cnt = (uint32_t)(end - start);
+        if (u + gridDim.x < nu) {
+            const uint64_t ns = c.ustart[u + gridDim.x], ne = min(c.n, ns + UNIT_QUANTUM);
+            prefetch_range(c.lo_in + ns, (ne - ns) * 8, UR_THREADS);
+            prefetch_range(c.id_in + ns, (ne - ns) * 4, UR_THREADS);
+        }
+        const uint64_t base = c.lo_in[start] >> lowbits << lowbits, top = c.lo_in[end - 1] - base;
+        bool whole = cnt <= (uint32_t)SS_SMALL_CAP;
+        if (whole) {
+            // bins: the top bits of the unit's key range
+            const uint64_t width = top >> lowbits;  // buckets after the first
+            const int wb = width ? 64 - __clzll((long long)width) : 0, sh = max(lowbits + wb - UR_BINBITS, 0);
+            reinterpret_cast<uint4 *>(sm.bin)[threadIdx.x * 2] = make_uint4(0, 0, 0, 0);
+            reinterpret_cast<uint4 *>(sm.bin)[threadIdx.x * 2 + 1] = make_uint4(0, 0, 0, 0);
+            uint64_t key[SS_ITEMS];
+            uint32_t rd[SS_ITEMS];  // bin << 16 | arrival in the bin
+#pragma unroll
+            for (int j = 0; j < SS_ITEMS; j++) {
+                const uint32_t e = threadIdx.x + j * UR_THREADS;
+                key[j] = e < cnt ? c.lo_in[start + e] - base : 0ull;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < SS_ITEMS; j++) {
+                const uint32_t e = threadIdx.x + j * UR_THREADS;
+                const uint32_t d = (uint32_t)(key[j] >> sh) & (UR_BINS - 1);
+                rd[j] = d << 16;
+                if (e < cnt) rd[j] |= atomicAdd(&sm.bin[d], 1u);
+            }
+            __syncthreads();
+            uint32_t v[8], tot = 0, most = 0;
+            {
+                const uint4 a = reinterpret_cast<const uint4 *>(sm.bin)[threadIdx.x * 2];
+                const uint4 b = reinterpret_cast<const uint4 *>(sm.bin)[threadIdx.x * 2 + 1];
+                v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                most = max(most, v[q]);
+                const uint32_t t = v[q];
+                v[q] = tot;
+                tot += t;
+            }
+            uint32_t x = tot;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULLM, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) sm.wsum[warp] = x;
+            whole = !__syncthreads_or(most > UR_MOST);
+            if (whole) {
+                uint32_t before = x - tot;
+                for (int w = 0; w < warp; w++) before += sm.wsum[w];
+                reinterpret_cast<uint4 *>(sm.bin)[threadIdx.x * 2] =
+                    make_uint4(before + v[0], before + v[1], before + v[2], before + v[3]);
+                reinterpret_cast<uint4 *>(sm.bin)[threadIdx.x * 2 + 1] =
+                    make_uint4(before + v[4], before + v[5], before + v[6], before + v[7]);
+                if (threadIdx.x == 0) sm.bin[UR_BINS] = cnt;
+                __syncthreads();
+#pragma unroll
+                for (int j = 0; j < SS_ITEMS; j++) {
+                    const uint32_t e = threadIdx.x + j * UR_THREADS;
+                    if (e >= cnt) continue;
+                    const uint32_t q = sm.bin[rd[j] >> 16] + (rd[j] & 0xFFFF);
+                    sm.key[q] = key[j];
+                    sm.id[q] = c.id_in[start + e];
+                    sm.at[q] = (uint16_t)e;
+                }
+                __syncthreads();
+                for (uint32_t p = threadIdx.x; p < cnt; p += UR_THREADS) {
+                    const uint64_t k = sm.key[p];
+                    const uint32_t e = sm.at[p], d = (uint32_t)(k >> sh) & (UR_BINS - 1);
+                    const uint32_t s = sm.bin[d], t = sm.bin[d + 1];
+                    uint32_t rank = s;
+                    for (uint32_t q = s; q < t; q++) {
+                        const uint64_t o = sm.key[q];
+                        rank += o < k || (o == k && sm.at[q] < e);
+                    }
+                    c.lo_out[start + rank] = k + base;
+                    c.id_out[start + rank] = sm.id[p];
+                }
+            }
+            __syncthreads();  // the next unit reuses the shared arrays
+        }
+        if (!whole && threadIdx.x == 0) {
+            uint32_t *l = c.list + 3ull * atomicAdd(c.nlist, 1u);
+            l[0] = (uint32_t)start;
+            l[1] = cnt;
+            l[2] = (uint32_t)((((c.lo_in[start] >> 8) | ((uint64_t)(c.hi_in ? c.hi_in[start] : 0) << 56)) >> c.bsh) & (NB - 1));
+        }
+    }
+}
+
+// Where the lines lie: 8,192 tuples take 258 us by passes and 146 by units, all of it launches and waits; above
+// 2^27 a bucket of evenly spread keys nears a unit, and keys that occur in few (digit, digit) pairs make buckets far
+// above one (they would be sorted twice).
+constexpr uint64_t UNIT_SORT_MIN = 1ull << 10, UNIT_SORT_MAX = 1ull << 27;
+
+static void sort_kernel_attrs()
+{
+    static std::once_flag once[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::call_once(once[dev & 63], [] {
+        cudaFuncSetAttribute(k_onesweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        cudaFuncSetAttribute(k_onesweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        cudaFuncSetAttribute(k_onesweep<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        cudaFuncSetAttribute(k_onesweep<2, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        cudaFuncSetAttribute(k_onesweep<2, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        cudaFuncSetAttribute(k_onesweep<2, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        cudaFuncSetAttribute(k_onesweep<2, 8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        cudaFuncSetAttribute(k_onesweep<2, 7, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        cudaFuncSetAttribute(k_onesweep<2, 6, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        cudaFuncSetAttribute(k_onesweep<2, 5, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem));
+        cudaFuncSetAttribute(k_unit_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(UnitRankSmem));
+        cudaFuncSetAttribute(k_segsort<1024, SS_CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SegSmemL));
+        cudaFuncSetAttribute(k_segsort<512, SS_SMALL_CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SegSmemS));
+    });
+}
+
+int unit_sort(const SortInput &in, SortBufs &b, uint64_t n, DeviceArena &arena, cudaStream_t st, bool *done)
+{
+    *done = false;
+    if (n < UNIT_SORT_MIN || n > UNIT_SORT_MAX) return 0;
+    struct Head {
+        KeyBits bits;
+        unsigned int occur[2], cnt[512];
+        uint32_t ctr[2], err, nlist;
+    };
+    const uint64_t tiles = (n + STILE - 1) / STILE;
+    Head *head = reinterpret_cast<Head *>(arena.alloc<uint64_t>((sizeof(Head) + 7) / 8));
+    uint64_t *dbase = arena.alloc<uint64_t>(512), *off = arena.alloc<uint64_t>(UW_BUCKETS + 2), *tot = arena.alloc<uint64_t>(1);
+    uint32_t *first = arena.alloc<uint32_t>(UW_BUCKETS), *end = arena.alloc<uint32_t>(UW_BUCKETS);
+    uint32_t *flag = arena.alloc<uint32_t>(UW_BUCKETS + 1), *ustart = arena.alloc<uint32_t>(UW_BUCKETS);
+    uint32_t *list = arena.alloc<uint32_t>(3 * UW_BUCKETS);
+    unsigned long long *status = arena.alloc<unsigned long long>(tiles * 256);
+    const size_t tb = scan_tmp_bytes(UW_BUCKETS + 1);
+    void *tmp = arena.alloc<uint8_t>(tb);
+    if (!head || !dbase || !off || !tot || !first || !end || !flag || !ustart || !list || !status || !tmp)
+        return set_error(MP_ENOMEM, "device memory for the unit sort");
+    sort_kernel_attrs();
+    MP_CUDA(cudaMemsetAsync(head, 0, sizeof(Head), st));
+    MP_CUDA(cudaMemsetAsync(end, 0, UW_BUCKETS * sizeof(uint32_t), st));
+    MP_CUDA(cudaMemsetAsync(flag + UW_BUCKETS, 0, sizeof(uint32_t), st));
+    MP_CUDA(cudaMemsetAsync(status, 0, tiles * 256 * sizeof(unsigned long long), st));
+    const unsigned grid = (unsigned)std::min<uint64_t>((n + 1023) / 1024, 8ull * (uint64_t)sm_count());
+    (mp::count_launch(), k_key_bits<<<grid, 256, 0, st>>>(in.lo, in.hi, n, &head->bits));
+    (mp::count_launch(), k_window_hist<<<grid, 256, 0, st>>>(in.lo, in.hi, n, &head->bits, head->cnt));
+    (mp::count_launch(), k_window_digits<<<2, 256, 0, st>>>(head->cnt, dbase, head->occur));
+    Head h;
+    MP_CUDA(cudaMemcpyAsync(&h, head, offsetof(Head, cnt), cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaStreamSynchronize(st));
+    const unsigned long long vh = h.bits.hi1 & h.bits.hi0 & 0xFF, vl = h.bits.lo1 & h.bits.lo0;
+    const int t = vh ? 127 - __builtin_clzll(vh) : vl ? 63 - __builtin_clzll(vl) : -1;
+    const int bsh = window_shift(t), lowbits = bsh + 8, r = std::min(UW_BITS, 64 - lowbits);
+    // (a listed unit carries its first bucket in 20 bits: constant bits above the window must be zero or leave the low word)
+    const unsigned long long above = ((h.bits.lo1 >> 8) | (h.bits.hi1 << 56)) >> bsh >> UW_BITS;
+    if (t < 0 || (above && lowbits < 44) || n > (uint64_t)(UNIT_QUANTUM / 2) * h.occur[0] * h.occur[1]) {
+        arena.free_scratch(status);
+        return 0;
+    }
+    const uint32_t pf = onesweep_prefetch_tiles();
+    // lo and id: in -> buffer 0 -> 1 -> (units) 0; hi, which the units leave as it is: in -> 1 -> 0
+    (mp::count_launch(), k_onesweep<2><<<(unsigned)tiles, ST, sizeof(SortSmem), st>>>(
+        in.lo, in.hi, in.id, b.lo[0], b.hi[1], b.id[0], n, bsh, 8, dbase, nullptr, status, head->ctr, 1u, &head->err, pf, nullptr,
+        Segs{}, arena.lim.lookback_spins));
+    (mp::count_launch(), k_onesweep<2><<<(unsigned)tiles, ST, sizeof(SortSmem), st>>>(
+        b.lo[0], b.hi[1], b.id[0], b.lo[1], b.hi[0], b.id[1], n, bsh + 8, 8, dbase + 256, nullptr, status, head->ctr + 1, 2u,
+        &head->err, pf, nullptr, Segs{}, arena.lim.lookback_spins));
+    (mp::count_launch(), k_bucket_bounds<<<grid, 256, 0, st>>>(b.lo[1], b.hi[0], n, bsh, first, end));
+    (mp::count_launch(), k_unit_flags<<<UW_BUCKETS / 256, 256, 0, st>>>(b.lo[1], b.hi[0], bsh, r, first, end, flag));
+    scan_u32_to_u64(flag, off, UW_BUCKETS + 1, tot, tmp, tb, st);
+    (mp::count_launch(), k_unit_starts<<<UW_BUCKETS / 256, 256, 0, st>>>(flag, off, first, ustart));
+    (mp::count_launch(), k_unit_rank<<<2 * sm_count(), UR_THREADS, sizeof(UnitRankSmem), st>>>(
+        UnitRank{b.lo[1], b.hi[0], b.id[1], b.lo[0], b.id[0], ustart, tot, n, bsh, &head->nlist, list}));
+    MP_CUDA(cudaMemcpyAsync(&h.err, &head->err, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaStreamSynchronize(st));
+    MP_CUDA(cudaGetLastError());
+    arena.free_scratch(status);
+    if (h.err) return set_error(MP_EDEVICE, "radix sort look-back gave up (device error flags 0x%x)", h.err);
+    if (h.nlist) {  // by size: a block's digit passes, a large block's, the device-wide sort
+        std::vector<uint32_t> l(3ull * h.nlist);
+        MP_CUDA(cudaMemcpyAsync(l.data(), list, l.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        MP_CUDA(cudaStreamSynchronize(st));
+        std::vector<uint32_t> order(h.nlist);
+        for (uint32_t i = 0; i < h.nlist; i++) order[i] = i;
+        std::sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return l[3ull * x] < l[3ull * y]; });
+        std::vector<uint64_t> us[3];
+        std::vector<uint32_t> uc[3], ub[3];
+        for (uint32_t i : order) {
+            const uint32_t c = l[3ull * i + 1], q = c <= (uint32_t)SS_SMALL_CAP ? 0 : c <= (uint32_t)SS_CAP ? 1 : 2;
+            us[q].push_back(l[3ull * i]);
+            uc[q].push_back(c);
+            ub[q].push_back(l[3ull * i + 2]);
+        }
+        SortBufs u = b;  // the units' hi is in buffer 0 already
+        u.hi[1] = b.hi[0];
+        const bool has_hi = in.hi != nullptr;
+        int rc = 0;
+        uint64_t nbig = 0;
+        if (!us[0].empty())
+            rc = sort_listed_units<512, SS_SMALL_CAP, SegSmemS>(us[0], uc[0], ub[0], u, 1, 0, has_hi, bsh, lowbits, SS_MAXBITS,
+                                                                nullptr, arena, st);
+        if (!rc && !us[1].empty())
+            rc = sort_listed_units<1024, SS_CAP, SegSmemL>(us[1], uc[1], ub[1], u, 1, 0, has_hi, bsh, lowbits, SS_MAXBITS,
+                                                           nullptr, arena, st);
+        if (!rc && !us[2].empty()) rc = sort_big_buckets(us[2], uc[2], ub[2], u, 1, 0, lowbits, arena, st, &nbig);
+        if (rc) return rc;
+    }
+    b.cur = 0;
+    *done = true;
     return 0;
 }
 
@@ -1300,6 +1726,16 @@ static bool bytes_overlap(const void *a, uint64_t an, const void *b, uint64_t bn
 {
     const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
     return an && bn && x < y + bn && y < x + an;
+}
+
+bool tuples_overlap(const SortInput &in, const SortBufs &b, int which, uint64_t n)
+{
+    const void *i[3] = {in.lo, in.hi, in.id}, *o[3] = {b.lo[which], b.hi[which], b.id[which]};
+    const uint64_t w[3] = {8, 1, 4};
+    for (int x = 0; x < 3; x++)
+        for (int y = 0; y < 3; y++)
+            if (i[x] && o[y] && bytes_overlap(i[x], n * w[x], o[y], n * w[y])) return true;
+    return false;
 }
 
 int sort_tuples_noalloc(const uint64_t *lo_in, const uint8_t *hi_in, const uint32_t *id_in, uint64_t *lo_out,

@@ -35,8 +35,23 @@ struct SortStats {
 int count_unsorted(const uint64_t *lo, const uint8_t *hi, uint64_t n, unsigned long long *d_count, cudaStream_t st,
                    uint64_t *out);
 
-// Stable sort of b[cur][0, n) by (hi, lo); on return b.cur names the sorted buffer.
-int radix_sort(SortBufs &b, uint64_t n, bool has_hi, DeviceArena &arena, cudaStream_t st, SortStats *stats);
+// A sort's input where it is not one of the buffers (hi null without the hi array).
+struct SortInput {
+    const uint64_t *lo;
+    const uint8_t *hi;
+    const uint32_t *id;
+};
+
+// Stable sort of b[cur][0, n) by (hi, lo); on return b.cur names the sorted buffer.  With from, of the tuples there
+// (which stay as they are and overlap neither buffer) into buffer 0.
+int radix_sort(SortBufs &b, uint64_t n, bool has_hi, DeviceArena &arena, cudaStream_t st, SortStats *stats,
+               const SortInput *from = nullptr);
+
+// The same by units, where the tuples lend themselves to it (*done says whether they did; if not, nothing is written).
+int unit_sort(const SortInput &in, SortBufs &b, uint64_t n, DeviceArena &arena, cudaStream_t st, bool *done);
+
+// The arrays share bytes.
+bool tuples_overlap(const SortInput &in, const SortBufs &b, int which, uint64_t n);
 
 // The tuning table or the environment shapes the bucket sort of a scan of n tuples (other digits than the default).
 bool sort_plan_chosen(int k, uint64_t n);

@@ -1526,12 +1526,18 @@ int mp_sort_tuples(mp_ctx *ctx, const uint64_t *lo_in, const uint8_t *hi_in, con
         arena.release_all();
         return set_error(MP_ENOMEM, "device memory for sorting %llu tuples", (unsigned long long)n);
     }
-    if (n) {
+    const SortInput in{lo_in, hi_in, id_in};
+    int rc = 0;
+    if (tuples_overlap(in, b, 0, n)) {  // sorted in place: a copy first
         MP_CUDA(cudaMemcpyAsync(lo_out, lo_in, n * 8, cudaMemcpyDeviceToDevice, st));
         MP_CUDA(cudaMemcpyAsync(id_out, id_in, n * 4, cudaMemcpyDeviceToDevice, st));
         if (has_hi) MP_CUDA(cudaMemcpyAsync(hi_out, hi_in, n, cudaMemcpyDeviceToDevice, st));
+        rc = radix_sort(b, n, has_hi, arena, st, nullptr);
+    } else {
+        bool done = false;
+        rc = unit_sort(in, b, n, arena, st, &done);
+        if (!rc && !done) rc = radix_sort(b, n, has_hi, arena, st, nullptr, &in);
     }
-    int rc = radix_sort(b, n, has_hi, arena, st, nullptr);
     if (!rc && b.cur == 1 && n) {
         cudaMemcpyAsync(lo_out, b.lo[1], n * 8, cudaMemcpyDeviceToDevice, st);
         cudaMemcpyAsync(id_out, b.id[1], n * 4, cudaMemcpyDeviceToDevice, st);

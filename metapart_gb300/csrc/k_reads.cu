@@ -174,32 +174,58 @@ __global__ void __launch_bounds__(NL_THREADS) k_nl_count(const uint8_t *buf, uin
     }
 }
 
+// Bit q: byte q of the sixteen at p is a newline of the parsed range.
+__device__ __forceinline__ uint32_t nl_mask16(const uint8_t *buf, uint64_t p, uint64_t end, uint32_t skip)
+{
+    if (p + 16 <= end && p >= skip) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(buf + p);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        uint32_t m = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) m |= ((((nl_in_word(w[q]) >> 7) * 0x01020408u) >> 24) & 0xFu) << (4 * q);
+        return m;
+    }
+    uint32_t m = 0;
+    for (uint32_t q = 0; q < 16; q++)
+        if (p + q < end && p + q >= skip && buf[p + q] == '\n') m |= 1u << q;
+    return m;
+}
+
+// A warp takes an eighth of the block's bytes and keeps its newlines as bits, so the block meets once, for the warps' counts.
+// Bound by its instructions, about 60 per 16 bytes (220 with every byte compared and a block scan every 4 KB): 6.2 GB
+// 2.73 -> 2.30 ms.
 __global__ void __launch_bounds__(NL_THREADS) k_nl_write(const uint8_t *buf, uint64_t n, uint32_t skip,
                                                          const uint64_t *seg_off, uint64_t *nl_pos)
 {
-    const uint64_t s0 = (uint64_t)blockIdx.x * NL_SEG, s1 = min(n, s0 + NL_SEG);
-    uint64_t out = seg_off[blockIdx.x];
-    for (uint64_t r = s0; r < s1; r += NL_THREADS * 16) {
-        const uint64_t p = r + (uint64_t)threadIdx.x * 16;
-        uint8_t b[16];
-        int cnt = 0;
-        if (p + 16 <= s1 && p >= skip) {
-            uint4 v = *reinterpret_cast<const uint4 *>(buf + p);
-            memcpy(b, &v, 16);
-            cnt = __popc(nl_in_word(v.x)) + __popc(nl_in_word(v.y)) + __popc(nl_in_word(v.z)) + __popc(nl_in_word(v.w));
-        } else {
-            for (int q = 0; q < 16; q++) {
-                b[q] = (p + q < s1 && p + q >= skip) ? buf[p + q] : 0;
-                cnt += b[q] == '\n';
-            }
-        }
-        uint64_t tot;
-        uint64_t pre = block_excl_scan((uint64_t)cnt, &tot);
-        uint64_t o = out + pre;
+    constexpr int WARPS = NL_THREADS / 32, TURNS = (int)(NL_SEG / (NL_THREADS * 16));
+    __shared__ uint32_t ws[WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t end = min(n, ((uint64_t)blockIdx.x + 1) * NL_SEG);
+    const uint64_t p0 = (uint64_t)blockIdx.x * NL_SEG + (uint64_t)warp * (NL_SEG / WARPS) + (uint64_t)lane * 16;
+    uint32_t m[TURNS], c = 0;
 #pragma unroll
-        for (int q = 0; q < 16; q++)
-            if (b[q] == '\n') nl_pos[o++] = p + q - skip;
-        out += tot;
+    for (int i = 0; i < TURNS; i++) {
+        const uint64_t p = p0 + (uint64_t)i * 512;
+        m[i] = p < end ? nl_mask16(buf, p, end, skip) : 0u;
+        c += (uint32_t)__popc(m[i]);
+    }
+    c = __reduce_add_sync(0xFFFFFFFFu, c);
+    if (lane == 0) ws[warp] = c;
+    __syncthreads();
+    uint64_t out = seg_off[blockIdx.x];
+    for (int w = 0; w < warp; w++) out += ws[w];
+#pragma unroll
+    for (int i = 0; i < TURNS; i++) {
+        const uint32_t cnt = (uint32_t)__popc(m[i]);
+        uint32_t x = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        uint64_t o = out + x - cnt;
+        for (uint32_t b = m[i]; b; b &= b - 1) nl_pos[o++] = p0 + (uint64_t)i * 512 + (uint32_t)(__ffs((int)b) - 1) - skip;
+        out += __shfl_sync(0xFFFFFFFFu, x, 31);
     }
 }
 

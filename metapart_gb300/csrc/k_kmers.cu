@@ -100,64 +100,117 @@ __global__ void __launch_bounds__(CT_THREADS) k_count_tiles(ReadTiles t, uint64_
 
 // ------------------------------------------------------- 3-minimizer core
 
-// One read, thread-sequential.  ENUM: apply the scan range and produce adjacency bytes.
-template <bool ENUM, class Emit>
+// The adjacency byte of a minimum: at = 4 position + 2 its strand + the strand of the k-mer that ended its window.
+__device__ __forceinline__ uint32_t min3_adj(const uint8_t *s, int L, int k, uint32_t at)
+{
+    const int m = (int)(at >> 2);
+    uint32_t pa = m == 0 ? 7u : a5_of(s[m - 1]), na = m == L - k ? 7u : a5_of(s[m + k]);
+    if (!(at & 2u)) {
+        pa = a5_cmpl(pa);
+        na = a5_cmpl(na);
+    }
+    return at & 1u ? ((pa << 3) | (na & 7)) : ((na << 3) | (pa & 7));
+}
+
+// One read, thread-sequential: emit(k-mer, at) for every window's minimum, at as min3_adj takes it.  ENUM: apply the scan
+// range.  HI: 2k >= 34 (KmerRoll).
+//
+// Bound by its integer instructions (41 a character when every character was loaded, tested for N and for the window's end,
+// and the minimum's neighbours kept along): eight characters are loaded and decoded at once, and eight k-mers of one window
+// take only the roll and the comparison, about twenty.  3 million reads of 250 bases: counting 1.25 -> 0.92 ms,
+// enumeration 3.5 (a counting and a writing pass) -> 1.43 ms.
+template <bool ENUM, bool HI, class Emit>
 __device__ __forceinline__ void min3_read(const uint8_t *s, int L, int k, uint32_t lo, uint32_t hi, Emit emit)
 {
     if (L <= k) return;
     const int last = L - k, sh = 2 * (k - 10), win = last / 3;
     const uint64_t mask = kmer_mask(k);
-    uint64_t fwd = 0, rc = 0, mn = 0;
-    uint32_t mps = 0, mns = 0;  // stored adjacency a5 values of the current minimum
-    int lastN = -1;
-    for (int j = 0; j < k; j++) {
-        const uint32_t c = s[j];
-        if (c == 'N') lastN = j;
-        rc |= (uint64_t)(3u - fcode(c)) << (2 * j);
-        fwd = (fwd << 2) | fcode(c);
-    }
-    if (lastN == -1) {
-        const bool f = fwd < rc;
-        const uint64_t v = f ? fwd : rc;
-        const uint32_t b = (uint32_t)(v >> sh);
-        if (!ENUM || (b >= lo && b < hi)) {
-            mn = v;
-            if (ENUM) {
-                const uint32_t pa = 7u, na = a5_of(s[k]);
-                mps = f ? pa : a5_cmpl(pa);
-                mns = f ? na : a5_cmpl(na);
+    const uint32_t mh = (uint32_t)(mask >> 32);
+    const int top = HI ? 2 * k - 34 : 2 * k - 2;
+    uint32_t fl = 0, fh = 0, rl = 0, rh = 0;
+    uint64_t mn1 = ~0ull;  // the current minimum less one: none, and the k-mer of code 0, give way to any (all ones)
+    uint32_t mpf = 0;      // its position and strand
+    int lastN = -1, next_win = win;
+    const bool all = lo == 0 && hi >= NB;
+    auto roll = [&](uint32_t fc) {
+        if constexpr (HI) {
+            fh = __funnelshift_l(fl, fh, 2) & mh;
+            fl = (fl << 2) | fc;
+            rl = __funnelshift_r(rl, rh, 2);
+            rh = (rh >> 2) | ((fc ^ 3u) << top);
+        } else {
+            const uint64_t f = (((((uint64_t)fh << 32) | fl) << 2) | fc) & mask;
+            const uint64_t r = ((((uint64_t)rh << 32) | rl) >> 2) | ((uint64_t)(fc ^ 3u) << top);
+            fl = (uint32_t)f, fh = (uint32_t)(f >> 32), rl = (uint32_t)r, rh = (uint32_t)(r >> 32);
+        }
+    };
+    auto flush = [&](bool f) {  // f: the strand of the k-mer that ends the window
+        if (mn1 != ~0ull) emit(mn1 + 1, 2 * mpf + f);
+    };
+    const uint64_t *w = reinterpret_cast<const uint64_t *>(reinterpret_cast<uintptr_t>(s) & ~(uintptr_t)7);
+    const uint32_t ws = (uint32_t)(reinterpret_cast<uintptr_t>(s) & 7) * 8;
+    uint64_t w0 = w[0], w1 = w[1];
+    for (int t0 = 0; t0 < L; t0 += 8) {
+        const uint64_t c8 = ws ? (w0 >> ws) | (w1 << (64 - ws)) : w0;
+        w0 = w1;
+        w1 = w[t0 / 8 + 2];  // a turn ahead: at most 23 bytes past the read, inside the buffer's spare bytes
+        const int i0 = t0 - (k - 1);  // the position whose last character is the first of these
+        const uint32_t cl = (uint32_t)c8, ch = (uint32_t)(c8 >> 32);
+        const bool plain = !(pack_n4(cl) | pack_n4(ch)) && t0 + 8 <= L;
+        if (plain && (i0 < -7 || (i0 > lastN && i0 + 7 <= next_win && (!ENUM || all)))) {
+            // eight characters of no k-mer yet, or eight k-mers of one window
+            uint32_t x[2] = {(cl >> 1) & 0x03030303u, (ch >> 1) & 0x03030303u};
+            x[0] ^= (x[0] >> 1) & 0x01010101u;
+            x[1] ^= (x[1] >> 1) & 0x01010101u;
+            if (i0 < -7) {
+#pragma unroll
+                for (int q = 0; q < 8; q++) roll((x[q >> 2] >> (8 * (q & 3))) & 3u);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    roll((x[q >> 2] >> (8 * (q & 3))) & 3u);
+                    const uint64_t fwd = ((uint64_t)fh << 32) | fl, rc = ((uint64_t)rh << 32) | rl;
+                    const bool f = fwd < rc;
+                    const uint64_t v = f ? fwd : rc;
+                    if (v <= mn1) {
+                        mn1 = v - 1;
+                        mpf = 2 * (uint32_t)(i0 + q) + f;
+                    }
+                }
+            }
+            continue;
+        }
+        const int e = min(8, L - t0);
+#pragma unroll 1
+        for (int q = 0; q < e; q++) {
+            const uint32_t c = (uint32_t)(c8 >> (8 * q)) & 0xFFu;
+            const int i = i0 + q;
+            roll(fcode(c));
+            if (c == 'N') lastN = t0 + q;
+            if (!(i > lastN && i >= 0)) continue;
+            const uint64_t fwd = ((uint64_t)fh << 32) | fl, rc = ((uint64_t)rh << 32) | rl;
+            const bool f = fwd < rc;
+            const uint64_t v = f ? fwd : rc;
+            if (ENUM && !all) {
+                const uint32_t b = (uint32_t)(v >> sh);
+                if (!(b >= lo && b < hi)) continue;
+            }
+            if (i > next_win) {
+                flush(f);
+                mn1 = ~0ull;
+                next_win += win;
+                if (next_win + win > last) next_win = last;
+            }
+            if (v <= mn1) {
+                mn1 = v - 1;
+                mpf = 2 * (uint32_t)i + f;
             }
         }
     }
-    int next_win = win;
-    for (int i = 1; i <= last; i++) {
-        const uint32_t c = s[i + k - 1];
-        rc = (rc >> 2) | ((uint64_t)(3u - fcode(c)) << (2 * (k - 1)));
-        fwd = ((fwd << 2) | fcode(c)) & mask;
-        if (c == 'N') lastN = i + k - 1;
-        if (!(i > lastN)) continue;
-        const bool f = fwd < rc;
-        const uint64_t v = f ? fwd : rc;
-        const uint32_t b = (uint32_t)(v >> sh);
-        if (ENUM && !(b >= lo && b < hi)) continue;
-        uint32_t pa = 0, na = 0;
-        if (ENUM) {
-            pa = a5_of(s[i - 1]);
-            na = (i == last) ? 7u : a5_of(s[i + k]);
-            if (!f) { pa = a5_cmpl(pa); na = a5_cmpl(na); }
-        }
-        if (i > next_win) {
-            if (mn != 0) emit(mn, f ? ((mps << 3) | (mns & 7)) : ((mns << 3) | (mps & 7)));
-            mn = v; mps = pa; mns = na;
-            next_win += win;
-            if (next_win + win > last) next_win = last;
-        } else if (v < mn || mn == 0) {
-            mn = v; mps = pa; mns = na;
-        }
-    }
-    if (mn != 0) emit(mn, (mns << 3) | (mps & 7));
+    flush(false);
 }
 
+template <bool HI>
 __global__ void k_count_min3(const uint8_t *fq, const uint64_t *seq_off, const uint32_t *seq_len, uint64_t r0, uint64_t r1,
                              int k, const uint64_t *chunk_rec, int nchunks, uint32_t *cc, unsigned long long *glob,
                              uint32_t *err)
@@ -168,7 +221,7 @@ __global__ void k_count_min3(const uint8_t *fq, const uint64_t *seq_off, const u
         const uint32_t L = seq_len[r];
         if (L > (uint32_t)MAX_READ_COUNT) { atomicOr(err, DERR_LONG_READ); continue; }
         uint32_t *ccc = cc ? cc + (size_t)chunk_of(chunk_rec, nchunks, r) * NB : nullptr;
-        min3_read<false>(fq + seq_off[r], (int)L, k, 0, 0, [&](uint64_t v, uint32_t) {
+        min3_read<false, HI>(fq + seq_off[r], (int)L, k, 0, 0, [&](uint64_t v, uint32_t) {
             const uint32_t b = (uint32_t)(v >> sh);
             if (ccc) atomicAdd(&ccc[b], 1u); else atomicAdd(&glob[b], 1ull);
         });
@@ -321,7 +374,7 @@ __global__ void __launch_bounds__(256) k_enum_count_scans(const uint8_t *fq, con
 
 // ------------------------------------------------------------- K2 3-min
 
-template <bool WRITE>
+template <bool WRITE, bool HI>
 __global__ void k_enum_min3(const uint8_t *fq, const uint64_t *seq_off, const uint32_t *seq_len, uint64_t n_reads, int k,
                             uint32_t lo, uint32_t hi, const uint32_t *label, const uint64_t *out_off, uint32_t *cnt,
                             uint64_t *o_lo, uint8_t *o_hi, uint32_t *o_id, uint32_t *err)
@@ -339,10 +392,10 @@ __global__ void k_enum_min3(const uint8_t *fq, const uint64_t *seq_off, const ui
         uint64_t pos = WRITE ? out_off[r] : 0;
         const uint64_t end = WRITE ? out_off[r + 1] : 0;
         uint32_t c = 0;
-        min3_read<true>(fq + seq_off[r], (int)L, k, lo, hi, [&](uint64_t v, uint32_t adj) {
+        min3_read<true, HI>(fq + seq_off[r], (int)L, k, lo, hi, [&](uint64_t v, uint32_t at) {
             if constexpr (WRITE) {
                 if (pos < end) {
-                    o_lo[pos] = (v << 8) | adj;
+                    o_lo[pos] = (v << 8) | min3_adj(fq + seq_off[r], (int)L, k, at);
                     if (o_hi) o_hi[pos] = (uint8_t)(v >> 56);
                     o_id[pos] = id;
                 } else {
@@ -356,6 +409,76 @@ __global__ void k_enum_min3(const uint8_t *fq, const uint64_t *seq_off, const ui
             cnt[r] = c;
             if (c > 255) atomicOr(err, DERR_TOO_MANY);
         }
+    }
+}
+
+// The same in one pass and no order: a block's reads keep their tuples in shared memory (three each, as a rule) and take
+// their places with one addition a block -- one a warp and window was bound by the additions to one address (1.8 ms for 3
+// million reads).  Tuples past n are counted and not written.
+constexpr int EM_THREADS = 128, EM_KEEP = 4;
+
+template <bool HI>
+__global__ void __launch_bounds__(EM_THREADS) k_enum_min3_any(const uint8_t *fq, const uint64_t *seq_off, const uint32_t *seq_len,
+                                                              uint64_t n_reads, int k, uint32_t lo, uint32_t hi, const uint32_t *label,
+                                                              unsigned long long *total, uint64_t n, uint64_t *o_lo, uint8_t *o_hi,
+                                                              uint32_t *o_id, uint32_t *err)
+{
+    __shared__ uint64_t kv[EM_KEEP][EM_THREADS];
+    __shared__ uint32_t ka[EM_KEEP][EM_THREADS];
+    __shared__ uint32_t ws[EM_THREADS / 32];
+    __shared__ unsigned long long place;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint64_t r0 = (uint64_t)blockIdx.x * EM_THREADS; r0 < n_reads; r0 += (uint64_t)gridDim.x * EM_THREADS) {
+        const uint64_t r = r0 + threadIdx.x;
+        const uint32_t L = r < n_reads ? seq_len[r] : 0u;
+        uint32_t id = (uint32_t)r, c = 0;
+        if (L > (uint32_t)k && L - (uint32_t)k >= 300u) {
+            atomicOr(err, DERR_LONG_READ);
+        } else if (L > (uint32_t)k) {
+            if (label && label[r] != BAD) id = label[r];
+            min3_read<true, HI>(fq + seq_off[r], (int)L, k, lo, hi, [&](uint64_t v, uint32_t at) {
+                if (c < (uint32_t)EM_KEEP) {
+                    kv[c][threadIdx.x] = v;
+                    ka[c][threadIdx.x] = at;
+                } else {  // (windows of no position: a short read)
+                    const unsigned long long pos = atomicAdd(total, 1ull);
+                    if (pos < n) {
+                        o_lo[pos] = (v << 8) | min3_adj(fq + seq_off[r], (int)L, k, at);
+                        if (o_hi) o_hi[pos] = (uint8_t)(v >> 56);
+                        o_id[pos] = id;
+                    }
+                }
+                c++;
+            });
+            if (c > 255) atomicOr(err, DERR_TOO_MANY);
+        }
+        const uint32_t m = min(c, (uint32_t)EM_KEEP);
+        uint32_t x = m;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) ws[warp] = x;
+        __syncthreads();
+        uint32_t before = x - m, all = 0;
+#pragma unroll
+        for (int q = 0; q < EM_THREADS / 32; q++) {
+            if (q < warp) before += ws[q];
+            all += ws[q];
+        }
+        if (threadIdx.x == 0) place = atomicAdd(total, (unsigned long long)all);
+        __syncthreads();
+#pragma unroll
+        for (uint32_t q = 0; q < (uint32_t)EM_KEEP; q++) {
+            const unsigned long long pos = place + before + q;
+            if (q >= m || pos >= n) continue;
+            const uint64_t v = kv[q][threadIdx.x];
+            o_lo[pos] = (v << 8) | min3_adj(fq + seq_off[r], (int)L, k, ka[q][threadIdx.x]);
+            if (o_hi) o_hi[pos] = (uint8_t)(v >> 56);
+            o_id[pos] = id;
+        }
+        __syncthreads();
     }
 }
 
@@ -375,7 +498,7 @@ void launch_count(const uint8_t *fq, const ParsedReads &pr, int k, int min3, con
                   uint32_t *cc, unsigned long long *glob, uint32_t *err, cudaStream_t st, bool odd)
 {
     if (min3)
-        (mp::count_launch(), k_count_min3<<<grid_for(pr.n_reads, 128, 32), 128, 0, st>>>(fq, pr.seq_off, pr.seq_len, 0, pr.n_reads, k,
+        (mp::count_launch(), (k >= 17 ? k_count_min3<true> : k_count_min3<false>)<<<grid_for(pr.n_reads, 128, 32), 128, 0, st>>>(fq, pr.seq_off, pr.seq_len, 0, pr.n_reads, k,
                                                                           chunk_rec, nchunks, cc, glob, err));
     else if (pr.max_len > (uint32_t)k) {
         const ReadTiles t = read_tiles(fq, pr, k, std::min<uint32_t>(pr.max_len, (uint32_t)MAX_READ_COUNT), CT_THREADS, 4096);
@@ -391,7 +514,8 @@ void launch_enum_count(const uint8_t *fq, const ParsedReads &pr, int k, int min3
                        uint32_t *cnt, uint32_t *err, cudaStream_t st)
 {
     if (min3)
-        (mp::count_launch(), k_enum_min3<false><<<grid_for(pr.n_reads, 128, 32), 128, 0, st>>>(
+        (mp::count_launch(), (k >= 17 ? k_enum_min3<false, true> : k_enum_min3<false, false>)<<<grid_for(pr.n_reads, 128, 32), 128, 0,
+                                                                                               st>>>(
             fq, pr.seq_off, pr.seq_len, pr.n_reads, k, lo, hi, nullptr, nullptr, cnt, nullptr, nullptr, nullptr, err));
     else
         (mp::count_launch(), k_enum_plain<false><<<grid_for(pr.n_reads, 8), 256, 0, st>>>(fq, pr.seq_off, pr.seq_len, pr.n_reads, k, lo, hi,
@@ -412,11 +536,21 @@ void launch_enum_write(const uint8_t *fq, const ParsedReads &pr, int k, int min3
                        uint32_t *err, cudaStream_t st)
 {
     if (min3)
-        (mp::count_launch(), k_enum_min3<true><<<grid_for(pr.n_reads, 128, 32), 128, 0, st>>>(
+        (mp::count_launch(), (k >= 17 ? k_enum_min3<true, true> : k_enum_min3<true, false>)<<<grid_for(pr.n_reads, 128, 32), 128, 0,
+                                                                                             st>>>(
             fq, pr.seq_off, pr.seq_len, pr.n_reads, k, lo, hi, label, off, nullptr, o_lo, o_hi, o_id, err));
     else
         (mp::count_launch(), k_enum_plain<true><<<grid_for(pr.n_reads, 8), 256, 0, st>>>(fq, pr.seq_off, pr.seq_len, pr.n_reads, k, lo, hi,
                                                                     label, off, nullptr, o_lo, o_hi, o_id, err));
+}
+
+void launch_enum_min3(const uint8_t *fq, const ParsedReads &pr, int k, uint32_t lo, uint32_t hi, const uint32_t *label,
+                      unsigned long long *total, uint64_t n, uint64_t *o_lo, uint8_t *o_hi, uint32_t *o_id, uint32_t *err,
+                      cudaStream_t st)
+{
+    (mp::count_launch(), (k >= 17 ? k_enum_min3_any<true> : k_enum_min3_any<false>)<<<grid_for(pr.n_reads, EM_THREADS, 64), EM_THREADS,
+                                                                                     0, st>>>(
+        fq, pr.seq_off, pr.seq_len, pr.n_reads, k, lo, hi, label, total, n, o_lo, o_hi, o_id, err));
 }
 
 }  // namespace mp

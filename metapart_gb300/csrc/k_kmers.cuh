@@ -25,4 +25,10 @@ void launch_enum_write(const uint8_t *fq, const ParsedReads &pr, int k, int min3
                        const uint32_t *label, const uint64_t *off, uint64_t *o_lo, uint8_t *o_hi, uint32_t *o_id,
                        uint32_t *err, cudaStream_t st);
 
+// K2 of the 3-minimizer variant in one pass, for readers that need no order: the tuples (as launch_enum_write's) at places
+// counted in *total (zero before); those past n are counted and not written.
+void launch_enum_min3(const uint8_t *fq, const ParsedReads &pr, int k, uint32_t lo, uint32_t hi, const uint32_t *label,
+                      unsigned long long *total, uint64_t n, uint64_t *o_lo, uint8_t *o_hi, uint32_t *o_id, uint32_t *err,
+                      cudaStream_t st);
+
 }  // namespace mp

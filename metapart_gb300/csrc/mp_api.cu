@@ -1141,6 +1141,35 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             j->arena.release_scratch();
             continue;
         }
+        if (grouped) {  // the 3-minimizer tuples: the splits need no order, and the histogram knows their number
+            uint64_t *tl = j->arena.alloc<uint64_t>(expect + 1);
+            uint8_t *th = has_hi ? j->arena.alloc<uint8_t>(expect + 1) : nullptr;
+            uint32_t *ti = j->arena.alloc<uint32_t>(expect + 1);
+            unsigned long long *ntot = j->arena.alloc<unsigned long long>(1);
+            if (!tl || !ti || (has_hi && !th) || !ntot)
+                return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)expect);
+            unsigned long long n = 0;
+            uint32_t cerr = 0;
+            {
+                StageTimer tm(j->clk, j->st, 2);
+                MP_CUDA(cudaMemsetAsync(ntot, 0, 8, j->st));
+                launch_enum_min3(j->d_fq, j->pr, k, (uint32_t)lo, (uint32_t)hi, s ? j->d_parent : nullptr, ntot, expect, tl, th, ti,
+                                 err, j->st);
+                MP_CUDA(cudaMemcpyAsync(&n, ntot, 8, cudaMemcpyDeviceToHost, j->st));
+                MP_CUDA(cudaMemcpyAsync(&cerr, err, 4, cudaMemcpyDeviceToHost, j->st));
+                MP_CUDA(cudaStreamSynchronize(j->st));
+            }
+            if (cerr & DERR_LONG_READ) return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
+            if (cerr & DERR_TOO_MANY)
+                return set_error(MP_EUNSUP, "a read has 256 or more k-mers in scan %d (the reference counts them "
+                                            "in 8 bits, enumerateKmers.c:152)", s);
+            if (n != expect)
+                return set_error(MP_EFMT, "scan %d: %llu tuples but the histogram holds %llu", s, n, (unsigned long long)expect);
+            if (cerr) return set_error(MP_EDEVICE, "enumeration flags 0x%x", cerr);
+            if ((rc = grouped_scan(j, gs, 1, s, tl, th, ti, err, hist))) return rc;
+            j->arena.release_scratch();
+            continue;
+        }
         if ((rc = count_scans())) return rc;
         uint32_t *cnt = cnt_all ? cnt_all + (size_t)s * (N + 1) : j->arena.alloc<uint32_t>(N + 1);
         uint64_t *off = j->arena.alloc<uint64_t>(N + 2), *ntot = j->arena.alloc<uint64_t>(1);
@@ -1168,7 +1197,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             if (n != expect)
                 return set_error(MP_EFMT, "scan %d: %llu tuples but the histogram holds %llu", s, (unsigned long long)n,
                                  (unsigned long long)expect);
-            for (int b = 0; b < (grouped ? 1 : 2); b++) {
+            for (int b = 0; b < 2; b++) {
                 sb.lo[b] = j->arena.alloc<uint64_t>(n + 1);
                 sb.id[b] = j->arena.alloc<uint32_t>(n + 1);
                 sb.hi[b] = has_hi ? j->arena.alloc<uint8_t>(n + 1) : nullptr;
@@ -1187,11 +1216,6 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
                                         "enumerateKmers.c:152)", s);
         if (herr) return set_error(MP_EDEVICE, "enumeration flags 0x%x", herr);
         if (rb_rc) return set_error(rb_rc, "%s", rb_msg.c_str());
-        if (grouped) {
-            if ((rc = grouped_scan(j, gs, 1, s, sb.lo[0], sb.hi[0], sb.id[0], err, hist))) return rc;
-            j->arena.release_scratch();
-            continue;
-        }
         snprintf(name, sizeof name, "scan%d_enum.bin", s);
         if ((rc = dump_tuples(j, name, sb.lo[0], sb.hi[0], sb.id[0], n))) return rc;
         {

@@ -530,12 +530,10 @@ __global__ void __launch_bounds__(256) k_edges_warp(EdgeCtx c)
 
 // printStats compression (metapart.c:3248-3262): every non-BAD read points at its root,
 // where a BAD parent also stops the walk (unionfind.h:25-32).
-__global__ void k_compress(uint32_t *parent, uint64_t n)
+__device__ __forceinline__ uint32_t compress_one(uint32_t *parent, uint64_t x)
 {
-    const uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= n) return;
     const uint32_t p = parent[x];
-    if (p == BAD || p == x) return;
+    if (p == BAD || p == x) return (uint32_t)x;
     uint32_t y = p;
     for (uint32_t it = 0; it < UF_CAP; it++) {
         const uint32_t q = parent[y];
@@ -543,18 +541,31 @@ __global__ void k_compress(uint32_t *parent, uint64_t n)
         y = q;
     }
     parent[x] = y;
+    return y;
+}
+
+__global__ void k_compress(uint32_t *parent, uint64_t n)
+{
+    const uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (x < n) compress_one(parent, x);
 }
 
 // compSizes after a reset to 1 and printStats (metapart.c:4010-4030): 1 + non-root members.
 // Component sizes (1 + members below each root).  The reads of a large component meet in most warps,
 // so the lanes of one root add together: one atomic per root and warp instead of one per read.
-__global__ void k_sizes(const uint32_t *parent, uint64_t n, uint32_t *size)
+// COMPRESS: the parents are compressed first, else they point at their roots.
+template <bool COMPRESS>
+__global__ void k_sizes(uint32_t *parent, uint64_t n, uint32_t *size)
 {
     const uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t r = 0xFFFFFFFFu;
     if (x < n) {
-        const uint32_t p = parent[x];
-        r = (p == BAD || p == x) ? (uint32_t)x : p;
+        if (COMPRESS) {
+            r = compress_one(parent, x);
+        } else {
+            const uint32_t p = parent[x];
+            r = (p == BAD || p == x) ? (uint32_t)x : p;
+        }
     }
     const uint32_t peers = __match_any_sync(FULLW, r);
     if (x < n && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&size[r], (uint32_t)__popc(peers));
@@ -1189,28 +1200,23 @@ int mate_union(uint32_t *parent, uint64_t n_reads, uint32_t *size, DeviceArena &
     const uint32_t limit = 1000;
     const uint64_t npairs = n_reads / 2;
     MP_CUDA(cudaMemsetAsync(size, 0, n_reads * sizeof(uint32_t), st));
-    (mp::count_launch(), k_sizes<<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads, size));
+    (mp::count_launch(), k_sizes<false><<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads, size));
     uint32_t *act = arena.alloc<uint32_t>(npairs + 1), *act2 = arena.alloc<uint32_t>(npairs + 1);
     uint32_t *pra = arena.alloc<uint32_t>(npairs + 1), *prb = arena.alloc<uint32_t>(npairs + 1);
     uint32_t *big = arena.alloc<uint32_t>(npairs + 1);
     uint32_t *psa = arena.alloc<uint32_t>(npairs + 1), *psb = arena.alloc<uint32_t>(npairs + 1);
-    unsigned long long *resv = arena.alloc<unsigned long long>(n_reads);
-    unsigned long long *hold = arena.alloc<unsigned long long>(n_reads), *first = arena.alloc<unsigned long long>(n_reads);
-    uint32_t *done = arena.alloc<uint32_t>(PEC_BLOCKS * PEC_PAIRS / 32);
-    unsigned long long *gmax = arena.alloc<unsigned long long>(n_reads);
-    unsigned long long *gadd = arena.alloc<unsigned long long>(n_reads);
+    // per read: resv, hold, first, gmax, gadd; then the cluster's done bits; one clearing for all
+    const size_t cleared = 5 * n_reads + PEC_BLOCKS * PEC_PAIRS / 64;
+    unsigned long long *resv = arena.alloc<unsigned long long>(cleared);
     constexpr int RB = 8;  // rounds launched between host synchronisations
     // per round r of a batch: [4r] reserved pairs, [4r+1] pairs left for the next round, [4r+2] big-small merges;
     // [4 RB + 1] the batch's first active count
     unsigned int *cnts = arena.alloc<unsigned int>(4 * RB + 4);
-    if (!act || !act2 || !pra || !prb || !big || !psa || !psb || !resv || !hold || !first || !done || !gmax || !gadd || !cnts)
+    if (!act || !act2 || !pra || !prb || !big || !psa || !psb || !resv || !cnts)
         return set_error(MP_ENOMEM, "device memory for the mate union");
-    MP_CUDA(cudaMemsetAsync(resv, 0, n_reads * sizeof(unsigned long long), st));
-    MP_CUDA(cudaMemsetAsync(hold, 0, n_reads * sizeof(unsigned long long), st));
-    MP_CUDA(cudaMemsetAsync(first, 0, n_reads * sizeof(unsigned long long), st));
-    MP_CUDA(cudaMemsetAsync(done, 0, PEC_BLOCKS * PEC_PAIRS / 8, st));
-    MP_CUDA(cudaMemsetAsync(gmax, 0, n_reads * sizeof(unsigned long long), st));
-    MP_CUDA(cudaMemsetAsync(gadd, 0, n_reads * sizeof(unsigned long long), st));
+    unsigned long long *hold = resv + n_reads, *first = hold + n_reads, *gmax = first + n_reads, *gadd = gmax + n_reads;
+    uint32_t *done = reinterpret_cast<uint32_t *>(gadd + n_reads);
+    MP_CUDA(cudaMemsetAsync(resv, 0, cleared * sizeof(unsigned long long), st));
     (mp::count_launch(), k_pe_prepare<<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads, act, npairs));
     uint32_t nact = (uint32_t)npairs, round = 0;
     const uint32_t most_blocks = (uint32_t)pe_cluster_blocks();
@@ -1270,9 +1276,8 @@ int mate_union(uint32_t *parent, uint64_t n_reads, uint32_t *size, DeviceArena &
     }
     if (rounds_out) *rounds_out = (int)round;
     // final printStats: compress and recount (metapart.c:4026-4030)
-    (mp::count_launch(), k_compress<<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads));
     MP_CUDA(cudaMemsetAsync(size, 0, n_reads * sizeof(uint32_t), st));
-    (mp::count_launch(), k_sizes<<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads, size));
+    (mp::count_launch(), k_sizes<true><<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads, size));
     return 0;
 }
 

@@ -195,8 +195,12 @@ __device__ __forceinline__ uint32_t nl_mask16(const uint8_t *buf, uint64_t p, ui
 // Bound by its instructions, about 60 per 16 bytes (220 with every byte compared and a block scan every 4 KB): 6.2 GB
 // 2.73 -> 2.30 ms.
 __global__ void __launch_bounds__(NL_THREADS) k_nl_write(const uint8_t *buf, uint64_t n, uint32_t skip,
-                                                         const uint64_t *seg_off, uint64_t *nl_pos)
+                                                         const uint64_t *seg_off, uint64_t *nl_pos, unsigned long long *stat)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // k_records' results
+        stat[0] = ~0ull;
+        stat[1] = 0;
+    }
     constexpr int WARPS = NL_THREADS / 32, TURNS = (int)(NL_SEG / (NL_THREADS * 16));
     __shared__ uint32_t ws[WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -230,7 +234,7 @@ __global__ void __launch_bounds__(NL_THREADS) k_nl_write(const uint8_t *buf, uin
 }
 
 // Record table from the newline positions; flags quality/sequence length mismatches.
-// stat: [0] first record with a mismatch, [1] the longest sequence.
+// stat: [0] first record with a mismatch, [1] the longest sequence (both set before), [2] the end of the last record.
 __global__ void k_records(const uint64_t *nl, uint64_t n_rec, uint64_t *rec_start, uint64_t *seq_off, uint32_t *seq_len,
                           unsigned long long *stat)
 {
@@ -249,7 +253,7 @@ __global__ void k_records(const uint64_t *nl, uint64_t n_rec, uint64_t *rec_star
     seq_off[r] = sq;
     seq_len[r] = (uint32_t)sl;
     if (ql != sl || sl > 0xFFFFFFFFull) atomicMin(&stat[0], (unsigned long long)r);
-    if (r == n_rec - 1) rec_start[n_rec] = nl[4 * r + 3] + 1;
+    if (r == n_rec - 1) stat[2] = rec_start[n_rec] = nl[4 * r + 3] + 1;
 }
 
 // For each query offset: the record whose start equals it, or ~0 when no record starts there.
@@ -297,19 +301,16 @@ int parse_fastq_range(const uint8_t *d_base, uint64_t begin, uint64_t end, Parse
     if (n_nl == 0 || n_nl % 4) return set_error(MP_EFMT, "FASTQ line count %llu is not a multiple of 4", (unsigned long long)n_nl);
     uint64_t *nl = arena.alloc<uint64_t>(n_nl);
     if (!nl) return set_error(MP_ENOMEM, "device memory for newline positions");
-    (mp::count_launch(), k_nl_write<<<(unsigned)segs, NL_THREADS, 0, st>>>(d_buf, na, skip, seg_off, nl));
     const uint64_t n_rec = n_nl / 4;
     pr->n_reads = n_rec;
     pr->rec_start = arena.alloc_persistent<uint64_t>(n_rec + 1);
     pr->seq_off = arena.alloc_persistent<uint64_t>(n_rec);
     pr->seq_len = arena.alloc_persistent<uint32_t>(n_rec);
-    unsigned long long *bad = arena.alloc<unsigned long long>(2);
+    unsigned long long *bad = arena.alloc<unsigned long long>(3);
     if (!pr->rec_start || !pr->seq_off || !pr->seq_len || !bad) return set_error(MP_ENOMEM, "device memory for the record table");
-    MP_CUDA(cudaMemsetAsync(bad, 0xFF, sizeof *bad, st));
-    MP_CUDA(cudaMemsetAsync(bad + 1, 0, sizeof *bad, st));
+    (mp::count_launch(), k_nl_write<<<(unsigned)segs, NL_THREADS, 0, st>>>(d_buf, na, skip, seg_off, nl, bad));
     (mp::count_launch(), k_records<<<(unsigned)((n_rec + 255) / 256), 256, 0, st>>>(nl, n_rec, pr->rec_start, pr->seq_off, pr->seq_len, bad));
-    MP_CUDA(cudaMemcpyAsync(&rb[1], bad, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    MP_CUDA(cudaMemcpyAsync(&rb[3], pr->rec_start + n_rec, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    MP_CUDA(cudaMemcpyAsync(&rb[1], bad, 3 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));
     const uint64_t hb[2] = {rb[1], rb[2]}, last_end = rb[3];
     MP_CUDA(cudaGetLastError());

@@ -269,12 +269,12 @@ int range_bounds(const uint64_t *hist, const uint64_t *ltr, int T, uint64_t scan
 }
 
 // Makes the pages of a caller's array present before the GPU copies into it: a page first touched by the copy costs about
-// 20 us, by the host 1.  The bytes stay as they are.
+// 20 us, by the host 1.  The bytes stay as they are; one access that writes (a read first would map the shared zero page).
 void touch_pages(void *p, size_t bytes)
 {
-    volatile char *c = static_cast<volatile char *>(p);
-    for (size_t i = 0; i < bytes; i += 4096) c[i] = c[i];
-    if (bytes) c[bytes - 1] = c[bytes - 1];
+    unsigned char *c = static_cast<unsigned char *>(p);
+    for (size_t i = 0; i < bytes; i += 4096) __atomic_fetch_or(c + i, (unsigned char)0, __ATOMIC_RELAXED);
+    if (bytes) __atomic_fetch_or(c + bytes - 1, (unsigned char)0, __ATOMIC_RELAXED);
 }
 
 int chunk_records(mp_job *j, const uint64_t *chunk_starts, int nchunks, std::vector<uint64_t> &rec)

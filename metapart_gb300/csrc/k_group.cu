@@ -673,7 +673,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
             ac[j] = (uint32_t)key[j] & 63u;
             if (j * THREADS + tid < cnt) {
                 const unsigned long long k = key[j] >> 6;
-                uint32_t h = key_hash(k) >> (32 - SLOT_BITS);
+                const uint32_t kh = key_hash(k), step = kh | 1u;
+                uint32_t h = kh >> (32 - SLOT_BITS);
                 for (;;) {
                     unsigned long long v = vkey[h];
                     if (v == EMPTY) {
@@ -681,7 +682,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
                         if (v == EMPTY) v = k;
                     }
                     if (v == k) break;
-                    h = (h + 1) & SMASK;
+                    h = (h + step) & SMASK;
                 }
                 const uint32_t bi = ac[j] & 7u, ai = ac[j] >> 3;
                 const uint32_t m = (bi < 7u ? 0x10000u << bi : 0u) | (ai < 7u ? 0x800000u << ai : 0u);

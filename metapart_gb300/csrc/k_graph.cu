@@ -579,16 +579,142 @@ __global__ void k_sizes(uint32_t *parent, uint64_t n, uint32_t *size)
 // depends on earlier pairs only through the small (<= limit) roots it touches, so in each
 // round a pair commits when it is the earliest remaining pair on each of its small roots;
 // large roots are shared: merging small components into a large one commutes.
-__global__ void k_pe_prepare(uint32_t *parent, uint64_t n, uint32_t *active, uint64_t npairs)
+//
+// Waiting pairs sleep.  A reservation holds until its pair is done: hold[x] is the first live pair of small root x, which
+// alone may merge x, so pairs on x have nothing to look at before that pair's bit in the bitmap of done pairs is set.
+// The pairs of both roots of a merge then wake together and reserve the new one.  (With every pair finding its roots and
+// reserving them again in every round, 3M reads took 32 rounds of 40 us and a tail of 9 us a round, nearly all of it for
+// pairs behind the few hundred of one component.)
+//
+// A single is a root of one read (or of one BAD read): its own pair is the only one that touches it, so a pair of a
+// single and a small component X merges whatever X's size, and matters to X's other pairs only through X's size.  All
+// pairs of X and singles that come before hold[X] therefore commit in one round, as if in order; they reserve nothing
+// (first[X] keeps the pair hold[X] back for that round).  One a round they were half of 1M reads' 152 rounds.
+struct PeArrays {
+    uint32_t *parent, *size;
+    unsigned long long *hold, *first;  // by root: the pair that holds it (pe_hold_key), this round's first pair with a single
+    unsigned long long *gmax, *gadd;   // by root: the largest root that joins it this round, the sizes that do
+    uint32_t *done;                    // a bit per pair (in the cluster: per place in its list)
+    uint32_t limit;
+};
+constexpr uint32_t PE_NONE = 0xFFFFFFFFu;
+// a pair's flags: not done, awake, which ends are small, which a single beside a small root, to join a shared root
+constexpr unsigned PE_LIVE = 1, PE_AWAKE = 2, PE_SA = 4, PE_SB = 8, PE_OA = 16, PE_OB = 32, PE_GROUP = 64;
+
+__global__ void k_pe_prepare(uint32_t *parent, uint64_t n, uint32_t *active, uint8_t *fl, uint64_t npairs)
 {
     const uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x < n && parent[x] == BAD) parent[x] = (uint32_t)x;  // a BAD read acts as its own root
-    if (x < npairs) active[x] = (uint32_t)x;
+    if (x < npairs) {
+        active[x] = (uint32_t)x;
+        fl[x] = PE_LIVE | PE_AWAKE;
+    }
 }
 
-__device__ __forceinline__ unsigned long long resv_key(uint32_t round, uint32_t j)
+// Earlier pairs have larger stamps; later rounds' are larger than any before.
+__device__ __forceinline__ unsigned long long pe_stamp(uint32_t round, uint32_t j)
 {
     return ((unsigned long long)round << 32) | (0xFFFFFFFFu - j);
+}
+
+// Earlier pairs have larger keys; the low half is the pair's bit in the bitmap.
+__device__ __forceinline__ unsigned long long pe_hold_key(uint32_t j, uint32_t bit)
+{
+    return ((unsigned long long)(0xFFFFFFFFu - j) << 32) | bit;
+}
+
+__device__ __forceinline__ bool pe_done(const uint32_t *done, uint32_t bit) { return (done[bit >> 5] >> (bit & 31)) & 1u; }
+
+__device__ __forceinline__ unsigned pe_flags(uint32_t za, uint32_t zb, uint32_t limit)
+{
+    const bool sa = za <= limit, sb = zb <= limit;
+    return (sa ? PE_SA : 0) | (sb ? PE_SB : 0) | (za <= 1 && zb > 1 && sb ? PE_OA : 0) | (zb <= 1 && za > 1 && sa ? PE_OB : 0);
+}
+
+// Key for a small root (none: key 0): over none, a later pair's key or that of a pair done before this round.
+__device__ __forceinline__ void pe_hold(unsigned long long *hold, unsigned long long key, const uint32_t *done)
+{
+    unsigned long long v = __ldcg(hold);
+    if (v && pe_done(done, (uint32_t)v)) {
+        const unsigned long long u = atomicCAS(hold, v, key);
+        if (u == v) return;
+        v = u;  // of this round
+    }
+    if (v < key) atomicMax(hold, key);
+}
+
+__device__ __forceinline__ void pe_reserve_ends(const PeArrays &c, unsigned f, uint32_t xa, uint32_t xb, unsigned long long key,
+                                                unsigned long long stamp, const uint32_t *done)
+{
+    if (f & (PE_OA | PE_OB)) {
+        const uint32_t x = f & PE_OA ? xb : xa;
+        atomicMax(&c.first[x], stamp);
+        pe_hold(&c.hold[x], 0, done);
+        return;
+    }
+    if (f & PE_SA) pe_hold(&c.hold[xa], key, done);
+    if (f & PE_SB) pe_hold(&c.hold[xb], key, done);
+}
+
+// Whether the pair commits: it holds its small roots, or, with a single, comes before the pair that holds the other
+// root.  If not, the pairs it waits for (their bits).
+__device__ __forceinline__ bool pe_decide(const PeArrays &c, unsigned f, uint32_t xa, uint32_t xb, unsigned long long key,
+                                          unsigned long long stamp, uint32_t &ha, uint32_t &hb)
+{
+    const unsigned long long va = __ldcg(&c.hold[xa]), vb = __ldcg(&c.hold[xb]);
+    const unsigned long long wa = __ldcg(&c.first[xa]), wb = __ldcg(&c.first[xb]);
+    ha = hb = PE_NONE;
+    bool ok = true;
+    if (f & (PE_OA | PE_OB)) {
+        const unsigned long long v = f & PE_OA ? vb : va;
+        if (v > key) ha = (uint32_t)v;
+        return v < key;
+    }
+    if (f & PE_SA) {
+        if (va != key) ha = (uint32_t)va;
+        ok = va == key && wa < stamp;
+    }
+    if (f & PE_SB) {
+        if (vb != key) hb = (uint32_t)vb;
+        ok = ok && vb == key && wb < stamp;
+    }
+    return ok;
+}
+
+// Two small roots merge at once (returns false); a single or a small root x joins g with the others of that root.
+__device__ __forceinline__ bool pe_commit(const PeArrays &c, unsigned f, uint32_t xa, uint32_t xb, uint32_t round, uint32_t &g, uint32_t &x)
+{
+    const uint32_t za = __ldcg(c.size + xa), zb = __ldcg(c.size + xb);  // (of a small root held here, as they were)
+    if ((f & (PE_SA | PE_SB)) == (PE_SA | PE_SB) && !(f & (PE_OA | PE_OB))) {
+        const uint32_t hi = max(xa, xb), lo = min(xa, xb);
+        c.parent[lo] = hi;
+        c.size[hi] = za + zb;
+        c.size[lo] = 0;
+        return false;
+    }
+    const bool a = (f & PE_SA) && !(f & PE_OB);  // a is the end that joins
+    g = a ? xb : xa;
+    x = a ? xa : xb;
+    atomicMax(&c.gmax[g], ((unsigned long long)round << 32) | x);
+    atomicAdd(&c.gadd[g], (unsigned long long)(a ? za : zb));
+    return true;
+}
+
+__device__ __forceinline__ void pe_join(const PeArrays &c, uint32_t g, uint32_t x)
+{
+    const uint32_t mx = (uint32_t)(__ldcg(&c.gmax[g]) & 0xFFFFFFFFu), R = max(mx, g);
+    if (x != mx) {
+        c.parent[x] = R;
+        c.size[x] = 0;
+        return;
+    }
+    // the group's one writer; a small root's first pair holds the new one as well
+    const uint32_t tot = __ldcg(&c.size[g]) + (uint32_t)__ldcg(&c.gadd[g]);
+    if (R != g) c.hold[R] = __ldcg(&c.hold[g]);
+    c.parent[R != g ? g : x] = R;
+    c.size[R != g ? g : x] = 0;
+    c.size[R] = tot;
+    c.gadd[g] = 0;
 }
 
 // The round kernels read their list lengths from device memory (written by the previous kernel),
@@ -607,122 +733,87 @@ __device__ __forceinline__ void warp_append(uint32_t *list, unsigned int *count,
     if (pred) list[base + __popc(m & ((1u << lane) - 1))] = v;
 }
 
-__global__ void k_pe_reserve(uint32_t *parent, const uint32_t *size, const uint32_t *act, const unsigned int *nact_p,
-                             uint32_t *act2, unsigned int *nact2, uint32_t *pra, uint32_t *prb, uint32_t *psa,
-                             uint32_t *psb, unsigned long long *resv, uint32_t round, uint32_t limit)
+struct PePairs {  // by pair: its ends' roots when it was last awake, the pairs it sleeps behind, flags
+    uint32_t *xa, *xb, *ha, *hb;
+    uint8_t *fl;
+};
+
+// The pairs of act that are awake to the list awake, the others to next.
+__global__ void k_pe_reserve(PeArrays c, PePairs s, const uint32_t *act, const unsigned int *nact_p, uint32_t *awake,
+                             unsigned int *nawake, uint32_t *next, unsigned int *nnext, uint32_t round)
 {
     const uint32_t nact = *nact_p;
     const int lane = threadIdx.x & 31;
     for (uint32_t w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < nact; w0 += gridDim.x * blockDim.x) {
         const uint32_t t = w0 + lane;
-        bool keep = false, sa = false, sb = false;
-        uint32_t j = 0, ra = 0, rb = 0;
-        if (t < nact) {
-            j = act[t];
-            ra = 2 * j;
-            rb = 2 * j + 1;
-            uf_find2(parent, ra, rb);
-            if (ra != rb) {
-                const uint32_t za = size[ra], zb = size[rb];
-                sa = za <= limit;
-                sb = zb <= limit;
-                keep = sa || sb;
-                if (keep) {
-                    pra[j] = ra;
-                    prb[j] = rb;
-                    psa[j] = za;  // sizes at the start of the round: the commit kernel changes sizes while it runs
-                    psb[j] = zb;
-                }
-            }
-        }
-        warp_append(act2, nact2, keep, j, lane);
-        if (keep) {
-            const unsigned long long key = resv_key(round, j);
-            if (sa) atomicMax(&resv[ra], key);
-            if (sb) atomicMax(&resv[rb], key);
-        }
-    }
-}
-
-// The commit of pair j: 0 = committed a small-small merge, 1 = back to the next round's list,
-// 2 = a small root under a large one (to k_pe_bigsmall).
-__device__ __forceinline__ int pe_commit_one(uint32_t *parent, uint32_t *size, uint32_t j, uint32_t *pra, uint32_t *prb,
-                                             const uint32_t *psa, const uint32_t *psb, const unsigned long long *resv,
-                                             unsigned long long *gmax, unsigned long long *gadd, uint32_t round,
-                                             uint32_t limit)
-{
-    const uint32_t ra = pra[j], rb = prb[j];
-    const uint32_t za = psa[j], zb = psb[j];
-    const bool sa = za <= limit, sb = zb <= limit;
-    const unsigned long long key = resv_key(round, j);
-    const bool own = (!sa || resv[ra] == key) && (!sb || resv[rb] == key);
-    if (!own) return 1;
-    if (sa && sb) {
-        const uint32_t hi = ra > rb ? ra : rb, lo = ra > rb ? rb : ra;
-        parent[lo] = hi;
-        size[hi] = za + zb;
-        size[lo] = 0;
-        return 0;
-    }
-    const uint32_t g = sa ? rb : ra, x = sa ? ra : rb;
-    atomicMax(&gmax[g], ((unsigned long long)round << 32) | x);
-    atomicAdd(&gadd[g], (unsigned long long)(sa ? za : zb));
-    pra[j] = g;  // k_pe_bigsmall reads the roles from here: sizes change while it runs
-    prb[j] = x;
-    return 2;
-}
-
-__global__ void k_pe_commit(uint32_t *parent, uint32_t *size, const uint32_t *act, const unsigned int *nact_p, uint32_t *next,
-                            unsigned int *nnext, uint32_t *pra, uint32_t *prb, const uint32_t *psa,
-                            const uint32_t *psb, const unsigned long long *resv, unsigned long long *gmax, unsigned long long *gadd,
-                            uint32_t *bigsmall, unsigned int *nbig, uint32_t round, uint32_t limit)
-{
-    const uint32_t nact = *nact_p;
-    const int lane = threadIdx.x & 31;
-    for (uint32_t w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < nact; w0 += gridDim.x * blockDim.x) {
-        const uint32_t t = w0 + lane;
-        int r = -1;
+        bool up = false, keep = false;
         uint32_t j = 0;
         if (t < nact) {
             j = act[t];
-            r = pe_commit_one(parent, size, j, pra, prb, psa, psb, resv, gmax, gadd, round, limit);
+            up = s.fl[j] & PE_AWAKE;
+            if (!up) {
+                const uint32_t ha = s.ha[j], hb = s.hb[j];
+                up = (ha != PE_NONE && pe_done(c.done, ha)) || (hb != PE_NONE && pe_done(c.done, hb));
+            }
+            keep = true;
+            if (up) {
+                uint32_t xa = 2 * j, xb = 2 * j + 1;
+                uf_find2(c.parent, xa, xb);
+                const unsigned f = xa == xb ? 0u : pe_flags(c.size[xa], c.size[xb], c.limit);
+                keep = f & (PE_SA | PE_SB);
+                if (keep) {
+                    s.xa[j] = xa;
+                    s.xb[j] = xb;
+                    s.fl[j] = (uint8_t)(PE_LIVE | PE_AWAKE | f);
+                    pe_reserve_ends(c, f, xa, xb, pe_hold_key(j, j), pe_stamp(round, j), c.done);
+                } else {
+                    atomicOr(c.done + (j >> 5), 1u << (j & 31));
+                }
+            }
         }
-        warp_append(next, nnext, r == 1, j, lane);
-        warp_append(bigsmall, nbig, r == 2, j, lane);
+        warp_append(awake, nawake, keep && up, j, lane);
+        warp_append(next, nnext, keep && !up, j, lane);
     }
 }
 
-__device__ __forceinline__ void pe_bigsmall_one(uint32_t *parent, uint32_t *size, uint32_t j, const uint32_t *pra,
-                                                const uint32_t *prb, const unsigned long long *gmax,
-                                                unsigned long long *gadd)
+__global__ void k_pe_commit(PeArrays c, PePairs s, const uint32_t *awake, const unsigned int *nawake_p, uint32_t *next,
+                            unsigned int *nnext, uint32_t *group, unsigned int *ngroup, uint32_t round)
 {
-    const uint32_t g = pra[j], x = prb[j];
-    const uint32_t mx = (uint32_t)(gmax[g] & 0xFFFFFFFFu);
-    const uint32_t R = mx > g ? mx : g;
-    if (x != mx) {  // not the designated pair of g
-        parent[x] = R;
-        size[x] = 0;
-        return;
+    const uint32_t n = *nawake_p;
+    const int lane = threadIdx.x & 31;
+    for (uint32_t w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < n; w0 += gridDim.x * blockDim.x) {
+        const uint32_t t = w0 + lane;
+        bool ok = false, join = false;
+        uint32_t j = 0;
+        if (t < n) {
+            j = awake[t];
+            const unsigned f = s.fl[j];
+            const uint32_t xa = s.xa[j], xb = s.xb[j];
+            uint32_t ha, hb, g, x;
+            ok = pe_decide(c, f, xa, xb, pe_hold_key(j, j), pe_stamp(round, j), ha, hb);
+            if (ok) {
+                atomicOr(c.done + (j >> 5), 1u << (j & 31));
+                join = pe_commit(c, f, xa, xb, round, g, x);
+                if (join) {
+                    s.xa[j] = g;
+                    s.xb[j] = x;
+                }
+            } else {
+                s.ha[j] = ha;
+                s.hb[j] = hb;
+                if (ha != PE_NONE || hb != PE_NONE) s.fl[j] = (uint8_t)(f & ~PE_AWAKE);
+            }
+        }
+        warp_append(next, nnext, t < n && !ok, j, lane);
+        warp_append(group, ngroup, join, j, lane);
     }
-    // designated pair (largest small root of g this round): finish the merge of g's group
-    const uint32_t tot = size[g] + (uint32_t)gadd[g];
-    if (R != g) {  // x is the new root
-        parent[g] = R;
-        size[g] = 0;
-    } else {       // g stays the root: x goes under it like the others
-        parent[x] = R;
-        size[x] = 0;
-    }
-    size[R] = tot;
-    gadd[g] = 0;
 }
 
-__global__ void k_pe_bigsmall(uint32_t *parent, uint32_t *size, const uint32_t *list, const unsigned int *nl_p,
-                              const uint32_t *pra, const uint32_t *prb, const unsigned long long *gmax, unsigned long long *gadd)
+__global__ void k_pe_join(PeArrays c, PePairs s, const uint32_t *list, const unsigned int *nl_p)
 {
     const uint32_t nl = *nl_p;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nl; t += gridDim.x * blockDim.x)
-        pe_bigsmall_one(parent, size, list[t], pra, prb, gmax, gadd);
+        pe_join(c, s.xa[list[t]], s.xb[list[t]]);
 }
 
 // All remaining rounds in one cluster of blocks: the steps of a round are parted by cluster barriers (hardware, about a
@@ -730,43 +821,10 @@ __global__ void k_pe_bigsmall(uint32_t *parent, uint32_t *size, const uint32_t *
 // between them took 14-21 us a round for 24,000 to 75,000 pairs.  Parents and sizes change under the kernel and are read
 // from L2.
 //
-// Waiting pairs sleep.  Scattered loads and atomics of 16 SMs bound a round in which every pair finds its roots and
-// reserves them again (9 us for 24,000 pairs, nearly all of them behind the few hundred pairs of one component).  Here a
-// reservation holds until its pair is done: hold[x] is the first live pair of small root x, which alone may merge x, so
-// pairs on x have nothing to look at before that pair's bit in the bitmap of done pairs is set.  The pairs of both roots
-// of a merge then wake together and reserve the new one.
-//
-// A single is a root of one read (or of one BAD read): its own pair is the only one that touches it, so a pair of a
-// single and a small component X merges whatever X's size, and matters to X's other pairs only through X's size.  All
-// pairs of X and singles that come before hold[X] therefore commit in one round, as if in order; they reserve nothing
-// (first[X] keeps the pair hold[X] back for that round).  One a round they were half of 1M reads' 152 rounds.
-//
-// What is left of a round is four dependent trips to L2 and three barriers, 7 us.  Mate union of 1M reads 3.1 -> 1.2 ms, of
-// 100k 1.08 -> 0.54 ms.
+// What is left of a round is about eight dependent trips to L2 and three barriers, 7 us.  Mate union, with the sleeping pairs
+// above: 100k reads 1.08 -> 0.52 ms, 1M 3.1 -> 1.07, 3M 5 -> 2.4, 20M 8 -> 6.3.
 constexpr int PEC_THREADS = 1024, PEC_ITEMS = 8, PEC_PAIRS = PEC_THREADS * PEC_ITEMS, PEC_BLOCKS = 16;
-constexpr uint32_t PEC_NONE = 0xFFFFFFFFu;
 constexpr unsigned PEC_COMMITTED = 1u << 20;  // above any count of pairs
-
-// Earlier pairs have larger keys; the low half is the pair's place in the list.
-__device__ __forceinline__ unsigned long long pe_hold_key(uint32_t j, uint32_t t)
-{
-    return ((unsigned long long)(0xFFFFFFFFu - j) << 32) | t;
-}
-
-// an item's flags
-constexpr unsigned PE_LIVE = 1, PE_AWAKE = 2, PE_SA = 4, PE_SB = 8, PE_OA = 16, PE_OB = 32, PE_GROUP = 64;
-
-// Key for a small root: over none, an earlier key or that of a pair that is done (the done ones before this round).
-__device__ __forceinline__ void pe_hold(unsigned long long *hold, unsigned long long key, const uint32_t *done)
-{
-    unsigned long long v = __ldcg(hold);
-    if (v && (done[(uint32_t)v >> 5] >> ((uint32_t)v & 31) & 1u)) {
-        const unsigned long long u = atomicCAS(hold, v, key);
-        if (u == v) return;
-        v = u;  // of this round
-    }
-    if (v < key) atomicMax(hold, key);
-}
 
 struct PeState {
     uint32_t pj[PEC_PAIRS];                // the pair
@@ -792,12 +850,10 @@ __device__ __forceinline__ void pe_sync()
 }
 
 struct PeCluster {
-    uint32_t *parent, *size;
+    PeArrays a;
     const uint32_t *act;
     uint32_t nact;
-    unsigned long long *hold, *first, *gmax, *gadd;
-    uint32_t *done;                           // a bit per place in act, clear
-    uint32_t round, limit, batch, max_round;  // rounds so far; ends are looked for as in batches of this many launched rounds
+    uint32_t round, batch, max_round;  // rounds so far; ends are looked for as in batches of this many launched rounds
     unsigned int *out;                        // [0] the last round, [1] pairs left when max_round came first
 };
 
@@ -821,7 +877,7 @@ __global__ void __launch_bounds__(PEC_THREADS, 1) k_pe_cluster(PeCluster c)
         s.pj[l] = j;
         s.xa[l] = 2 * j;
         s.xb[l] = 2 * j + 1;
-        s.ha[l] = s.hb[l] = PEC_NONE;
+        s.ha[l] = s.hb[l] = PE_NONE;
         s.fl[l] = PE_LIVE | PE_AWAKE;
         s.awake[l] = (uint16_t)l;
     }
@@ -838,88 +894,52 @@ __global__ void __launch_bounds__(PEC_THREADS, 1) k_pe_cluster(PeCluster c)
             const uint32_t l = s.awake[i], j = s.pj[l];
             uint32_t xa = s.xa[l], xb = s.xb[l], za = 0, zb = 0;
             for (uint32_t it = 0; it < UF_CAP; it++) {
-                const uint32_t pa = __ldcg(c.parent + xa), pb = __ldcg(c.parent + xb);
-                za = __ldcg(c.size + xa);
-                zb = __ldcg(c.size + xb);
+                const uint32_t pa = __ldcg(c.a.parent + xa), pb = __ldcg(c.a.parent + xb);
+                za = __ldcg(c.a.size + xa);
+                zb = __ldcg(c.a.size + xb);
                 const bool end = pa == pb || (pa == xa && pb == xb);
                 xa = pa;
                 xb = pb;
                 if (end) break;
             }
-            const bool sa = za <= c.limit, sb = zb <= c.limit;
-            if (xa == xb || !(sa || sb)) {
-                const uint32_t t = l * nb + me;
+            const unsigned f = xa == xb ? 0u : pe_flags(za, zb, c.a.limit);
+            const uint32_t t = l * nb + me;
+            if (!(f & (PE_SA | PE_SB))) {
                 s.fl[l] = 0;
                 atomicSub(&s.live, 1u);
-                atomicOr(c.done + (t >> 5), 1u << (t & 31));
+                atomicOr(c.a.done + (t >> 5), 1u << (t & 31));
                 continue;
             }
             s.xa[l] = xa;
             s.xb[l] = xb;
-            const bool oa = za <= 1 && zb > 1 && sb, ob = zb <= 1 && za > 1 && sa;
-            s.fl[l] = (uint8_t)(PE_LIVE | PE_AWAKE | (sa ? PE_SA : 0) | (sb ? PE_SB : 0) | (oa ? PE_OA : 0) | (ob ? PE_OB : 0));
-            if (oa || ob) {
-                atomicMax(&c.first[oa ? xb : xa], resv_key(round, j));
-            } else {
-                const unsigned long long key = pe_hold_key(j, l * nb + me);
-                if (sa) pe_hold(&c.hold[xa], key, s.done);
-                if (sb) pe_hold(&c.hold[xb], key, s.done);
-            }
+            s.fl[l] = (uint8_t)(PE_LIVE | PE_AWAKE | f);
+            pe_reserve_ends(c.a, f, xa, xb, pe_hold_key(j, t), pe_stamp(round, j), s.done);
         }
         pe_sync();
-        // a pair commits when it holds its small roots, or, with a single, comes before the pair that holds the other root;
-        // two small roots merge at once, a single or a small root beside a large one with the others of that root
+        // commits
         bool any_group = false, any_commit = false;
         for (uint32_t i = threadIdx.x; i < nawake; i += PEC_THREADS) {
             const uint32_t l = s.awake[i], t = l * nb + me;
             const unsigned f = s.fl[l];
             if (!(f & PE_LIVE)) continue;
             const uint32_t j = s.pj[l], xa = s.xa[l], xb = s.xb[l];
-            const unsigned long long key = pe_hold_key(j, t), stamp = resv_key(round, j);
-            const unsigned long long va = __ldcg(&c.hold[xa]), vb = __ldcg(&c.hold[xb]);
-            const unsigned long long wa = __ldcg(&c.first[xa]), wb = __ldcg(&c.first[xb]);
-            const uint32_t za = __ldcg(c.size + xa), zb = __ldcg(c.size + xb);  // (of a small root held here, as they were)
-            uint32_t ha = PEC_NONE, hb = PEC_NONE;
-            bool ok = true;
-            if (f & (PE_OA | PE_OB)) {
-                unsigned long long v = f & PE_OA ? vb : va;
-                if (v && (s.done[(uint32_t)v >> 5] >> ((uint32_t)v & 31) & 1u)) v = 0;
-                if (v > key) ha = (uint32_t)v;
-                ok = v < key;
-            } else {
-                if (f & PE_SA) {
-                    if (va != key) ha = (uint32_t)va;
-                    ok = va == key && wa < stamp;
-                }
-                if (f & PE_SB) {
-                    if (vb != key) hb = (uint32_t)vb;
-                    ok = ok && vb == key && wb < stamp;
-                }
-            }
-            if (!ok) {
+            uint32_t ha, hb, g, x;
+            if (!pe_decide(c.a, f, xa, xb, pe_hold_key(j, t), pe_stamp(round, j), ha, hb)) {
                 s.ha[l] = ha;
                 s.hb[l] = hb;
-                if (ha != PEC_NONE || hb != PEC_NONE) s.fl[l] = (uint8_t)(f & ~PE_AWAKE);
+                if (ha != PE_NONE || hb != PE_NONE) s.fl[l] = (uint8_t)(f & ~PE_AWAKE);
                 continue;
             }
             any_commit = true;
             atomicSub(&s.live, 1u);
-            atomicOr(c.done + (t >> 5), 1u << (t & 31));
-            if ((f & (PE_SA | PE_SB)) == (PE_SA | PE_SB) && !(f & (PE_OA | PE_OB))) {
-                const uint32_t hi = max(xa, xb), lo = min(xa, xb);
-                c.parent[lo] = hi;
-                c.size[hi] = za + zb;
-                c.size[lo] = 0;
-                s.fl[l] = 0;
-            } else {
-                const bool a = (f & PE_SA) && !(f & PE_OB);  // a is the end that joins
-                const uint32_t g = a ? xb : xa, x = a ? xa : xb;
-                atomicMax(&c.gmax[g], ((unsigned long long)round << 32) | x);
-                atomicAdd(&c.gadd[g], (unsigned long long)(a ? za : zb));
+            atomicOr(c.a.done + (t >> 5), 1u << (t & 31));
+            if (pe_commit(c.a, f, xa, xb, round, g, x)) {
                 s.xa[l] = g;
                 s.xb[l] = x;
                 s.fl[l] = PE_GROUP;
                 any_group = true;
+            } else {
+                s.fl[l] = 0;
             }
         }
         any_group = __syncthreads_or(any_group);
@@ -935,7 +955,7 @@ __global__ void __launch_bounds__(PEC_THREADS, 1) k_pe_cluster(PeCluster c)
         }
         pe_sync();
         const unsigned left = s.state[slot] % PEC_COMMITTED;
-        const bool last = (round - c.round) % c.batch == 0;
+        const bool last = round % c.batch == 0;
         if (left == 0 || (last && round + c.batch > c.max_round)) {
             // (a round that committed pairs is followed by the one that finds none left, unless a batch ends with it)
             if (first) {
@@ -949,25 +969,12 @@ __global__ void __launch_bounds__(PEC_THREADS, 1) k_pe_cluster(PeCluster c)
                 const uint32_t l = s.awake[i];
                 if (!(s.fl[l] & PE_GROUP)) continue;
                 s.fl[l] = 0;
-                const uint32_t g = s.xa[l], x = s.xb[l];
-                const uint32_t mx = (uint32_t)(__ldcg(&c.gmax[g]) & 0xFFFFFFFFu), R = max(mx, g);
-                if (x != mx) {
-                    c.parent[x] = R;
-                    c.size[x] = 0;
-                    continue;
-                }
-                // the group's one writer; a small root's first pair holds the new one as well
-                const uint32_t tot = __ldcg(&c.size[g]) + (uint32_t)__ldcg(&c.gadd[g]);
-                if (R != g) c.hold[R] = __ldcg(&c.hold[g]);
-                c.parent[R != g ? g : x] = R;
-                c.size[R != g ? g : x] = 0;
-                c.size[R] = tot;
-                c.gadd[g] = 0;
+                pe_join(c.a, s.xa[l], s.xb[l]);
             }
         }
         if (over) break;
         // who is awake in the next round
-        for (uint32_t w = threadIdx.x; w < (nact + 31) / 32; w += PEC_THREADS) s.done[w] = __ldcg(c.done + w);
+        for (uint32_t w = threadIdx.x; w < (nact + 31) / 32; w += PEC_THREADS) s.done[w] = __ldcg(c.a.done + w);
         __syncthreads();
         for (uint32_t l0 = threadIdx.x & ~31u; l0 < mine; l0 += PEC_THREADS) {
             const uint32_t l = l0 + lane;
@@ -975,7 +982,7 @@ __global__ void __launch_bounds__(PEC_THREADS, 1) k_pe_cluster(PeCluster c)
             bool up = (f & PE_LIVE) && (f & PE_AWAKE);
             if ((f & PE_LIVE) && !up) {
                 const uint32_t ha = s.ha[l], hb = s.hb[l];
-                up = (ha != PEC_NONE && (s.done[ha >> 5] >> (ha & 31) & 1u)) || (hb != PEC_NONE && (s.done[hb >> 5] >> (hb & 31) & 1u));
+                up = (ha != PE_NONE && (s.done[ha >> 5] >> (ha & 31) & 1u)) || (hb != PE_NONE && (s.done[hb >> 5] >> (hb & 31) & 1u));
             }
             const uint32_t m = __ballot_sync(FULLW, up);
             uint32_t base = 0;
@@ -1197,36 +1204,42 @@ static int pe_cluster_blocks()
 
 int mate_union(uint32_t *parent, uint64_t n_reads, uint32_t *size, DeviceArena &arena, cudaStream_t st, int *rounds_out)
 {
-    const uint32_t limit = 1000;
     const uint64_t npairs = n_reads / 2;
     MP_CUDA(cudaMemsetAsync(size, 0, n_reads * sizeof(uint32_t), st));
     (mp::count_launch(), k_sizes<false><<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads, size));
     uint32_t *act = arena.alloc<uint32_t>(npairs + 1), *act2 = arena.alloc<uint32_t>(npairs + 1);
-    uint32_t *pra = arena.alloc<uint32_t>(npairs + 1), *prb = arena.alloc<uint32_t>(npairs + 1);
-    uint32_t *big = arena.alloc<uint32_t>(npairs + 1);
-    uint32_t *psa = arena.alloc<uint32_t>(npairs + 1), *psb = arena.alloc<uint32_t>(npairs + 1);
-    // per read: resv, hold, first, gmax, gadd; then the cluster's done bits; one clearing for all
-    const size_t cleared = 5 * n_reads + PEC_BLOCKS * PEC_PAIRS / 64;
-    unsigned long long *resv = arena.alloc<unsigned long long>(cleared);
+    uint32_t *awake = arena.alloc<uint32_t>(npairs + 1), *group = arena.alloc<uint32_t>(npairs + 1);
+    PePairs s{arena.alloc<uint32_t>(npairs + 1), arena.alloc<uint32_t>(npairs + 1), arena.alloc<uint32_t>(npairs + 1),
+              arena.alloc<uint32_t>(npairs + 1), arena.alloc<uint8_t>(npairs + 1)};
     constexpr int RB = 8;  // rounds launched between host synchronisations
-    // per round r of a batch: [4r] reserved pairs, [4r+1] pairs left for the next round, [4r+2] big-small merges;
+    // per round r of a batch: [4r] pairs awake, [4r+1] pairs left for the next round, [4r+2] joins;
     // [4 RB + 1] the batch's first active count
     unsigned int *cnts = arena.alloc<unsigned int>(4 * RB + 4);
-    if (!act || !act2 || !pra || !prb || !big || !psa || !psb || !resv || !cnts)
+    // per read: hold, first, gmax, gadd; then the done bits of the pairs, or of the cluster's places; one clearing for all
+    const size_t done_words = std::max<size_t>(npairs / 32 + 1, PEC_BLOCKS * PEC_PAIRS / 32), cleared = 4 * n_reads + (done_words + 1) / 2;
+    unsigned long long *hold = arena.alloc<unsigned long long>(cleared);
+    if (!act || !act2 || !awake || !group || !s.xa || !s.xb || !s.ha || !s.hb || !s.fl || !cnts || !hold)
         return set_error(MP_ENOMEM, "device memory for the mate union");
-    unsigned long long *hold = resv + n_reads, *first = hold + n_reads, *gmax = first + n_reads, *gadd = gmax + n_reads;
-    uint32_t *done = reinterpret_cast<uint32_t *>(gadd + n_reads);
-    MP_CUDA(cudaMemsetAsync(resv, 0, cleared * sizeof(unsigned long long), st));
-    (mp::count_launch(), k_pe_prepare<<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads, act, npairs));
+    const PeArrays c{parent, size, hold, hold + n_reads, hold + 2 * n_reads, hold + 3 * n_reads,
+                     reinterpret_cast<uint32_t *>(hold + 4 * n_reads), 1000};
+    MP_CUDA(cudaMemsetAsync(hold, 0, cleared * sizeof(unsigned long long), st));
+    (mp::count_launch(), k_pe_prepare<<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads, act, s.fl, npairs));
     uint32_t nact = (uint32_t)npairs, round = 0;
     const uint32_t most_blocks = (uint32_t)pe_cluster_blocks();
     while (nact > 0) {
-        if (round + RB <= arena.lim.mate_rounds && nact <= most_blocks * (round ? PEC_PAIRS : PEC_THREADS + PEC_THREADS / 2)) {
+        // (the limit is looked at every RB rounds)
+        if (round / RB * RB + RB > arena.lim.mate_rounds)
+            return set_error(MP_EDEVICE, "mate union did not converge within %u rounds", arena.lim.mate_rounds);
+        if (nact <= most_blocks * (round ? PEC_PAIRS : PEC_THREADS + PEC_THREADS / 2)) {
             // the rest (not many fresh pairs: all of them are awake in the first round, 66 us for 50,000 on 16 SMs where a
             // launched one takes 16) in one cluster, of as few blocks as give each thread a pair (cheaper barriers)
             uint32_t cluster = 1;
             while (cluster < most_blocks && cluster * PEC_THREADS < nact) cluster *= 2;
-            PeCluster c{parent, size, act, nact, hold, first, gmax, gadd, done, round, limit, (uint32_t)RB, arena.lim.mate_rounds, cnts};
+            if (round) {  // its bits are by place
+                MP_CUDA(cudaMemsetAsync(c.hold, 0, n_reads * sizeof(unsigned long long), st));
+                MP_CUDA(cudaMemsetAsync(c.done, 0, PEC_BLOCKS * PEC_PAIRS / 8, st));
+            }
+            PeCluster pc{c, act, nact, round, (uint32_t)RB, arena.lim.mate_rounds, cnts};
             cudaLaunchConfig_t cfg{};
             cudaLaunchAttribute at{};
             at.id = cudaLaunchAttributeClusterDimension;
@@ -1238,7 +1251,7 @@ int mate_union(uint32_t *parent, uint64_t n_reads, uint32_t *size, DeviceArena &
             cfg.attrs = &at;
             cfg.numAttrs = 1;
             mp::count_launch();
-            MP_CUDA(cudaLaunchKernelEx(&cfg, k_pe_cluster, c));
+            MP_CUDA(cudaLaunchKernelEx(&cfg, k_pe_cluster, pc));
             ReadBack<unsigned int> h(arena, 2);
             MP_CUDA(cudaMemcpyAsync(h.p, cnts, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
             MP_CUDA(cudaStreamSynchronize(st));
@@ -1246,30 +1259,29 @@ int mate_union(uint32_t *parent, uint64_t n_reads, uint32_t *size, DeviceArena &
             if (h[1]) return set_error(MP_EDEVICE, "mate union did not converge within %u rounds", arena.lim.mate_rounds);
             break;
         }
-        if (round + RB > arena.lim.mate_rounds)
-            return set_error(MP_EDEVICE, "mate union did not converge within %u rounds", arena.lim.mate_rounds);
+        // two rounds leave at most half of the pairs, nearly all asleep: where that fits the cluster it takes over
+        const int rb = round == 0 && nact <= 2 * most_blocks * PEC_PAIRS ? 2 : RB - (int)(round % RB);
         // counts only shrink, so nact bounds every list of the batch
         const unsigned g = (unsigned)std::min<uint64_t>(blocks_for(nact, 256), 8ull * (uint64_t)sm_count());
         MP_CUDA(cudaMemsetAsync(cnts, 0, (4 * RB + 4) * sizeof(unsigned int), st));
         MP_CUDA(cudaMemcpyAsync(cnts + 4 * RB + 1, &nact, sizeof(unsigned int), cudaMemcpyHostToDevice, st));
-        for (int r = 0; r < RB; r++) {
+        for (int r = 0; r < rb; r++) {
             ++round;
             const unsigned int *nin = r ? cnts + 4 * (r - 1) + 1 : cnts + 4 * RB + 1;
-            (mp::count_launch(), k_pe_reserve<<<g, 256, 0, st>>>(parent, size, act, nin, act2, cnts + 4 * r, pra, prb, psa,
-                                                                 psb, resv, round, limit));
-            (mp::count_launch(), k_pe_commit<<<g, 256, 0, st>>>(parent, size, act2, cnts + 4 * r, act, cnts + 4 * r + 1, pra,
-                                                                prb, psa, psb, resv, gmax, gadd, big, cnts + 4 * r + 2,
-                                                                round, limit));
-            (mp::count_launch(), k_pe_bigsmall<<<g, 256, 0, st>>>(parent, size, big, cnts + 4 * r + 2, pra, prb, gmax, gadd));
+            (mp::count_launch(), k_pe_reserve<<<g, 256, 0, st>>>(c, s, act, nin, awake, cnts + 4 * r, act2, cnts + 4 * r + 1, round));
+            (mp::count_launch(), k_pe_commit<<<g, 256, 0, st>>>(c, s, awake, cnts + 4 * r, act2, cnts + 4 * r + 1, group,
+                                                                cnts + 4 * r + 2, round));
+            (mp::count_launch(), k_pe_join<<<g, 256, 0, st>>>(c, s, group, cnts + 4 * r + 2));
+            std::swap(act, act2);
         }
         ReadBack<unsigned int> h(arena, 4 * RB + 4);
         MP_CUDA(cudaMemcpyAsync(h.p, cnts, (4 * RB + 4) * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
         MP_CUDA(cudaStreamSynchronize(st));
-        nact = h[4 * (RB - 1) + 1];
+        nact = h[4 * (rb - 1) + 1];
         // rounds that reserved nothing leave nothing active: stop counting at the first empty one
-        for (int r = 0; r < RB; r++)
-            if (h[4 * r] == 0) {
-                round -= (uint32_t)(RB - 1 - r);
+        for (int r = 0; r < rb; r++)
+            if (h[4 * r] == 0 && h[4 * r + 1] == 0) {
+                round -= (uint32_t)(rb - 1 - r);
                 nact = 0;
                 break;
             }

@@ -5,6 +5,7 @@ the oracle at the sizes where they change: one block and more of a cluster (1,02
 The reads give the mate union what its rounds part on: components around the 1,000-read limit, many small ones, singles
 beside both, and BAD reads; the labels, sizes and all partition files are compared byte for byte.
 """
+import numpy as np
 import pytest
 
 import pipeline_util as pu
@@ -41,3 +42,31 @@ def test_mate_union_and_output_in_a_batch(built_gpu):
     with native.Context(0) as ctx:
         res, outs, fs, labs, _ = _batched(ctx, data, shapes, 27)
         _check(ctx, data, shapes, 27, res, outs, fs, labs)
+
+
+def test_output_copies_records_of_all_lengths(built_gpu):
+    """Records of 60 to 2,700 bytes (one turn of a warp and several) at every alignment: each file holds its records whole
+    and in input order, and together they are the input."""
+    rng = np.random.default_rng(3)
+    recs = []
+    for i in range(6_000):
+        L = int(rng.integers(20, 270))
+        seq = bytes(rng.choice(np.frombuffer(b"ACGT", np.uint8), L))
+        name = b"@%d " % i + b"h" * int(rng.integers(0, 40) if i % 3 else rng.integers(0, 2_100))
+        recs.append(name + b"\n" + seq + b"\n+\n" + b"I" * L + b"\n")
+    data = b"".join(recs)
+    with native.Context(0) as ctx, native.Job(ctx) as job:
+        job.load(data)
+        cnt = job.count(21, [0, len(data)])
+        job.partition(21, 1, 1, [0, len(data)], cnt.chunk_first_read, cnt.hist)
+        out, sizes = job.output()
+    at, seen = 0, []
+    for size in sizes:
+        part, last = bytes(out[at:at + int(size)]), -1
+        at += int(size)
+        while part:
+            i = int(part[1:part.index(b" ")])
+            assert i > last and part.startswith(recs[i])
+            part, last = part[len(recs[i]):], i
+            seen.append(i)
+    assert at == len(data) and sorted(seen) == list(range(len(recs)))

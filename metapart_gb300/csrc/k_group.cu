@@ -38,7 +38,7 @@ struct PlanCtx {
     const uint32_t *brk;      // a bit per bucket (from lo): a thread range starts there
     const uint32_t *seg_sh;   // per segment: its bins hold 2^seg_sh buckets
     const uint32_t *seg_bin0; // per segment: its first bin
-    uint32_t seg_lo;          // first bucket of a segment (lo, or 0 with several)
+    uint32_t seg_lo;          // where a segment's bins count from (GroupScan::anchor, or 0 with several)
 };
 
 // The bin width of a segment of n tuples over `span` buckets.  A bin of at most 1024 buckets has at most 1024 units, so
@@ -184,11 +184,12 @@ __global__ void __launch_bounds__(GP_COUNT_BLOCK) k_gp_write(PlanCtx c, const ui
     uint32_t u = (uint32_t)blk[blockIdx.x] + (uint32_t)__popc(m & ((1u << lane) - 1));  // units that start before b
     for (int w = 0; w < warp; w++) u += ws[w];
     const uint32_t seg = (uint32_t)(b / NB), rel = ((uint32_t)b & (NB - 1)) - c.seg_lo, sh = c.seg_sh[seg];
-    if ((rel & ((1u << sh) - 1)) == 0) {
+    if ((rel & ((1u << sh) - 1)) == 0 || b == c.lo) {  // (a merged scan's first bin may begin before the scan)
         const uint32_t bin = c.seg_bin0[seg] + (rel >> sh);
-        bstart[bin] = bcur[bin] = (uint32_t)s;
+        bstart[bin] = (uint32_t)s;
+        if (bcur) bcur[bin] = (uint32_t)s;
         bu0[bin] = u;
-        bfirst[bin] = (uint32_t)(b - c.lo);
+        bfirst[bin] = (uint32_t)(b - c.lo) - (rel & ((1u << sh) - 1));
         bsh[bin] = sh;
     }
     unit_of[b - c.lo] = u + (f & 1u) - 1u;  // (before the first unit: ~0)
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(GP_COUNT_BLOCK) k_gp_write(PlanCtx c, const ui
 // ------------------------------------------------------------------ split
 
 constexpr int SP_THREADS = 512, SP_ITEMS = 12, SP_TILE = SP_THREADS * SP_ITEMS;
+constexpr uint32_t SP_EXTRA = GROUP_MAX_MERGED - 1;  // digits above GP_DIGITS: a bin that a scan's bounds cut counts once more
 
 // Tiles of the second pass, every bin's own: first tuple, tuples, bin.
 __global__ void __launch_bounds__(1024) k_gp_tiles(const uint32_t *bstart, uint32_t nb, uint32_t *ctr, uint4 *tiles)
@@ -229,8 +231,8 @@ struct SplitSmem {
     uint64_t key[SP_TILE];
     uint32_t id[SP_TILE];
     uint16_t dig[SP_TILE];      // a place's digit, times 4
-    uint32_t hist[GP_DIGITS];   // tuples per digit, then the digit's first place in the tile
-    uint32_t delta[GP_DIGITS];  // global place of a digit's first tuple less its place in the tile
+    uint32_t hist[GP_DIGITS + SP_EXTRA];   // tuples per digit, then the digit's first place in the tile
+    uint32_t delta[GP_DIGITS + SP_EXTRA];  // global place of a digit's first tuple less its place in the tile
     uint32_t ws[SP_THREADS / 32];
 };
 constexpr uint32_t SP_PACKED = 4096;  // words of packed reads
@@ -248,10 +250,11 @@ __device__ __forceinline__ uint32_t &at_byte(uint32_t *p, uint32_t off) { return
 
 // Unstable, so there are no ballots and no look-back: ranks by shared-memory atomics, places by one global atomic per
 // digit and tile (the order of a digit's tuples is free; its latency passes while the tile is reordered), a
-// shared-memory reorder so that a digit's tuples are stored side by side.  rd: digit times 4 (bits 0-11) and the tuple's rank
+// shared-memory reorder so that a digit's tuples are stored side by side.  rd: digit times 4 (bits 0-15) and the tuple's rank
 // in it (16-31), or ~0 for none, as the caller's atomics on sm.hist gave them.  Returns the tile's tuples, 0 when one
-// would land past the n tuples (the histogram is not the tuples': the group kernel reports it).
-template <class LoadId>
+// would land past the n tuples (the histogram is not the tuples': the group kernel reports it).  EXTRA: with the SP_EXTRA
+// digits above GP_DIGITS.
+template <bool EXTRA, class LoadId>
 __device__ __forceinline__ uint32_t split_order(SplitSmem &sm, const uint32_t (&kl)[SP_ITEMS], const uint32_t (&kh)[SP_ITEMS],
                                                 const uint32_t (&rd)[SP_ITEMS], uint32_t *cur, uint32_t nd, LoadId load_id, uint32_t n)
 {
@@ -264,6 +267,14 @@ __device__ __forceinline__ uint32_t split_order(SplitSmem &sm, const uint32_t (&
     const uint2 c = *reinterpret_cast<const uint2 *>(&sm.hist[2 * tid]);
     const uint32_t g0 = c.x && 2 * tid < nd ? atomicAdd(&cur[2 * tid], c.x) : 0u;
     const uint32_t g1 = c.y && 2 * tid + 1 < nd ? atomicAdd(&cur[2 * tid + 1], c.y) : 0u;
+    static_assert(SP_EXTRA == 2, "two extra digits");
+    uint32_t ex = 0, ey = 0, ge = 0;  // the extra digits' tuples, the place of this thread's one
+    if constexpr (EXTRA) {
+        ex = sm.hist[GP_DIGITS];
+        ey = sm.hist[GP_DIGITS + 1];
+        const uint32_t n0 = tid ? ey : ex;
+        if (tid < 2 && n0 && GP_DIGITS + tid < nd) ge = atomicAdd(&cur[GP_DIGITS + tid], n0);
+    }
     uint32_t x = c.x + c.y;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -280,20 +291,31 @@ __device__ __forceinline__ uint32_t split_order(SplitSmem &sm, const uint32_t (&
         nv += v;
     }
     *reinterpret_cast<uint2 *>(&sm.hist[2 * tid]) = make_uint2(before, before + c.x);
+    bool past = false;
+    if constexpr (EXTRA) {
+        if (tid < 2) {
+            const uint32_t at = nv + (tid ? ex : 0u), n0 = tid ? ey : ex;
+            sm.hist[GP_DIGITS + tid] = at;
+            sm.delta[GP_DIGITS + tid] = ge - at;
+            past = n0 && (uint64_t)ge + n0 > n;
+        }
+        nv += ex + ey;
+    }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < SP_ITEMS; j++) {
         if (rd[j] != ~0u) {
-            const uint32_t d = rd[j] & 0xFFFu, p = at_byte(sm.hist, d) + (rd[j] >> 16);
+            const uint32_t d = rd[j] & 0xFFFFu, p = at_byte(sm.hist, d) + (rd[j] >> 16);
             sm.key[p] = ((uint64_t)kh[j] << 32) | kl[j];
             sm.id[p] = id[j];
             sm.dig[p] = (uint16_t)d;
         }
     }
     *reinterpret_cast<uint2 *>(&sm.delta[2 * tid]) = make_uint2(g0 - before, g1 - before - c.x);
-    return __syncthreads_or((c.x && (uint64_t)g0 + c.x > n) || (c.y && (uint64_t)g1 + c.y > n)) ? 0u : nv;
+    return __syncthreads_or(past || (c.x && (uint64_t)g0 + c.x > n) || (c.y && (uint64_t)g1 + c.y > n)) ? 0u : nv;
 }
 
+template <bool EXTRA>
 __device__ __forceinline__ void split_store(SplitSmem &sm, uint32_t nv, uint64_t *out_k, uint32_t *out_id)
 {
 #pragma unroll 4
@@ -303,6 +325,7 @@ __device__ __forceinline__ void split_store(SplitSmem &sm, uint32_t nv, uint64_t
         out_id[o] = sm.id[p];
     }
     *reinterpret_cast<uint2 *>(&sm.hist[2 * threadIdx.x]) = make_uint2(0, 0);
+    if (EXTRA && threadIdx.x < SP_EXTRA) sm.hist[GP_DIGITS + threadIdx.x] = 0;
 }
 
 // The tiles of a pass over segments: tile0[q] the segment's first tile, start[q] its first read or tuple, tile_seg the
@@ -334,6 +357,8 @@ struct BinCtx {
     SegTiles sg;
     uint64_t *out_k = nullptr;
     uint32_t *out_id = nullptr;
+    uint32_t m_digits = 0, m_sh = 0;                    // merged scans (group_bins_scans): the digits, the bins' width
+    uint64_t m_start[SP_EXTRA] = {~0ull, ~0ull};        // the first k-mer of every scan but the first, less k_lo
 };
 
 __device__ __forceinline__ void bin_tile(const BinCtx &c, uint32_t tile, uint32_t per, uint32_t all, uint32_t &seg, uint32_t &base,
@@ -354,14 +379,16 @@ __device__ __forceinline__ void bin_tile(const BinCtx &c, uint32_t tile, uint32_
 // 150 bp, 2 scans: 35.4 ms for what counting (6.1), enumerating (14.3) and a first split over 13-byte tuples (29.3) took.
 //
 // HI: 2k >= 34 and bins of at least 2^32 k-mers, so a k-mer's bin is a shift of its high word.
-template <bool HI>
+//
+// MERGED: the tuples of all scans (group_bins_scans).  Packing the reads and rolling through them was half of the pass.
+template <bool HI, bool MERGED>
 __global__ void __launch_bounds__(SP_THREADS, 2) k_split_reads(BinCtx c)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     BinSmem &sm = *reinterpret_cast<BinSmem *>(smraw);
     __shared__ uint32_t many[SP_THREADS];
     const int tid = threadIdx.x;
-    for (uint32_t d = tid; d < GP_DIGITS; d += SP_THREADS) sm.hist[d] = 0;
+    for (uint32_t d = tid; d < GP_DIGITS + SP_EXTRA; d += SP_THREADS) sm.hist[d] = 0;
     const uint32_t per = c.t.rpt, rr = tid / c.t.spr, i0 = (tid - rr * c.t.spr) * c.t.P;
     uint32_t seg, base, end;
     if (blockIdx.x < c.tiles) {
@@ -369,8 +396,8 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_reads(BinCtx c)
         rt_pack(c.t, base, end - base, sm.packed);
     }
     for (uint32_t tile = blockIdx.x; tile < c.tiles; tile += gridDim.x) {
-        const uint32_t d0 = c.seg_bin0[seg], nd = c.seg_bin0[seg + 1] - d0;
-        const int bits = c.bsh + (int)c.seg_sh[seg];  // a k-mer's bits within its bin
+        const uint32_t d0 = MERGED ? 0u : c.seg_bin0[seg], nd = MERGED ? c.m_digits : c.seg_bin0[seg + 1] - d0;
+        const int bits = c.bsh + (int)(MERGED ? c.m_sh : c.seg_sh[seg]);  // a k-mer's bits within its bin
         const uint64_t mask = (1ull << bits) - 1;
         const uint32_t r = base + rr, L = rr < per && r < end ? c.t.seq_len[r] : 0u;
         uint32_t id = r;
@@ -396,7 +423,11 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_reads(BinCtx c)
                 const uint32_t a6 = s.template adj6<j>(fw, cn, cp);
                 rd[j] = ~0u;
                 if (((s.vm >> j) & 1u) && rel < c.k_span) {
-                    const uint32_t d = HI ? (uint32_t)(rel >> 32) >> dsh : (uint32_t)(rel >> dsh);
+                    uint32_t d = HI ? (uint32_t)(rel >> 32) >> dsh : (uint32_t)(rel >> dsh);
+                    if constexpr (MERGED) {  // one more for every scan that began
+#pragma unroll
+                        for (uint32_t q = 0; q < SP_EXTRA; q++) d += rel >= c.m_start[q];
+                    }
                     if constexpr (HI) {
                         kl[j] = ((uint32_t)rel << 6) | a6;
                         kh[j] = __funnelshift_l((uint32_t)rel, (uint32_t)(rel >> 32) & mh, 6);
@@ -426,8 +457,8 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_reads(BinCtx c)
             // the reference counts a read's k-mers of one scan in 8 bits (enumerateKmers.c:152)
             if (c.check_many && got && atomicAdd(&many[rr], got) + got > 255u) atomicOr(c.err, 4u);
         }
-        const uint32_t nv = split_order(sm, kl, kh, rd, c.bcur + d0, nd, [&](int) { return id; }, c.n);
-        split_store(sm, nv, c.out_k, c.out_id);
+        const uint32_t nv = split_order<MERGED>(sm, kl, kh, rd, c.bcur + d0, nd, [&](int) { return id; }, c.n);
+        split_store<MERGED>(sm, nv, c.out_k, c.out_id);
         // the next tile's reads while others store (its bytes fetched before the stores instead cost registers that spill: 37.5
         // against 35.7 ms at 20M x 150 bp, 2 scans)
         const uint32_t next = tile + gridDim.x;
@@ -468,10 +499,10 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_tuples(BinCtx c)
                 }
             }
         }
-        const uint32_t got = split_order(
+        const uint32_t got = split_order<false>(
             sm, kl, kh, rd, c.bcur + d0, nd,
             [&](int j) { const uint32_t e = j * SP_THREADS + tid; return e < nv ? c.id[base + e] : 0u; }, c.n);
-        split_store(sm, got, c.out_k, c.out_id);
+        split_store<false>(sm, got, c.out_k, c.out_id);
     }
 }
 
@@ -488,7 +519,8 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_units(const uint64_t *_
                                                                const uint32_t *__restrict__ bin_sh,
                                                                const uint32_t *__restrict__ ub0, uint32_t *ucur,
                                                                const uint32_t *__restrict__ unit_of, uint32_t nbk,
-                                                               const uint4 *__restrict__ tile_of, uint64_t *out_k,
+                                                               const uint4 *__restrict__ tile_of, uint32_t tuple0,
+                                                               const uint32_t *__restrict__ label, uint64_t *out_k,
                                                                uint32_t *out_id)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -520,7 +552,7 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_units(const uint64_t *_
         __syncthreads();  // the tile before is stored
         if (bin != have) {
             have = bin;
-            whole = bcur[bin] == bstart[bin + 1];  // else the histogram is not the tuples' (the bin's units stay short: k_group)
+            whole = bcur[bin] - tuple0 == bstart[bin + 1];  // else the histogram is not the tuples' (the bin's units stay short: k_group)
             d0 = bu0[bin];
             nd = min(bu0[bin + 1] - d0, GP_DIGITS);
             const uint32_t s = bin_sh[bin], b0 = bfirst[bin];
@@ -545,13 +577,23 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_units(const uint64_t *_
                 rd[j] = j * SP_THREADS + tid < nv ? d4 | (atomicAdd(&at_byte(sm.hist, d4), 1u) << 16) : ~0u;
             }
             const uint32_t *ip = id + base + tid;
-            got = split_order(sm, kl, kh, rd, ucur + d0, nd, [&](int j) { return j * SP_THREADS + tid < nv ? ip[j * SP_THREADS] : 0u; }, n);
+            got = split_order<false>(
+                sm, kl, kh, rd, ucur + d0, nd,
+                [&](int j) {
+                    uint32_t v = j * SP_THREADS + tid < nv ? ip[j * SP_THREADS] : 0u;
+                    if (label) {
+                        const uint32_t p = label[v];
+                        v = p == BAD ? v : p;
+                    }
+                    return v;
+                },
+                n);
         }
         if (tile_at(i + 1) < tiles) {  // the next tile's keys on their way while this one's tuples are stored
             now = tile_of[tile_at(i + 1)];
             load(now);
         }
-        split_store(sm, got, out_k, out_id);
+        split_store<false>(sm, got, out_k, out_id);
     }
 }
 
@@ -1006,8 +1048,8 @@ static void group_kernel_attrs()
     int dev = 0;
     cudaGetDevice(&dev);
     std::call_once(once[dev & 63], [] {
-        cudaFuncSetAttribute(k_split_reads<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinSmem));
-        cudaFuncSetAttribute(k_split_reads<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinSmem));
+        for (auto f : {k_split_reads<true, false>, k_split_reads<false, false>, k_split_reads<true, true>, k_split_reads<false, true>})
+            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinSmem));
         cudaFuncSetAttribute(k_split_tuples, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SplitSmem));
         cudaFuncSetAttribute(k_split_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(UnitSmem));
         cudaFuncSetAttribute(k_group<512, 12, 13>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmemS));
@@ -1026,14 +1068,14 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
     uint32_t *bin0 = h.data(), *sh = bin0 + nseg + 1, *lrs = sh + nseg;
     for (int q = 0, t = 0; q < nseg; q++) {
         const uint64_t n = g.seg_tstart[q + 1] - g.seg_tstart[q], span = nseg > 1 ? (uint64_t)NB : nbk;
-        sh[q] = (uint32_t)bin_width(n, span);
-        bin0[q + 1] = bin0[q] + (uint32_t)((span - 1) >> sh[q]) + 1;
+        sh[q] = g.merged ? (uint32_t)g.merged->sh : (uint32_t)bin_width(n, span);
+        bin0[q + 1] = bin0[q] + (uint32_t)((g.merged ? g.hi - 1 - g.anchor : span - 1) >> sh[q]) + 1;
         uint64_t b = g.seg_tstart[q];
         for (; t < (int)nbounds && g.bounds[t] < g.seg_tstart[q + 1]; t++) b = std::max(b, g.bounds[t]);
         lrs[q] = (uint32_t)b;
     }
     g.bins = bin0[nseg];
-    g.seg_lo = nseg > 1 ? 0u : (uint32_t)g.lo;
+    g.seg_lo = nseg > 1 ? 0u : (uint32_t)(g.merged ? g.anchor : g.lo);
     // units: a start per thread range, segment and bin, and at most two per 2^GP_UNIT_SHIFT tuples
     g.max_units = 2 * (uint32_t)(g.n >> GP_UNIT_SHIFT) + nbounds + g.bins + 2u * (uint32_t)nseg + 8;
     g.max_tiles = (uint32_t)(g.n / SP_TILE) + g.bins + 1;
@@ -1053,8 +1095,8 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
     g.ub0 = g.ustart + g.max_units + 1;
     g.ucur = g.ub0 + g.max_units + 1;
     g.bu0 = g.bstart + g.bins + 1;
-    g.bcur = g.bu0 + g.bins + 1;
-    g.bin_sh = g.bcur + g.bins + 1;
+    g.bcur = g.merged ? g.merged->cur + g.digit0 : g.bu0 + g.bins + 1;
+    g.bin_sh = g.bu0 + 2 * (size_t)(g.bins + 1);
     g.bfirst = g.bin_sh + g.bins + 1;
     g.seg_sh = g.seg_bin0 + nseg + 1;
     g.lrs = g.seg_sh + nseg;
@@ -1068,8 +1110,8 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
     (count_launch(), k_gp_marks<<<blocks_of(nbounds, 64), 64, 0, st>>>(g.d_hist, g.lo, g.hi, d_bounds, (int)nbounds, brk));
     (count_launch(), k_gp_count<<<nblk, GP_COUNT_BLOCK, 0, st>>>(c, blk));
     (count_launch(), k_gp_scan<<<1, 1024, 0, st>>>(blk, nblk, (uint32_t)g.n, g.bins, g.ctr, g.ustart, g.bstart, g.bu0));
-    (count_launch(), k_gp_write<<<nblk, GP_COUNT_BLOCK, 0, st>>>(c, blk, g.ctr, g.ustart, g.ub0, g.ucur, g.bstart, g.bu0, g.bcur,
-                                                                  g.bin_sh, g.bfirst, g.unit_of, g.mid, g.big));
+    (count_launch(), k_gp_write<<<nblk, GP_COUNT_BLOCK, 0, st>>>(c, blk, g.ctr, g.ustart, g.ub0, g.ucur, g.bstart, g.bu0,
+                                                                  g.merged ? nullptr : g.bcur, g.bin_sh, g.bfirst, g.unit_of, g.mid, g.big));
     (count_launch(), k_gp_tiles<<<1, 1024, 0, st>>>(g.bstart, g.bins, g.ctr, g.tiles));
     ReadBack<uint32_t> rb(arena, GC_N, PLAN_MAIL);
     if (!arena.mail) {
@@ -1126,7 +1168,7 @@ static int launch_bins(GroupScan &g, BinCtx &c, const std::vector<uint64_t> &seg
     c.err = g.ctr + GC_ERR;
     uint32_t least = 16;  // the narrowest bins
     for (int q = 0; q < nseg; q++) least = std::min(least, g.h_plan[(size_t)nseg + 1 + q]);
-    auto kern = !reads ? k_split_tuples : g.k >= 17 && c.bsh + (int)least >= 32 ? k_split_reads<true> : k_split_reads<false>;
+    auto kern = !reads ? k_split_tuples : g.k >= 17 && c.bsh + (int)least >= 32 ? k_split_reads<true, false> : k_split_reads<false, false>;
     const unsigned blocks = std::min<unsigned>(c.tiles, 2u * (unsigned)sm_count());
     if (blocks) (count_launch(), kern<<<blocks, SP_THREADS, reads ? sizeof(BinSmem) : sizeof(SplitSmem), st>>>(c));
     MP_CUDA(cudaGetLastError());
@@ -1158,11 +1200,82 @@ int group_bins_tuples(GroupScan &g, const uint64_t *lo, const uint8_t *hi, const
     return launch_bins(g, c, g.seg_tstart, arena, st);
 }
 
+// The first tuple of every bin of the merged scans.
+__global__ void k_gp_cursors(const uint64_t *hist, uint64_t lo, uint64_t hi, int sh, uint64_t s1, uint64_t s2, uint32_t digits,
+                             uint32_t *cur)
+{
+    const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
+    if (d >= digits) return;
+    uint32_t s = 0;
+    uint64_t first = lo;  // of the digit's scan
+    if (s1 < hi && d >= (uint32_t)((s1 - lo) >> sh) + 1) s = 1, first = s1;
+    if (s2 < hi && d >= (uint32_t)((s2 - lo) >> sh) + 2) s = 2, first = s2;
+    const uint64_t b = max(first, lo + ((uint64_t)(d - s) << sh));
+    cur[d] = (uint32_t)(hist[min(b, hi)] - hist[lo]);
+}
+
+bool group_merge(MergedScans &m, const uint64_t *hist, const std::vector<uint32_t> &scan, uint32_t max_len, int k)
+{
+    const int S = (int)scan.size() - 1;
+    if (S < 2 || S > GROUP_MAX_MERGED || max_len > (uint32_t)k + 254u) return false;
+    int small = 0;
+    bool large = false;
+    for (int s = 0; s < S; s++) {
+        if (scan[s] >= scan[s + 1]) return false;
+        const uint64_t n = hist[scan[s + 1]] - hist[scan[s]];
+        small = std::max(small, bin_width(n, scan[s + 1] - scan[s]));
+        large |= n > GP_SMALL;
+    }
+    m.scan = scan;
+    m.n = hist[scan[S]] - hist[scan[0]];
+    m.sh = large ? 10 : small;
+    m.digits = ((scan[S] - 1 - scan[0]) >> m.sh) + (uint32_t)S;
+    return m.digits <= GP_DIGITS + SP_EXTRA && m.n >= 1 && m.n <= GROUP_MAX_TUPLES;
+}
+
+int group_bins_scans(MergedScans &m, const uint64_t *d_hist, int k, const uint8_t *fq, const ParsedReads &pr, cudaStream_t st)
+{
+    group_kernel_attrs();
+    const int S = (int)m.scan.size() - 1;
+    const uint64_t lo = m.scan[0], hi = m.scan[S];
+    (count_launch(), k_gp_cursors<<<blocks_of(m.digits, 256), 256, 0, st>>>(d_hist, lo, hi, m.sh, m.scan[1], S > 2 ? m.scan[2] : hi,
+                                                                           m.digits, m.cur));
+    BinCtx c;
+    c.t = read_tiles(fq, pr, k, pr.max_len, SP_THREADS, SP_PACKED);
+    c.n_reads = (uint32_t)pr.n_reads;
+    c.out_k = m.k1;
+    c.out_id = m.id1;
+    c.n = (uint32_t)m.n;
+    c.tiles = blocks_of(c.n_reads, (int)c.t.rpt);
+    c.bsh = 2 * (k - 10);
+    c.k_lo = lo << c.bsh;
+    c.k_span = (hi - lo) << c.bsh;
+    c.bcur = m.cur;
+    c.m_digits = m.digits;
+    c.m_sh = (uint32_t)m.sh;
+    for (int s = 1; s < S; s++) c.m_start[s - 1] = (m.scan[s] - lo) << c.bsh;
+    auto kern = k >= 17 && c.bsh + m.sh >= 32 ? k_split_reads<true, true> : k_split_reads<false, true>;
+    const unsigned blocks = std::min<unsigned>(c.tiles, 2u * (unsigned)sm_count());
+    if (blocks) (count_launch(), kern<<<blocks, SP_THREADS, sizeof(BinSmem), st>>>(c));
+    MP_CUDA(cudaGetLastError());
+    return 0;
+}
+
+void group_take(GroupScan &g, const MergedScans &m, int s, const uint32_t *label, const std::vector<uint64_t> &tuple0)
+{
+    const uint64_t rel = g.lo - m.scan[0];
+    g.merged = &m;
+    g.anchor = m.scan[0] + (rel >> m.sh << m.sh);
+    g.digit0 = (uint32_t)(rel >> m.sh) + (uint32_t)s;
+    g.tuple0 = (uint32_t)tuple0[s];
+    g.late_label = s ? label : nullptr;
+}
+
 int group_units(GroupScan &g, const uint64_t *k1, const uint32_t *id1, uint64_t *k2, uint32_t *id2, cudaStream_t st)
 {
     (count_launch(), k_split_units<<<std::min(g.max_tiles, 2u * (unsigned)sm_count()), SP_THREADS, sizeof(UnitSmem), st>>>(
         k1, id1, (uint32_t)g.n, 2 * (g.k - 10), g.seg_lo, g.ctr, g.bstart, g.bfirst, g.bu0, g.bcur, g.bin_sh, g.ub0,
-        g.ucur, g.unit_of, (uint32_t)(g.hi - g.lo), g.tiles, k2, id2));
+        g.ucur, g.unit_of, (uint32_t)(g.hi - g.lo), g.tiles, g.tuple0, g.late_label, k2, id2));
     MP_CUDA(cudaGetLastError());
     return 0;
 }

@@ -17,6 +17,21 @@ namespace mp {
 constexpr uint64_t GROUP_MAX_TUPLES = 4000000000ull;  // tuple positions are 32 bits
 constexpr uint64_t GROUP_MAX_READS = 0x7FFFFFFFull;   // a grouped id keeps its top bit for the group's first tuple
 
+// The first split pass of all scans of a job at once: the reads are packed and rolled through once.  Needs the tuples of
+// every scan at once, so it is for the callers whose memory holds them, and the components of later scans are looked up in
+// the second pass.  The scans' bins count from the first scan's first bucket, in the same widths; a bin that a scan's
+// bounds cut is two.
+constexpr int GROUP_MAX_MERGED = 3;  // scans
+struct MergedScans {
+    std::vector<uint32_t> scan;  // the scans' buckets, consecutive
+    uint64_t n = 0;              // their tuples
+    int sh = 0;                  // bins of 2^sh buckets
+    uint32_t digits = 0;         // bins
+    uint32_t *cur = nullptr;     // the bins' fill (digits words, the caller's), from the first scan's first tuple
+    uint64_t *k1 = nullptr;      // the split tuples (n, the caller's)
+    uint32_t *id1 = nullptr;
+};
+
 // One scan (or every sample's scan of a batch, as segments) to split and group.
 struct GroupScan {
     int k = 0;
@@ -25,6 +40,12 @@ struct GroupScan {
     uint64_t lo = 0, hi = 0;
     std::vector<uint64_t> bounds;      // thread ranges' tuple bounds, every segment's after the other (ascending)
     std::vector<uint64_t> seg_tstart;  // nseg + 1 tuple offsets ({0, n} for one scan)
+
+    // a scan of merged ones (group_take)
+    const MergedScans *merged = nullptr;
+    uint64_t anchor = 0;                     // where its bins count from
+    uint32_t digit0 = 0, tuple0 = 0;         // its first bin's digit and its first tuple among the merged
+    const uint32_t *late_label = nullptr;    // the reads' components, for the second pass
 
     // the plan (device), from group_plan
     uint32_t bins = 0, seg_lo = 0, max_units = 0, max_tiles = 0;
@@ -70,6 +91,12 @@ int group_bins_reads(GroupScan &g, const uint8_t *fq, const ParsedReads &pr, con
                      const uint32_t *label, uint64_t *k1, uint32_t *id1, DeviceArena &arena, cudaStream_t st);
 int group_bins_tuples(GroupScan &g, const uint64_t *lo, const uint8_t *hi, const uint32_t *id, uint64_t *k1, uint32_t *id1,
                       DeviceArena &arena, cudaStream_t st);
+// Whether the scans [scan[s], scan[s + 1]) can be split together, and how (m's arrays are then the caller's to set).
+bool group_merge(MergedScans &m, const uint64_t *hist, const std::vector<uint32_t> &scan, uint32_t max_len, int k);
+// Their first split pass, from the reads; ids are the reads'.
+int group_bins_scans(MergedScans &m, const uint64_t *d_hist, int k, const uint8_t *fq, const ParsedReads &pr, cudaStream_t st);
+// Before group_plan: g is scan s of m (tuple0: every scan's first tuple among the merged).
+void group_take(GroupScan &g, const MergedScans &m, int s, const uint32_t *label, const std::vector<uint64_t> &tuple0);
 // Second pass: the bins' tuples into units.
 int group_units(GroupScan &g, const uint64_t *k1, const uint32_t *id1, uint64_t *k2, uint32_t *id2, cudaStream_t st);
 // The mischief filter over the split tuples (kk, ids), and every k-mer's reads side by side in out (n ids).

@@ -956,8 +956,9 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
 {
     const uint64_t N = j->pr.n_reads, n = gs.n;
     int rc = 0;
-    uint64_t *k1 = j->arena.alloc<uint64_t>(n + 1), *k2 = nullptr;
-    uint32_t *id1 = j->arena.alloc<uint32_t>(n + 1), *id2 = nullptr;
+    const MergedScans *m = gs.merged;  // its first split pass is done
+    uint64_t *k1 = m ? m->k1 + gs.tuple0 : j->arena.alloc<uint64_t>(n + 1), *k2 = nullptr;
+    uint32_t *id1 = m ? m->id1 + gs.tuple0 : j->arena.alloc<uint32_t>(n + 1), *id2 = nullptr;
     {
         StageTimer tm(j->clk, j->st, min3 ? 3 : 2, SPLIT_SLOT);
         if ((rc = group_plan(gs, j->arena, j->st))) return rc;
@@ -970,8 +971,8 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
         }
         if (!k1 || !id1 || !k2 || !id2)
             return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)n);
-        rc = min3 ? group_bins_tuples(gs, lo, hi, id, k1, id1, j->arena, j->st)
-                  : group_bins_reads(gs, j->d_fq, j->pr, {0, N}, s ? j->d_parent : nullptr, k1, id1, j->arena, j->st);
+        rc = m ? 0 : min3 ? group_bins_tuples(gs, lo, hi, id, k1, id1, j->arena, j->st)
+                 : group_bins_reads(gs, j->d_fq, j->pr, {0, N}, s ? j->d_parent : nullptr, k1, id1, j->arena, j->st);
         if (rc) return rc;
     }
     {
@@ -1001,6 +1002,41 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
     ss.big_tuples = gs.hctr[GC_BIG_TUPLES];
     add_sort_stats(j, ss, n);
     return 0;
+}
+
+// The first split pass of all scans at once (MergedScans), where every scan is to be grouped and one scan of all the tuples
+// would not have to go in pieces (its two buffers take more than the one of all tuples and a second one of a scan's).  Else
+// m.k1 stays null and every scan makes its own.
+static int merge_scans(mp_job *j, int k, int T, const std::vector<uint64_t> &scanR, const std::vector<uint64_t> &thrR,
+                       const uint64_t *hist, const uint64_t *d_hist, uint64_t piece_cap, MergedScans &m,
+                       std::vector<uint64_t> &tuple0)
+{
+    const int S = (int)scanR.size() - 1;
+    if (S > GROUP_MAX_MERGED || (j->pr.max_len > (uint32_t)k && j->pr.max_len - (uint32_t)k >= 300u)) return 0;
+    for (int s = 0; s < S; s++) {
+        if (scanR[s] >= scanR[s + 1] || scanR[s + 1] > NB || hist[scanR[s]] > hist[scanR[s + 1]]) return 0;
+        const uint64_t n = hist[scanR[s + 1]] - hist[scanR[s]];
+        if (!scan_is_grouped(j, k, n)) return 0;
+        std::vector<uint64_t> rb;
+        if (range_bounds(hist, thrR.data() + (size_t)s * T, T, scanR[s], scanR[s + 1], rb)) return 0;
+        tuple0.push_back(hist[scanR[s]] - hist[scanR[0]]);
+    }
+    if (!group_merge(m, hist, std::vector<uint32_t>(scanR.begin(), scanR.end()), j->pr.max_len, k)) return 0;
+    if (m.n > piece_cap) return 0;
+    m.k1 = j->arena.alloc_persistent<uint64_t>(m.n + 1);
+    m.id1 = j->arena.alloc_persistent<uint32_t>(m.n + 1);
+    m.cur = j->arena.alloc_persistent<uint32_t>(m.digits);
+    if (!m.k1 || !m.id1 || !m.cur) {
+        j->arena.free_persistent(m.k1);
+        j->arena.free_persistent(m.id1);
+        j->arena.free_persistent(m.cur);
+        m.k1 = nullptr;
+        m.id1 = nullptr;
+        m.cur = nullptr;
+        return 0;
+    }
+    StageTimer tm(j->clk, j->st, 2, SPLIT_SLOT);
+    return group_bins_scans(m, d_hist, k, j->d_fq, j->pr, j->st);
 }
 
 int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_starts, const uint64_t *chunk_first_read,
@@ -1089,6 +1125,9 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
     j->pieces_total = 0;
     j->hooked_bad = ~0u;
     const uint64_t piece_cap = p->min3 ? ~0ull : scan_piece_cap(j);  // the 3-minimizer choice depends on the range
+    MergedScans merged;
+    std::vector<uint64_t> tuple0;
+    if (S > 1 && !p->min3 && (rc = merge_scans(j, k, T, scanR, thrR, hist, d_hist, piece_cap, merged, tuple0))) return rc;
     for (int s = 0; s < S; s++) {
         const uint64_t lo = scanR[s], hi = scanR[s + 1];
         const uint64_t expect = hist[hi] - hist[lo];
@@ -1133,6 +1172,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             gs.hi = hi;
             gs.bounds = rb;
             gs.seg_tstart = {0, expect};
+            if (merged.k1) group_take(gs, merged, s, j->d_parent, tuple0);
         }
         if (grouped && !p->min3) {
             if (j->pr.max_len > (uint32_t)k && j->pr.max_len - (uint32_t)k >= 300u)
@@ -1255,6 +1295,9 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         snprintf(name, sizeof name, "stats%d_parent.bin", s);
         if ((rc = dump_state(j, name, nullptr))) return rc;
     }
+    j->arena.free_persistent(merged.k1);
+    j->arena.free_persistent(merged.id1);
+    j->arena.free_persistent(merged.cur);
     j->arena.free_persistent(cnt_all);
     j->arena.free_persistent(d_b);
     j->arena.free_persistent(d_hist);

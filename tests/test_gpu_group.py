@@ -111,3 +111,27 @@ def test_random_tiny(ctx, seed):
                 except native.MetapartError as e:  # ranges the planner refuses are refused on both paths
                     res.append(str(e))
         assert res[0] == res[1]
+
+
+@pytest.mark.parametrize("k", [11, 17, 21, 31])
+@pytest.mark.parametrize("scans", [2, 3])
+@pytest.mark.parametrize("n", [600, 60_000])
+def test_scans_split_together(ctx, n, scans, k):
+    """Two and three scans whose first split pass is one, against a pass per scan (a piece limit that all scans
+    together exceed): bins of every width, small scans' and (60,000 reads) the 1024-bucket bins that the scans' bounds cut."""
+    data = synth.fastq_bytes(synth.workload("plain_large", n, seed=5 + k))
+    fno, ofs = native.fastq_index(4, [data], False)
+    starts = native.chunk_starts_of(fno, ofs, [len(data)])
+    res = []
+    for cap in (0, 1):
+        with native.Job(ctx) as job:
+            job.load(data)
+            cnt = job.count(k, starts)
+            total = int(cnt.hist[-1])
+            if cap:
+                job.set_scan_piece_tuples(total - 1)  # more than a scan, less than all
+            b = job.partition(k, scans, 4, starts, cnt.chunk_first_read, cnt.hist)
+            assert job.scan_pieces == scans
+            out, sizes = job.output()
+            res.append((b.tolist(), job.labels().tolist(), sizes.tolist(), bytes(out)))
+    assert res[0] == res[1]

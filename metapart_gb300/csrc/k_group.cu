@@ -636,9 +636,10 @@ struct GroupCtx {
     uint8_t *filtered;
 };
 
-// Bound by shared memory (random accesses and atomics: about five per tuple) and the block's barriers; two
-// 512-thread blocks per SM overlap each other's.  20M x 150 bp, 2 scans (2.39 G tuples): 31.4 ms for both block
-// shapes, where sorting the units (66.8 ms) and judging the sorted runs (31.9 ms) took 98.7.
+// Bound by shared memory (random accesses and atomics: about five per tuple), its instructions and the block's barriers;
+// two 512-thread blocks per SM overlap each other's.  20M x 150 bp, 2 scans (2.39 G tuples): 28 ms for both block
+// shapes, where sorting the units (66.8 ms) and judging the sorted runs (31.9 ms) took 98.7.  30.4 with every tuple's info
+// read again for the marks and the rare tests in the probe loop; probing pairs of slots at once gained nothing.
 //
 // One block per unit (persistent, units handed out by a counter): the unit's tuples into a hash table of its
 // k-mers (open addressing in shared memory), the filter's judgement of every k-mer, its marks, and the reads of
@@ -728,13 +729,22 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
                     if (v == k) break;
                     h = (h + step) & SMASK;
                 }
-                const uint32_t bi = ac[j] & 7u, ai = ac[j] >> 3;
-                const uint32_t m = (bi < 7u ? 0x10000u << bi : 0u) | (ai < 7u ? 0x800000u << ai : 0u);
+                const uint32_t m = ((0x10000u << (ac[j] & 7u)) & 0x7F0000u) | ((0x800000u << (ac[j] >> 3)) & 0x3F800000u);
                 const uint32_t old = atomicAdd(&sm.info[h], 1u);
                 if (m & ~old) atomicOr(&sm.info[h], m);
-                sr[j] = h | ((old & 0xFFFFu) << 16);
-                if (k == 0) ac[j] |= 64u;
-                if (ends && k == sm.maxkey) sm.slot_ex = h;
+                sr[j] = h | (old << 16);
+            }
+        }
+        const bool zero_bucket = (b0 & (NB - 1)) == 0;
+        if (ends || zero_bucket) {
+            const unsigned long long mx = sm.maxkey;
+#pragma unroll
+            for (int j = 0; j < ITEMS; j++) {
+                if (j * THREADS + tid < cnt) {
+                    const unsigned long long k = key[j] >> 6;
+                    if (zero_bucket && k == 0) ac[j] |= 64u;
+                    if (ends && k == mx) sm.slot_ex = sr[j] & 0xFFFFu;
+                }
             }
         }
         uint32_t id[ITEMS];
@@ -746,7 +756,6 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
         __syncthreads();
         // ---- a slot's first tuple decides its side, its counters and whether its reads are kept
         const uint32_t ex = sm.slot_ex;
-        const bool zero_bucket = (b0 & (NB - 1)) == 0;
         uint32_t kept = 0;
 #pragma unroll
         for (int j = 0; j < ITEMS; j++) {
@@ -760,7 +769,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
                     reinterpret_cast<uint4 *>(sm.u.b.pool)[p] = make_uint4(0, 0, 0, h << 16);
                     ni |= p << 16;
                 }
-                if (side != 3u && !(zero_bucket && (ac[j] & 64u)) && (n >= 2u || singles)) {
+                if (side != 3u && !(ac[j] & 64u) && (n >= 2u || singles)) {
                     ni |= GI_KEPT;
                     kept += n;
                     ac[j] |= 128u;
@@ -776,12 +785,14 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
         }
         if (lane == 31) sm.ws[warp] = x;
         __syncthreads();
-        uint32_t at = x - kept, total = 0;
-        for (int q = 0; q < THREADS / 32; q++) {
-            const uint32_t t = sm.ws[q];
-            at += q < warp ? t : 0u;
-            total += t;
+        uint32_t at = x - kept, sums = lane < THREADS / 32 ? sm.ws[lane] : 0u;  // the warps', then up to each
+#pragma unroll
+        for (int o = 1; o < THREADS / 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULLG, sums, o);
+            if (lane >= o) sums += y;
         }
+        const uint32_t total = __shfl_sync(FULLG, sums, THREADS / 32 - 1), before = __shfl_sync(FULLG, sums, (warp + 31) & 31);
+        at += warp ? before : 0u;
         if (tid == 0) sm.base = atomicAdd(&c.ctr[GC_OUT], total);
 #pragma unroll
         for (int j = 0; j < ITEMS; j++) {
@@ -791,14 +802,17 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
                 at += sm.info[h] & 0x3FFFu;
             }
         }
-        // ---- code counts of the runs branching on one side
+        // ---- code counts of the runs branching on one side; ac: such a run's tuple (bit 6) and its code there, kept (bit 7)
 #pragma unroll
         for (int j = 0; j < ITEMS; j++) {
             if (j * THREADS + tid < cnt) {
                 const uint32_t inf = sm.info[sr[j] & 0xFFFFu], side = (inf >> 14) & 3u;
                 const uint32_t code = side == 1u ? ac[j] & 7u : (ac[j] >> 3) & 7u;
-                if ((side == 1u || side == 2u) && code < 7u)
-                    atomicAdd(&sm.u.b.pool[((inf >> 16) & 0x1FFFu) * 4 + (code >> 1)], 1u << (16 * (code & 1)));
+                ac[j] = (inf & GI_KEPT) >> 24;
+                if (side == 1u || side == 2u) {
+                    ac[j] |= 64u | code;
+                    if (code < 7u) atomicAdd(&sm.u.b.pool[((inf >> 16) & 0x1FFFu) * 4 + (code >> 1)], 1u << (16 * (code & 1)));
+                }
             }
         }
         __syncthreads();
@@ -824,13 +838,15 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
 #pragma unroll
         for (int j = 0; j < ITEMS; j++) {
             if (j * THREADS + tid < cnt) {
-                const uint32_t h = sr[j] & 0xFFFFu, inf = sm.info[h], side = (inf >> 14) & 3u;
-                const uint32_t code = side == 1u ? ac[j] & 7u : (ac[j] >> 3) & 7u;
-                if ((side == 1u || side == 2u) && (code != ((inf >> 16) & 7u) || (inf & (1u << 19)))) {
-                    c.parent[id[j]] = BAD;
-                    c.filtered[id[j]] = 1;
+                const uint32_t h = sr[j] & 0xFFFFu;
+                if (ac[j] & 64u) {
+                    const uint32_t inf = sm.info[h];
+                    if ((ac[j] & 7u) != ((inf >> 16) & 7u) || (inf & (1u << 19))) {
+                        c.parent[id[j]] = BAD;
+                        c.filtered[id[j]] = 1;
+                    }
                 }
-                if (inf & GI_KEPT) stage[sm.u.b.off[h] + (sr[j] >> 16)] = id[j] | ((sr[j] >> 16) == 0 ? 0x80000000u : 0u);
+                if (ac[j] & 128u) stage[sm.u.b.off[h] + (sr[j] >> 16)] = id[j] | ((sr[j] >> 16) == 0 ? 0x80000000u : 0u);
             }
         }
         if (singles && tid == 0) {

@@ -551,24 +551,56 @@ __global__ void k_compress(uint32_t *parent, uint64_t n)
 }
 
 // compSizes after a reset to 1 and printStats (metapart.c:4010-4030): 1 + non-root members.
-// Component sizes (1 + members below each root).  The reads of a large component meet in most warps,
-// so the lanes of one root add together: one atomic per root and warp instead of one per read.
+// Component sizes (1 + members below each root).  Bound by the additions to the few hundred roots of the large components:
+// a block counts its stretch of reads by root in shared memory and adds once per root (a root that finds no slot, and a
+// read that is its own root, add by themselves).  20M reads 1.17 (COMPRESS: 1.44) -> 0.11 (0.16) ms against one addition
+// per root and warp.
 // COMPRESS: the parents are compressed first, else they point at their roots.
+constexpr int SZ_THREADS = 256, SZ_SLOTS_LOG = 11, SZ_SLOTS = 1 << SZ_SLOTS_LOG;
 template <bool COMPRESS>
-__global__ void k_sizes(uint32_t *parent, uint64_t n, uint32_t *size)
+__global__ void __launch_bounds__(SZ_THREADS) k_sizes(uint32_t *parent, uint64_t n, uint64_t per, uint32_t *size)
 {
-    const uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t r = 0xFFFFFFFFu;
-    if (x < n) {
+    __shared__ uint32_t root[SZ_SLOTS], cnt[SZ_SLOTS];
+    for (int i = threadIdx.x; i < SZ_SLOTS; i += SZ_THREADS) {
+        root[i] = 0xFFFFFFFFu;
+        cnt[i] = 0;
+    }
+    __syncthreads();
+    const uint64_t end = min(n, (blockIdx.x + 1) * per);
+#pragma unroll 4
+    for (uint64_t x = blockIdx.x * per + threadIdx.x; x < end; x += SZ_THREADS) {
+        uint32_t r;
         if (COMPRESS) {
             r = compress_one(parent, x);
         } else {
             const uint32_t p = parent[x];
             r = (p == BAD || p == x) ? (uint32_t)x : p;
         }
+        bool in = false;
+        if (r != x) {
+            uint32_t h = (r * 0x9E3779B1u) >> (32 - SZ_SLOTS_LOG);
+            for (int q = 0; q < 4 && !in; q++, h = (h + 1) & (SZ_SLOTS - 1)) {
+                uint32_t v = *(volatile uint32_t *)&root[h];
+                if (v == 0xFFFFFFFFu) v = atomicCAS(&root[h], 0xFFFFFFFFu, r);
+                if (v == 0xFFFFFFFFu || v == r) {
+                    atomicAdd(&cnt[h], 1u);
+                    in = true;
+                }
+            }
+        }
+        if (!in) atomicAdd(&size[r], 1u);
     }
-    const uint32_t peers = __match_any_sync(FULLW, r);
-    if (x < n && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&size[r], (uint32_t)__popc(peers));
+    __syncthreads();
+    for (int i = threadIdx.x; i < SZ_SLOTS; i += SZ_THREADS)
+        if (cnt[i]) atomicAdd(&size[root[i]], cnt[i]);
+}
+
+template <bool COMPRESS> static void launch_sizes(uint32_t *parent, uint64_t n, uint32_t *size, cudaStream_t st)
+{
+    if (n == 0) return;
+    const uint64_t blocks = std::min<uint64_t>((n + SZ_THREADS - 1) / SZ_THREADS, 8u * (uint64_t)sm_count());
+    const uint64_t per = ((n + blocks - 1) / blocks + SZ_THREADS - 1) / SZ_THREADS * SZ_THREADS;
+    (mp::count_launch(), k_sizes<COMPRESS><<<(unsigned)((n + per - 1) / per), SZ_THREADS, 0, st>>>(parent, n, per, size));
 }
 
 // -------------------------------------------------------------- K6 mate union
@@ -681,8 +713,9 @@ __device__ __forceinline__ bool pe_decide(const PeArrays &c, unsigned f, uint32_
     return ok;
 }
 
-// Two small roots merge at once (returns false); a single or a small root x joins g with the others of that root.
-__device__ __forceinline__ bool pe_commit(const PeArrays &c, unsigned f, uint32_t xa, uint32_t xb, uint32_t round, uint32_t &g, uint32_t &x)
+// Two small roots merge at once (returns false); a single or a small root x of size z is to join g with the others of that
+// root (pe_group).
+__device__ __forceinline__ bool pe_commit(const PeArrays &c, unsigned f, uint32_t xa, uint32_t xb, uint32_t &g, uint32_t &x, uint32_t &z)
 {
     const uint32_t za = __ldcg(c.size + xa), zb = __ldcg(c.size + xb);  // (of a small root held here, as they were)
     if ((f & (PE_SA | PE_SB)) == (PE_SA | PE_SB) && !(f & (PE_OA | PE_OB))) {
@@ -695,9 +728,14 @@ __device__ __forceinline__ bool pe_commit(const PeArrays &c, unsigned f, uint32_
     const bool a = (f & PE_SA) && !(f & PE_OB);  // a is the end that joins
     g = a ? xb : xa;
     x = a ? xa : xb;
-    atomicMax(&c.gmax[g], ((unsigned long long)round << 32) | x);
-    atomicAdd(&c.gadd[g], (unsigned long long)(a ? za : zb));
+    z = a ? za : zb;
     return true;
+}
+
+__device__ __forceinline__ void pe_group(const PeArrays &c, uint32_t g, uint32_t x, uint32_t z, uint32_t round)
+{
+    atomicMax(&c.gmax[g], ((unsigned long long)round << 32) | x);
+    atomicAdd(&c.gadd[g], (unsigned long long)z);
 }
 
 __device__ __forceinline__ void pe_join(const PeArrays &c, uint32_t g, uint32_t x)
@@ -723,14 +761,39 @@ __device__ __forceinline__ void pe_join(const PeArrays &c, uint32_t g, uint32_t 
 // with one atomic (the order of a list's entries does not matter: a commit is decided by the round's
 // reservations, not by list position).
 
-// Appends v (where pred) to list; all 32 lanes call it.
-__device__ __forceinline__ void warp_append(uint32_t *list, unsigned int *count, bool pred, uint32_t v, int lane)
+constexpr int PE_THREADS = 256;
+struct PeAppend {  // one list's counts by warp, then their places; two in turn, so that one barrier less is needed
+    uint32_t at[2][2][PE_THREADS / 32];
+};
+
+// v to list a or list b; all threads of the block come here, with turns counted from 0.  One addition to a list's count per
+// block: with one per warp the round was a queue at that address (60 us for a million pairs, nearly all of them asleep).
+__device__ __forceinline__ void pe_append(PeAppend &m, int turn, uint32_t *a, unsigned int *ca, bool pa, uint32_t *b, unsigned int *cb,
+                                          bool pb, uint32_t v)
 {
-    const uint32_t m = __ballot_sync(FULLW, pred);
-    uint32_t base = 0;
-    if (lane == 0 && m) base = atomicAdd(count, (unsigned int)__popc(m));
-    base = __shfl_sync(FULLW, base, 0);
-    if (pred) list[base + __popc(m & ((1u << lane) - 1))] = v;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t(&at)[2][PE_THREADS / 32] = m.at[turn & 1];
+    const uint32_t ma = __ballot_sync(FULLW, pa), mb = __ballot_sync(FULLW, pb), lt = (1u << lane) - 1;
+    if (lane == 0) {
+        at[0][warp] = (uint32_t)__popc(ma);
+        at[1][warp] = (uint32_t)__popc(mb);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        uint32_t *p = at[threadIdx.x], sum = 0;
+#pragma unroll
+        for (int w = 0; w < PE_THREADS / 32; w++) sum += p[w];
+        uint32_t base = sum ? atomicAdd(threadIdx.x ? cb : ca, sum) : 0u;
+#pragma unroll
+        for (int w = 0; w < PE_THREADS / 32; w++) {
+            const uint32_t c = p[w];
+            p[w] = base;
+            base += c;
+        }
+    }
+    __syncthreads();
+    if (pa) a[at[0][warp] + __popc(ma & lt)] = v;
+    if (pb) b[at[1][warp] + __popc(mb & lt)] = v;
 }
 
 struct PePairs {  // by pair: its ends' roots when it was last awake, the pairs it sleeps behind, flags
@@ -739,13 +802,14 @@ struct PePairs {  // by pair: its ends' roots when it was last awake, the pairs 
 };
 
 // The pairs of act that are awake to the list awake, the others to next.
-__global__ void k_pe_reserve(PeArrays c, PePairs s, const uint32_t *act, const unsigned int *nact_p, uint32_t *awake,
+__global__ void __launch_bounds__(PE_THREADS) k_pe_reserve(PeArrays c, PePairs s, const uint32_t *act, const unsigned int *nact_p, uint32_t *awake,
                              unsigned int *nawake, uint32_t *next, unsigned int *nnext, uint32_t round)
 {
     const uint32_t nact = *nact_p;
-    const int lane = threadIdx.x & 31;
-    for (uint32_t w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < nact; w0 += gridDim.x * blockDim.x) {
-        const uint32_t t = w0 + lane;
+    __shared__ PeAppend ap;
+    int turn = 0;
+    for (uint32_t b0 = blockIdx.x * PE_THREADS; b0 < nact; b0 += gridDim.x * PE_THREADS) {
+        const uint32_t t = b0 + threadIdx.x;
         bool up = false, keep = false;
         uint32_t j = 0;
         if (t < nact) {
@@ -771,29 +835,30 @@ __global__ void k_pe_reserve(PeArrays c, PePairs s, const uint32_t *act, const u
                 }
             }
         }
-        warp_append(awake, nawake, keep && up, j, lane);
-        warp_append(next, nnext, keep && !up, j, lane);
+        pe_append(ap, turn++, awake, nawake, keep && up, next, nnext, keep && !up, j);
     }
 }
 
-__global__ void k_pe_commit(PeArrays c, PePairs s, const uint32_t *awake, const unsigned int *nawake_p, uint32_t *next,
+__global__ void __launch_bounds__(PE_THREADS) k_pe_commit(PeArrays c, PePairs s, const uint32_t *awake, const unsigned int *nawake_p, uint32_t *next,
                             unsigned int *nnext, uint32_t *group, unsigned int *ngroup, uint32_t round)
 {
     const uint32_t n = *nawake_p;
     const int lane = threadIdx.x & 31;
-    for (uint32_t w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < n; w0 += gridDim.x * blockDim.x) {
-        const uint32_t t = w0 + lane;
+    __shared__ PeAppend ap;
+    int turn = 0;
+    for (uint32_t b0 = blockIdx.x * PE_THREADS; b0 < n; b0 += gridDim.x * PE_THREADS) {
+        const uint32_t t = b0 + threadIdx.x;
         bool ok = false, join = false;
-        uint32_t j = 0;
+        uint32_t j = 0, g = 0, x = 0, z = 0;
         if (t < n) {
             j = awake[t];
             const unsigned f = s.fl[j];
             const uint32_t xa = s.xa[j], xb = s.xb[j];
-            uint32_t ha, hb, g, x;
+            uint32_t ha, hb;
             ok = pe_decide(c, f, xa, xb, pe_hold_key(j, j), pe_stamp(round, j), ha, hb);
             if (ok) {
                 atomicOr(c.done + (j >> 5), 1u << (j & 31));
-                join = pe_commit(c, f, xa, xb, round, g, x);
+                join = pe_commit(c, f, xa, xb, g, x, z);
                 if (join) {
                     s.xa[j] = g;
                     s.xb[j] = x;
@@ -804,8 +869,14 @@ __global__ void k_pe_commit(PeArrays c, PePairs s, const uint32_t *awake, const 
                 if (ha != PE_NONE || hb != PE_NONE) s.fl[j] = (uint8_t)(f & ~PE_AWAKE);
             }
         }
-        warp_append(next, nnext, t < n && !ok, j, lane);
-        warp_append(group, ngroup, join, j, lane);
+        // the lanes that join one root together (20M reads: the roots of a few large components take most joins; all rounds'
+        // commits 2.7 -> 1.5 ms)
+        const uint32_t joins = __ballot_sync(FULLW, join);
+        if (join) {
+            const uint32_t peers = __match_any_sync(joins, g), most = __reduce_max_sync(peers, x), sum = __reduce_add_sync(peers, z);
+            if (lane == __ffs(peers) - 1) pe_group(c, g, most, sum, round);
+        }
+        pe_append(ap, turn++, next, nnext, t < n && !ok, group, ngroup, join, j);
     }
 }
 
@@ -923,7 +994,7 @@ __global__ void __launch_bounds__(PEC_THREADS, 1) k_pe_cluster(PeCluster c)
             const unsigned f = s.fl[l];
             if (!(f & PE_LIVE)) continue;
             const uint32_t j = s.pj[l], xa = s.xa[l], xb = s.xb[l];
-            uint32_t ha, hb, g, x;
+            uint32_t ha, hb, g, x, z;
             if (!pe_decide(c.a, f, xa, xb, pe_hold_key(j, t), pe_stamp(round, j), ha, hb)) {
                 s.ha[l] = ha;
                 s.hb[l] = hb;
@@ -933,7 +1004,8 @@ __global__ void __launch_bounds__(PEC_THREADS, 1) k_pe_cluster(PeCluster c)
             any_commit = true;
             atomicSub(&s.live, 1u);
             atomicOr(c.a.done + (t >> 5), 1u << (t & 31));
-            if (pe_commit(c.a, f, xa, xb, round, g, x)) {
+            if (pe_commit(c.a, f, xa, xb, g, x, z)) {
+                pe_group(c.a, g, x, z, round);
                 s.xa[l] = g;
                 s.xb[l] = x;
                 s.fl[l] = PE_GROUP;
@@ -1206,7 +1278,7 @@ int mate_union(uint32_t *parent, uint64_t n_reads, uint32_t *size, DeviceArena &
 {
     const uint64_t npairs = n_reads / 2;
     MP_CUDA(cudaMemsetAsync(size, 0, n_reads * sizeof(uint32_t), st));
-    (mp::count_launch(), k_sizes<false><<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads, size));
+    launch_sizes<false>(parent, n_reads, size, st);
     uint32_t *act = arena.alloc<uint32_t>(npairs + 1), *act2 = arena.alloc<uint32_t>(npairs + 1);
     uint32_t *awake = arena.alloc<uint32_t>(npairs + 1), *group = arena.alloc<uint32_t>(npairs + 1);
     PePairs s{arena.alloc<uint32_t>(npairs + 1), arena.alloc<uint32_t>(npairs + 1), arena.alloc<uint32_t>(npairs + 1),
@@ -1268,8 +1340,8 @@ int mate_union(uint32_t *parent, uint64_t n_reads, uint32_t *size, DeviceArena &
         for (int r = 0; r < rb; r++) {
             ++round;
             const unsigned int *nin = r ? cnts + 4 * (r - 1) + 1 : cnts + 4 * RB + 1;
-            (mp::count_launch(), k_pe_reserve<<<g, 256, 0, st>>>(c, s, act, nin, awake, cnts + 4 * r, act2, cnts + 4 * r + 1, round));
-            (mp::count_launch(), k_pe_commit<<<g, 256, 0, st>>>(c, s, awake, cnts + 4 * r, act2, cnts + 4 * r + 1, group,
+            (mp::count_launch(), k_pe_reserve<<<g, PE_THREADS, 0, st>>>(c, s, act, nin, awake, cnts + 4 * r, act2, cnts + 4 * r + 1, round));
+            (mp::count_launch(), k_pe_commit<<<g, PE_THREADS, 0, st>>>(c, s, awake, cnts + 4 * r, act2, cnts + 4 * r + 1, group,
                                                                 cnts + 4 * r + 2, round));
             (mp::count_launch(), k_pe_join<<<g, 256, 0, st>>>(c, s, group, cnts + 4 * r + 2));
             std::swap(act, act2);
@@ -1289,7 +1361,7 @@ int mate_union(uint32_t *parent, uint64_t n_reads, uint32_t *size, DeviceArena &
     if (rounds_out) *rounds_out = (int)round;
     // final printStats: compress and recount (metapart.c:4026-4030)
     MP_CUDA(cudaMemsetAsync(size, 0, n_reads * sizeof(uint32_t), st));
-    (mp::count_launch(), k_sizes<true><<<blocks_for(n_reads, 256), 256, 0, st>>>(parent, n_reads, size));
+    launch_sizes<true>(parent, n_reads, size, st);
     return 0;
 }
 

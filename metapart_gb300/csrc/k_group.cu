@@ -54,30 +54,60 @@ static int bin_width(uint64_t n, uint64_t span)
     return s;
 }
 
-// The populated bucket before b within b's segment: its index, or ~0 when b is the segment's first.
-__device__ __forceinline__ uint64_t prev_bucket(const PlanCtx &c, uint64_t b)
+constexpr uint64_t GP_NO_BUCKET = ~0ull;
+
+// The last index of [a, z) whose prefix is below x, by one warp; hist[a] < x <= hist[z].
+__device__ __forceinline__ uint64_t last_below(const uint64_t *hist, uint64_t a, uint64_t z, uint64_t x)
 {
-    const uint64_t s = c.hist[b], first = max(c.lo, b & ~(uint64_t)(NB - 1));
-    if (c.hist[first] == s) return ~0ull;
-    uint64_t p = b - 1;
-    for (int i = 0; i < 4; i++, p--)
-        if (c.hist[p] != s) return p;
-    uint64_t a = first, z = p + 1;  // the first index whose prefix is s ends the bucket before b
-    while (a < z) {
-        const uint64_t m = (a + z) >> 1;
-        if (c.hist[m] < s) a = m + 1; else z = m;
+    const int lane = threadIdx.x & 31;
+    while (z - a > 1) {
+        const uint64_t step = (z - a + 32) / 33, m = a + (uint64_t)(lane + 1) * step;
+        const int n = __popc(__ballot_sync(FULLG, m < z && hist[m] < x));
+        a += (uint64_t)n * step;
+        z = min(z, a + step);
     }
-    return a - 1;
+    return a;
 }
 
-// Whether bucket b (populated, prefix [s, e) from the scan's start) starts a unit (bit 0) and a thread range (bit 3).
+struct PrevSmem {
+    int last[GP_COUNT_BLOCK / 32];
+    uint64_t before;
+};
+
+// The populated bucket before b within b's segment (GP_NO_BUCKET: none), for a block's buckets b0 + thread, which are of
+// one segment; s: b's prefix; populated: b is asked for.  All threads come here.  Only the block's first populated bucket
+// has to search (every one of a sparse histogram searching for itself was 20 dependent loads: 20 us of each planning kernel
+// for 10,000 reads).
+__device__ __forceinline__ uint64_t prev_bucket(const PlanCtx &c, uint64_t b0, bool populated, PrevSmem &sm)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t m = __ballot_sync(FULLG, populated);
+    if (lane == 0) sm.last[warp] = m ? warp * 32 + 31 - __clz(m) : -1;
+    if (warp == 0) {
+        const uint64_t first = max(c.lo, b0 & ~(uint64_t)(NB - 1)), s0 = c.hist[b0];
+        uint64_t p = GP_NO_BUCKET;
+        if (b0 > first && c.hist[first] != s0) {
+            const uint64_t q = b0 - 1 - lane;
+            const uint32_t near = __ballot_sync(FULLG, q >= first && q < b0 && c.hist[q] < s0);
+            p = near ? b0 - (uint64_t)__ffs(near) : last_below(c.hist, first, b0, s0);
+        }
+        if (lane == 0) sm.before = p;
+    }
+    __syncthreads();
+    const uint32_t lower = m & ((1u << lane) - 1);
+    if (lower) return b0 + (uint64_t)(warp * 32 + 31 - __clz(lower));
+    for (int w = warp - 1; w >= 0; w--)
+        if (sm.last[w] >= 0) return b0 + (uint64_t)sm.last[w];
+    return sm.before;
+}
+
+// Whether bucket b (populated, prefix [s, e) from the scan's start, p the one before) starts a unit (bit 0) and a thread range (bit 3).
 // Units never cross a thread range, a segment, a bin or a multiple of 2^GP_UNIT_SHIFT tuples, except that a bucket which
 // would make its unit larger than GP_CAP_S is a unit of its own: every decision is local to the bucket and its
 // predecessor, so the plan is two parallel passes (a greedy packing by one thread per 256 buckets took 140-210 us).
-__device__ __forceinline__ uint32_t plan_flags(const PlanCtx &c, uint64_t b, uint64_t s, uint64_t e)
+__device__ __forceinline__ uint32_t plan_flags(const PlanCtx &c, uint64_t b, uint64_t s, uint64_t e, uint64_t p)
 {
-    const uint64_t p = prev_bucket(c, b);
-    if (p == ~0ull) return 9u;
+    if (p == GP_NO_BUCKET) return 9u;
     const uint64_t sp = c.hist[p] - c.hist[c.lo];
     const uint64_t rel = b - c.lo;
     const bool brk = (c.brk[rel >> 5] >> (rel & 31)) & 1u;
@@ -88,18 +118,16 @@ __device__ __forceinline__ uint32_t plan_flags(const PlanCtx &c, uint64_t b, uin
     return (unit ? 1u : 0u) | (brk ? 8u : 0u);
 }
 
-// The bucket that starts at each thread range's first tuple.
+// The bucket that starts at each thread range's first tuple, a warp each: the last one whose prefix is not above that is the
+// populated one.
 __global__ void k_gp_marks(const uint64_t *hist, uint64_t lo, uint64_t hi, const uint64_t *bounds, int nb, uint32_t *brk)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (t >= nb) return;
     const uint64_t x = bounds[t] + hist[lo];
-    uint64_t a = lo, z = hi;  // the last bucket whose prefix is x is the populated one
-    while (a < z) {
-        const uint64_t m = (a + z) >> 1;
-        if (hist[m + 1] <= x) a = m + 1; else z = m;
-    }
-    if (a < hi) atomicOr(&brk[(a - lo) >> 5], 1u << ((a - lo) & 31));
+    if (x >= hist[hi]) return;
+    const uint64_t a = last_below(hist, lo, hi, x + 1);
+    if ((threadIdx.x & 31) == 0) atomicOr(&brk[(a - lo) >> 5], 1u << ((a - lo) & 31));
 }
 
 __device__ __forceinline__ uint64_t block_scan_excl(uint64_t v, uint64_t *total, uint64_t *ws)
@@ -127,12 +155,15 @@ __device__ __forceinline__ uint64_t block_scan_excl(uint64_t v, uint64_t *total,
 // Units starting in each block of GP_COUNT_BLOCK buckets.
 __global__ void __launch_bounds__(GP_COUNT_BLOCK) k_gp_count(PlanCtx c, uint64_t *blk)
 {
-    const uint64_t b = c.lo + (uint64_t)blockIdx.x * GP_COUNT_BLOCK + threadIdx.x;
-    bool f = false;
+    __shared__ PrevSmem ps;
+    const uint64_t b0 = c.lo + (uint64_t)blockIdx.x * GP_COUNT_BLOCK, b = b0 + threadIdx.x;
+    uint64_t s = 0, e = 0;
     if (b < c.hi) {
-        const uint64_t h0 = c.hist[c.lo], s = c.hist[b], e = c.hist[b + 1];
-        f = s != e && (plan_flags(c, b, s - h0, e - h0) & 1u);
+        s = c.hist[b];
+        e = c.hist[b + 1];
     }
+    const uint64_t h0 = c.hist[c.lo], p = prev_bucket(c, b0, s != e, ps);
+    const bool f = s != e && (plan_flags(c, b, s - h0, e - h0, p) & 1u);
     const int n = __syncthreads_count(f);
     if (threadIdx.x == 0) blk[blockIdx.x] = (uint64_t)n;
 }
@@ -168,15 +199,16 @@ __global__ void __launch_bounds__(GP_COUNT_BLOCK) k_gp_write(PlanCtx c, const ui
 {
     __shared__ uint32_t ws[GP_COUNT_BLOCK / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t b = c.lo + (uint64_t)blockIdx.x * GP_COUNT_BLOCK + threadIdx.x;
+    __shared__ PrevSmem ps;
+    const uint64_t b0 = c.lo + (uint64_t)blockIdx.x * GP_COUNT_BLOCK, b = b0 + threadIdx.x;
     uint64_t s = 0, e = 0;
-    uint32_t f = 0;
     if (b < c.hi) {
         const uint64_t h0 = c.hist[c.lo];
         s = c.hist[b] - h0;
         e = c.hist[b + 1] - h0;
-        if (s != e) f = plan_flags(c, b, s, e);
     }
+    const uint64_t p = prev_bucket(c, b0, s != e, ps);
+    const uint32_t f = s != e ? plan_flags(c, b, s, e, p) : 0u;
     const uint32_t m = __ballot_sync(FULLG, f & 1u);
     if (lane == 0) ws[warp] = (uint32_t)__popc(m);
     __syncthreads();
@@ -211,20 +243,32 @@ __global__ void __launch_bounds__(GP_COUNT_BLOCK) k_gp_write(PlanCtx c, const ui
 constexpr int SP_THREADS = 512, SP_ITEMS = 12, SP_TILE = SP_THREADS * SP_ITEMS;
 constexpr uint32_t SP_EXTRA = GROUP_MAX_MERGED - 1;  // digits above GP_DIGITS: a bin that a scan's bounds cut counts once more
 
-// Tiles of the second pass, every bin's own: first tuple, tuples, bin.
+// Tiles of the second pass, every bin's own: first tuple, tuples, bin.  Every block counts the tiles and writes its share
+// (one block with a bin's tiles per thread took 115 us at 200,000 tiles).
 __global__ void __launch_bounds__(1024) k_gp_tiles(const uint32_t *bstart, uint32_t nb, uint32_t *ctr, uint4 *tiles)
 {
     __shared__ uint64_t ws[32];
-    uint64_t carry = 0;
+    __shared__ uint32_t at[1024], sb[1025];
+    uint32_t carry = 0;
     for (uint32_t i0 = 0; i0 < nb; i0 += 1024) {
-        const uint32_t i = i0 + threadIdx.x, s = i < nb ? bstart[i] : 0, e = i < nb ? bstart[i + 1] : 0;
-        const uint32_t t = (e - s + SP_TILE - 1) / SP_TILE;
+        const uint32_t i = i0 + threadIdx.x, s = bstart[min(i, nb)], e = bstart[min(i + 1, nb)];
         uint64_t tot;
-        const uint64_t x = carry + block_scan_excl(t, &tot, ws);
-        for (uint32_t q = 0; q < t; q++) tiles[x + q] = make_uint4(s + q * SP_TILE, min((uint32_t)SP_TILE, e - s - q * SP_TILE), i, 0);
-        carry += tot;
+        at[threadIdx.x] = (uint32_t)block_scan_excl((e - s + SP_TILE - 1) / SP_TILE, &tot, ws);
+        sb[threadIdx.x] = s;
+        if (threadIdx.x == 1023) sb[1024] = e;
+        __syncthreads();
+        for (uint32_t t = blockIdx.x * 1024 + threadIdx.x; t < (uint32_t)tot; t += gridDim.x * 1024) {
+            uint32_t x = 0;  // the last bin whose first tile is not after t (it has tiles)
+#pragma unroll
+            for (uint32_t w = 512; w; w >>= 1)
+                if (at[x + w] <= t) x += w;
+            const uint32_t o = (t - at[x]) * SP_TILE;
+            tiles[carry + t] = make_uint4(sb[x] + o, min((uint32_t)SP_TILE, sb[x + 1] - sb[x] - o), i0 + x, 0);
+        }
+        __syncthreads();
+        carry += (uint32_t)tot;
     }
-    if (threadIdx.x == 0) ctr[GC_TILES] = (uint32_t)carry;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctr[GC_TILES] = carry;
 }
 
 struct SplitSmem {
@@ -950,25 +994,33 @@ __global__ void k_gbig_reserve(uint32_t *ctr, uint32_t n, uint32_t *base) { *bas
 // read when it carries the scan's last k-mer, which only the last range with tuples can hold and only if no
 // smaller k-mer of that range has a read that is not BAD.  Per segment, over the grouped stretches of its last
 // range: [0] a read outside the last run, [1] one inside, [2] its id.
+// A block looks at a segment's stretches until it or another has found a read outside, and asks for that once a stretch
+// (asked for at every read by every thread, and set by every one that found it, the words of one segment were a queue: 245
+// us of 20M reads' scans).
 __global__ void __launch_bounds__(256) k_gp_quirk(const uint32_t *ctr, const uint32_t *qlist, const uint32_t *out,
-                                                  const uint8_t *filtered, uint32_t *quirk)
+                                                  const uint8_t *filtered, int nseg, uint32_t *quirk)
 {
     volatile uint32_t *vq = quirk;
     const uint32_t nq = ctr[GC_QLIST];
+    uint32_t known = ~0u;  // a segment with a read outside
     for (uint32_t q = blockIdx.x; q < nq; q += gridDim.x) {
         const uint32_t o = qlist[3 * (size_t)q], len = qlist[3 * (size_t)q + 1], seg = qlist[3 * (size_t)q + 2];
-        const uint32_t l0 = quirk[seg * QW + 3], l1 = l0 + quirk[seg * QW + 4];
-        for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) {
-            if (vq[seg * QW]) break;
-            const uint32_t id = out[o + i] & 0x7FFFFFFFu;
-            if (id == GP_NONE || filtered[id]) continue;
-            if (o + i >= l0 && o + i < l1) {
-                quirk[seg * QW + 2] = id;
-                quirk[seg * QW + 1] = 1;
-            } else {
-                quirk[seg * QW] = 1;
+        if (seg != known) {
+            const uint32_t l0 = quirk[seg * QW + 3], l1 = l0 + quirk[seg * QW + 4];
+            bool found = __syncthreads_or(threadIdx.x == 0 && vq[seg * QW]);
+            for (uint32_t i0 = 0; i0 < len && !found; i0 += blockDim.x) {
+                const uint32_t i = i0 + threadIdx.x, id = i < len ? out[o + i] & 0x7FFFFFFFu : GP_NONE;
+                const bool good = id != GP_NONE && !filtered[id], in = o + i >= l0 && o + i < l1;
+                if (good && in) {
+                    quirk[seg * QW + 2] = id;
+                    quirk[seg * QW + 1] = 1;
+                }
+                found = __syncthreads_or(good && !in);
+                if (found && threadIdx.x == 0) quirk[seg * QW] = 1;
             }
+            if (found) known = seg;
         }
+        if (nseg == 1 && known == seg) return;
     }
 }
 
@@ -1123,12 +1175,12 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
     MP_CUDA(cudaMemcpyAsync(d_bounds, g.bounds.data(), nbounds * 8, cudaMemcpyHostToDevice, st));
     MP_CUDA(cudaMemcpyAsync(g.seg_bin0, h.data(), h.size() * 4, cudaMemcpyHostToDevice, st));
     const PlanCtx c{g.d_hist, g.lo, g.hi, brk, g.seg_sh, g.seg_bin0, g.seg_lo};
-    (count_launch(), k_gp_marks<<<blocks_of(nbounds, 64), 64, 0, st>>>(g.d_hist, g.lo, g.hi, d_bounds, (int)nbounds, brk));
+    (count_launch(), k_gp_marks<<<blocks_of(nbounds, 4), 128, 0, st>>>(g.d_hist, g.lo, g.hi, d_bounds, (int)nbounds, brk));
     (count_launch(), k_gp_count<<<nblk, GP_COUNT_BLOCK, 0, st>>>(c, blk));
     (count_launch(), k_gp_scan<<<1, 1024, 0, st>>>(blk, nblk, (uint32_t)g.n, g.bins, g.ctr, g.ustart, g.bstart, g.bu0));
     (count_launch(), k_gp_write<<<nblk, GP_COUNT_BLOCK, 0, st>>>(c, blk, g.ctr, g.ustart, g.ub0, g.ucur, g.bstart, g.bu0,
                                                                   g.merged ? nullptr : g.bcur, g.bin_sh, g.bfirst, g.unit_of, g.mid, g.big));
-    (count_launch(), k_gp_tiles<<<1, 1024, 0, st>>>(g.bstart, g.bins, g.ctr, g.tiles));
+    (count_launch(), k_gp_tiles<<<std::min(32u, g.max_tiles / 2048 + 1), 1024, 0, st>>>(g.bstart, g.bins, g.ctr, g.tiles));
     ReadBack<uint32_t> rb(arena, GC_N, PLAN_MAIL);
     if (!arena.mail) {
         g.h_ctr.assign(GC_N, 0);
@@ -1378,7 +1430,8 @@ int group_union(GroupScan &g, const uint32_t *out, uint32_t *parent, const uint8
 {
     const int nseg = (int)g.seg_tstart.size() - 1;
     open.clear();
-    (count_launch(), k_gp_quirk<<<64, 256, 0, st>>>(g.ctr, g.qlist, out, filtered, g.quirk));
+    (count_launch(), k_gp_quirk<<<std::min(2u * (unsigned)sm_count(), g.hctr[GC_UNITS] / 16 + 1), 256, 0, st>>>(g.ctr, g.qlist, out, filtered, nseg,
+                                                                                                            g.quirk));
     const unsigned blocks = std::min<unsigned>(8u * (unsigned)sm_count(), blocks_of(g.n, (int)GE_SEG * 8));
     uint32_t *err = arena.alloc<uint32_t>(1);
     if (!err) return set_error(MP_ENOMEM, "device memory");

@@ -23,7 +23,7 @@ constexpr unsigned FULLG = 0xFFFFFFFFu;
 // ------------------------------------------------------------------ plan
 
 constexpr int GP_UNIT_SHIFT = 12;        // units end where the tuple prefix crosses a multiple of 4096
-constexpr int GP_CAP_S = 6128;           // most tuples of a unit for the 512-thread blocks (two per SM)
+constexpr int GP_CAP_S = 6128;           // most tuples of a unit for the small blocks (two per SM)
 constexpr int GP_CAP_L = 12288;          // and for the 1024-thread blocks; a larger bucket takes the device-wide sort
 constexpr uint32_t GP_DIGITS = 1024;     // digits of a split pass: bins of a segment, units of a bin
 constexpr uint64_t GP_SMALL = 1500000;   // tuples of a segment that fit GP_DIGITS units however they are spread
@@ -681,9 +681,11 @@ struct GroupCtx {
 };
 
 // Bound by shared memory (random accesses and atomics: about five per tuple), its instructions and the block's barriers;
-// two 512-thread blocks per SM overlap each other's.  20M x 150 bp, 2 scans (2.39 G tuples): 28 ms for both block
-// shapes, where sorting the units (66.8 ms) and judging the sorted runs (31.9 ms) took 98.7.  30.4 with every tuple's info
-// read again for the marks and the rare tests in the probe loop; probing pairs of slots at once gained nothing.
+// two small blocks per SM overlap each other's.  20M x 150 bp, 2 scans (2.39 G tuples): 26.3 ms for both block shapes,
+// where sorting the units (66.8 ms) and judging the sorted runs (31.9 ms) took 98.7.  A tuple's slot, its number there
+// and its codes share a word, so that 768 threads of 8 tuples keep 40 registers: 512 of 12 took 27.9 ms, 1024 of 6 27.2;
+// every tuple's info read again for the marks and the rare tests in the probe loop 30.4; probing pairs of slots at once
+// gained nothing.
 //
 // One block per unit (persistent, units handed out by a counter): the unit's tuples into a hash table of its
 // k-mers (open addressing in shared memory), the filter's judgement of every k-mer, its marks, and the reads of
@@ -696,7 +698,7 @@ struct GroupCtx {
 // Later use of info: count (0-13), branching side (14-15: 0 none, 1 before, 2 after, 3 both), the run's counters
 // in pool (16-28), then the judgement (16-18 most frequent code, 19 second count above 0.2), kept (31).
 template <int THREADS, int ITEMS, int SLOT_BITS>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
+__global__ void __launch_bounds__(THREADS, SLOT_BITS == 13 ? 2 : 1) k_group(GroupCtx c)
 {
     typedef GroupSmem<THREADS, ITEMS, SLOT_BITS> Smem;
     constexpr uint32_t SLOTS = Smem::SLOTS, SMASK = SLOTS - 1;
@@ -754,15 +756,21 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
             if (lane == 0) atomicMax(&sm.maxkey, m);
             __syncthreads();
         }
-        // ---- every tuple's slot and its number within the slot (sr: slot 0-13, number 16-29), codes in ac
-        uint32_t sr[ITEMS], ac[ITEMS];
+        // ---- every tuple's slot, its number within the slot and its codes, in one word where they fit
+        constexpr bool PACK = 2 * SLOT_BITS + 6 <= 32;
+        uint32_t sr[ITEMS] = {}, ac[PACK ? 1 : ITEMS] = {};
+        auto slot = [&](int j) { return sr[j] & SMASK; };
+        auto number = [&](int j) { return (sr[j] >> SLOT_BITS) & SMASK; };
+        auto code6 = [&](int j) { return PACK ? sr[j] >> 26 : ac[PACK ? 0 : j]; };
+        auto set_code6 = [&](int j, uint32_t v) {
+            if (PACK) sr[j] = (sr[j] & 0x3FFFFFFu) | (v << 26);
+            else ac[PACK ? 0 : j] = v;
+        };
 #pragma unroll
         for (int j = 0; j < ITEMS; j++) {
-            sr[j] = 0;
-            ac[j] = (uint32_t)key[j] & 63u;
             if (j * THREADS + tid < cnt) {
                 const unsigned long long k = key[j] >> 6;
-                const uint32_t kh = key_hash(k), step = kh | 1u;
+                const uint32_t kh = key_hash(k), step = kh | 1u, code = (uint32_t)key[j] & 63u;
                 uint32_t h = kh >> (32 - SLOT_BITS);
                 for (;;) {
                     unsigned long long v = vkey[h];
@@ -773,12 +781,14 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
                     if (v == k) break;
                     h = (h + step) & SMASK;
                 }
-                const uint32_t m = ((0x10000u << (ac[j] & 7u)) & 0x7F0000u) | ((0x800000u << (ac[j] >> 3)) & 0x3F800000u);
+                const uint32_t m = ((0x10000u << (code & 7u)) & 0x7F0000u) | ((0x800000u << (code >> 3)) & 0x3F800000u);
                 const uint32_t old = atomicAdd(&sm.info[h], 1u);
                 if (m & ~old) atomicOr(&sm.info[h], m);
-                sr[j] = h | (old << 16);
+                sr[j] = h | ((old & SMASK) << SLOT_BITS);
+                set_code6(j, code);
             }
         }
+        uint32_t zeros = 0, kept_here = 0;  // a bit per tuple: the zero k-mer's; the first of a slot whose reads are kept
         const bool zero_bucket = (b0 & (NB - 1)) == 0;
         if (ends || zero_bucket) {
             const unsigned long long mx = sm.maxkey;
@@ -786,8 +796,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
             for (int j = 0; j < ITEMS; j++) {
                 if (j * THREADS + tid < cnt) {
                     const unsigned long long k = key[j] >> 6;
-                    if (zero_bucket && k == 0) ac[j] |= 64u;
-                    if (ends && k == mx) sm.slot_ex = sr[j] & 0xFFFFu;
+                    if (zero_bucket && k == 0) zeros |= 1u << j;
+                    if (ends && k == mx) sm.slot_ex = slot(j);
                 }
             }
         }
@@ -803,8 +813,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
         uint32_t kept = 0;
 #pragma unroll
         for (int j = 0; j < ITEMS; j++) {
-            if (j * THREADS + tid < cnt && (sr[j] >> 16) == 0) {
-                const uint32_t h = sr[j], inf = sm.info[h], n = inf & 0xFFFFu;
+            if (j * THREADS + tid < cnt && number(j) == 0) {
+                const uint32_t h = slot(j), inf = sm.info[h], n = inf & 0xFFFFu;
                 uint32_t side = 0;
                 if (h != ex) side = (__popc(inf & 0x7F0000u) > 1 ? 1u : 0u) | (__popc(inf & 0x3F800000u) > 1 ? 2u : 0u);
                 uint32_t ni = n | (side << 14);
@@ -813,10 +823,10 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
                     reinterpret_cast<uint4 *>(sm.u.b.pool)[p] = make_uint4(0, 0, 0, h << 16);
                     ni |= p << 16;
                 }
-                if (side != 3u && !(ac[j] & 64u) && (n >= 2u || singles)) {
+                if (side != 3u && !((zeros >> j) & 1u) && (n >= 2u || singles)) {
                     ni |= GI_KEPT;
                     kept += n;
-                    ac[j] |= 128u;
+                    kept_here |= 1u << j;
                 }
                 sm.info[h] = ni;
             }
@@ -840,23 +850,24 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
         if (tid == 0) sm.base = atomicAdd(&c.ctr[GC_OUT], total);
 #pragma unroll
         for (int j = 0; j < ITEMS; j++) {
-            if (ac[j] & 128u) {
-                const uint32_t h = sr[j] & 0xFFFFu;
+            if ((kept_here >> j) & 1u) {
+                const uint32_t h = slot(j);
                 sm.u.b.off[h] = (uint16_t)at;
                 at += sm.info[h] & 0x3FFFu;
             }
         }
-        // ---- code counts of the runs branching on one side; ac: such a run's tuple (bit 6) and its code there, kept (bit 7)
+        // ---- code counts of the runs branching on one side; then code6: such a run's tuple (bit 3) and its code there, kept (4)
 #pragma unroll
         for (int j = 0; j < ITEMS; j++) {
             if (j * THREADS + tid < cnt) {
-                const uint32_t inf = sm.info[sr[j] & 0xFFFFu], side = (inf >> 14) & 3u;
-                const uint32_t code = side == 1u ? ac[j] & 7u : (ac[j] >> 3) & 7u;
-                ac[j] = (inf & GI_KEPT) >> 24;
+                const uint32_t inf = sm.info[slot(j)], side = (inf >> 14) & 3u;
+                const uint32_t code = side == 1u ? code6(j) & 7u : code6(j) >> 3;
+                uint32_t v = inf & GI_KEPT ? 16u : 0u;
                 if (side == 1u || side == 2u) {
-                    ac[j] |= 64u | code;
+                    v |= 8u | code;
                     if (code < 7u) atomicAdd(&sm.u.b.pool[((inf >> 16) & 0x1FFFu) * 4 + (code >> 1)], 1u << (16 * (code & 1)));
                 }
+                set_code6(j, v);
             }
         }
         __syncthreads();
@@ -882,15 +893,15 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
 #pragma unroll
         for (int j = 0; j < ITEMS; j++) {
             if (j * THREADS + tid < cnt) {
-                const uint32_t h = sr[j] & 0xFFFFu;
-                if (ac[j] & 64u) {
+                const uint32_t h = slot(j), v = code6(j);
+                if (v & 8u) {
                     const uint32_t inf = sm.info[h];
-                    if ((ac[j] & 7u) != ((inf >> 16) & 7u) || (inf & (1u << 19))) {
+                    if ((v & 7u) != ((inf >> 16) & 7u) || (inf & (1u << 19))) {
                         c.parent[id[j]] = BAD;
                         c.filtered[id[j]] = 1;
                     }
                 }
-                if (ac[j] & 128u) stage[sm.u.b.off[h] + (sr[j] >> 16)] = id[j] | ((sr[j] >> 16) == 0 ? 0x80000000u : 0u);
+                if (v & 16u) stage[sm.u.b.off[h] + number(j)] = id[j] | (number(j) == 0 ? 0x80000000u : 0u);
             }
         }
         if (singles && tid == 0) {
@@ -911,7 +922,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_group(GroupCtx c)
         for (uint32_t i = tid; i < total; i += THREADS) o[i] = stage[i];
     }
 }
-typedef GroupSmem<512, 12, 13> GroupSmemS;
+constexpr int GP_THREADS = 768, GP_ITEMS = 8;  // small blocks (k_group)
+typedef GroupSmem<GP_THREADS, GP_ITEMS, 13> GroupSmemS;
 typedef GroupSmem<1024, 12, 14> GroupSmemL;
 static_assert(GP_CAP_S <= GroupSmemS::CAP && GP_CAP_L <= GroupSmemL::CAP, "a unit fits its block's slots");
 static_assert(GP_CAP_S * 8 <= GroupSmemS::SLOTS * 6 && GP_CAP_L * 8 <= GroupSmemL::SLOTS * 6,
@@ -1120,7 +1132,7 @@ static void group_kernel_attrs()
             cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinSmem));
         cudaFuncSetAttribute(k_split_tuples, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SplitSmem));
         cudaFuncSetAttribute(k_split_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(UnitSmem));
-        cudaFuncSetAttribute(k_group<512, 12, 13>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmemS));
+        cudaFuncSetAttribute(k_group<GP_THREADS, GP_ITEMS, 13>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmemS));
         cudaFuncSetAttribute(k_group<1024, 12, 14>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GroupSmemL));
     });
 }
@@ -1357,7 +1369,7 @@ int group_filter(GroupScan &g, const uint64_t *kk, const uint32_t *ids, uint32_t
     GroupCtx c{kk, ids, g.ustart, g.ub0, fill, g.lrs, nullptr, g.ctr, g.qlist, g.quirk, GC_WORK_S, GC_UNITS, 0, (uint32_t)GP_CAP_S,
                out, parent, filtered};
     const unsigned sms = (unsigned)sm_count();
-    (count_launch(), k_group<512, 12, 13><<<std::min(2 * sms, std::max(1u, g.hctr[GC_UNITS])), 512, sizeof(GroupSmemS), st>>>(c));
+    (count_launch(), k_group<GP_THREADS, GP_ITEMS, 13><<<std::min(2 * sms, std::max(1u, g.hctr[GC_UNITS])), GP_THREADS, sizeof(GroupSmemS), st>>>(c));
     if (g.hctr[GC_MID]) {
         c.list = g.mid;
         c.work = GC_WORK_L;

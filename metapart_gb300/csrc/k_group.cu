@@ -376,6 +376,7 @@ __device__ __forceinline__ void split_store(SplitSmem &sm, uint32_t nv, uint64_t
 // segment of every tile; null for one segment.
 struct SegTiles {
     const uint32_t *tile_seg = nullptr, *tile0 = nullptr, *start = nullptr;
+    const uint4 *shape = nullptr;  // of reads: the tiling of each segment's reads (P, spr, rounds, rpt of ReadTiles)
 };
 
 __global__ void k_gp_segtiles(const uint32_t *tile0, int nseg, uint32_t *tile_seg)
@@ -424,8 +425,11 @@ __device__ __forceinline__ void bin_tile(const BinCtx &c, uint32_t tile, uint32_
 //
 // HI: 2k >= 34 and bins of at least 2^32 k-mers, so a k-mer's bin is a shift of its high word.
 //
-// MERGED: the tuples of all scans (group_bins_scans).  Packing the reads and rolling through them was half of the pass.
-template <bool HI, bool MERGED>
+// SR_MERGED: the tuples of all scans (group_bins_scans).  Packing the reads and rolling through them was half of the pass.
+// SR_SEGMENTS: each segment's reads have their own tiling (samples of reads of 100 bases tiled as ones of 250 left two
+// threads of three idle).
+enum { SR_ONE = 0, SR_MERGED = 1, SR_SEGMENTS = 2 };
+template <bool HI, int MODE>
 __global__ void __launch_bounds__(SP_THREADS, 2) k_split_reads(BinCtx c)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -433,17 +437,28 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_reads(BinCtx c)
     __shared__ uint32_t many[SP_THREADS];
     const int tid = threadIdx.x;
     for (uint32_t d = tid; d < GP_DIGITS + SP_EXTRA; d += SP_THREADS) sm.hist[d] = 0;
-    const uint32_t per = c.t.rpt, rr = tid / c.t.spr, i0 = (tid - rr * c.t.spr) * c.t.P;
-    uint32_t seg, base, end;
-    if (blockIdx.x < c.tiles) {
-        bin_tile(c, blockIdx.x, per, c.n_reads, seg, base, end);
-        rt_pack(c.t, base, end - base, sm.packed);
-    }
+    constexpr bool MERGED = MODE == SR_MERGED;
+    ReadTiles t = c.t;
+    uint32_t seg = 0, base = 0, end = 0, rr = tid / t.spr, i0 = (tid - rr * t.spr) * t.P;
+    auto take = [&](uint32_t tile) {  // the tile's reads, packed
+        if constexpr (MODE == SR_SEGMENTS) {
+            const uint4 s = c.sg.shape[c.sg.tile_seg[tile]];
+            t.P = s.x;
+            t.spr = s.y;
+            t.rounds = s.z;
+            t.rpt = s.w;
+            rr = tid / t.spr;
+            i0 = (tid - rr * t.spr) * t.P;
+        }
+        bin_tile(c, tile, t.rpt, c.n_reads, seg, base, end);
+        rt_pack(t, base, end - base, sm.packed);
+    };
+    if (blockIdx.x < c.tiles) take(blockIdx.x);
     for (uint32_t tile = blockIdx.x; tile < c.tiles; tile += gridDim.x) {
         const uint32_t d0 = MERGED ? 0u : c.seg_bin0[seg], nd = MERGED ? c.m_digits : c.seg_bin0[seg + 1] - d0;
         const int bits = c.bsh + (int)(MERGED ? c.m_sh : c.seg_sh[seg]);  // a k-mer's bits within its bin
         const uint64_t mask = (1ull << bits) - 1;
-        const uint32_t r = base + rr, L = rr < per && r < end ? c.t.seq_len[r] : 0u;
+        const uint32_t r = base + rr, L = rr < t.rpt && r < end ? c.t.seq_len[r] : 0u;
         uint32_t id = r;
         if (c.label && L) {
             const uint32_t p = c.label[r];
@@ -454,7 +469,7 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_reads(BinCtx c)
         uint32_t kl[SP_ITEMS], kh[SP_ITEMS], rd[SP_ITEMS];
         {
             KmerRoll<HI> s = {};
-            if (L > (uint32_t)c.t.k && i0 <= L - (uint32_t)c.t.k) s.init(c.t, sm.packed + rr * rt_stride(c.t), L, i0);
+            if (L > (uint32_t)c.t.k && i0 <= L - (uint32_t)c.t.k) s.init(t, sm.packed + rr * rt_stride(t), L, i0);
             const uint32_t mh = (uint32_t)(mask >> 32), dsh = HI ? bits - 32 : bits;
             const uint32_t cn[2] = {s.compl_nibbles(s.an[0]), s.compl_nibbles(s.an[1])};
             const uint32_t cp[2] = {s.compl_nibbles(s.ap[0]), s.compl_nibbles(s.ap[1])};
@@ -506,10 +521,7 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_reads(BinCtx c)
         // the next tile's reads while others store (its bytes fetched before the stores instead cost registers that spill: 37.5
         // against 35.7 ms at 20M x 150 bp, 2 scans)
         const uint32_t next = tile + gridDim.x;
-        if (next < c.tiles) {
-            bin_tile(c, next, per, c.n_reads, seg, base, end);
-            rt_pack(c.t, base, end - base, sm.packed);
-        }
+        if (next < c.tiles) take(next);
     }
 }
 
@@ -1128,7 +1140,8 @@ static void group_kernel_attrs()
     int dev = 0;
     cudaGetDevice(&dev);
     std::call_once(once[dev & 63], [] {
-        for (auto f : {k_split_reads<true, false>, k_split_reads<false, false>, k_split_reads<true, true>, k_split_reads<false, true>})
+        for (auto f : {k_split_reads<true, SR_ONE>, k_split_reads<false, SR_ONE>, k_split_reads<true, SR_MERGED>, k_split_reads<false, SR_MERGED>,
+                       k_split_reads<true, SR_SEGMENTS>, k_split_reads<false, SR_SEGMENTS>})
             cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BinSmem));
         cudaFuncSetAttribute(k_split_tuples, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SplitSmem));
         cudaFuncSetAttribute(k_split_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(UnitSmem));
@@ -1214,7 +1227,9 @@ static int group_counts(GroupScan &g, DeviceArena &arena)
     return 0;
 }
 
-static int launch_bins(GroupScan &g, BinCtx &c, const std::vector<uint64_t> &seg_start, DeviceArena &arena, cudaStream_t st)
+// seg_shape: every segment's tiling of its reads (null: c.t for all).
+static int launch_bins(GroupScan &g, BinCtx &c, const std::vector<uint64_t> &seg_start, const std::vector<uint32_t> *seg_shape,
+                       DeviceArena &arena, cudaStream_t st)
 {
     group_kernel_attrs();
     const int nseg = (int)g.seg_tstart.size() - 1;
@@ -1223,20 +1238,23 @@ static int launch_bins(GroupScan &g, BinCtx &c, const std::vector<uint64_t> &seg
     c.tiles = blocks_of(reads ? c.n_reads : g.n, (int)per);
     if (nseg > 1) {
         std::vector<uint32_t> &h = g.h_tiles;
-        h.assign(2 * (size_t)nseg + 2, 0);
+        const size_t shapes = seg_shape ? 4 * (size_t)nseg : 0;  // first: they are read 16 bytes at a time
+        h.assign(shapes + 2 * (size_t)nseg + 2, 0);
         c.tiles = 0;
         for (int q = 0; q <= nseg; q++) {
-            h[q] = c.tiles;
-            h[nseg + 1 + q] = (uint32_t)seg_start[q];
-            if (q < nseg) c.tiles += blocks_of(seg_start[q + 1] - seg_start[q], (int)per);
+            h[shapes + q] = c.tiles;
+            h[shapes + nseg + 1 + q] = (uint32_t)seg_start[q];
+            if (q < nseg) c.tiles += blocks_of(seg_start[q + 1] - seg_start[q], seg_shape ? (int)(*seg_shape)[4 * q + 3] : (int)per);
         }
+        if (seg_shape) std::copy(seg_shape->begin(), seg_shape->end(), h.begin());
         uint32_t *d = arena.alloc<uint32_t>(h.size() + c.tiles);
         if (!d) return set_error(MP_ENOMEM, "device memory for the scan's tiles");
         MP_CUDA(cudaMemcpyAsync(d, h.data(), h.size() * 4, cudaMemcpyHostToDevice, st));
-        c.sg.tile0 = d;
-        c.sg.start = d + nseg + 1;
+        if (shapes) c.sg.shape = reinterpret_cast<const uint4 *>(d);
+        c.sg.tile0 = d + shapes;
+        c.sg.start = d + shapes + nseg + 1;
         c.sg.tile_seg = d + h.size();
-        (count_launch(), k_gp_segtiles<<<nseg, 256, 0, st>>>(d, nseg, d + h.size()));
+        (count_launch(), k_gp_segtiles<<<nseg, 256, 0, st>>>(d + shapes, nseg, d + h.size()));
     }
     c.n = (uint32_t)g.n;
     c.bsh = 2 * (g.k - 10);
@@ -1248,7 +1266,10 @@ static int launch_bins(GroupScan &g, BinCtx &c, const std::vector<uint64_t> &seg
     c.err = g.ctr + GC_ERR;
     uint32_t least = 16;  // the narrowest bins
     for (int q = 0; q < nseg; q++) least = std::min(least, g.h_plan[(size_t)nseg + 1 + q]);
-    auto kern = !reads ? k_split_tuples : g.k >= 17 && c.bsh + (int)least >= 32 ? k_split_reads<true, false> : k_split_reads<false, false>;
+    const bool high = g.k >= 17 && c.bsh + (int)least >= 32;
+    auto kern = !reads        ? k_split_tuples
+                : c.sg.shape ? (high ? k_split_reads<true, SR_SEGMENTS> : k_split_reads<false, SR_SEGMENTS>)
+                             : (high ? k_split_reads<true, SR_ONE> : k_split_reads<false, SR_ONE>);
     const unsigned blocks = std::min<unsigned>(c.tiles, 2u * (unsigned)sm_count());
     if (blocks) (count_launch(), kern<<<blocks, SP_THREADS, reads ? sizeof(BinSmem) : sizeof(SplitSmem), st>>>(c));
     MP_CUDA(cudaGetLastError());
@@ -1256,8 +1277,14 @@ static int launch_bins(GroupScan &g, BinCtx &c, const std::vector<uint64_t> &seg
 }
 
 int group_bins_reads(GroupScan &g, const uint8_t *fq, const ParsedReads &pr, const std::vector<uint64_t> &seg_reads,
-                     const uint32_t *label, uint64_t *k1, uint32_t *id1, DeviceArena &arena, cudaStream_t st)
+                     const uint32_t *label, uint64_t *k1, uint32_t *id1, DeviceArena &arena, cudaStream_t st,
+                     const std::vector<uint32_t> &seg_len)
 {
+    std::vector<uint32_t> shape;
+    for (uint32_t n : seg_len) {
+        const ReadTiles t = read_tiles(fq, pr, g.k, std::max(n, 1u), SP_THREADS, SP_PACKED);
+        shape.insert(shape.end(), {t.P, t.spr, t.rounds, t.rpt});
+    }
     BinCtx c;
     c.t = read_tiles(fq, pr, g.k, pr.max_len, SP_THREADS, SP_PACKED);
     c.n_reads = (uint32_t)pr.n_reads;
@@ -1265,7 +1292,7 @@ int group_bins_reads(GroupScan &g, const uint8_t *fq, const ParsedReads &pr, con
     c.label = label;
     c.out_k = k1;
     c.out_id = id1;
-    return launch_bins(g, c, seg_reads, arena, st);
+    return launch_bins(g, c, seg_reads, shape.empty() ? nullptr : &shape, arena, st);
 }
 
 int group_bins_tuples(GroupScan &g, const uint64_t *lo, const uint8_t *hi, const uint32_t *id, uint64_t *k1, uint32_t *id1,
@@ -1277,7 +1304,7 @@ int group_bins_tuples(GroupScan &g, const uint64_t *lo, const uint8_t *hi, const
     c.id = id;
     c.out_k = k1;
     c.out_id = id1;
-    return launch_bins(g, c, g.seg_tstart, arena, st);
+    return launch_bins(g, c, g.seg_tstart, nullptr, arena, st);
 }
 
 // The first tuple of every bin of the merged scans.
@@ -1334,7 +1361,7 @@ int group_bins_scans(MergedScans &m, const uint64_t *d_hist, int k, const uint8_
     c.m_digits = m.digits;
     c.m_sh = (uint32_t)m.sh;
     for (int s = 1; s < S; s++) c.m_start[s - 1] = (m.scan[s] - lo) << c.bsh;
-    auto kern = k >= 17 && c.bsh + m.sh >= 32 ? k_split_reads<true, true> : k_split_reads<false, true>;
+    auto kern = k >= 17 && c.bsh + m.sh >= 32 ? k_split_reads<true, SR_MERGED> : k_split_reads<false, SR_MERGED>;
     const unsigned blocks = std::min<unsigned>(c.tiles, 2u * (unsigned)sm_count());
     if (blocks) (count_launch(), kern<<<blocks, SP_THREADS, sizeof(BinSmem), st>>>(c));
     MP_CUDA(cudaGetLastError());

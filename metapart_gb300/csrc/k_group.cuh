@@ -85,10 +85,12 @@ struct GroupQuirk {
 bool group_fits(uint64_t n, uint64_t n_reads, const SortSegments *segs);
 // Plans g (its inputs set) on the device; its counts are on their way to the host (group_filter takes them).
 int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st);
-// First split pass, into bins, of n tuples to (k1, id1): enumerated from the reads (seg_reads: nseg + 1 read offsets; label: the reads' components, null in the first scan; every read at
-// most 300 positions), or of tuples enumerated before, segment-major.
+// First split pass, into bins, of n tuples to (k1, id1): enumerated from the reads (seg_reads: nseg + 1 read offsets; label:
+// the reads' components, null in the first scan; every read at most 300 positions; seg_len: with several segments, each
+// one's longest read, else empty), or of tuples enumerated before, segment-major.
 int group_bins_reads(GroupScan &g, const uint8_t *fq, const ParsedReads &pr, const std::vector<uint64_t> &seg_reads,
-                     const uint32_t *label, uint64_t *k1, uint32_t *id1, DeviceArena &arena, cudaStream_t st);
+                     const uint32_t *label, uint64_t *k1, uint32_t *id1, DeviceArena &arena, cudaStream_t st,
+                     const std::vector<uint32_t> &seg_len = {});
 int group_bins_tuples(GroupScan &g, const uint64_t *lo, const uint8_t *hi, const uint32_t *id, uint64_t *k1, uint32_t *id1,
                       DeviceArena &arena, cudaStream_t st);
 // Whether the scans [scan[s], scan[s + 1]) can be split together, and how (m's arrays are then the caller's to set).

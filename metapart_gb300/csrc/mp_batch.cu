@@ -50,6 +50,18 @@ __device__ __forceinline__ uint64_t lower_bound_dev(const uint64_t *h, uint64_t 
     return lo;
 }
 
+// Every sample's longest read (set to 0 before), LONGEST_BLOCKS blocks each.
+constexpr unsigned LONGEST_BLOCKS = 16;
+__global__ void __launch_bounds__(256) k_longest(const uint32_t *seq_len, const uint64_t *first, uint32_t *longest)
+{
+    uint32_t m = 0;
+#pragma unroll 4
+    for (uint64_t r = first[blockIdx.x] + blockIdx.y * 256 + threadIdx.x; r < first[blockIdx.x + 1]; r += LONGEST_BLOCKS * 256)
+        m = max(m, seq_len[r]);
+    m = __reduce_max_sync(0xFFFFFFFFu, m);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(&longest[blockIdx.x], m);
+}
+
 __global__ void k_batch_plan(const uint64_t *shist, int nseg, const uint32_t *T, const uint32_t *rb0, uint64_t *rb,
                              int *status)
 {
@@ -357,7 +369,10 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     int *dstat = A.alloc<int>(nseg);
     const size_t tbh = scan_tmp_bytes((size_t)nseg * NB);
     void *tmph = A.alloc<uint8_t>(tbh);
-    if (!shist || !dT || !drb0 || !drb || !dstat || !tmph) return set_error(MP_ENOMEM, "device memory for the group's plan");
+    uint64_t *dR = A.alloc<uint64_t>(nseg + 1);
+    uint32_t *dlongest = A.alloc<uint32_t>(nseg);
+    std::vector<uint32_t> longest(nseg, 0);  // every sample's longest read
+    if (!shist || !dT || !drb0 || !drb || !dstat || !tmph || !dR || !dlongest) return set_error(MP_ENOMEM, "device memory for the group's plan");
     std::vector<uint64_t> rb(Rn + 1);
     std::vector<int> hstat(nseg);
     uint32_t herr = 0;
@@ -367,6 +382,10 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
         MP_CUDA(cudaMemcpyAsync(dT, hT.data(), nseg * 4, cudaMemcpyHostToDevice, st));
         MP_CUDA(cudaMemcpyAsync(drb0, hrb0.data(), (nseg + 1) * 4, cudaMemcpyHostToDevice, st));
         (count_launch(), k_batch_plan<<<(nseg + 63) / 64, 64, 0, st>>>(shist, nseg, dT, drb0, drb, dstat));
+        MP_CUDA(cudaMemcpyAsync(dR, R.data(), (nseg + 1) * 8, cudaMemcpyHostToDevice, st));
+        MP_CUDA(cudaMemsetAsync(dlongest, 0, nseg * 4, st));
+        (count_launch(), k_longest<<<dim3((unsigned)nseg, LONGEST_BLOCKS), 256, 0, st>>>(pr.seq_len, dR, dlongest));
+        MP_CUDA(cudaMemcpyAsync(longest.data(), dlongest, nseg * 4, cudaMemcpyDeviceToHost, st));
         MP_CUDA(cudaMemcpyAsync(rb.data(), drb, (Rn + 1) * 8, cudaMemcpyDeviceToHost, st));
         MP_CUDA(cudaMemcpyAsync(hstat.data(), dstat, nseg * sizeof(int), cudaMemcpyDeviceToHost, st));
         MP_CUDA(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
@@ -411,7 +430,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
         {
             StageTimer tm(b->clk, st, 2, SPLIT_SLOT);
             if ((rc = group_plan(gs, A, st))) return rc;
-            if ((rc = group_bins_reads(gs, d_fq, pr, R, nullptr, sb.lo[1], sb.id[1], A, st))) return rc;
+            if ((rc = group_bins_reads(gs, d_fq, pr, R, nullptr, sb.lo[1], sb.id[1], A, st, nseg > 1 ? longest : std::vector<uint32_t>()))) return rc;
         }
         {
             StageTimer tm(b->clk, st, 3, SPLIT_SLOT);

@@ -287,7 +287,7 @@ struct UnitSmem : SplitSmem {
     uint16_t cell[GP_DIGITS];   // the bin's buckets in 1024 cells: the digit (times 4) of a cell's first bucket
     uint16_t b0[GP_DIGITS];     // first bucket of every unit within the bin (bins of more than 1024 buckets)
 };
-constexpr uint32_t SP_CHUNK = 4;  // tiles of the second pass a block takes at a time
+constexpr uint32_t SP_CHUNK = 4;  // most tiles of the second pass a block takes at a time
 static_assert(2 * (sizeof(UnitSmem) + 1024) <= 228 * 1024 && 2 * (sizeof(BinSmem) + 3 * 1024) <= 228 * 1024, "two split blocks per SM");
 
 __device__ __forceinline__ uint32_t &at_byte(uint32_t *p, uint32_t off) { return *reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(p) + off); }
@@ -587,7 +587,8 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_units(const uint64_t *_
     int cs = 0;  // buckets per cell: 2^cs, 0 for bins of at most 1024 buckets
     bool whole = false;
     for (uint32_t d = tid; d < GP_DIGITS; d += SP_THREADS) sm.hist[d] = 0;
-    auto tile_at = [&](uint32_t i) { return ((i / SP_CHUNK) * gridDim.x + blockIdx.x) * SP_CHUNK + i % SP_CHUNK; };
+    const uint32_t chunk = min(SP_CHUNK, max(1u, tiles / gridDim.x));  // (few tiles: one for each block)
+    auto tile_at = [&](uint32_t i) { return ((i / chunk) * gridDim.x + blockIdx.x) * chunk + i % chunk; };
     uint32_t kl[SP_ITEMS], kh[SP_ITEMS];
     auto load = [&](const uint4 &t) {
         const uint64_t *kp = kk + t.x + tid;
@@ -1048,7 +1049,8 @@ __global__ void __launch_bounds__(256) k_gp_quirk(const uint32_t *ctr, const uin
     }
 }
 
-constexpr uint32_t GE_SEG = 1024;  // grouped ids per warp and turn
+constexpr uint32_t GE_SEG = 1024;  // most grouped ids per warp and turn
+constexpr uint32_t GE_BLOCKS = 8;   // blocks per SM
 
 // Bound by the random reads of the BAD flags and parents in L2.  It reads 4 bytes per joining tuple where the
 // sweep over sorted tuples read 13 per tuple: 6.7 ms against 21.0 at 20M x 150 bp, 2 scans.
@@ -1057,14 +1059,14 @@ constexpr uint32_t GE_SEG = 1024;  // grouped ids per warp and turn
 // of the stretch.  A stretch that starts inside a run looks back for one read of it, so long runs are shared by
 // many warps.
 __global__ void __launch_bounds__(256) k_gp_union(const uint32_t *ctr, const uint32_t *__restrict__ out, uint32_t *parent,
-                                                  const uint8_t *__restrict__ filtered, uint32_t *err, uint32_t uf_cap)
+                                                  const uint8_t *__restrict__ filtered, uint32_t per, uint32_t *err, uint32_t uf_cap)
 {
     const uint32_t m = ctr[GC_OUT];
     const int lane = threadIdx.x & 31;
     const uint32_t le = (lane == 31) ? FULLG : ((2u << lane) - 1);
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5, nseg = (m + GE_SEG - 1) / GE_SEG;
+    const uint32_t nw = (gridDim.x * blockDim.x) >> 5, nseg = (m + per - 1) / per;
     for (uint32_t sgm = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; sgm < nseg; sgm += nw) {
-        const uint32_t p0 = sgm * GE_SEG, p1 = min(m, p0 + GE_SEG);
+        const uint32_t p0 = sgm * per, p1 = min(m, p0 + per);
         bool has = false;
         uint32_t anchor = 0;
         if (!(out[p0] >> 31)) {  // the run's reads before the stretch, a window at a time
@@ -1471,11 +1473,15 @@ int group_union(GroupScan &g, const uint32_t *out, uint32_t *parent, const uint8
     open.clear();
     (count_launch(), k_gp_quirk<<<std::min(2u * (unsigned)sm_count(), g.hctr[GC_UNITS] / 16 + 1), 256, 0, st>>>(g.ctr, g.qlist, out, filtered, nseg,
                                                                                                             g.quirk));
-    const unsigned blocks = std::min<unsigned>(8u * (unsigned)sm_count(), blocks_of(g.n, (int)GE_SEG * 8));
+    // a stretch for every warp there is room for, of whole windows (600 reads: stretches of 1024 ids on a few
+    // warps took 23 us, of 32 take 6)
+    const uint64_t warps = 8ull * GE_BLOCKS * (uint64_t)sm_count();
+    const uint32_t per = std::min(GE_SEG, ((uint32_t)(g.n / warps) + 63u) / 32u * 32u);
+    const unsigned blocks = std::min<unsigned>(GE_BLOCKS * (unsigned)sm_count(), blocks_of(g.n, (int)per * 8));
     uint32_t *err = arena.alloc<uint32_t>(1);
     if (!err) return set_error(MP_ENOMEM, "device memory");
     MP_CUDA(cudaMemsetAsync(err, 0, 4, st));
-    (count_launch(), k_gp_union<<<blocks, 256, 0, st>>>(g.ctr, out, parent, filtered, err, arena.lim.union_retries));
+    (count_launch(), k_gp_union<<<blocks, 256, 0, st>>>(g.ctr, out, parent, filtered, per, err, arena.lim.union_retries));
     compress_parents(parent, n_reads, st);
     const size_t words = GC_N + (size_t)nseg * QW;
     ReadBack<uint32_t> h(arena, words + 1);

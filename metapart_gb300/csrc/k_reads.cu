@@ -147,33 +147,6 @@ __device__ __forceinline__ uint32_t nl_in_word(uint32_t w)
     return ~(y | x | 0x7F7F7F7Fu);
 }
 
-// buf is 16-byte aligned; its first `skip` (< 16) bytes are not part of the parsed range, whose byte 0 is
-// buf[skip] (newline positions are written relative to it).
-__global__ void __launch_bounds__(NL_THREADS) k_nl_count(const uint8_t *buf, uint64_t n, uint32_t skip, uint32_t *seg_counts)
-{
-    const uint64_t s0 = (uint64_t)blockIdx.x * NL_SEG, s1 = min(n, s0 + NL_SEG);
-    uint32_t c = 0;
-    for (uint64_t p = s0 + (uint64_t)threadIdx.x * 16; p < s1; p += NL_THREADS * 16) {
-        if (p + 16 <= s1 && p >= skip) {
-            uint4 v = *reinterpret_cast<const uint4 *>(buf + p);
-            c += __popc(nl_in_word(v.x)) + __popc(nl_in_word(v.y)) + __popc(nl_in_word(v.z)) + __popc(nl_in_word(v.w));
-        } else {
-            for (uint64_t q = max(p, (uint64_t)skip); q < min(s1, p + 16); q++) c += buf[q] == '\n';
-        }
-    }
-    uint64_t tot;
-    uint64_t x = c;
-    for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xFFFFFFFFu, x, o);
-    __shared__ uint64_t ws[NL_THREADS / 32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        tot = 0;
-        for (int w = 0; w < NL_THREADS / 32; w++) tot += ws[w];
-        seg_counts[blockIdx.x] = (uint32_t)tot;
-    }
-}
-
 // Bit q: byte q of the sixteen at p is a newline of the parsed range.
 __device__ __forceinline__ uint32_t nl_mask16(const uint8_t *buf, uint64_t p, uint64_t end, uint32_t skip)
 {
@@ -189,6 +162,32 @@ __device__ __forceinline__ uint32_t nl_mask16(const uint8_t *buf, uint64_t p, ui
     for (uint32_t q = 0; q < 16; q++)
         if (p + q < end && p + q >= skip && buf[p + q] == '\n') m |= 1u << q;
     return m;
+}
+
+// buf is 16-byte aligned; its first `skip` (< 16) bytes are not part of the parsed range, whose byte 0 is
+// buf[skip] (newline positions are written relative to it).  mask (nullable): a bit per byte of the blocks, for k_nl_place.
+__global__ void __launch_bounds__(NL_THREADS) k_nl_count(const uint8_t *buf, uint64_t n, uint32_t skip, uint32_t *seg_counts,
+                                                         uint16_t *mask)
+{
+    const uint64_t s0 = (uint64_t)blockIdx.x * NL_SEG, s1 = min(n, s0 + NL_SEG);
+    uint32_t c = 0;
+#pragma unroll 4
+    for (uint64_t p = s0 + (uint64_t)threadIdx.x * 16; p < s0 + NL_SEG; p += NL_THREADS * 16) {
+        const uint32_t m = p < s1 ? nl_mask16(buf, p, s1, skip) : 0u;
+        if (mask) mask[p >> 4] = (uint16_t)m;
+        c += (uint32_t)__popc(m);
+    }
+    uint64_t tot;
+    uint64_t x = c;
+    for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xFFFFFFFFu, x, o);
+    __shared__ uint64_t ws[NL_THREADS / 32];
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        tot = 0;
+        for (int w = 0; w < NL_THREADS / 32; w++) tot += ws[w];
+        seg_counts[blockIdx.x] = (uint32_t)tot;
+    }
 }
 
 // A warp takes an eighth of the block's bytes and keeps its newlines as bits, so the block meets once, for the warps' counts.
@@ -231,6 +230,38 @@ __global__ void __launch_bounds__(NL_THREADS) k_nl_write(const uint8_t *buf, uin
         for (uint32_t b = m[i]; b; b &= b - 1) nl_pos[o++] = p0 + (uint64_t)i * 512 + (uint32_t)(__ffs((int)b) - 1) - skip;
         out += __shfl_sync(0xFFFFFFFFu, x, 31);
     }
+}
+
+// The same from the count's bits: a lane takes 256 bytes, so a warp's counts meet once.  6.2 GB: 0.33 ms where the bytes read
+// again took 2.29, and the bits cost the count 0.36.
+__global__ void __launch_bounds__(NL_THREADS) k_nl_place(const uint16_t *mask, uint32_t skip, const uint64_t *seg_off, uint64_t *nl_pos,
+                                                         unsigned long long *stat)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // k_records' results
+        stat[0] = ~0ull;
+        stat[1] = 0;
+    }
+    static_assert(NL_SEG == (uint64_t)NL_THREADS * 256, "256 bytes per thread");
+    __shared__ uint32_t ws[NL_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t p0 = (uint64_t)blockIdx.x * NL_SEG + (uint64_t)threadIdx.x * 256;
+    const ulonglong2 *mp = reinterpret_cast<const ulonglong2 *>(mask + (p0 >> 4));
+    const ulonglong2 a = mp[0], b = mp[1];
+    const unsigned long long w[4] = {a.x, a.y, b.x, b.y};
+    const uint32_t c = (uint32_t)(__popcll(w[0]) + __popcll(w[1]) + __popcll(w[2]) + __popcll(w[3]));
+    uint32_t x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) ws[warp] = x;
+    __syncthreads();
+    uint64_t o = seg_off[blockIdx.x] + x - c;
+    for (int v = 0; v < warp; v++) o += ws[v];
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        for (unsigned long long m = w[q]; m; m &= m - 1) nl_pos[o++] = p0 + (uint32_t)(64 * q + __ffsll((long long)m) - 1) - skip;
 }
 
 // Record table from the newline positions; flags quality/sequence length mismatches.
@@ -292,7 +323,15 @@ int parse_fastq_range(const uint8_t *d_base, uint64_t begin, uint64_t end, Parse
     size_t tb = scan_tmp_bytes(segs);
     void *tmp = arena.alloc<uint8_t>(tb);
     if (!seg_counts || !seg_off || !total || !tmp) return set_error(MP_ENOMEM, "device memory for the FASTQ parse");
-    (mp::count_launch(), k_nl_count<<<(unsigned)segs, NL_THREADS, 0, st>>>(d_buf, na, skip, seg_counts));
+    // the newlines as bits, where there is room for them beside what has to be held
+    uint16_t *mask = arena.alloc<uint16_t>(segs * (NL_SEG / 16));
+    auto without_mask = [&] {
+        const bool had = mask != nullptr;
+        if (had) arena.free_scratch(mask);
+        mask = nullptr;
+        return had;
+    };
+    (mp::count_launch(), k_nl_count<<<(unsigned)segs, NL_THREADS, 0, st>>>(d_buf, na, skip, seg_counts, mask));
     scan_u32_to_u64(seg_counts, seg_off, segs, total, tmp, tb, st);
     ReadBack<uint64_t> rb(arena, 4);
     MP_CUDA(cudaMemcpyAsync(&rb[0], total, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
@@ -300,15 +339,23 @@ int parse_fastq_range(const uint8_t *d_base, uint64_t begin, uint64_t end, Parse
     const uint64_t n_nl = rb[0];
     if (n_nl == 0 || n_nl % 4) return set_error(MP_EFMT, "FASTQ line count %llu is not a multiple of 4", (unsigned long long)n_nl);
     uint64_t *nl = arena.alloc<uint64_t>(n_nl);
+    if (!nl && without_mask()) nl = arena.alloc<uint64_t>(n_nl);
     if (!nl) return set_error(MP_ENOMEM, "device memory for newline positions");
     const uint64_t n_rec = n_nl / 4;
     pr->n_reads = n_rec;
     pr->rec_start = arena.alloc_persistent<uint64_t>(n_rec + 1);
     pr->seq_off = arena.alloc_persistent<uint64_t>(n_rec);
     pr->seq_len = arena.alloc_persistent<uint32_t>(n_rec);
+    if (!(pr->rec_start && pr->seq_off && pr->seq_len) && without_mask()) {
+        if (!pr->rec_start) pr->rec_start = arena.alloc_persistent<uint64_t>(n_rec + 1);
+        if (!pr->seq_off) pr->seq_off = arena.alloc_persistent<uint64_t>(n_rec);
+        if (!pr->seq_len) pr->seq_len = arena.alloc_persistent<uint32_t>(n_rec);
+    }
     unsigned long long *bad = arena.alloc<unsigned long long>(3);
+    if (!bad && without_mask()) bad = arena.alloc<unsigned long long>(3);
     if (!pr->rec_start || !pr->seq_off || !pr->seq_len || !bad) return set_error(MP_ENOMEM, "device memory for the record table");
-    (mp::count_launch(), k_nl_write<<<(unsigned)segs, NL_THREADS, 0, st>>>(d_buf, na, skip, seg_off, nl, bad));
+    if (mask) (mp::count_launch(), k_nl_place<<<(unsigned)segs, NL_THREADS, 0, st>>>(mask, skip, seg_off, nl, bad));
+    else (mp::count_launch(), k_nl_write<<<(unsigned)segs, NL_THREADS, 0, st>>>(d_buf, na, skip, seg_off, nl, bad));
     (mp::count_launch(), k_records<<<(unsigned)((n_rec + 255) / 256), 256, 0, st>>>(nl, n_rec, pr->rec_start, pr->seq_off, pr->seq_len, bad));
     MP_CUDA(cudaMemcpyAsync(&rb[1], bad, 3 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     MP_CUDA(cudaStreamSynchronize(st));

@@ -1,16 +1,16 @@
 """Benchmark of the GB300 read-partitioning path (one JSON line on rank 0).
 
 A step is one pass of the whole path over one read set: chunk index, GPU FASTQ parse, m-mer histogram,
-then per scan tuple enumeration, onesweep radix sort, branching-k-mer filter and union-find, the mate
+then the scans' tuples split into units, grouped by k-mer and filtered, and joined by union-find, the mate
 union, the 16 work partitions and the partition-FASTQ gather.
 
   value  -- bases/s with the FASTQ already in HBM (the step copies it into the job and runs every stage)
   e2e    -- the same through the C ABI from pinned host memory: FASTQ upload and partition-file download
             inside the timed region
-  roofline -- the dominant kernel, the shared-memory unit sort (k_segsort: one launch per block shape and
-            scan): algorithmic bytes (25 B per tuple read and written) over its CUDA-event time, against the
-            measured HBM copy bandwidth; it is bound by shared memory, not HBM
-  roofline_digit_pass -- the same for the bucket-digit radix passes (k_onesweep), the HBM-streaming kernel
+  roofline -- the split passes (k_split_reads, k_split_units), the largest share of the step: algorithmic bytes
+            (36 B per tuple: 12 written, 12 read and 12 written) over their CUDA-event time per step, against the
+            measured HBM copy bandwidth; they are bound on chip, not by HBM
+  roofline_group -- the same for the grouping and filter (k_group): 12 B per tuple read; bound by shared memory
   cpu_baseline -- the CPU oracle (the reference's algorithm restated in C/OpenMP, all host cores) on a
             bounded sample of the same read set; the GPU's partition files of that sample are compared with
             the oracle's ("parity")
@@ -40,8 +40,7 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 METRIC = "bases/sec partitioned (k=31) batched vs plain on 1 GB300; p50/p99 job latency"
-ROOFLINE_TRAFFIC_FILE = ROOT / "profiles" / "onesweep_traffic.json"
-UNIT_SORT_TRAFFIC_FILE = ROOT / "profiles" / "unit_sort_traffic.json"
+TRAFFIC_FILE = ROOT / "profiles" / "split_group_traffic.json"
 
 
 def parse_args():
@@ -141,7 +140,7 @@ def measured_peak():
     return 6800.0, "fallback"
 
 
-def traffic_per_tuple(path=ROOFLINE_TRAFFIC_FILE, key="dram_bytes_per_tuple_per_pass"):
+def traffic_per_tuple(key, path=TRAFFIC_FILE):
     """DRAM bytes per tuple of one launch from a committed ncu capture (null when absent)."""
     try:
         return float(json.loads(path.read_text())[key])
@@ -255,7 +254,7 @@ def main():
         device_step()
     # ---- device-resident timed region
     sort_bytes = sort_ms = 0.0
-    sort_passes = sort_tuples = 0
+    sort_tuples = 0
     stage = {}
     split = {}
     l0 = native.launch_count()
@@ -270,7 +269,6 @@ def main():
             s = job.sort_stats()
             sort_bytes += s["bytes"]
             sort_ms += s["pass_ms"]
-            sort_passes += s["passes"]
             sort_tuples += s["tuples"]
             for kk, v in job.stage_ms().items():
                 stage[kk] = stage.get(kk, 0.0) + v
@@ -332,19 +330,12 @@ def main():
     link = link_bandwidth(host_in, dev_in[:nbytes], out_host)
 
     peak, peak_kind = measured_peak()
-    achieved = (sort_bytes / 1e9) / (sort_ms / 1e3) if sort_ms > 0 else 0.0
-    per_launch_bytes = sort_bytes / max(sort_passes, 1)
-    elt = 13 if 2 * args.k + 8 > 64 else 12   # bytes of one tuple: key (8) + read id (4) [+ high k-mer byte]
-    tuples_per_launch = sort_bytes / (2 * elt) / max(sort_passes, 1)
-    tpt = traffic_per_tuple()
-    traffic = tpt * tuples_per_launch if tpt else None
-    # the unit sort: every tuple outside the oversized buckets, read (key, high byte, id) and written (key, id)
-    # once per scan; its time per scan covers both block shapes
-    unit_tuples = (sort_tuples - split.get("big_tuples", 0)) / args.steps / max(args.scans, 1)
-    unit_ms = split.get("unit_sort_ms", 0.0) / args.steps / max(args.scans, 1)
-    unit_bytes = unit_tuples * (elt + 12)
-    unit_achieved = (unit_bytes / 1e9) / (unit_ms / 1e3) if unit_ms > 0 else 0.0
-    utpt = traffic_per_tuple(UNIT_SORT_TRAFFIC_FILE, "dram_bytes_per_tuple")
+    split_ms, tuples = sort_ms / args.steps, sort_tuples / args.steps
+    split_bytes = sort_bytes / args.steps
+    achieved = (split_bytes / 1e9) / (split_ms / 1e3) if split_ms > 0 else 0.0
+    group_ms, group_bytes = stage.get("filter", 0.0) / args.steps, 12 * tuples
+    group_achieved = (group_bytes / 1e9) / (group_ms / 1e3) if group_ms > 0 else 0.0
+    split_tpt, group_tpt = traffic_per_tuple("split_dram_bytes_per_tuple"), traffic_per_tuple("group_dram_bytes_per_tuple")
     line = {
         "metric": METRIC,
         "value": round(value, 1),
@@ -368,18 +359,18 @@ def main():
                 "scan_pieces": e2e_pieces,
                 "phase_ms": {kk: round(v / args.steps, 2) for kk, v in phase.items()},
                 "link_gbs": link, "host": host_placement(dev), "clocks": clk_e2e.summary()},
-        "roofline": {"bound": "hbm", "achieved": round(unit_achieved, 1), "peak": peak, "unit": "GB/s",
-                     "frac": round(unit_achieved / peak, 4), "peak_kind": peak_kind,
-                     "kernel": "k_segsort (shared-memory unit sort, per scan)",
-                     "limiter": "shared memory: the dependent gathers and scatters of its digit passes",
-                     "bytes_per_launch": int(unit_bytes), "launch_ms": round(unit_ms, 4),
-                     "traffic": (round(utpt * unit_tuples) if utpt else None)},
-        "roofline_digit_pass": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                                "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
-                                "kernel": "k_onesweep (radix digit pass)",
-                                "bytes_per_launch": int(per_launch_bytes),
-                                "launch_ms": round(sort_ms / max(sort_passes, 1), 4),
-                                "traffic": (round(traffic) if traffic else None)},
+        "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
+                     "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
+                     "kernel": "k_split_reads + k_split_units (split passes, per step)",
+                     "limiter": "the instructions of the k-mers and the shared-memory reorder",
+                     "bytes_per_step": int(split_bytes), "ms_per_step": round(split_ms, 4),
+                     "traffic": (round(split_tpt * tuples) if split_tpt else None)},
+        "roofline_group": {"bound": "hbm", "achieved": round(group_achieved, 1), "peak": peak, "unit": "GB/s",
+                           "frac": round(group_achieved / peak, 4), "peak_kind": peak_kind,
+                           "kernel": "k_group (grouping and filter, per step)",
+                           "limiter": "shared memory: the hash table's random accesses",
+                           "bytes_per_step": int(group_bytes), "ms_per_step": round(group_ms, 4),
+                           "traffic": (round(group_tpt * tuples) if group_tpt else None)},
         "read_stores": stores,
         "gpu_launches": int(launches),
         "stage_ms": {kk: round(v / args.steps, 3) for kk, v in stage.items()},

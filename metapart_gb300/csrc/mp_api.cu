@@ -1013,10 +1013,12 @@ static int merge_scans(mp_job *j, int k, int T, const std::vector<uint64_t> &sca
 {
     const int S = (int)scanR.size() - 1;
     if (S > GROUP_MAX_MERGED || (j->pr.max_len > (uint32_t)k && j->pr.max_len - (uint32_t)k >= 300u)) return 0;
+    uint64_t most = 0;
     for (int s = 0; s < S; s++) {
         if (scanR[s] >= scanR[s + 1] || scanR[s + 1] > NB || hist[scanR[s]] > hist[scanR[s + 1]]) return 0;
         const uint64_t n = hist[scanR[s + 1]] - hist[scanR[s]];
         if (!scan_is_grouped(j, k, n)) return 0;
+        most = std::max(most, n);
         std::vector<uint64_t> rb;
         if (range_bounds(hist, thrR.data() + (size_t)s * T, T, scanR[s], scanR[s + 1], rb)) return 0;
         tuple0.push_back(hist[scanR[s]] - hist[scanR[0]]);
@@ -1026,7 +1028,10 @@ static int merge_scans(mp_job *j, int k, int T, const std::vector<uint64_t> &sca
     m.k1 = j->arena.alloc_persistent<uint64_t>(m.n + 1);
     m.id1 = j->arena.alloc_persistent<uint32_t>(m.n + 1);
     m.cur = j->arena.alloc_persistent<uint32_t>(m.digits);
-    if (!m.k1 || !m.id1 || !m.cur) {
+    // the largest scan's second buffers and plan have to fit beside them (piece_cap may be the caller's own)
+    uint8_t *room = m.k1 && m.id1 ? j->arena.alloc_persistent<uint8_t>(13 * most + (64u << 20)) : nullptr;
+    if (room) j->arena.free_persistent(room);
+    if (!m.k1 || !m.id1 || !m.cur || !room) {
         j->arena.free_persistent(m.k1);
         j->arena.free_persistent(m.id1);
         j->arena.free_persistent(m.cur);

@@ -295,12 +295,11 @@ __device__ __forceinline__ uint32_t &at_byte(uint32_t *p, uint32_t off) { return
 // Unstable, so there are no ballots and no look-back: ranks by shared-memory atomics, places by one global atomic per
 // digit and tile (the order of a digit's tuples is free; its latency passes while the tile is reordered), a
 // shared-memory reorder so that a digit's tuples are stored side by side.  rd: digit times 4 (bits 0-15) and the tuple's rank
-// in it (16-31), or ~0 for none, as the caller's atomics on sm.hist gave them.  Returns the tile's tuples, 0 when one
-// would land past the n tuples (the histogram is not the tuples': the group kernel reports it).  EXTRA: with the SP_EXTRA
-// digits above GP_DIGITS.
+// in it (16-31), or ~0 for none, as the caller's atomics on sm.hist gave them.  Returns the tile's tuples.  EXTRA: with
+// the SP_EXTRA digits above GP_DIGITS.
 template <bool EXTRA, class LoadId>
 __device__ __forceinline__ uint32_t split_order(SplitSmem &sm, const uint32_t (&kl)[SP_ITEMS], const uint32_t (&kh)[SP_ITEMS],
-                                                const uint32_t (&rd)[SP_ITEMS], uint32_t *cur, uint32_t nd, LoadId load_id, uint32_t n)
+                                                const uint32_t (&rd)[SP_ITEMS], uint32_t *cur, uint32_t nd, LoadId load_id)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t id[SP_ITEMS];
@@ -335,13 +334,11 @@ __device__ __forceinline__ uint32_t split_order(SplitSmem &sm, const uint32_t (&
         nv += v;
     }
     *reinterpret_cast<uint2 *>(&sm.hist[2 * tid]) = make_uint2(before, before + c.x);
-    bool past = false;
     if constexpr (EXTRA) {
         if (tid < 2) {
-            const uint32_t at = nv + (tid ? ex : 0u), n0 = tid ? ey : ex;
+            const uint32_t at = nv + (tid ? ex : 0u);
             sm.hist[GP_DIGITS + tid] = at;
             sm.delta[GP_DIGITS + tid] = ge - at;
-            past = n0 && (uint64_t)ge + n0 > n;
         }
         nv += ex + ey;
     }
@@ -356,17 +353,23 @@ __device__ __forceinline__ uint32_t split_order(SplitSmem &sm, const uint32_t (&
         }
     }
     *reinterpret_cast<uint2 *>(&sm.delta[2 * tid]) = make_uint2(g0 - before, g1 - before - c.x);
-    return __syncthreads_or(past || (c.x && (uint64_t)g0 + c.x > n) || (c.y && (uint64_t)g1 + c.y > n)) ? 0u : nv;
+    __syncthreads();
+    return nv;
 }
 
+// A digit with more tuples than the histogram gave it (which is then not the tuples': k_split_units and k_group tell) runs on
+// into the next one's places, and past all n of them the tuples are left out: every place that a cursor passed holds a
+// tuple, so what is read of it later is in range.
 template <bool EXTRA>
-__device__ __forceinline__ void split_store(SplitSmem &sm, uint32_t nv, uint64_t *out_k, uint32_t *out_id)
+__device__ __forceinline__ void split_store(SplitSmem &sm, uint32_t nv, uint64_t *out_k, uint32_t *out_id, uint32_t n)
 {
 #pragma unroll 4
     for (uint32_t p = threadIdx.x; p < nv; p += SP_THREADS) {
         const uint32_t o = p + at_byte(sm.delta, sm.dig[p]);
-        out_k[o] = sm.key[p];
-        out_id[o] = sm.id[p];
+        if (o < n) {
+            out_k[o] = sm.key[p];
+            out_id[o] = sm.id[p];
+        }
     }
     *reinterpret_cast<uint2 *>(&sm.hist[2 * threadIdx.x]) = make_uint2(0, 0);
     if (EXTRA && threadIdx.x < SP_EXTRA) sm.hist[GP_DIGITS + threadIdx.x] = 0;
@@ -516,8 +519,8 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_reads(BinCtx c)
             // the reference counts a read's k-mers of one scan in 8 bits (enumerateKmers.c:152)
             if (c.check_many && got && atomicAdd(&many[rr], got) + got > 255u) atomicOr(c.err, 4u);
         }
-        const uint32_t nv = split_order<MERGED>(sm, kl, kh, rd, c.bcur + d0, nd, [&](int) { return id; }, c.n);
-        split_store<MERGED>(sm, nv, c.out_k, c.out_id);
+        const uint32_t nv = split_order<MERGED>(sm, kl, kh, rd, c.bcur + d0, nd, [&](int) { return id; });
+        split_store<MERGED>(sm, nv, c.out_k, c.out_id, c.n);
         // the next tile's reads while others store (its bytes fetched before the stores instead cost registers that spill: 37.5
         // against 35.7 ms at 20M x 150 bp, 2 scans)
         const uint32_t next = tile + gridDim.x;
@@ -557,8 +560,8 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_tuples(BinCtx c)
         }
         const uint32_t got = split_order<false>(
             sm, kl, kh, rd, c.bcur + d0, nd,
-            [&](int j) { const uint32_t e = j * SP_THREADS + tid; return e < nv ? c.id[base + e] : 0u; }, c.n);
-        split_store<false>(sm, got, c.out_k, c.out_id);
+            [&](int j) { const uint32_t e = j * SP_THREADS + tid; return e < nv ? c.id[base + e] : 0u; });
+        split_store<false>(sm, got, c.out_k, c.out_id, c.n);
     }
 }
 
@@ -567,7 +570,7 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_tuples(BinCtx c)
 // evicted their half-filled lines, and 2.39 G tuples moved 102 GB through DRAM where they take 57 (26.5 ms; 15.1 now, 3.8
 // TB/s, at 20M x 150 bp, 2 scans).
 __global__ void __launch_bounds__(SP_THREADS, 2) k_split_units(const uint64_t *__restrict__ kk, const uint32_t *__restrict__ id,
-                                                               uint32_t n, int bsh, uint32_t seg_lo, const uint32_t *__restrict__ ctr,
+                                                               uint32_t n, int bsh, uint32_t seg_lo, uint32_t *ctr, uint32_t nbins,
                                                                const uint32_t *__restrict__ bstart,
                                                                const uint32_t *__restrict__ bfirst,
                                                                const uint32_t *__restrict__ bu0,
@@ -587,6 +590,9 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_units(const uint64_t *_
     int cs = 0;  // buckets per cell: 2^cs, 0 for bins of at most 1024 buckets
     bool whole = false;
     for (uint32_t d = tid; d < GP_DIGITS; d += SP_THREADS) sm.hist[d] = 0;
+    // every bin, those without a tuple in the histogram too, holds as many as that says, or the histogram is not the tuples'
+    for (uint32_t x = blockIdx.x * SP_THREADS + tid; x < nbins; x += gridDim.x * SP_THREADS)
+        if (bcur[x] - tuple0 != bstart[x + 1]) atomicOr(&ctr[GC_ERR], 2u);
     const uint32_t chunk = min(SP_CHUNK, max(1u, tiles / gridDim.x));  // (few tiles: one for each block)
     auto tile_at = [&](uint32_t i) { return ((i / chunk) * gridDim.x + blockIdx.x) * chunk + i % chunk; };
     uint32_t kl[SP_ITEMS], kh[SP_ITEMS];
@@ -609,7 +615,7 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_units(const uint64_t *_
         __syncthreads();  // the tile before is stored
         if (bin != have) {
             have = bin;
-            whole = bcur[bin] - tuple0 == bstart[bin + 1];  // else the histogram is not the tuples' (the bin's units stay short: k_group)
+            whole = bcur[bin] - tuple0 == bstart[bin + 1];  // else some of its places may hold nothing
             d0 = bu0[bin];
             nd = min(bu0[bin + 1] - d0, GP_DIGITS);
             const uint32_t s = bin_sh[bin], b0 = bfirst[bin];
@@ -628,7 +634,7 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_units(const uint64_t *_
 #pragma unroll
             for (int j = 0; j < SP_ITEMS; j++) {
                 const uint32_t b = bits >= 32 ? kh[j] >> (bits - 32) : __funnelshift_r(kl[j], kh[j], bits);
-                uint32_t d4 = sm.cell[b >> cs];
+                uint32_t d4 = sm.cell[(b >> cs) & (GP_DIGITS - 1)];  // (a tuple of another bin, where that one runs over)
                 if (cs)
                     while (d4 / 4 + 1 < nd && sm.b0[d4 / 4 + 1] <= b) d4 += 4;
                 rd[j] = j * SP_THREADS + tid < nv ? d4 | (atomicAdd(&at_byte(sm.hist, d4), 1u) << 16) : ~0u;
@@ -643,14 +649,13 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_units(const uint64_t *_
                         v = p == BAD ? v : p;
                     }
                     return v;
-                },
-                n);
+                });
         }
         if (tile_at(i + 1) < tiles) {  // the next tile's keys on their way while this one's tuples are stored
             now = tile_of[tile_at(i + 1)];
             load(now);
         }
-        split_store<false>(sm, got, out_k, out_id);
+        split_store<false>(sm, got, out_k, out_id, n);
     }
 }
 
@@ -1383,7 +1388,7 @@ void group_take(GroupScan &g, const MergedScans &m, int s, const uint32_t *label
 int group_units(GroupScan &g, const uint64_t *k1, const uint32_t *id1, uint64_t *k2, uint32_t *id2, cudaStream_t st)
 {
     (count_launch(), k_split_units<<<std::min(g.max_tiles, 2u * (unsigned)sm_count()), SP_THREADS, sizeof(UnitSmem), st>>>(
-        k1, id1, (uint32_t)g.n, 2 * (g.k - 10), g.seg_lo, g.ctr, g.bstart, g.bfirst, g.bu0, g.bcur, g.bin_sh, g.ub0,
+        k1, id1, (uint32_t)g.n, 2 * (g.k - 10), g.seg_lo, g.ctr, g.bins, g.bstart, g.bfirst, g.bu0, g.bcur, g.bin_sh, g.ub0,
         g.ucur, g.unit_of, (uint32_t)(g.hi - g.lo), g.tiles, g.tuple0, g.late_label, k2, id2));
     MP_CUDA(cudaGetLastError());
     return 0;

@@ -940,6 +940,7 @@ static int scan_first_read(mp_job *j, int k, int min3, uint64_t lo, uint64_t hi,
     uint64_t n = 0;
     MP_CUDA(cudaMemcpyAsync(&n, ntot, 8, cudaMemcpyDeviceToHost, j->st));
     MP_CUDA(cudaStreamSynchronize(j->st));
+    if (n != hist[b1] - hist[b0]) return set_error(MP_EFMT, "the histogram does not match the scan's tuples");
     const bool has_hi = 2 * k + 8 > 64;
     uint64_t *tl = j->arena.alloc<uint64_t>(n + 1);
     uint8_t *th = has_hi ? j->arena.alloc<uint8_t>(n + 1) : nullptr;

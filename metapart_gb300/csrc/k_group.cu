@@ -955,7 +955,7 @@ struct BigUnit {
 };
 
 __global__ void k_big_units(const uint32_t *big, uint32_t nb, const uint32_t *ustart, const uint32_t *ub0, uint32_t nunits,
-                            const uint32_t *fill, uint32_t *err, uint32_t *out)
+                            const uint32_t *fill, uint32_t *out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nb) return;
@@ -964,10 +964,7 @@ __global__ void k_big_units(const uint32_t *big, uint32_t nb, const uint32_t *us
     out[4 * i + 1] = ustart[u];
     out[4 * i + 2] = ustart[u + 1] - ustart[u];
     out[4 * i + 3] = (u + 1 == nunits || (ub0[u + 1] >> 31)) ? 1u : 0u;  // ends a thread range
-    if (fill[u] != ustart[u + 1]) {  // the histogram is not the tuples'
-        atomicOr(err, 2u);
-        out[4 * i + 2] = 0;
-    }
+    if (fill[u] != ustart[u + 1]) out[4 * i + 2] = 0;  // the histogram is not the tuples': the caller stops here
 }
 
 // Gathered keys: unit index << (2 (k - 10) + 8) | low k-mer bits << 8 | adjacency codes.
@@ -1420,11 +1417,12 @@ int group_filter(GroupScan &g, const uint64_t *kk, const uint32_t *ids, uint32_t
         BigUnit *d_b = arena.alloc<BigUnit>(nb);
         uint32_t *d_base = arena.alloc<uint32_t>(1);
         if (!d_l || !d_b || !d_base) return set_error(MP_ENOMEM, "device memory for oversized buckets");
-        (count_launch(), k_big_units<<<blocks_of(nb, 128), 128, 0, st>>>(g.big, nb, g.ustart, g.ub0, g.hctr[GC_UNITS], fill,
-                                                                        g.ctr + GC_ERR, d_l));
+        (count_launch(), k_big_units<<<blocks_of(nb, 128), 128, 0, st>>>(g.big, nb, g.ustart, g.ub0, g.hctr[GC_UNITS], fill, d_l));
         std::vector<uint32_t> hl(4 * (size_t)nb);
         MP_CUDA(cudaMemcpyAsync(hl.data(), d_l, hl.size() * 4, cudaMemcpyDeviceToHost, st));
         MP_CUDA(cudaStreamSynchronize(st));
+        for (size_t i = 0; i < nb; i++)
+            if (hl[4 * i + 2] == 0) return set_error(MP_EFMT, "the histogram does not match the scan's tuples");
         const size_t per_batch = lowbits >= 44 ? ((size_t)1 << (64 - lowbits)) : ((size_t)1 << 20);
         std::vector<BigUnit> hb(nb);
         uint64_t most = 0;

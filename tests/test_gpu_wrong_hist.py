@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from metapart_gb300 import native, synth
+from test_gpu_batch import _poly_c
 from test_gpu_errors import EFMT, code
 
 pytestmark = pytest.mark.gpu
@@ -102,3 +103,29 @@ def test_histogram_of_another_k(ctx):
                 with pytest.raises(native.MetapartError) as e:
                     job.partition(k, scans, 4, st, cnt.chunk_first_read, cnt.hist)
                 assert code(e.value) == EFMT
+
+
+@pytest.mark.parametrize("threads", [1, 2])
+@pytest.mark.parametrize("to", [0, 5, -300_000], ids=["more", "after", "before"])
+def test_bucket_above_a_block(ctx, to, threads):
+    """One bucket of 210,000 tuples, the scan's last unit: it takes the device-wide sort, which has to see the mismatch."""
+    data = _poly_c(3000)
+    fno, ofs = native.fastq_index(4, [data])
+    st = native.chunk_starts_of(fno, ofs, [len(data)])
+    with native.Job(ctx) as job:
+        job.load(data)
+        cnt = job.count(31, st)
+        job.partition(31, 1, threads, st, cnt.chunk_first_read, cnt.hist)
+        want = job.labels()
+        c = np.diff(cnt.hist.astype(np.int64))
+        b = int(np.argmax(c))
+        assert c[b] > 12_288 and b > 300_000
+        c[b + to] += 1
+        if to:
+            c[b] -= 1
+        bad = np.r_[0, np.cumsum(c)].astype(np.uint64)
+        with pytest.raises(native.MetapartError) as e:
+            job.partition(31, 1, threads, st, cnt.chunk_first_read, bad)
+        assert code(e.value) == EFMT
+        job.partition(31, 1, threads, st, cnt.chunk_first_read, cnt.hist)
+        assert np.array_equal(job.labels(), want)

@@ -152,8 +152,9 @@ __device__ __forceinline__ uint64_t block_scan_excl(uint64_t v, uint64_t *total,
     return before + x - v;
 }
 
-// Units starting in each block of GP_COUNT_BLOCK buckets.
-__global__ void __launch_bounds__(GP_COUNT_BLOCK) k_gp_count(PlanCtx c, uint64_t *blk)
+// Units starting in each block of GP_COUNT_BLOCK buckets.  The plan's arrays have room for the units of a prefix that never
+// falls; the caller's may come from a file, so one that does is told here (GC_ERR), and nothing is planned.
+__global__ void __launch_bounds__(GP_COUNT_BLOCK) k_gp_count(PlanCtx c, uint64_t *blk, uint32_t *ctr)
 {
     __shared__ PrevSmem ps;
     const uint64_t b0 = c.lo + (uint64_t)blockIdx.x * GP_COUNT_BLOCK, b = b0 + threadIdx.x;
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(GP_COUNT_BLOCK) k_gp_count(PlanCtx c, uint64_t
     const bool f = s != e && (plan_flags(c, b, s - h0, e - h0, p) & 1u);
     const int n = __syncthreads_count(f);
     if (threadIdx.x == 0) blk[blockIdx.x] = (uint64_t)n;
+    if (e < s) atomicOr(&ctr[GC_ERR], 2u);
 }
 
 // Exclusive scan of the blocks' counts by one block; the sentinels past the last unit and bin.
@@ -174,6 +176,7 @@ __global__ void __launch_bounds__(1024) k_gp_scan(uint64_t *blk, uint32_t nblk, 
 {
     __shared__ uint64_t ws[32];
     uint64_t carry = 0;
+    if (ctr[GC_ERR]) nblk = 0;  // no units
     for (uint32_t i0 = 0; i0 < nblk; i0 += 1024) {
         const uint32_t i = i0 + threadIdx.x;
         uint64_t tot;
@@ -200,6 +203,7 @@ __global__ void __launch_bounds__(GP_COUNT_BLOCK) k_gp_write(PlanCtx c, const ui
     __shared__ uint32_t ws[GP_COUNT_BLOCK / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ PrevSmem ps;
+    if (ctr[GC_ERR]) return;  // (set by k_gp_count alone until here)
     const uint64_t b0 = c.lo + (uint64_t)blockIdx.x * GP_COUNT_BLOCK, b = b0 + threadIdx.x;
     uint64_t s = 0, e = 0;
     if (b < c.hi) {
@@ -250,6 +254,7 @@ __global__ void __launch_bounds__(1024) k_gp_tiles(const uint32_t *bstart, uint3
     __shared__ uint64_t ws[32];
     __shared__ uint32_t at[1024], sb[1025];
     uint32_t carry = 0;
+    if (ctr[GC_ERR]) nb = 0;  // no tiles
     for (uint32_t i0 = 0; i0 < nb; i0 += 1024) {
         const uint32_t i = i0 + threadIdx.x, s = bstart[min(i, nb)], e = bstart[min(i + 1, nb)];
         uint64_t tot;
@@ -1205,7 +1210,7 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
     MP_CUDA(cudaMemcpyAsync(g.seg_bin0, h.data(), h.size() * 4, cudaMemcpyHostToDevice, st));
     const PlanCtx c{g.d_hist, g.lo, g.hi, brk, g.seg_sh, g.seg_bin0, g.seg_lo};
     (count_launch(), k_gp_marks<<<blocks_of(nbounds, 4), 128, 0, st>>>(g.d_hist, g.lo, g.hi, d_bounds, (int)nbounds, brk));
-    (count_launch(), k_gp_count<<<nblk, GP_COUNT_BLOCK, 0, st>>>(c, blk));
+    (count_launch(), k_gp_count<<<nblk, GP_COUNT_BLOCK, 0, st>>>(c, blk, g.ctr));
     (count_launch(), k_gp_scan<<<1, 1024, 0, st>>>(blk, nblk, (uint32_t)g.n, g.bins, g.ctr, g.ustart, g.bstart, g.bu0));
     (count_launch(), k_gp_write<<<nblk, GP_COUNT_BLOCK, 0, st>>>(c, blk, g.ctr, g.ustart, g.ub0, g.ucur, g.bstart, g.bu0,
                                                                   g.merged ? nullptr : g.bcur, g.bin_sh, g.bfirst, g.unit_of, g.mid, g.big));

@@ -11,6 +11,7 @@ from test_gpu_errors import EFMT, code
 pytestmark = pytest.mark.gpu
 
 NB = 1 << 20
+EUNSUP = -5
 
 
 @pytest.fixture(scope="module")
@@ -128,4 +129,39 @@ def test_bucket_above_a_block(ctx, to, threads):
             job.partition(31, 1, threads, st, cnt.chunk_first_read, bad)
         assert code(e.value) == EFMT
         job.partition(31, 1, threads, st, cnt.chunk_first_read, cnt.hist)
+        assert np.array_equal(job.labels(), want)
+
+
+def _dip(h):  # one value below the one before
+    b = int(np.searchsorted(h, h[-1] // 2)) + 50
+    h[b] = h[b - 1] - 1
+
+
+def _saw(h):  # every second one: a unit at most buckets, where the right prefix has a hundredth of them
+    h[2001:900_001:2] += np.uint64(50_000)
+
+
+def _past(h):  # a bucket that seems to hold a million tuples
+    h[300_000] += np.uint64(1 << 20)
+
+
+@pytest.mark.parametrize("fall", [_dip, _saw, _past], ids=["dip", "saw", "past"])
+@pytest.mark.parametrize("n,k,scans,threads", [(600, 27, 1, 1), (60_000, 31, 1, 1), (60_000, 31, 1, 4), (60_000, 31, 2, 4)],
+                         ids=["600", "60000", "60000-t4", "60000-s2"])
+def test_falling_prefix(ctx, n, k, scans, threads, fall):
+    """A prefix that somewhere falls.  (The planner may refuse the ranges that it finds in it.)"""
+    data = synth.fastq_bytes(synth.workload("plain_large", n, seed=23))
+    fno, ofs = native.fastq_index(4, [data])
+    st = native.chunk_starts_of(fno, ofs, [len(data)])
+    with native.Job(ctx) as job:
+        job.load(data)
+        cnt = job.count(k, st)
+        job.partition(k, scans, threads, st, cnt.chunk_first_read, cnt.hist)
+        want = job.labels()
+        bad = cnt.hist.copy()
+        fall(bad)
+        with pytest.raises(native.MetapartError) as e:
+            job.partition(k, scans, threads, st, cnt.chunk_first_read, bad)
+        assert code(e.value) in (EFMT, EUNSUP)
+        job.partition(k, scans, threads, st, cnt.chunk_first_read, cnt.hist)
         assert np.array_equal(job.labels(), want)

@@ -1132,6 +1132,35 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
     j->hooked_bad = ~0u;
     const uint64_t piece_cap = p->min3 ? ~0ull : scan_piece_cap(j);  // the 3-minimizer choice depends on the range
     MergedScans merged;
+    struct Hold {  // what the scans share goes back on every return
+        DeviceArena &arena;
+        MergedScans &m;
+        uint32_t *&cnt_all, *&d_b;
+        uint64_t *&d_hist;
+        void drop_merged()
+        {
+            arena.free_persistent(m.k1);
+            arena.free_persistent(m.id1);
+            arena.free_persistent(m.cur);
+            m.k1 = nullptr;
+            m.id1 = nullptr;
+            m.cur = nullptr;
+        }
+        void drop()
+        {
+            drop_merged();
+            arena.free_persistent(cnt_all);
+            arena.free_persistent(d_b);
+            arena.free_persistent(d_hist);
+            cnt_all = d_b = nullptr;
+            d_hist = nullptr;
+        }
+        ~Hold()
+        {
+            drop();
+            arena.release_scratch();
+        }
+    } hold{j->arena, merged, cnt_all, d_b, d_hist};
     std::vector<uint64_t> tuple0;
     if (S > 1 && !p->min3 && (rc = merge_scans(j, k, T, scanR, thrR, hist, d_hist, piece_cap, merged, tuple0))) return rc;
     for (int s = 0; s < S; s++) {
@@ -1301,12 +1330,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         snprintf(name, sizeof name, "stats%d_parent.bin", s);
         if ((rc = dump_state(j, name, nullptr))) return rc;
     }
-    j->arena.free_persistent(merged.k1);
-    j->arena.free_persistent(merged.id1);
-    j->arena.free_persistent(merged.cur);
-    j->arena.free_persistent(cnt_all);
-    j->arena.free_persistent(d_b);
-    j->arena.free_persistent(d_hist);
+    hold.drop();
     j->kc_pieces = 0;
     {
         StageTimer tm(j->clk, j->st, 6);

@@ -10,7 +10,6 @@ from test_gpu_errors import EFMT, code
 
 pytestmark = pytest.mark.gpu
 
-NB = 1 << 20
 EUNSUP = -5
 
 
@@ -41,8 +40,9 @@ def _near(c):  # two units on
     _moved(c, p[len(p) // 3], np.searchsorted(np.cumsum(c), c[:p[len(p) // 3]].sum() + 13_000))
 
 
-def _emptied(c):  # tuples arrive where the histogram has none in a whole bin
-    lo, hi = (512 << 10, 513 << 10) if c.sum() > 2_000_000 else (NB // 2, NB)
+def _emptied(c):  # tuples arrive where the histogram has none (many reads: in a whole bin)
+    p = np.flatnonzero(c)
+    lo, hi = (512 << 10, 513 << 10) if c.sum() > 2_000_000 else (p[4 * len(p) // 10], p[6 * len(p) // 10])
     n = c[lo:hi].sum()
     c[lo:hi] = 0
     c[np.flatnonzero(c)[0]] += n
@@ -52,8 +52,9 @@ def _more(c):
     c[np.flatnonzero(c)[-1]] += 7
 
 
-def _less(c):
-    c[np.flatnonzero(c)[-1]] -= 1
+def _less(c):  # (not the last bucket's, which the scans then end before)
+    p = np.flatnonzero(c)
+    c[p[len(p) // 2]] -= 1
 
 
 def _halved(c):

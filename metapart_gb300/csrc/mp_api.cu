@@ -684,14 +684,9 @@ static void add_sort_stats(mp_job *j, const SortStats &ss, uint64_t n)
     for (int q = 0; q < 7; q++) j->pass_cycles_total[q] += ss.pass_cycles[q];
 }
 
-// Most tuples one scan may hold in HBM at once: MP_SCAN_PIECE_TUPLES, else the job's setting, else what
-// the context's budget (or the device, counting the pool's cached memory) has left at ~32 B per tuple
-// (two tuple buffers of 13 B, the sort's status and plans, the filter's marks).
-static uint64_t scan_piece_cap(mp_job *j)
+// Bytes that the context's budget (or the device, counting the pool's cached memory) has left.
+static uint64_t device_room(mp_job *j)
 {
-    const char *e = getenv("MP_SCAN_PIECE_TUPLES");
-    if (e && *e) return std::max<uint64_t>(1, strtoull(e, nullptr, 10));
-    if (j->piece_tuples) return j->piece_tuples;
     size_t fr = 0, tot = 0;
     uint64_t avail = cudaMemGetInfo(&fr, &tot) == cudaSuccess ? fr : 0;
     cudaMemPool_t pool;
@@ -708,7 +703,17 @@ static uint64_t scan_piece_cap(mp_job *j)
         const uint64_t u = j->arena.budget_used->load();
         avail = std::min<uint64_t>(avail, u < j->arena.budget_limit ? j->arena.budget_limit - u : 0);
     }
-    return std::max<uint64_t>(1, avail / 32);
+    return avail;
+}
+
+// Most tuples one scan may hold in HBM at once: MP_SCAN_PIECE_TUPLES, else the job's setting, else the bytes left at ~32 B
+// per tuple (two tuple buffers of 13 B, the sort's status and plans, the filter's marks).
+static uint64_t scan_piece_cap(const mp_job *j, uint64_t room)
+{
+    const char *e = getenv("MP_SCAN_PIECE_TUPLES");
+    if (e && *e) return std::max<uint64_t>(1, strtoull(e, nullptr, 10));
+    if (j->piece_tuples) return j->piece_tuples;
+    return std::max<uint64_t>(1, room / 32);
 }
 
 // Bucket-range pieces of the scan [lo, hi): consecutive buckets while their tuples stay within cap (a bucket
@@ -1006,10 +1011,11 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
 }
 
 // The first split pass of all scans at once (MergedScans), where every scan is to be grouped and one scan of all the tuples
-// would not have to go in pieces (its two buffers take more than the one of all tuples and a second one of a scan's).  Else
-// m.k1 stays null and every scan makes its own.
+// would not have to go in pieces, and where the bytes left (room) hold, beside the split tuples of all, what the largest scan
+// takes at most: its second buffers (12 a tuple), the two buffers of oversized buckets (24), the plan.  Else m.k1 stays null
+// and every scan makes its own.
 static int merge_scans(mp_job *j, int k, int T, const std::vector<uint64_t> &scanR, const std::vector<uint64_t> &thrR,
-                       const uint64_t *hist, const uint64_t *d_hist, uint64_t piece_cap, MergedScans &m,
+                       const uint64_t *hist, const uint64_t *d_hist, uint64_t piece_cap, uint64_t room_left, MergedScans &m,
                        std::vector<uint64_t> &tuple0)
 {
     const int S = (int)scanR.size() - 1;
@@ -1025,11 +1031,11 @@ static int merge_scans(mp_job *j, int k, int T, const std::vector<uint64_t> &sca
         tuple0.push_back(hist[scanR[s]] - hist[scanR[0]]);
     }
     if (!group_merge(m, hist, std::vector<uint32_t>(scanR.begin(), scanR.end()), j->pr.max_len, k)) return 0;
-    if (m.n > piece_cap) return 0;
+    if (m.n > piece_cap || 12 * m.n + 36 * most + (64ull << 20) > room_left) return 0;
     m.k1 = j->arena.alloc_persistent<uint64_t>(m.n + 1);
     m.id1 = j->arena.alloc_persistent<uint32_t>(m.n + 1);
     m.cur = j->arena.alloc_persistent<uint32_t>(m.digits);
-    // the largest scan's second buffers and plan have to fit beside them (piece_cap may be the caller's own)
+    // (what is left may be in pieces that are too small)
     uint8_t *room = m.k1 && m.id1 ? j->arena.alloc_persistent<uint8_t>(13 * most + (64u << 20)) : nullptr;
     if (room) j->arena.free_persistent(room);
     if (!m.k1 || !m.id1 || !m.cur || !room) {
@@ -1130,7 +1136,8 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
     };
     j->pieces_total = 0;
     j->hooked_bad = ~0u;
-    const uint64_t piece_cap = p->min3 ? ~0ull : scan_piece_cap(j);  // the 3-minimizer choice depends on the range
+    const uint64_t room = p->min3 ? 0 : device_room(j);
+    const uint64_t piece_cap = p->min3 ? ~0ull : scan_piece_cap(j, room);  // the 3-minimizer choice depends on the range
     MergedScans merged;
     struct Hold {  // what the scans share goes back on every return
         DeviceArena &arena;
@@ -1162,7 +1169,8 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         }
     } hold{j->arena, merged, cnt_all, d_b, d_hist};
     std::vector<uint64_t> tuple0;
-    if (S > 1 && !p->min3 && (rc = merge_scans(j, k, T, scanR, thrR, hist, d_hist, piece_cap, merged, tuple0))) return rc;
+    if (S > 1 && !p->min3 && (rc = merge_scans(j, k, T, scanR, thrR, hist, d_hist, piece_cap, room, merged, tuple0)))
+        return rc;
     for (int s = 0; s < S; s++) {
         const uint64_t lo = scanR[s], hi = scanR[s + 1];
         const uint64_t expect = hist[hi] - hist[lo];
@@ -1245,6 +1253,7 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
             j->arena.release_scratch();
             continue;
         }
+        hold.drop_merged();  // (a sorted scan takes 26 bytes a tuple; a later grouped one makes its own first pass)
         if ((rc = count_scans())) return rc;
         uint32_t *cnt = cnt_all ? cnt_all + (size_t)s * (N + 1) : j->arena.alloc<uint32_t>(N + 1);
         uint64_t *off = j->arena.alloc<uint64_t>(N + 2), *ntot = j->arena.alloc<uint64_t>(1);

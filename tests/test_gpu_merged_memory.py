@@ -1,5 +1,7 @@
-"""Device memory of scans that are split together: the split tuples of all scans go back when a partition fails.
+"""Device memory of scans that are split together: the split tuples of all scans go back when a partition fails, and
+when a later scan has to be sorted (a read that the scan before hooked below a component) and needs the room itself.
 """
+import numpy as np
 import pytest
 
 from metapart_gb300 import native, synth
@@ -28,3 +30,45 @@ def test_failed_partition_keeps_no_split_tuples(built_gpu):
         assert used[2] - used[0] < 1 << 20 < 12 * tuples
         job.set_wait_limits()
         job.partition(27, 2, 4, st, cnt.chunk_first_read, cnt.hist)
+
+
+def _hooked(n):
+    """Two scans of n reads, the second after a BAD read was hooked in the first (bad_anchor_fastq's "two_scans", larger)."""
+    L = 100
+    reads = ["A" * (L - 1) + c for c in "CGTC"] + ["C" * L] * n + [("GC" * L)[:L]] * n
+    return "".join(f"@b{i}\n{s}\n+\n{'I' * len(s)}\n" for i, s in enumerate(reads)).encode()
+
+
+def test_sorted_scan_after_merged_ones_fits_where_it_did(built_gpu):
+    """Every budget that holds the two scans one after another holds them when they may be split together."""
+    data = _hooked(60_000)
+    st = _starts(data)
+
+    def run(budget, together):
+        with native.Context(0, hbm_budget=budget) as ctx, native.Job(ctx) as job:
+            job.load(data)
+            cnt = job.count(27, st)
+            total = int(cnt.hist[-1])
+            job.set_scan_piece_tuples(total if together else total - 1)
+            try:
+                job.partition(27, 2, 1, st, cnt.chunk_first_read, cnt.hist)
+            except native.MetapartError as e:
+                assert "(-4)" in str(e)  # MP_ENOMEM
+                return None
+            assert job.scan_pieces == 2
+            return job.labels()
+
+    mb = 1 << 20
+    lo, hi = 64, 2048  # does not fit, fits
+    want = run(hi * mb, False)
+    assert want is not None
+    while hi - lo > 8:
+        m = (lo + hi) // 2
+        if run(m * mb, False) is None:
+            lo = m
+        else:
+            hi = m
+    for b in range(hi, hi + 320, 16):
+        got = run(b * mb, True)
+        assert got is not None, f"budget {b} MB (one after another: {hi} MB)"
+        assert np.array_equal(got, want)

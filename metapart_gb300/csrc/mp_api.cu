@@ -123,11 +123,14 @@ struct mp_job {
     uint64_t units_total = 0, big_buckets_total = 0, big_tuples_total = 0;
     uint64_t unit_passes_total = 0, phase_total[3] = {0, 0, 0}, pass_cycles_total[7] = {};
     int pe_rounds = 0;
+    uint64_t share = 0;         // device bytes that its caller set aside for it (job_set_share; 0: none)
     uint64_t piece_tuples = 0;  // most tuples a scan holds in HBM at once (0: from the free device memory)
     int pieces_total = 0;       // bucket-range pieces of the last partition, over all scans
     uint32_t hooked_bad = ~0u;  // a flagged read the last scan's unions hooked below a component (next scan: BAD)
     bool checks = false;        // self-checks of the sorted tuples and the final forest (mp_job_set_checks)
 };
+
+void mp::job_set_share(mp_job *job, uint64_t bytes) { job->share = bytes; }
 
 // ------------------------------------------------------------------ helpers
 
@@ -1012,8 +1015,9 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
 
 // The first split pass of all scans at once (MergedScans), where every scan is to be grouped and one scan of all the tuples
 // would not have to go in pieces, and where the bytes left (room) hold, beside the split tuples of all, what the largest scan
-// takes at most: its second buffers (12 a tuple), the two buffers of oversized buckets (24), the plan.  Else m.k1 stays null
-// and every scan makes its own.
+// takes at most: its second buffers (12 a tuple), the two buffers of oversized buckets (24), the plan.  A request of the loop
+// also stays within what was set aside for it, where each scan by itself would.  Else m.k1 stays null and every scan makes its
+// own.
 static int merge_scans(mp_job *j, int k, int T, const std::vector<uint64_t> &scanR, const std::vector<uint64_t> &thrR,
                        const uint64_t *hist, const uint64_t *d_hist, uint64_t piece_cap, uint64_t room_left, MergedScans &m,
                        std::vector<uint64_t> &tuple0)
@@ -1031,6 +1035,7 @@ static int merge_scans(mp_job *j, int k, int T, const std::vector<uint64_t> &sca
         tuple0.push_back(hist[scanR[s]] - hist[scanR[0]]);
     }
     if (!group_merge(m, hist, std::vector<uint32_t>(scanR.begin(), scanR.end()), j->pr.max_len, k)) return 0;
+    if (j->share && j->arena.live + 12 * m.n + 13 * most + (64ull << 20) > j->share) return 0;
     if (m.n > piece_cap || 12 * m.n + 36 * most + (64ull << 20) > room_left) return 0;
     m.k1 = j->arena.alloc_persistent<uint64_t>(m.n + 1);
     m.id1 = j->arena.alloc_persistent<uint32_t>(m.n + 1);

@@ -15,6 +15,9 @@ constexpr int STORE_FASTQ = MP_STORE_FASTQ, STORE_KMER_CACHE = MP_STORE_KMER_CAC
 int ctx_device(const mp_ctx *ctx);
 void ctx_budget(mp_ctx *ctx, std::atomic<uint64_t> **used, uint64_t *limit);
 
+// The device bytes that are set aside for a job's input (a request's footprint): it takes no more than these by choice.
+void job_set_share(mp_job *job, uint64_t bytes);
+
 // parent[x] = x for every read.
 void launch_init_parent(uint32_t *parent, uint64_t n, cudaStream_t st);
 

@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "metapart_gpu.h"
+#include "mp_internal.cuh"
 
 namespace {
 
@@ -105,6 +106,7 @@ void run_request(mp_server *s, mp_job *job, Request &rq, mp_result &res)
                             ofs.data(), &nrec);
     if (!rc && nrec != C + 1) rc = MP_EFMT;
     if (!rc) rc = mp_job_set_read_store(job, p.read_store);
+    if (!rc) mp::job_set_share(job, rq.footprint);
     if (!rc) {
         starts.assign(ofs.begin(), ofs.begin() + nrec);
         starts[nrec - 1] = rq.nbytes;

@@ -1,10 +1,13 @@
 """Device memory of scans that are split together: the split tuples of all scans go back when a partition fails, and
-when a later scan has to be sorted (a read that the scan before hooked below a component) and needs the room itself.
+when a later scan has to be sorted (a read that the scan before hooked below a component) and needs the room itself; a
+request of the loop takes no more for them than was set aside for it.
 """
+import threading
+
 import numpy as np
 import pytest
 
-from metapart_gb300 import native, synth
+from metapart_gb300 import native, serve, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -72,3 +75,31 @@ def test_sorted_scan_after_merged_ones_fits_where_it_did(built_gpu):
         got = run(b * mb, True)
         assert got is not None, f"budget {b} MB (one after another: {hi} MB)"
         assert np.array_equal(got, want)
+
+
+def test_request_stays_within_its_footprint(built_gpu):
+    """A small k, long reads and three scans without a store: the scans split together would take more than the request's
+    reservation, one after another they do not."""
+    import torch
+    spec = synth.workload("plain_large", 300_000, seed=33)
+    spec.lengths = (250,)
+    data = synth.fastq_to(spec, lambda n: (lambda t: (t, t.data_ptr()))(torch.empty(n, dtype=torch.uint8, pin_memory=True)))
+    out = torch.empty(data.numel() + 64, dtype=torch.uint8, pin_memory=True)
+    p = serve.RequestParams(k=11, num_scans=3, num_threads=4, num_chunks=8, read_store=0)
+    with native.Context(0) as ctx, serve.Server(ctx, slots=1) as srv:
+        ticket = srv.submit(data.data_ptr(), data.numel(), p, out.data_ptr(), out.numel())
+        peak, done = [0], threading.Event()
+
+        def watch():
+            while not done.is_set():
+                peak[0] = max(peak[0], ctx.hbm_in_use())
+
+        w = threading.Thread(target=watch)
+        w.start()
+        try:
+            r = srv.result(ticket)
+        finally:
+            done.set()
+            w.join()
+    assert r.status == 0, r.error
+    assert data.numel() < peak[0] <= serve.footprint(data.data_ptr(), data.numel(), p)

@@ -984,7 +984,8 @@ __global__ void k_gbig_gather(const BigUnit *bu, const uint64_t *kk, const uint3
     }
 }
 
-// The sorted units' ids into out, as k_group leaves them (a zeroed tuple or the zero k-mer's stands for no read).
+// The sorted units' ids into out, as k_group leaves them (a zeroed tuple or the zero k-mer's stands for no read, each a run
+// of its own: nothing looks back through them).
 __global__ void k_gbig_emit(const BigUnit *bu, const uint32_t *base, const uint64_t *tk, const uint32_t *tid, const uint32_t *z,
                             const uint32_t *ub0, uint32_t nunits, const uint32_t *lrs, int bsh, uint32_t *ctr, uint32_t *qlist,
                             uint32_t *quirk, uint32_t *out)
@@ -998,7 +999,7 @@ __global__ void k_gbig_emit(const BigUnit *bu, const uint32_t *base, const uint6
         const uint64_t km = tk[i] >> 8;
         const bool head = e == 0 || (tk[i - 1] >> 8) != km;
         const bool none = ((z[i >> 5] >> (i & 31)) & 1u) || (zero_bucket && (km & lowmask) == 0);
-        out[o + e] = (none ? GP_NONE : tid[i]) | (head ? 0x80000000u : 0u);
+        out[o + e] = (none ? GP_NONE : tid[i]) | (head || none ? 0x80000000u : 0u);
     }
     if (blockIdx.y == 0 && threadIdx.x == 0 && b.start >= lrs[seg]) {
         uint32_t *q = qlist + 3 * (size_t)atomicAdd(&ctr[GC_QLIST], 1u);
@@ -1018,7 +1019,12 @@ __global__ void k_gbig_emit(const BigUnit *bu, const uint32_t *base, const uint6
     }
 }
 
-__global__ void k_gbig_reserve(uint32_t *ctr, uint32_t n, uint32_t *base) { *base = atomicAdd(&ctr[GC_OUT], n); }
+// first: the first batch of oversized units; their ids are out's last (GC_LONG).
+__global__ void k_gbig_reserve(uint32_t *ctr, uint32_t n, uint32_t *base, bool first)
+{
+    *base = atomicAdd(&ctr[GC_OUT], n);
+    if (first) ctr[GC_LONG] = *base;
+}
 
 // ------------------------------------------------------------------ unions
 
@@ -1059,14 +1065,37 @@ __global__ void __launch_bounds__(256) k_gp_quirk(const uint32_t *ctr, const uin
 constexpr uint32_t GE_SEG = 1024;  // most grouped ids per warp and turn
 constexpr uint32_t GE_BLOCKS = 8;   // blocks per SM
 
+// Whether a stretch among the oversized units' ids has neither a run's start nor a read that is not BAD: k_gp_union passes by
+// it when it looks for a read of a run that began earlier.  A run of a few million tuples whose reads are all BAD (the inner
+// k-mers of an adapter, when its ends' branches make its reads BAD) was looked through from every stretch of it: 2M reads, 33
+// runs of 1.8M, the unions 142 -> 0.8 ms.
+__global__ void __launch_bounds__(256) k_gp_blank(const uint32_t *ctr, const uint32_t *__restrict__ out,
+                                                  const uint8_t *__restrict__ filtered, uint32_t per, uint8_t *blank)
+{
+    const uint32_t m = ctr[GC_OUT], first = (ctr[GC_LONG] + per - 1) / per, nseg = (m + per - 1) / per;
+    const int lane = threadIdx.x & 31;
+    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t sgm = first + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); sgm < nseg; sgm += nw) {
+        const uint32_t p0 = sgm * per, p1 = min(m, p0 + per);
+        bool some = false;
+        for (uint32_t p = p0; p < p1 && !some; p += 32) {
+            const uint32_t v = p + lane < p1 ? out[p + lane] : GP_NONE, id = v & 0x7FFFFFFFu;
+            some = __any_sync(FULLG, (v >> 31) || (id != GP_NONE && !filtered[id]));
+        }
+        if (lane == 0) blank[sgm] = !some;
+    }
+}
+
 // Bound by the random reads of the BAD flags and parents in L2.  It reads 4 bytes per joining tuple where the
 // sweep over sorted tuples read 13 per tuple: 6.7 ms against 21.0 at 20M x 150 bp, 2 scans.
 //
 // The unions of every k-mer's reads (metapart.c:2537-2727): each read that is not BAD joins its k-mer's first one
 // of the stretch.  A stretch that starts inside a run looks back for one read of it, so long runs are shared by
-// many warps.
+// many warps (at most a large block's tuples back, or past stretches known to be blank: k_gp_blank; null without oversized
+// units).
 __global__ void __launch_bounds__(256) k_gp_union(const uint32_t *ctr, const uint32_t *__restrict__ out, uint32_t *parent,
-                                                  const uint8_t *__restrict__ filtered, uint32_t per, uint32_t *err, uint32_t uf_cap)
+                                                  const uint8_t *__restrict__ filtered, const uint8_t *__restrict__ blank,
+                                                  uint32_t per, uint32_t *err, uint32_t uf_cap)
 {
     const uint32_t m = ctr[GC_OUT];
     const int lane = threadIdx.x & 31;
@@ -1077,7 +1106,16 @@ __global__ void __launch_bounds__(256) k_gp_union(const uint32_t *ctr, const uin
         bool has = false;
         uint32_t anchor = 0;
         if (!(out[p0] >> 31)) {  // the run's reads before the stretch, a window at a time
-            for (uint32_t q = p0; q >= 32;) {
+            uint32_t back = sgm;
+            if (blank) {
+                const uint32_t first = (ctr[GC_LONG] + per - 1) / per;
+                for (uint32_t n = 32; n == 32 && back > first;) {
+                    const uint32_t some = __ballot_sync(FULLG, back < first + 1 + lane || !blank[back - 1 - lane]);
+                    n = some ? (uint32_t)__ffs(some) - 1 : 32u;
+                    back -= n;
+                }
+            }
+            for (uint32_t q = back * per; q >= 32;) {
                 q -= 32;
                 const uint32_t v = out[q + lane], id = v & 0x7FFFFFFFu;
                 const uint32_t H = __ballot_sync(FULLG, v >> 31);
@@ -1464,7 +1502,7 @@ int group_filter(GroupScan &g, const uint64_t *kk, const uint32_t *ids, uint32_t
             tp.id = t.id[t.cur];
             tp.n = acc;
             if ((rc = filter_scan(tp, ends, parent, filtered, arena, st, false))) return rc;
-            (count_launch(), k_gbig_reserve<<<1, 1, 0, st>>>(g.ctr, (uint32_t)acc, d_base));
+            (count_launch(), k_gbig_reserve<<<1, 1, 0, st>>>(g.ctr, (uint32_t)acc, d_base, b0 == 0));
             (count_launch(), k_gbig_emit<<<grid, 256, 0, st>>>(d_b + b0, d_base, tp.lo, tp.id, tp.z, g.ub0, g.hctr[GC_UNITS], g.lrs,
                                                               bsh, g.ctr, g.qlist, g.quirk, out));
             MP_CUDA(cudaStreamSynchronize(st));  // ends is this turn's
@@ -1487,9 +1525,11 @@ int group_union(GroupScan &g, const uint32_t *out, uint32_t *parent, const uint8
     const uint32_t per = std::min(GE_SEG, ((uint32_t)(g.n / warps) + 63u) / 32u * 32u);
     const unsigned blocks = std::min<unsigned>(GE_BLOCKS * (unsigned)sm_count(), blocks_of(g.n, (int)per * 8));
     uint32_t *err = arena.alloc<uint32_t>(1);
-    if (!err) return set_error(MP_ENOMEM, "device memory");
+    uint8_t *blank = g.hctr[GC_BIG] ? arena.alloc<uint8_t>(g.n / per + 1) : nullptr;
+    if (!err || (g.hctr[GC_BIG] && !blank)) return set_error(MP_ENOMEM, "device memory");
     MP_CUDA(cudaMemsetAsync(err, 0, 4, st));
-    (count_launch(), k_gp_union<<<blocks, 256, 0, st>>>(g.ctr, out, parent, filtered, per, err, arena.lim.union_retries));
+    if (blank) (count_launch(), k_gp_blank<<<blocks, 256, 0, st>>>(g.ctr, out, filtered, per, blank));
+    (count_launch(), k_gp_union<<<blocks, 256, 0, st>>>(g.ctr, out, parent, filtered, blank, per, err, arena.lim.union_retries));
     compress_parents(parent, n_reads, st);
     const size_t words = GC_N + (size_t)nseg * QW;
     ReadBack<uint32_t> h(arena, words + 1);

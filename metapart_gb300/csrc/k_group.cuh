@@ -72,7 +72,7 @@ struct GroupScan {
 
 enum GroupCounter : int {
     GC_UNITS = 0, GC_TILES, GC_MID, GC_BIG, GC_BIG_TUPLES,  // the plan's counts
-    GC_WORK_S, GC_WORK_L, GC_OUT, GC_QLIST, GC_ERR, GC_N = 16
+    GC_WORK_S, GC_WORK_L, GC_OUT, GC_QLIST, GC_ERR, GC_LONG, GC_N = 16
 };
 
 // What a scan's unions left open, per segment: the segment's last run is to be united with the segment's first

@@ -699,7 +699,7 @@ __global__ void k_big_gather(const uint64_t *__restrict__ bstart, const uint32_t
 {
     const uint32_t b = blockIdx.x;
     const uint64_t lowmask = (1ull << lowbits) - 1, s = bstart[b], o = boff[b];
-    for (uint32_t e = threadIdx.x; e < bcount[b]; e += blockDim.x) {
+    for (uint32_t e = blockIdx.y * blockDim.x + threadIdx.x; e < bcount[b]; e += gridDim.y * blockDim.x) {
         tk[o + e] = ((uint64_t)b << lowbits) | (lo_in[s + e] & lowmask);
         tid[o + e] = id_in[s + e];
     }
@@ -713,7 +713,7 @@ __global__ void k_big_scatter(const uint64_t *__restrict__ bstart, const uint32_
     const uint32_t b = blockIdx.x;
     const uint64_t lowmask = (1ull << lowbits) - 1, s = bstart[b], o = boff[b];
     const uint64_t hibits = (uint64_t)(bbucket[b] & (NB - 1)) << lowbits;  // the bucket within its segment
-    for (uint32_t e = threadIdx.x; e < bcount[b]; e += blockDim.x) {
+    for (uint32_t e = blockIdx.y * blockDim.x + threadIdx.x; e < bcount[b]; e += gridDim.y * blockDim.x) {
         lo_out[s + e] = hibits | (tk[o + e] & lowmask);
         id_out[s + e] = tid[o + e];
     }
@@ -1020,15 +1020,21 @@ static int sort_big_buckets(const std::vector<uint64_t> &bs, const std::vector<u
     }
     for (size_t b0 = 0; b0 < nb; b0 += per_batch) {
         const size_t b1 = std::min<size_t>(nb, b0 + per_batch);
-        uint64_t acc = 0;
-        for (size_t q = b0; q < b1; q++) { bo[q] = acc; acc += bc[q]; }
+        uint64_t acc = 0, most = 0;
+        for (size_t q = b0; q < b1; q++) {
+            bo[q] = acc;
+            acc += bc[q];
+            most = std::max<uint64_t>(most, bc[q]);
+        }
+        // blocks for the largest bucket (one block for one of 21 million tuples took 40 ms each way)
+        const dim3 grid((unsigned)(b1 - b0), (unsigned)std::min<uint64_t>({256, most / 8192 + 1, 65536 / (b1 - b0) + 1}));
         MP_CUDA(cudaMemcpyAsync(d_bo + b0, bo.data() + b0, (b1 - b0) * 8, cudaMemcpyHostToDevice, st));
         t.cur = 0;
-        (mp::count_launch(), k_big_gather<<<(unsigned)(b1 - b0), 256, 0, st>>>(d_bs + b0, d_bc + b0, d_bo + b0, b.lo[in],
+        (mp::count_launch(), k_big_gather<<<grid, 256, 0, st>>>(d_bs + b0, d_bc + b0, d_bo + b0, b.lo[in],
                                                                               b.id[in], t.lo[0], t.id[0], lowbits));
         int rc = radix_sort(t, acc, false, arena, st, nullptr);
         if (rc) return rc;
-        (mp::count_launch(), k_big_scatter<<<(unsigned)(b1 - b0), 256, 0, st>>>(d_bs + b0, d_bc + b0, d_bb + b0, d_bo + b0,
+        (mp::count_launch(), k_big_scatter<<<grid, 256, 0, st>>>(d_bs + b0, d_bc + b0, d_bb + b0, d_bo + b0,
                                                                                t.lo[t.cur], t.id[t.cur], b.lo[out],
                                                                                b.id[out], lowbits));
     }
@@ -1339,9 +1345,16 @@ __global__ void __launch_bounds__(256) k_key_bits(const uint64_t *__restrict__ l
     }
 }
 
-// Counts of the window's two digits.
+// A sample of the tuples by window bucket: every (mask + 1)-th.  big: those in buckets of at least `large` of them.
+struct BucketSample {
+    uint32_t mask, large;
+    uint32_t *bucket;
+    unsigned int *big;
+};
+
+// Counts of the window's two digits, and the sample.
 __global__ void __launch_bounds__(256) k_window_hist(const uint64_t *__restrict__ lo, const uint8_t *__restrict__ hi, uint64_t n,
-                                                     const KeyBits *bits, unsigned int *cnt)
+                                                     const KeyBits *bits, unsigned int *cnt, BucketSample sm)
 {
     __shared__ uint32_t h[512];
     h[threadIdx.x] = h[threadIdx.x + 256] = 0;
@@ -1352,8 +1365,13 @@ __global__ void __launch_bounds__(256) k_window_hist(const uint64_t *__restrict_
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const uint64_t k = lo[i];
         const uint32_t x = hi ? (uint32_t)hi[i] : 0u;
-        atomicAdd(&h[digit_of<2>(k, x, bsh)], 1u);
-        atomicAdd(&h[256 + digit_of<2>(k, x, bsh + 8)], 1u);
+        const uint32_t d0 = digit_of<2>(k, x, bsh), d1 = digit_of<2>(k, x, bsh + 8);
+        atomicAdd(&h[d0], 1u);
+        atomicAdd(&h[256 + d1], 1u);
+        if (((uint32_t)i & sm.mask) == 0) {
+            const uint32_t c = atomicAdd(&sm.bucket[d1 << 8 | d0], 1u) + 1;
+            if (c >= sm.large) atomicAdd(sm.big, c == sm.large ? c : 1u);
+        }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < 512; i += 256)
@@ -1556,7 +1574,7 @@ __global__ void __launch_bounds__(UR_THREADS, 2) k_unit_rank(UnitRank c)
 // Where the lines lie: 8,192 tuples take 258 us by passes and 146 by units, all of it launches and waits; above
 // 2^27 a bucket of evenly spread keys nears a unit, and keys that occur in few (digit, digit) pairs make buckets far
 // above one (they would be sorted twice).
-constexpr uint64_t UNIT_SORT_MIN = 1ull << 10, UNIT_SORT_MAX = 1ull << 27;
+constexpr uint64_t UNIT_SORT_MIN = 1ull << 10, UNIT_SORT_MAX = 1ull << 27, UNIT_SORT_FEW = 3ull << 19;
 
 static void sort_kernel_attrs()
 {
@@ -1586,13 +1604,13 @@ int unit_sort(const SortInput &in, SortBufs &b, uint64_t n, DeviceArena &arena, 
     if (n < UNIT_SORT_MIN || n > UNIT_SORT_MAX) return 0;
     struct Head {
         KeyBits bits;
-        unsigned int occur[2], cnt[512];
+        unsigned int occur[2], big, pad, cnt[512];
         uint32_t ctr[2], err, nlist;
     };
     const uint64_t tiles = (n + STILE - 1) / STILE;
     Head *head = reinterpret_cast<Head *>(arena.alloc<uint64_t>((sizeof(Head) + 7) / 8));
     uint64_t *dbase = arena.alloc<uint64_t>(512), *off = arena.alloc<uint64_t>(UW_BUCKETS + 2), *tot = arena.alloc<uint64_t>(1);
-    uint32_t *first = arena.alloc<uint32_t>(UW_BUCKETS), *end = arena.alloc<uint32_t>(UW_BUCKETS);
+    uint32_t *first = arena.alloc<uint32_t>(2 * UW_BUCKETS), *end = first ? first + UW_BUCKETS : nullptr;
     uint32_t *flag = arena.alloc<uint32_t>(UW_BUCKETS + 1), *ustart = arena.alloc<uint32_t>(UW_BUCKETS);
     uint32_t *list = arena.alloc<uint32_t>(3 * UW_BUCKETS);
     unsigned long long *status = arena.alloc<unsigned long long>(tiles * 256);
@@ -1602,12 +1620,16 @@ int unit_sort(const SortInput &in, SortBufs &b, uint64_t n, DeviceArena &arena, 
         return set_error(MP_ENOMEM, "device memory for the unit sort");
     sort_kernel_attrs();
     MP_CUDA(cudaMemsetAsync(head, 0, sizeof(Head), st));
-    MP_CUDA(cudaMemsetAsync(end, 0, UW_BUCKETS * sizeof(uint32_t), st));
+    MP_CUDA(cudaMemsetAsync(first, 0, 2 * UW_BUCKETS * sizeof(uint32_t), st));  // (the sample's counts, until the bounds)
     MP_CUDA(cudaMemsetAsync(flag + UW_BUCKETS, 0, sizeof(uint32_t), st));
     MP_CUDA(cudaMemsetAsync(status, 0, tiles * 256 * sizeof(unsigned long long), st));
     const unsigned grid = (unsigned)std::min<uint64_t>((n + 1023) / 1024, 8ull * (uint64_t)sm_count());
+    uint32_t step = 1;  // 16,384 samples, and twelve of a bucket that a large block just takes
+    while (step < 1024 && n / (2 * step) >= 16384) step *= 2;
+    const uint64_t samples = (n + step - 1) / step;
     (mp::count_launch(), k_key_bits<<<grid, 256, 0, st>>>(in.lo, in.hi, n, &head->bits));
-    (mp::count_launch(), k_window_hist<<<grid, 256, 0, st>>>(in.lo, in.hi, n, &head->bits, head->cnt));
+    (mp::count_launch(), k_window_hist<<<grid, 256, 0, st>>>(in.lo, in.hi, n, &head->bits, head->cnt,
+                                                               BucketSample{step - 1, (uint32_t)(SS_CAP * samples / n) + 1, first, &head->big}));
     (mp::count_launch(), k_window_digits<<<2, 256, 0, st>>>(head->cnt, dbase, head->occur));
     Head h;
     MP_CUDA(cudaMemcpyAsync(&h, head, offsetof(Head, cnt), cudaMemcpyDeviceToHost, st));
@@ -1617,7 +1639,12 @@ int unit_sort(const SortInput &in, SortBufs &b, uint64_t n, DeviceArena &arena, 
     const int bsh = window_shift(t), lowbits = bsh + 8, r = std::min(UW_BITS, 64 - lowbits);
     // (a listed unit carries its first bucket in 20 bits: constant bits above the window must be zero or leave the low word)
     const unsigned long long above = ((h.bits.lo1 >> 8) | (h.bits.hi1 << 56)) >> bsh >> UW_BITS;
-    if (t < 0 || (above && lowbits < 44) || n > (uint64_t)(UNIT_QUANTUM / 2) * h.occur[0] * h.occur[1]) {
+    // Buckets above a large block are gathered and take the digit passes after all.  Where few tuples are in such buckets that
+    // costs less than the passes saved (a third of one k-mer: 24 million tuples 2.0 against 3.0 ms, 2 million 0.50 against
+    // 0.58); where most are, or with few tuples any (the gather's launches and waits), it does not (24 million of 1,200 k-mers 3.6
+    // against 3.0; a tenth of one k-mer: 1.2 million 0.45 against 0.39, 200,000 0.39 against 0.30).
+    const bool heavy = h.big > samples / 2 || (h.big && n < UNIT_SORT_FEW);
+    if (t < 0 || heavy || (above && lowbits < 44) || n > (uint64_t)(UNIT_QUANTUM / 2) * h.occur[0] * h.occur[1]) {
         arena.free_scratch(status);
         return 0;
     }

@@ -1630,9 +1630,9 @@ int mp_sort_tuples(mp_ctx *ctx, const uint64_t *lo_in, const uint8_t *hi_in, con
     b.lo[0] = lo_out;
     b.id[0] = id_out;
     b.hi[0] = hi_out;
-    b.lo[1] = arena.alloc<uint64_t>(n + 1);
-    b.id[1] = arena.alloc<uint32_t>(n + 1);
-    b.hi[1] = has_hi ? arena.alloc<uint8_t>(n + 1) : nullptr;
+    b.lo[1] = arena.alloc_persistent<uint64_t>(n + 1);
+    b.id[1] = arena.alloc_persistent<uint32_t>(n + 1);
+    b.hi[1] = has_hi ? arena.alloc_persistent<uint8_t>(n + 1) : nullptr;
     if (!b.lo[1] || !b.id[1] || (has_hi && !b.hi[1])) {
         arena.release_all();
         return set_error(MP_ENOMEM, "device memory for sorting %llu tuples", (unsigned long long)n);
@@ -1647,6 +1647,10 @@ int mp_sort_tuples(mp_ctx *ctx, const uint64_t *lo_in, const uint8_t *hi_in, con
     } else {
         bool done = false;
         rc = unit_sort(in, b, n, arena, st, &done);
+        if (rc == MP_ENOMEM) {  // (its tables and its buckets above a block take more than the digit passes do)
+            arena.release_scratch();
+            rc = 0;
+        }
         if (!rc && !done) rc = radix_sort(b, n, has_hi, arena, st, nullptr, &in);
     }
     if (!rc && b.cur == 1 && n) {

@@ -66,3 +66,33 @@ def test_one_kmer_is_not_one_block_s(built_gpu, share):
             o = [torch.empty_like(x) for x in d]
             t.append(min(_sort(ctx, d, o) for _ in range(6)))
     assert t[1] < 6 * t[0], t
+
+
+@pytest.mark.parametrize("n,share", [(2_000, 0.0), (40_000, 0.0), (3_000_000, 0.4)])
+def test_budget_of_the_digit_passes_is_enough(built_gpu, n, share):
+    """The smallest budget that the sort in place fits (digit passes alone), to a few KB, is enough for the other."""
+    lo, hi, ids = _keys(n, share, 7)
+    order = np.lexsort((lo, hi))
+
+    def sort(budget, in_place):
+        import torch
+        d = _dev(lo, hi, ids)
+        o = d if in_place else [torch.empty_like(x) for x in d]
+        with native.Context(0, hbm_budget=budget) as ctx:
+            try:
+                _sort(ctx, d, o)
+            except native.MetapartError as e:
+                assert "(-4)" in str(e)  # MP_ENOMEM
+                return None
+        return o[2].cpu().numpy().view(np.uint32)
+
+    small, fits = 1024, 256 << 20
+    while fits - small > 4096:
+        m = (small + fits) // 2
+        if sort(m, True) is None:
+            small = m
+        else:
+            fits = m
+    for more in (0, 64 << 10, 1 << 20, 3 << 20, 5 << 20, 20 << 20, 40 << 20):
+        got = sort(fits + more, False)
+        assert got is not None and np.array_equal(got, ids[order]), (fits, more)

@@ -13,9 +13,10 @@ namespace mp {
 //
 // Allocations of up to SLAB_PIECE bytes are cut from two slabs of SLAB bytes (one each for scratch and persistent ones,
 // reused in stream order, given back by release_all): a small job makes 140 allocations of which all but a few are
-// small, at 1-2 us each to take and to free.
+// small, at 1-2 us each to take and to free.  Where the budget has less than SLAB_ROOM left, a slab would be more than a few
+// thousandths of it, and every allocation is exact.
 struct DeviceArena {
-    static constexpr size_t SLAB = 1u << 20, SLAB_PIECE = 64u << 10;
+    static constexpr size_t SLAB = 1u << 20, SLAB_PIECE = 64u << 10, SLAB_ROOM = 256 * SLAB;
     struct Slab {
         char *p = nullptr;
         size_t at = 0;
@@ -55,7 +56,7 @@ struct DeviceArena {
         if (bytes == 0) bytes = 256;
         if (bytes <= SLAB_PIECE) {
             Slab &s = slab[keep];
-            if (!s.p) {
+            if (!s.p && (!budget_used || budget_limit == ~0ull || budget_used->load() + SLAB_ROOM <= budget_limit)) {
                 s.p = (char *)exact(SLAB, persistent);  // (both slabs stay until release_all)
                 s.at = 0;
             }

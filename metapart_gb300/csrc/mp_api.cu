@@ -476,12 +476,12 @@ int mp_job_count(mp_job *j, int k, int min3, const uint64_t *chunk_starts, int n
     j->clk.clear(1);
     uint64_t *d_rec = j->arena.alloc<uint64_t>(nchunks + 1);
     unsigned long long *glob = j->arena.alloc<unsigned long long>(NB + 1);
-    uint64_t *prefix = j->arena.alloc<uint64_t>(NB + 1);
-    const size_t tb = scan_tmp_bytes(NB + 1);
-    void *tmp = j->arena.alloc<uint8_t>(tb);
     uint32_t *cc = chunk_counts_out ? j->arena.alloc<uint32_t>((size_t)nchunks * NB) : nullptr;
     uint32_t *err = j->arena.alloc<uint32_t>(1);
-    if (!d_rec || !glob || !prefix || !tmp || !err || (chunk_counts_out && !cc)) return set_error(MP_ENOMEM, "device memory for counting");
+    if (!d_rec || !glob || !err || (chunk_counts_out && !cc)) return set_error(MP_ENOMEM, "device memory for counting");
+    const size_t tb = scan_tmp_bytes(NB + 1);
+    uint64_t *prefix = j->arena.alloc<uint64_t>(NB + 1);
+    void *tmp = prefix ? j->arena.alloc<uint8_t>(tb) : nullptr;
     MP_CUDA(cudaMemcpyAsync(d_rec, rec.data(), (nchunks + 1) * 8, cudaMemcpyHostToDevice, j->st));
     MP_CUDA(cudaMemsetAsync(glob, 0, (NB + 1) * 8, j->st));
     MP_CUDA(cudaMemsetAsync(err, 0, 4, j->st));
@@ -491,17 +491,26 @@ int mp_job_count(mp_job *j, int k, int min3, const uint64_t *chunk_starts, int n
         launch_count(j->d_fq, j->pr, k, min3, d_rec, nchunks, cc, glob, err, j->st, j->store == STORE_PACKED);
         j->kc_pieces = j->store != STORE_FASTQ && !min3 ? 1 : 0;
     }
-    // the prefix straight into the caller's array (on the host, two 8 MB arrays were first touched and walked: 1 ms)
-    scan_u64((const uint64_t *)glob, prefix, NB + 1, nullptr, tmp, tb, j->st);
+    // the prefix straight into the caller's array (on the host, two 8 MB arrays were first touched and walked: 1 ms), or the counts
+    // where there is no room for it
+    if (tmp) scan_u64((const uint64_t *)glob, prefix, NB + 1, nullptr, tmp, tb, j->st);
     ReadBack<uint32_t> rb(j->arena, 1);
     MP_CUDA(cudaMemcpyAsync(rb.p, err, 4, cudaMemcpyDeviceToHost, j->st));
     touch_pages(hist_out, (NB + 1) * 8);
-    MP_CUDA(cudaMemcpyAsync(hist_out, prefix, (NB + 1) * 8, cudaMemcpyDeviceToHost, j->st));
+    MP_CUDA(cudaMemcpyAsync(hist_out, tmp ? prefix : (const uint64_t *)glob, (NB + 1) * 8, cudaMemcpyDeviceToHost, j->st));
     if (cc) MP_CUDA(cudaMemcpyAsync(chunk_counts_out, cc, (size_t)nchunks * NB * 4, cudaMemcpyDeviceToHost, j->st));
     MP_CUDA(cudaStreamSynchronize(j->st));
     MP_CUDA(cudaGetLastError());
     const uint32_t herr = rb[0];
     j->arena.release_scratch();
+    if (!tmp) {
+        uint64_t acc = 0;
+        for (uint64_t b = 0; b <= NB; b++) {
+            const uint64_t c = hist_out[b];
+            hist_out[b] = acc;
+            acc += c;
+        }
+    }
     if (herr & DERR_LONG_READ) {
         j->kc_pieces = 0;
         return set_error(MP_EUNSUP, "a read is longer than %d bases", MAX_READ_COUNT);

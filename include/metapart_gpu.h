@@ -305,9 +305,11 @@ int mp_job_set_scan_piece_tuples(mp_job *job, uint64_t max_tuples);
 int mp_job_set_wait_limits(mp_job *job, uint32_t lookback_spins, uint32_t union_retries, uint32_t mate_rounds);
 
 /* Self-checks of the job's intermediate results (off by default; the environment variable MP_CHECK=1
- * turns them on for every job): after every scan's sort (or every piece's), that no adjacent tuple pair is
- * out of (k-mer, adjacency) order; after the mate union, that every read's parent is a root or BAD.  A
- * failed check makes mp_job_partition return MP_EDEVICE naming it.  The reference checks neither. */
+ * turns them on for every job): every scan that is grouped (the default path) is sorted as well, on its own copy of the
+ * forest, and both have to leave the same parents and BAD flags (where the memory holds both; else the scan is sorted
+ * only); after every scan's sort (or every piece's), that no adjacent tuple pair is out of (k-mer, adjacency) order;
+ * after the mate union, that every read's parent is a root or BAD.  A failed check makes mp_job_partition return
+ * MP_EDEVICE naming it.  The reference checks neither. */
 int mp_job_set_checks(mp_job *job, int on);
 
 /* Adjacent pairs out of (k-mer, adjacency) order in a device tuple array (lo and hi as mp_sort_tuples;

@@ -4,6 +4,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -146,14 +147,19 @@ int write_file(const std::string &path, const void *buf, size_t n, bool append =
     return 0;
 }
 
+// The scans' tuple streams are dumped ("0": the per-read dumps only, for large inputs).
+bool dumps_tuples(const mp_job *j)
+{
+    const char *tu = getenv("MP_DUMP_TUPLES");
+    return !j->dump_dir.empty() && !(tu && strcmp(tu, "0") == 0);
+}
+
 // Dump of tuples in the reference's 14-byte record format (enumerateKmers.c:352-365); append: after the
 // file's earlier pieces.
 int dump_tuples(mp_job *j, const char *name, const uint64_t *lo, const uint8_t *hi, const uint32_t *id, uint64_t n,
                 bool append = false)
 {
-    if (j->dump_dir.empty()) return 0;
-    const char *tu = getenv("MP_DUMP_TUPLES");  // "0": the per-read dumps only (large inputs)
-    if (tu && strcmp(tu, "0") == 0) return 0;
+    if (!dumps_tuples(j)) return 0;
     std::vector<uint64_t> hl(n);
     std::vector<uint8_t> hh(hi ? n : 0);
     std::vector<uint32_t> hid(n);
@@ -198,6 +204,15 @@ int dump_state(mp_job *j, const char *pname, const char *sname, bool with_parent
     return rc;
 }
 
+// A scan's BAD flags.
+int dump_bad(mp_job *j, int s)
+{
+    if (j->dump_dir.empty()) return 0;
+    std::vector<uint8_t> f(j->pr.n_reads);
+    MP_CUDA(cudaMemcpyAsync(f.data(), j->d_filtered, f.size(), cudaMemcpyDeviceToHost, j->st));
+    MP_CUDA(cudaStreamSynchronize(j->st));
+    return write_file(j->dump_dir + "/scan" + std::to_string(s) + "_bad.bin", f.data(), f.size());
+}
 
 __global__ void k_sizes_raw(const uint32_t *parent, uint64_t n, uint32_t *size)
 {
@@ -871,14 +886,7 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
         }
         MP_CUDA(cudaStreamSynchronize(j->st));
     }
-    if (!j->dump_dir.empty()) {
-        std::vector<uint8_t> f(N);
-        MP_CUDA(cudaMemcpyAsync(f.data(), j->d_filtered, N, cudaMemcpyDeviceToHost, j->st));
-        MP_CUDA(cudaStreamSynchronize(j->st));
-        snprintf(name, sizeof name, "scan%d_bad.bin", s);
-        rc = write_file(j->dump_dir + "/" + name, f.data(), N);
-        if (rc) return rc;
-    }
+    if ((rc = dump_bad(j, s))) return rc;
     // ---- sweep 2: the unions, piece by piece, from the scan's initial state
     rebad_read(j->d_parent, j->hooked_bad, j->st);
     j->hooked_bad = ~0u;
@@ -927,11 +935,12 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
 }
 
 // Whether a scan of n tuples is grouped instead of sorted (k_group.cuh).  The sorted scan is for who looks at
-// it or shapes its making: stage dumps, the self-checks, a tuning row or a limit of the sort's look-back; a read
+// it or shapes its making: dumps of its tuples, a tuning row or a limit of the sort's look-back; a read
 // that the previous scan hooked below a component (its label changes as this scan's unions begin) takes it too.
+// With the self-checks a grouped scan is sorted as well and the two are compared (CheckedScan).
 static bool scan_is_grouped(const mp_job *j, int k, uint64_t n)
 {
-    return j->dump_dir.empty() && !j->checks && j->arena.lim.lookback_spins == WaitLimits{}.lookback_spins &&
+    return (j->checks || !dumps_tuples(j)) && j->arena.lim.lookback_spins == WaitLimits{}.lookback_spins &&
            j->hooked_bad == ~0u && !sort_plan_chosen(k, n) && group_fits(n, j->pr.n_reads, nullptr);
 }
 
@@ -1022,6 +1031,70 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
     return 0;
 }
 
+// Reads whose parent or BAD flag differs.
+__global__ void k_count_differing(const uint32_t *pa, const uint32_t *pb, const uint8_t *fa, const uint8_t *fb, uint64_t n,
+                                  unsigned long long *out)
+{
+    const uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = __syncthreads_count(x < n && (pa[x] != pb[x] || fa[x] != fb[x]));
+    if (threadIdx.x == 0 && c) atomicAdd(out, (unsigned long long)c);
+}
+
+// The self-check of a grouped scan (mp_job_set_checks): it runs on a copy of the forest, then the scan is sorted, on the forest
+// itself, and both have to leave the same parents, BAD flags and hooked read.  (The root of a component is its largest read, so
+// the compressed parents do not depend on the order of the unions.)
+struct CheckedScan {
+    mp_job *j;
+    uint32_t *parent = nullptr;
+    uint8_t *filtered = nullptr;
+    uint32_t hooked = ~0u;
+
+    explicit CheckedScan(mp_job *job) : j(job) {}
+    ~CheckedScan()
+    {
+        j->arena.free_persistent(parent);
+        j->arena.free_persistent(filtered);
+    }
+    void swap()
+    {
+        std::swap(parent, j->d_parent);
+        std::swap(filtered, j->d_filtered);
+        std::swap(hooked, j->hooked_bad);
+    }
+    // run: the grouped scan.
+    int grouped(const std::function<int()> &run)
+    {
+        const uint64_t n = j->pr.n_reads + 1;
+        parent = j->arena.alloc_persistent<uint32_t>(n);
+        filtered = j->arena.alloc_persistent<uint8_t>(n);
+        if (!parent || !filtered) return set_error(MP_ENOMEM, "device memory for the self-check's copy of the forest");
+        MP_CUDA(cudaMemcpyAsync(parent, j->d_parent, n * 4, cudaMemcpyDeviceToDevice, j->st));
+        MP_CUDA(cudaMemcpyAsync(filtered, j->d_filtered, n, cudaMemcpyDeviceToDevice, j->st));
+        swap();
+        const int rc = run();
+        j->arena.release_scratch();
+        swap();
+        return rc;
+    }
+    int compare(int scan)
+    {
+        unsigned long long *dc = j->arena.alloc<unsigned long long>(1);
+        if (!dc) return set_error(MP_ENOMEM, "device memory");
+        const uint64_t n = j->pr.n_reads;
+        uint64_t bad = 0;
+        MP_CUDA(cudaMemsetAsync(dc, 0, 8, j->st));
+        (mp::count_launch(), k_count_differing<<<(unsigned)((n + 255) / 256), 256, 0, j->st>>>(j->d_parent, parent, j->d_filtered,
+                                                                                          filtered, n, dc));
+        MP_CUDA(cudaMemcpyAsync(&bad, dc, 8, cudaMemcpyDeviceToHost, j->st));
+        MP_CUDA(cudaStreamSynchronize(j->st));
+        MP_CUDA(cudaGetLastError());
+        if (bad || hooked != j->hooked_bad)
+            return set_error(MP_EDEVICE, "check: scan %d grouped and sorted differ in %llu reads' parents or flags", scan,
+                             (unsigned long long)bad);
+        return 0;
+    }
+};
+
 // The first split pass of all scans at once (MergedScans), where every scan is to be grouped and one scan of all the tuples
 // would not have to go in pieces, and where the bytes left (room) hold, beside the split tuples of all, what the largest scan
 // takes at most: its second buffers (12 a tuple), the two buffers of oversized buckets (24), the plan.  A request of the loop
@@ -1045,7 +1118,8 @@ static int merge_scans(mp_job *j, int k, int T, const std::vector<uint64_t> &sca
     }
     if (!group_merge(m, hist, std::vector<uint32_t>(scanR.begin(), scanR.end()), j->pr.max_len, k)) return 0;
     if (j->share && j->arena.live + 12 * m.n + 13 * most + (64ull << 20) > j->share) return 0;
-    if (m.n > piece_cap || 12 * m.n + 36 * most + (64ull << 20) > room_left) return 0;
+    const uint64_t checks = j->checks ? 28 * most + 5 * j->pr.n_reads : 0;  // the sorted scan and the copy of the forest
+    if (m.n > piece_cap || 12 * m.n + 36 * most + checks + (64ull << 20) > room_left) return 0;
     m.k1 = j->arena.alloc_persistent<uint64_t>(m.n + 1);
     m.id1 = j->arena.alloc_persistent<uint32_t>(m.n + 1);
     m.cur = j->arena.alloc_persistent<uint32_t>(m.digits);
@@ -1185,6 +1259,48 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
     std::vector<uint64_t> tuple0;
     if (S > 1 && !p->min3 && (rc = merge_scans(j, k, T, scanR, thrR, hist, d_hist, piece_cap, room, merged, tuple0)))
         return rc;
+    // scan s, grouped
+    auto run_grouped = [&](int s, uint64_t n, const std::vector<uint64_t> &rb) -> int {
+        GroupScan gs;
+        gs.k = k;
+        gs.n = n;
+        gs.d_hist = d_hist;
+        gs.lo = scanR[s];
+        gs.hi = scanR[s + 1];
+        gs.bounds = rb;
+        gs.seg_tstart = {0, n};
+        if (merged.k1) group_take(gs, merged, s, j->d_parent, tuple0);
+        if (!p->min3) {
+            if (j->pr.max_len > (uint32_t)k && j->pr.max_len - (uint32_t)k >= 300u)
+                return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
+            return grouped_scan(j, gs, 0, s, nullptr, nullptr, nullptr, err, hist);
+        }
+        // the 3-minimizer tuples: the splits need no order, and the histogram knows their number
+        uint64_t *tl = j->arena.alloc<uint64_t>(n + 1);
+        uint8_t *th = has_hi ? j->arena.alloc<uint8_t>(n + 1) : nullptr;
+        uint32_t *ti = j->arena.alloc<uint32_t>(n + 1);
+        unsigned long long *ntot = j->arena.alloc<unsigned long long>(1), got = 0;
+        if (!tl || !ti || (has_hi && !th) || !ntot)
+            return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)n);
+        uint32_t cerr = 0;
+        {
+            StageTimer tm(j->clk, j->st, 2);
+            MP_CUDA(cudaMemsetAsync(ntot, 0, 8, j->st));
+            launch_enum_min3(j->d_fq, j->pr, k, (uint32_t)gs.lo, (uint32_t)gs.hi, s ? j->d_parent : nullptr, ntot, n, tl, th, ti, err,
+                             j->st);
+            MP_CUDA(cudaMemcpyAsync(&got, ntot, 8, cudaMemcpyDeviceToHost, j->st));
+            MP_CUDA(cudaMemcpyAsync(&cerr, err, 4, cudaMemcpyDeviceToHost, j->st));
+            MP_CUDA(cudaStreamSynchronize(j->st));
+        }
+        if (cerr & DERR_LONG_READ) return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
+        if (cerr & DERR_TOO_MANY)
+            return set_error(MP_EUNSUP, "a read has 256 or more k-mers in scan %d (the reference counts them "
+                                        "in 8 bits, enumerateKmers.c:152)", s);
+        if (got != n)
+            return set_error(MP_EFMT, "scan %d: %llu tuples but the histogram holds %llu", s, got, (unsigned long long)n);
+        if (cerr) return set_error(MP_EDEVICE, "enumeration flags 0x%x", cerr);
+        return grouped_scan(j, gs, 1, s, tl, th, ti, err, hist);
+    };
     for (int s = 0; s < S; s++) {
         const uint64_t lo = scanR[s], hi = scanR[s + 1];
         const uint64_t expect = hist[hi] - hist[lo];
@@ -1219,55 +1335,24 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         std::vector<uint64_t> rb;
         const int rb_rc = range_bounds(hist, thrR.data() + (size_t)s * T, T, lo, hi, rb);
         const std::string rb_msg = rb_rc ? g_err : std::string();
-        const bool grouped = !rb_rc && scan_is_grouped(j, k, expect);
-        GroupScan gs;
+        bool grouped = !rb_rc && scan_is_grouped(j, k, expect);
+        CheckedScan checked(j);
         if (grouped) {
-            gs.k = k;
-            gs.n = expect;
-            gs.d_hist = d_hist;
-            gs.lo = lo;
-            gs.hi = hi;
-            gs.bounds = rb;
-            gs.seg_tstart = {0, expect};
-            if (merged.k1) group_take(gs, merged, s, j->d_parent, tuple0);
-        }
-        if (grouped && !p->min3) {
-            if (j->pr.max_len > (uint32_t)k && j->pr.max_len - (uint32_t)k >= 300u)
-                return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
-            if ((rc = grouped_scan(j, gs, 0, s, nullptr, nullptr, nullptr, err, hist))) return rc;
-            j->arena.release_scratch();
-            continue;
-        }
-        if (grouped) {  // the 3-minimizer tuples: the splits need no order, and the histogram knows their number
-            uint64_t *tl = j->arena.alloc<uint64_t>(expect + 1);
-            uint8_t *th = has_hi ? j->arena.alloc<uint8_t>(expect + 1) : nullptr;
-            uint32_t *ti = j->arena.alloc<uint32_t>(expect + 1);
-            unsigned long long *ntot = j->arena.alloc<unsigned long long>(1);
-            if (!tl || !ti || (has_hi && !th) || !ntot)
-                return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)expect);
-            unsigned long long n = 0;
-            uint32_t cerr = 0;
-            {
-                StageTimer tm(j->clk, j->st, 2);
-                MP_CUDA(cudaMemsetAsync(ntot, 0, 8, j->st));
-                launch_enum_min3(j->d_fq, j->pr, k, (uint32_t)lo, (uint32_t)hi, s ? j->d_parent : nullptr, ntot, expect, tl, th, ti,
-                                 err, j->st);
-                MP_CUDA(cudaMemcpyAsync(&n, ntot, 8, cudaMemcpyDeviceToHost, j->st));
-                MP_CUDA(cudaMemcpyAsync(&cerr, err, 4, cudaMemcpyDeviceToHost, j->st));
-                MP_CUDA(cudaStreamSynchronize(j->st));
+            rc = j->checks ? checked.grouped([&] { return run_grouped(s, expect, rb); }) : run_grouped(s, expect, rb);
+            if (rc == MP_ENOMEM && j->checks) {  // no room for both: the sorted scan's checks alone
+                rc = 0;
+                grouped = false;
+                hold.drop_merged();
             }
-            if (cerr & DERR_LONG_READ) return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
-            if (cerr & DERR_TOO_MANY)
-                return set_error(MP_EUNSUP, "a read has 256 or more k-mers in scan %d (the reference counts them "
-                                            "in 8 bits, enumerateKmers.c:152)", s);
-            if (n != expect)
-                return set_error(MP_EFMT, "scan %d: %llu tuples but the histogram holds %llu", s, n, (unsigned long long)expect);
-            if (cerr) return set_error(MP_EDEVICE, "enumeration flags 0x%x", cerr);
-            if ((rc = grouped_scan(j, gs, 1, s, tl, th, ti, err, hist))) return rc;
+            if (rc) return rc;
             j->arena.release_scratch();
+        }
+        if (grouped && !j->checks) {
+            snprintf(name, sizeof name, "stats%d_parent.bin", s);
+            if ((rc = dump_bad(j, s)) || (rc = dump_state(j, name, nullptr))) return rc;
             continue;
         }
-        hold.drop_merged();  // (a sorted scan takes 26 bytes a tuple; a later grouped one makes its own first pass)
+        if (!j->checks) hold.drop_merged();  // (a sorted scan takes 26 bytes a tuple; a later grouped one makes its own first pass)
         if ((rc = count_scans())) return rc;
         uint32_t *cnt = cnt_all ? cnt_all + (size_t)s * (N + 1) : j->arena.alloc<uint32_t>(N + 1);
         uint64_t *off = j->arena.alloc<uint64_t>(N + 2), *ntot = j->arena.alloc<uint64_t>(1);
@@ -1336,19 +1421,13 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         }
         snprintf(name, sizeof name, "scan%d_filtered.bin", s);
         if ((rc = dump_tuples(j, name, tp.lo, tp.hi, tp.id, n))) return rc;
-        if (!j->dump_dir.empty()) {
-            std::vector<uint8_t> f(N);
-            MP_CUDA(cudaMemcpyAsync(f.data(), j->d_filtered, N, cudaMemcpyDeviceToHost, j->st));
-            MP_CUDA(cudaStreamSynchronize(j->st));
-            snprintf(name, sizeof name, "scan%d_bad.bin", s);
-            rc = write_file(j->dump_dir + "/" + name, f.data(), N);
-            if (rc) return rc;
-        }
+        if ((rc = dump_bad(j, s))) return rc;
         {
             StageTimer tm(j->clk, j->st, 5);
             if ((rc = union_scan(tp, rb, j->d_parent, j->d_filtered, N, j->arena, j->st, j->hooked_bad, &j->hooked_bad)))
                 return rc;
         }
+        if (grouped && (rc = checked.compare(s))) return rc;
         j->arena.release_scratch();
         snprintf(name, sizeof name, "stats%d_parent.bin", s);
         if ((rc = dump_state(j, name, nullptr))) return rc;

@@ -239,7 +239,7 @@ class Job:
         _check(lib().mp_job_set_scan_piece_tuples(self.h, int(max_tuples)), "set_scan_piece_tuples")
 
     def set_checks(self, on: bool = True):
-        """Self-checks of the sorted tuples and the final forest (mp_job_set_checks)."""
+        """Self-checks of the grouped scans against sorted ones, the sorted tuples and the final forest (mp_job_set_checks)."""
         _check(lib().mp_job_set_checks(self.h, int(bool(on))), "set_checks")
 
     def set_wait_limits(self, lookback_spins: int = 0, union_retries: int = 0, mate_rounds: int = 0):

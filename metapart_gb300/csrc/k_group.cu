@@ -698,6 +698,7 @@ struct GroupCtx {
     const uint32_t *ustart, *ub0, *fill, *lrs, *list;  // list: the units to take (null: all)
     uint32_t *ctr, *qlist, *quirk;
     int work, count;          // counters of the units taken and of the units there are
+    bool ends_range, ends_scan;  // of the last unit (GroupScan)
     uint32_t cap_lo, cap_hi;  // takes units of cap_lo < tuples <= cap_hi
     uint32_t *out, *parent;
     uint8_t *filtered;
@@ -741,7 +742,7 @@ __global__ void __launch_bounds__(THREADS, SLOT_BITS == 13 ? 2 : 1) k_group(Grou
         const bool take = cnt > c.cap_lo && cnt <= c.cap_hi;
         const bool last = u + 1 == nall;
         const uint32_t nextb = last ? ~0u : c.ub0[u + 1];
-        const bool ends = last || (nextb >> 31), seg_last = last || ((nextb & 0x7FFFFFFFu) / NB != b0 / NB);
+        const bool ends = last ? c.ends_range : nextb >> 31, seg_last = last ? c.ends_scan : (nextb & 0x7FFFFFFFu) / NB != b0 / NB;
         const uint32_t seg = b0 / NB;
         const bool singles = start >= c.lrs[seg];  // in the segment's last range every read that may join counts (k_gp_quirk)
         __syncthreads();
@@ -960,7 +961,7 @@ struct BigUnit {
 };
 
 __global__ void k_big_units(const uint32_t *big, uint32_t nb, const uint32_t *ustart, const uint32_t *ub0, uint32_t nunits,
-                            const uint32_t *fill, uint32_t *out)
+                            const uint32_t *fill, bool ends_range, uint32_t *out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nb) return;
@@ -968,7 +969,7 @@ __global__ void k_big_units(const uint32_t *big, uint32_t nb, const uint32_t *us
     out[4 * i] = u;
     out[4 * i + 1] = ustart[u];
     out[4 * i + 2] = ustart[u + 1] - ustart[u];
-    out[4 * i + 3] = (u + 1 == nunits || (ub0[u + 1] >> 31)) ? 1u : 0u;  // ends a thread range
+    out[4 * i + 3] = (u + 1 == nunits ? ends_range : ub0[u + 1] >> 31) ? 1u : 0u;  // ends a thread range
     if (fill[u] != ustart[u + 1]) out[4 * i + 2] = 0;  // the histogram is not the tuples': the caller stops here
 }
 
@@ -987,8 +988,8 @@ __global__ void k_gbig_gather(const BigUnit *bu, const uint64_t *kk, const uint3
 // The sorted units' ids into out, as k_group leaves them (a zeroed tuple or the zero k-mer's stands for no read, each a run
 // of its own: nothing looks back through them).
 __global__ void k_gbig_emit(const BigUnit *bu, const uint32_t *base, const uint64_t *tk, const uint32_t *tid, const uint32_t *z,
-                            const uint32_t *ub0, uint32_t nunits, const uint32_t *lrs, int bsh, uint32_t *ctr, uint32_t *qlist,
-                            uint32_t *quirk, uint32_t *out)
+                            const uint32_t *ub0, uint32_t nunits, bool ends_scan, const uint32_t *lrs, int bsh, uint32_t *ctr,
+                            uint32_t *qlist, uint32_t *quirk, uint32_t *out)
 {
     const BigUnit b = bu[blockIdx.x];
     const uint32_t b0 = ub0[b.u] & 0x7FFFFFFFu, seg = b0 / NB, o = *base + b.off;
@@ -1006,7 +1007,7 @@ __global__ void k_gbig_emit(const BigUnit *bu, const uint32_t *base, const uint6
         q[0] = o;
         q[1] = b.cnt;
         q[2] = seg;
-        if (b.u + 1 == nunits || (ub0[b.u + 1] & 0x7FFFFFFFu) / NB != seg) {  // the segment's last run
+        if (b.u + 1 == nunits ? ends_scan : (ub0[b.u + 1] & 0x7FFFFFFFu) / NB != seg) {  // the segment's last run
             const uint64_t km = tk[b.off + b.cnt - 1] >> 8;
             uint32_t a = b.off, y = b.off + b.cnt - 1;
             while (a < y) {
@@ -1212,7 +1213,7 @@ int group_plan(GroupScan &g, DeviceArena &arena, cudaStream_t st)
         bin0[q + 1] = bin0[q] + (uint32_t)((g.merged ? g.hi - 1 - g.anchor : span - 1) >> sh[q]) + 1;
         uint64_t b = g.seg_tstart[q];
         for (; t < (int)nbounds && g.bounds[t] < g.seg_tstart[q + 1]; t++) b = std::max(b, g.bounds[t]);
-        lrs[q] = (uint32_t)b;
+        lrs[q] = g.part ? g.last_range : (uint32_t)b;
     }
     g.bins = bin0[nseg];
     g.seg_lo = nseg > 1 ? 0u : (uint32_t)(g.merged ? g.anchor : g.lo);
@@ -1440,8 +1441,8 @@ int group_filter(GroupScan &g, const uint64_t *kk, const uint32_t *ids, uint32_t
     group_kernel_attrs();
     if (const int rc = group_counts(g, arena)) return rc;
     const uint32_t *fill = g.ucur;
-    GroupCtx c{kk, ids, g.ustart, g.ub0, fill, g.lrs, nullptr, g.ctr, g.qlist, g.quirk, GC_WORK_S, GC_UNITS, 0, (uint32_t)GP_CAP_S,
-               out, parent, filtered};
+    GroupCtx c{kk, ids, g.ustart, g.ub0, fill, g.lrs, nullptr, g.ctr, g.qlist, g.quirk, GC_WORK_S, GC_UNITS,
+               g.ends_range, g.ends_scan, 0, (uint32_t)GP_CAP_S, out, parent, filtered};
     const unsigned sms = (unsigned)sm_count();
     (count_launch(), k_group<GP_THREADS, GP_ITEMS, 13><<<std::min(2 * sms, std::max(1u, g.hctr[GC_UNITS])), GP_THREADS, sizeof(GroupSmemS), st>>>(c));
     if (g.hctr[GC_MID]) {
@@ -1460,7 +1461,8 @@ int group_filter(GroupScan &g, const uint64_t *kk, const uint32_t *ids, uint32_t
         BigUnit *d_b = arena.alloc<BigUnit>(nb);
         uint32_t *d_base = arena.alloc<uint32_t>(1);
         if (!d_l || !d_b || !d_base) return set_error(MP_ENOMEM, "device memory for oversized buckets");
-        (count_launch(), k_big_units<<<blocks_of(nb, 128), 128, 0, st>>>(g.big, nb, g.ustart, g.ub0, g.hctr[GC_UNITS], fill, d_l));
+        (count_launch(), k_big_units<<<blocks_of(nb, 128), 128, 0, st>>>(g.big, nb, g.ustart, g.ub0, g.hctr[GC_UNITS], fill,
+                                                                        g.ends_range, d_l));
         std::vector<uint32_t> hl(4 * (size_t)nb);
         MP_CUDA(cudaMemcpyAsync(hl.data(), d_l, hl.size() * 4, cudaMemcpyDeviceToHost, st));
         MP_CUDA(cudaStreamSynchronize(st));
@@ -1503,7 +1505,7 @@ int group_filter(GroupScan &g, const uint64_t *kk, const uint32_t *ids, uint32_t
             tp.n = acc;
             if ((rc = filter_scan(tp, ends, parent, filtered, arena, st, false))) return rc;
             (count_launch(), k_gbig_reserve<<<1, 1, 0, st>>>(g.ctr, (uint32_t)acc, d_base, b0 == 0));
-            (count_launch(), k_gbig_emit<<<grid, 256, 0, st>>>(d_b + b0, d_base, tp.lo, tp.id, tp.z, g.ub0, g.hctr[GC_UNITS], g.lrs,
+            (count_launch(), k_gbig_emit<<<grid, 256, 0, st>>>(d_b + b0, d_base, tp.lo, tp.id, tp.z, g.ub0, g.hctr[GC_UNITS], g.ends_scan, g.lrs,
                                                               bsh, g.ctr, g.qlist, g.quirk, out));
             MP_CUDA(cudaStreamSynchronize(st));  // ends is this turn's
         }
@@ -1545,6 +1547,9 @@ int group_union(GroupScan &g, const uint32_t *out, uint32_t *parent, const uint8
     if (herr) return set_error(MP_EDEVICE, "union-find retry limit reached (flags 0x%x)", herr);
     for (int q = 0; q < nseg; q++) {
         const uint32_t *w = h.p + GC_N + (size_t)q * QW;
+        g.outside = w[0];
+        g.inside = w[1];
+        g.anchor_read = w[2];
         if (!w[0] && w[1]) open.push_back(GroupQuirk{q, w[2]});
     }
     return 0;

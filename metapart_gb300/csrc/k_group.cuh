@@ -41,6 +41,14 @@ struct GroupScan {
     std::vector<uint64_t> bounds;      // thread ranges' tuple bounds, every segment's after the other (ascending)
     std::vector<uint64_t> seg_tstart;  // nseg + 1 tuple offsets ({0, n} for one scan)
 
+    // a bucket-range piece of a scan: whether a thread range ends with its last tuple, whether it holds the scan's last tuple, and
+    // its first tuple of the scan's last range with tuples (~0: none)
+    bool part = false, ends_range = true, ends_scan = true;
+    uint32_t last_range = 0;
+    // after group_union, of a scan or piece: the last range's reads that are not BAD, outside and inside the scan's last run
+    bool outside = false, inside = false;
+    uint32_t anchor_read = 0;
+
     // a scan of merged ones (group_take)
     const MergedScans *merged = nullptr;
     uint64_t anchor = 0;                     // where its bins count from

@@ -930,7 +930,6 @@ static int scan_in_pieces(mp_job *j, int s, int k, bool has_hi, uint64_t lo, uin
         MP_CUDA(cudaStreamSynchronize(j->st));
         MP_CUDA(cudaGetLastError());
     }
-    j->pieces_total += P;
     return 0;
 }
 
@@ -1028,6 +1027,111 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
     ss.big_buckets = gs.hctr[GC_BIG];
     ss.big_tuples = gs.hctr[GC_BIG_TUPLES];
     add_sort_stats(j, ss, n);
+    return 0;
+}
+
+// scan_in_pieces with grouped pieces: the same two sweeps, each piece split and grouped instead of enumerated and sorted.  The
+// second sweep's filter only repeats marks (a flagged read joins nothing, so its parent is still BAD), and what of the unions
+// depends on the scan's ends, the last range's reads outside and inside the scan's last run, is gathered over the pieces.
+// (Sorted pieces took their k-mers from the count's cache of them, 9 bytes a position, when there was one.  4M x 150 bp, 2
+// scans in 4 pieces each: 115 ms so, 155 enumerated twice from the reads, 65 grouped.)
+static int scan_in_grouped_pieces(mp_job *j, int s, int k, uint64_t lo, uint64_t hi, const std::vector<uint64_t> &pcs,
+                                  const std::vector<uint64_t> &rb, const uint64_t *hist, const uint64_t *d_hist, uint32_t *err)
+{
+    const uint64_t N = j->pr.n_reads, scan0 = hist[lo], n = hist[hi] - scan0;
+    const int P = (int)pcs.size() - 1;
+    uint64_t maxn = 0, last_range = 0;
+    for (int i = 0; i < P; i++) maxn = std::max<uint64_t>(maxn, hist[pcs[i + 1]] - hist[pcs[i]]);
+    for (uint64_t b : rb)
+        if (b < n) last_range = std::max(last_range, b);
+    struct Bufs {  // of every piece, beside each one's scratch
+        DeviceArena &arena;
+        uint32_t *roots = nullptr, *id1 = nullptr, *id2 = nullptr;
+        uint64_t *k1 = nullptr, *k2 = nullptr;
+        ~Bufs()
+        {
+            for (void *p : {(void *)roots, (void *)id1, (void *)id2, (void *)k1, (void *)k2}) arena.free_persistent(p);
+        }
+    } m{j->arena};
+    m.k1 = j->arena.alloc_persistent<uint64_t>(maxn + 1);
+    m.k2 = j->arena.alloc_persistent<uint64_t>(maxn + 1);
+    m.id1 = j->arena.alloc_persistent<uint32_t>(maxn + 1);
+    m.id2 = j->arena.alloc_persistent<uint32_t>(maxn + 1);
+    m.roots = s ? j->arena.alloc_persistent<uint32_t>(N + 1) : nullptr;
+    if (!m.k1 || !m.k2 || !m.id1 || !m.id2 || (s && !m.roots))
+        return set_error(MP_ENOMEM, "device memory for %llu tuples", (unsigned long long)maxn);
+    if (s) MP_CUDA(cudaMemcpyAsync(m.roots, j->d_parent, (N + 1) * 4, cudaMemcpyDeviceToDevice, j->st));
+    int rc = 0;
+    // piece i through the filter; its grouped ids are then in id1
+    auto filtered_piece = [&](int i, GroupScan &g) -> int {
+        const uint64_t p0 = hist[pcs[i]] - scan0, p1 = hist[pcs[i + 1]] - scan0;
+        g.k = k;
+        g.n = p1 - p0;
+        g.d_hist = d_hist;
+        g.lo = pcs[i];
+        g.hi = pcs[i + 1];
+        g.seg_tstart = {0, g.n};
+        g.part = true;
+        g.ends_range = false;
+        g.bounds = {0};
+        for (uint64_t b : rb) {
+            if (b > p0 && b < p1) g.bounds.push_back(b - p0);
+            if (b == p1) g.ends_range = true;
+        }
+        g.bounds.push_back(g.n);
+        g.ends_scan = p1 == n;
+        g.last_range = last_range >= p1 ? ~0u : (uint32_t)(last_range > p0 ? last_range - p0 : 0);
+        {
+            StageTimer tm(j->clk, j->st, 2, SPLIT_SLOT);
+            if ((rc = group_plan(g, j->arena, j->st))) return rc;
+            if ((rc = group_bins_reads(g, j->d_fq, j->pr, {0, N}, m.roots, m.k1, m.id1, j->arena, j->st))) return rc;
+        }
+        {
+            StageTimer tm(j->clk, j->st, 3, SPLIT_SLOT);
+            if ((rc = group_units(g, m.k1, m.id1, m.k2, m.id2, j->st))) return rc;
+        }
+        StageTimer tm(j->clk, j->st, 4);
+        if ((rc = group_filter(g, m.k2, m.id2, m.id1, j->d_parent, j->d_filtered, j->arena, j->st))) return rc;
+        SortStats ss;
+        ss.passes = 2;
+        ss.bytes = g.n * 36;
+        ss.units = g.hctr[GC_UNITS];
+        ss.big_buckets = g.hctr[GC_BIG];
+        ss.big_tuples = g.hctr[GC_BIG_TUPLES];
+        add_sort_stats(j, ss, g.n);
+        return 0;
+    };
+    for (int i = 0; i < P; i++) {
+        if (hist[pcs[i]] == hist[pcs[i + 1]]) continue;
+        GroupScan g;
+        if ((rc = filtered_piece(i, g))) return rc;
+        j->arena.release_scratch();
+    }
+    if ((rc = dump_bad(j, s))) return rc;
+    bool outside = false, inside = false;
+    uint32_t anchor = 0;
+    for (int i = 0; i < P; i++) {
+        if (hist[pcs[i]] == hist[pcs[i + 1]]) continue;
+        GroupScan g;
+        std::vector<GroupQuirk> open;
+        if ((rc = filtered_piece(i, g))) return rc;
+        {
+            StageTimer tm(j->clk, j->st, 5);
+            if ((rc = group_union(g, m.id1, j->d_parent, j->d_filtered, N, j->arena, j->st, open))) return rc;
+        }
+        outside = outside || g.outside;
+        if (g.ends_scan) {
+            inside = g.inside;
+            anchor = g.anchor_read;
+        }
+        j->arena.release_scratch();
+    }
+    if (!outside && inside) {
+        StageTimer tm(j->clk, j->st, 5);
+        uint32_t first = 0;
+        if ((rc = scan_first_read(j, k, 0, lo, hi, hist, s > 0, err, &first))) return rc;
+        if ((rc = group_finish(j->d_parent, N, first, anchor, j->arena, j->st, &j->hooked_bad))) return rc;
+    }
     return 0;
 }
 
@@ -1307,8 +1411,14 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
         if (expect > piece_cap) {
             const std::vector<uint64_t> pcs = plan_pieces(hist, lo, hi, piece_cap);
             if (pcs.size() > 2) {
-                if ((rc = count_scans())) return rc;
-                {  // the per-read checks of the whole scan (its counts, when the pass over all scans did not make them)
+                uint64_t most = 0;
+                for (size_t i = 0; i + 1 < pcs.size(); i++) most = std::max<uint64_t>(most, hist[pcs[i + 1]] - hist[pcs[i]]);
+                bool grouped = scan_is_grouped(j, k, most);
+                if (grouped && j->pr.max_len > (uint32_t)k && j->pr.max_len - (uint32_t)k >= 300u)
+                    return set_error(MP_EUNSUP, "a read has 300 or more k-mer positions");
+                if (!grouped || j->checks || j->pr.max_len > (uint32_t)k + 254u) {
+                    if ((rc = count_scans())) return rc;
+                    // the per-read checks of the whole scan (its counts, when the pass over all scans did not make them)
                     uint32_t cerr = 0, *c1 = cnt_all ? nullptr : j->arena.alloc<uint32_t>(N + 1);
                     if (!cnt_all && !c1) return set_error(MP_ENOMEM, "device memory for enumeration counts");
                     if (c1) launch_enum_count(j->d_fq, j->pr, k, 0, (uint32_t)lo, (uint32_t)hi, c1, err, j->st);
@@ -1323,7 +1433,22 @@ int mp_job_partition(mp_job *j, const mp_part_params *p, const uint64_t *chunk_s
                 }
                 std::vector<uint64_t> rb;
                 if ((rc = range_bounds(hist, thrR.data() + (size_t)s * T, T, lo, hi, rb))) return rc;
-                if ((rc = scan_in_pieces(j, s, k, has_hi, lo, hi, pcs, rb, hist, d_hist, err))) return rc;
+                CheckedScan checked(j);
+                auto run = [&] { return scan_in_grouped_pieces(j, s, k, lo, hi, pcs, rb, hist, d_hist, err); };
+                if (grouped) {
+                    rc = j->checks ? checked.grouped(run) : run();
+                    if (rc == MP_ENOMEM && j->checks) {
+                        rc = 0;
+                        grouped = false;
+                    }
+                    if (rc) return rc;
+                    j->arena.release_scratch();
+                }
+                if (!grouped || j->checks) {
+                    if ((rc = scan_in_pieces(j, s, k, has_hi, lo, hi, pcs, rb, hist, d_hist, err))) return rc;
+                    if (grouped && (rc = checked.compare(s))) return rc;
+                }
+                j->pieces_total += (int)pcs.size() - 1;
                 j->arena.release_scratch();
                 snprintf(name, sizeof name, "stats%d_parent.bin", s);
                 if ((rc = dump_state(j, name, nullptr))) return rc;

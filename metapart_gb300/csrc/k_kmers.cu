@@ -61,40 +61,76 @@ __device__ __forceinline__ uint32_t chunk_of(const uint64_t *chunk_rec, int nchu
 // ------------------------------------------------------------ K1 plain
 
 constexpr int CT_THREADS = 256;
+// Where a read is longer than CT_SPLIT, those above CT_LONG are counted by themselves, a block each: the longest sets the tiling
+// of all, and from about 1,540 bases a tile is one read (600,000 reads of 100 bases and one of 4,000: counting 1.8 ms, apart
+// 0.5; and one of 1,000: 0.7.  Apart wherever a read is above 512, a tenth of 900 bases 0.9 -> 1.15).
+constexpr uint32_t CT_LONG = 512, CT_SPLIT = 1536;
 
-// m-mer counts of the reads, a tile of reads per block and turn (k_readtile.cuh).  One reduction per k-mer: neighbouring
+struct CountOut {
+    const uint64_t *chunk_rec;
+    int nchunks;
+    uint32_t *cc;
+    unsigned long long *glob;
+    uint32_t *err;
+};
+
+// The k-mers of the reads [r0, r0 + n) by one block; of those of at most `most` bases.  One reduction per k-mer: neighbouring
 // positions almost never share a bucket, so grouping equal buckets first costs more than it saves.  ODD: a byte other
 // than A, C, G, T, N sets DERR_NONACGT.
 template <bool ODD, bool HI>
-__global__ void __launch_bounds__(CT_THREADS) k_count_tiles(ReadTiles t, uint64_t n_reads, const uint64_t *chunk_rec, int nchunks,
-                                                            uint32_t *cc, unsigned long long *glob, uint32_t *err)
+__device__ __forceinline__ void count_tile(const ReadTiles &t, uint64_t r0, uint32_t n, uint32_t most, const CountOut &o, uint32_t *packed)
 {
-    extern __shared__ __align__(16) uint32_t packed[];
     const uint32_t stride = rt_stride(t);
     const int sh = 2 * (t.k - 10);
+    if (rt_pack<ODD>(t, r0, n, packed)) atomicOr(o.err, DERR_NONACGT);
+    __syncthreads();
+    for (uint32_t x = threadIdx.x; x < n * t.spr; x += CT_THREADS) {
+        const uint32_t rr = x / t.spr, i0 = (x - rr * t.spr) * t.P, L = t.seq_len[r0 + rr];
+        if (L <= (uint32_t)t.k || L > most || i0 > L - (uint32_t)t.k) continue;
+        uint32_t *ccc = o.cc ? o.cc + (size_t)chunk_of(o.chunk_rec, o.nchunks, r0 + rr) * NB : nullptr;
+        KmerRoll<HI> s;
+        s.template init<false>(t, packed + rr * stride, L, i0);
+#pragma unroll
+        for (int j = 0; j < RT_P; j++) {
+            if ((s.vm >> j) & 1u) {
+                const uint64_t f = s.fwd(), r = s.rc();
+                const uint32_t b = (uint32_t)((f < r ? f : r) >> sh);
+                if (ccc) atomicAdd(&ccc[b], 1u);
+                else atomicAdd(&o.glob[b], 1ull);
+            }
+            s.next();
+        }
+    }
+    __syncthreads();
+}
+
+// m-mer counts of the reads of at most `most` bases, a tile of reads per block and turn (k_readtile.cuh).
+template <bool ODD, bool HI>
+__global__ void __launch_bounds__(CT_THREADS) k_count_tiles(ReadTiles t, uint64_t n_reads, uint32_t most, CountOut o)
+{
+    extern __shared__ __align__(16) uint32_t packed[];
     const uint64_t tiles = (n_reads + t.rpt - 1) / t.rpt;
     for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const uint64_t r0 = tile * t.rpt, r1 = min(n_reads, r0 + t.rpt);
-        if (rt_pack<ODD>(t, r0, (uint32_t)(r1 - r0), packed)) atomicOr(err, DERR_NONACGT);
+        const uint64_t r0 = tile * t.rpt;
+        count_tile<ODD, HI>(t, r0, (uint32_t)(min(n_reads, r0 + t.rpt) - r0), most, o, packed);
+    }
+}
+
+// And of the longer ones, found among CT_THREADS reads at a time.
+template <bool ODD, bool HI>
+__global__ void __launch_bounds__(CT_THREADS) k_count_long(ReadTiles t, uint64_t n_reads, CountOut o)
+{
+    extern __shared__ __align__(16) uint32_t packed[];
+    __shared__ uint16_t list[CT_THREADS];
+    __shared__ uint32_t nl;
+    for (uint64_t r0 = (uint64_t)blockIdx.x * CT_THREADS; r0 < n_reads; r0 += (uint64_t)gridDim.x * CT_THREADS) {
+        const bool is_long = r0 + threadIdx.x < n_reads && t.seq_len[r0 + threadIdx.x] > CT_LONG;
+        if (threadIdx.x == 0) nl = 0;
+        if (!__syncthreads_or(is_long)) continue;
+        if (is_long) list[atomicAdd(&nl, 1u)] = (uint16_t)threadIdx.x;
         __syncthreads();
-        for (uint32_t x = threadIdx.x; x < (uint32_t)(r1 - r0) * t.spr; x += CT_THREADS) {
-            const uint32_t rr = x / t.spr, i0 = (x - rr * t.spr) * t.P, L = t.seq_len[r0 + rr];
-            if (L <= (uint32_t)t.k || i0 > L - (uint32_t)t.k) continue;
-            uint32_t *ccc = cc ? cc + (size_t)chunk_of(chunk_rec, nchunks, r0 + rr) * NB : nullptr;
-            KmerRoll<HI> s;
-            s.template init<false>(t, packed + rr * stride, L, i0);
-#pragma unroll
-            for (int j = 0; j < RT_P; j++) {
-                if ((s.vm >> j) & 1u) {
-                    const uint64_t f = s.fwd(), r = s.rc();
-                    const uint32_t b = (uint32_t)((f < r ? f : r) >> sh);
-                    if (ccc) atomicAdd(&ccc[b], 1u);
-                    else atomicAdd(&glob[b], 1ull);
-                }
-                s.next();
-            }
-        }
-        __syncthreads();
+        const uint32_t n = nl;
+        for (uint32_t q = 0; q < n; q++) count_tile<ODD, HI>(t, r0 + list[q], 1, ~0u, o, packed);
     }
 }
 
@@ -501,11 +537,19 @@ void launch_count(const uint8_t *fq, const ParsedReads &pr, int k, int min3, con
         (mp::count_launch(), (k >= 17 ? k_count_min3<true> : k_count_min3<false>)<<<grid_for(pr.n_reads, 128, 32), 128, 0, st>>>(fq, pr.seq_off, pr.seq_len, 0, pr.n_reads, k,
                                                                           chunk_rec, nchunks, cc, glob, err));
     else if (pr.max_len > (uint32_t)k) {
-        const ReadTiles t = read_tiles(fq, pr, k, std::min<uint32_t>(pr.max_len, (uint32_t)MAX_READ_COUNT), CT_THREADS, 4096);
+        const CountOut o{chunk_rec, nchunks, cc, glob, err};
+        const uint32_t most = pr.max_len > CT_SPLIT ? CT_LONG : pr.max_len;
+        const ReadTiles t = read_tiles(fq, pr, k, most, CT_THREADS, 4096);
         auto kern = odd ? (k >= 17 ? k_count_tiles<true, true> : k_count_tiles<true, false>)
                         : (k >= 17 ? k_count_tiles<false, true> : k_count_tiles<false, false>);
-        (mp::count_launch(), kern<<<grid_for(pr.n_reads, (int)t.rpt, 16), CT_THREADS, t.words() * 4, st>>>(t, pr.n_reads, chunk_rec,
-                                                                                                     nchunks, cc, glob, err));
+        (mp::count_launch(), kern<<<grid_for(pr.n_reads, (int)t.rpt, 16), CT_THREADS, t.words() * 4, st>>>(t, pr.n_reads, most, o));
+        if (pr.max_len > CT_SPLIT) {
+            ReadTiles l = read_tiles(fq, pr, k, std::min<uint32_t>(pr.max_len, (uint32_t)MAX_READ_COUNT), CT_THREADS, 4096);
+            l.rpt = 1;
+            auto kern_long = odd ? (k >= 17 ? k_count_long<true, true> : k_count_long<true, false>)
+                                 : (k >= 17 ? k_count_long<false, true> : k_count_long<false, false>);
+            (mp::count_launch(), kern_long<<<grid_for(pr.n_reads, CT_THREADS, 8), CT_THREADS, l.words() * 4, st>>>(l, pr.n_reads, o));
+        }
     }
     if (cc && glob) (mp::count_launch(), k_sum_chunks<<<NB / 256, 256, 0, st>>>(cc, nchunks, glob));
 }

@@ -71,7 +71,7 @@ def parse_args():
                     help="plain mode: seconds of Poisson arrivals for the line's p50/p99 (0: none)")
     ap.add_argument("--no-batch", action="store_true", help="plain mode: leave out the batched-vs-plain run")
     ap.add_argument("--store", default="kmer_cache", choices=["kmer_cache", "packed", "fastq"],
-                    help="plain mode: what the count pass keeps of the reads for the partition")
+                    help="plain mode: the job's read store (it sets what a request reserves; nothing is held)")
     return ap.parse_args()
 
 
@@ -306,27 +306,6 @@ def main():
     e2e_pieces = job.scan_pieces
     e2e_ms = dist.max(e0.elapsed_time(e1) / args.steps)
     e2e_value = dist.world * bases / (e2e_ms / 1e3)
-    # the other stores of the reads (what the count pass keeps for the enumeration), device-resident, a few
-    # steps each: their times and device bytes
-    stores = {}
-    reads_pos = args.reads * max(0, spec.lengths[0] - args.k + 1)
-    rounds = args.reads * ((spec.lengths[0] + 31) // 32)
-    store_bytes = {"kmer_cache": 9 * reads_pos + 8 * args.reads, "packed": 12 * rounds + 8 * args.reads, "fastq": 0}
-    for other in [x for x in ("kmer_cache", "packed", "fastq") if x != args.store] if not min3 else []:
-        job.set_read_store(other)
-        device_step()
-        e_a = torch.cuda.Event(enable_timing=True)
-        e_b = torch.cuda.Event(enable_timing=True)
-        e_a.record(stream)
-        for _ in range(3):
-            device_step()
-        e_b.record(stream)
-        e_b.synchronize()
-        stores[other] = {"ms_per_step": round(e_a.elapsed_time(e_b) / 3, 3),
-                         "enumerate_ms": round(job.stage_ms()["enumerate"], 3), "device_bytes": store_bytes[other]}
-        job.set_read_store(args.store)
-    stores[args.store] = {"ms_per_step": round(ms, 3), "enumerate_ms": round(stage.get("enumerate", 0) / args.steps, 3),
-                          "device_bytes": store_bytes[args.store]}
     link = link_bandwidth(host_in, dev_in[:nbytes], out_host)
 
     peak, peak_kind = measured_peak()
@@ -371,7 +350,7 @@ def main():
                            "limiter": "shared memory: the hash table's random accesses",
                            "bytes_per_step": int(group_bytes), "ms_per_step": round(group_ms, 4),
                            "traffic": (round(group_tpt * tuples) if group_tpt else None)},
-        "read_stores": stores,
+        "read_store": args.store,
         "gpu_launches": int(launches),
         "stage_ms": {kk: round(v / args.steps, 3) for kk, v in stage.items()},
         "sort_split": {kk: ({k2: int(v2 / args.steps) for k2, v2 in v.items()} if isinstance(v, dict) else

@@ -43,7 +43,7 @@ struct PlanCtx {
 
 // The bin width of a segment of n tuples over `span` buckets.  A bin of at most 1024 buckets has at most 1024 units, so
 // the second pass finds a tuple's unit in a table of the bin's buckets; the widest such bins, as the first pass stores a
-// tile's tuples in runs by bin (20M x 150 bp, 2 scans: 512 bins 33.3 + 16.6 ms for the two passes, 1024 bins 35.6 + 15.4).
+// tile's tuples in runs by bin (20M x 150 bp, 2 scans, each with both passes: 512 bins 33.3 + 16.6 ms, 1024 bins 35.6 + 15.4).
 // A segment of at most GP_SMALL tuples has at most 1024 units in all and takes bins of about 16384 tuples instead, which
 // fill the second pass's tiles.
 static int bin_width(uint64_t n, uint64_t span)
@@ -429,7 +429,8 @@ __device__ __forceinline__ void bin_tile(const BinCtx &c, uint32_t tile, uint32_
 
 // Bound by the instructions of the k-mers (about 90 per position at 38 % issue; two blocks' 64 registers a thread hold 32
 // warps per SM) and the shared-memory reorder; the random stores and the ranks' atomics are about a fifth each.  20M x
-// 150 bp, 2 scans: 35.4 ms for what counting (6.1), enumerating (14.3) and a first split over 13-byte tuples (29.3) took.
+// 150 bp, 2 scans: 23.9 ms together (33.6 with a pass per scan) for what counting (6.1), enumerating (14.3) and a first split
+// over 13-byte tuples (29.3) took.
 //
 // HI: 2k >= 34 and bins of at least 2^32 k-mers, so a k-mer's bin is a shift of its high word.
 //
@@ -527,7 +528,7 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_reads(BinCtx c)
         const uint32_t nv = split_order<MERGED>(sm, kl, kh, rd, c.bcur + d0, nd, [&](int) { return id; });
         split_store<MERGED>(sm, nv, c.out_k, c.out_id, c.n);
         // the next tile's reads while others store (its bytes fetched before the stores instead cost registers that spill: 37.5
-        // against 35.7 ms at 20M x 150 bp, 2 scans)
+        // against 35.7 ms at 20M x 150 bp, 2 scans with a pass each)
         const uint32_t next = tile + gridDim.x;
         if (next < c.tiles) take(next);
     }
@@ -572,8 +573,8 @@ __global__ void __launch_bounds__(SP_THREADS, 2) k_split_tuples(BinCtx c)
 
 // Second pass: a bin's tuples into its units.  Blocks take four consecutive tiles at a time, so all of them work in a few
 // neighbouring bins: with long stretches per block instead (a bin or more), 300 bins of 560 units were open at once, L2
-// evicted their half-filled lines, and 2.39 G tuples moved 102 GB through DRAM where they take 57 (26.5 ms; 15.1 now, 3.8
-// TB/s, at 20M x 150 bp, 2 scans).
+// evicted their half-filled lines, and 2.39 G tuples moved 102 GB through DRAM where they take 57 (26.5 ms; 17.5 in stretches
+// of four, and 21.5 with a later scan's component lookups, at 20M x 150 bp, 2 scans).
 __global__ void __launch_bounds__(SP_THREADS, 2) k_split_units(const uint64_t *__restrict__ kk, const uint32_t *__restrict__ id,
                                                                uint32_t n, int bsh, uint32_t seg_lo, uint32_t *ctr, uint32_t nbins,
                                                                const uint32_t *__restrict__ bstart,
@@ -1088,7 +1089,7 @@ __global__ void __launch_bounds__(256) k_gp_blank(const uint32_t *ctr, const uin
 }
 
 // Bound by the random reads of the BAD flags and parents in L2.  It reads 4 bytes per joining tuple where the
-// sweep over sorted tuples read 13 per tuple: 6.7 ms against 21.0 at 20M x 150 bp, 2 scans.
+// sweep over sorted tuples read 13 per tuple: 6.2 ms against 21.0 at 20M x 150 bp, 2 scans.
 //
 // The unions of every k-mer's reads (metapart.c:2537-2727): each read that is not BAD joins its k-mer's first one
 // of the stretch.  A stretch that starts inside a run looks back for one read of it, so long runs are shared by

@@ -672,7 +672,7 @@ int mp_job_load_count(mp_job *j, const char *bytes, uint64_t nbytes, const uint6
         int rc = mp_job_load_fastq(j, bytes, nbytes, file_sizes, nfiles, interleaved);
         return rc ? rc : mp_job_count(j, k, min3, chunk_starts, nchunks, hist_out, nullptr, chunk_reads_out);
     };
-    // pinned input (asynchronous copies), the k-mer cache variant, ascending chunks over the whole input
+    // pinned input (asynchronous copies), the plain variant, a read store, ascending chunks over the whole input
     cudaPointerAttributes pa{};
     const bool pinned = cudaPointerGetAttributes(&pa, bytes) == cudaSuccess && pa.type == cudaMemoryTypeHost;
     cudaGetLastError();
@@ -1033,8 +1033,8 @@ static int grouped_scan(mp_job *j, GroupScan &gs, int min3, int s, uint64_t *lo,
 // scan_in_pieces with grouped pieces: the same two sweeps, each piece split and grouped instead of enumerated and sorted.  The
 // second sweep's filter only repeats marks (a flagged read joins nothing, so its parent is still BAD), and what of the unions
 // depends on the scan's ends, the last range's reads outside and inside the scan's last run, is gathered over the pieces.
-// (Sorted pieces took their k-mers from the count's cache of them, 9 bytes a position, when there was one.  4M x 150 bp, 2
-// scans in 4 pieces each: 115 ms so, 155 enumerated twice from the reads, 65 grouped.)
+// 4M x 150 bp, 2 scans in 4 pieces each: 65 ms of partition, 155 with the pieces enumerated from the reads and sorted (115 where
+// their k-mers, 9 bytes a position, were kept from the count).
 static int scan_in_grouped_pieces(mp_job *j, int s, int k, uint64_t lo, uint64_t hi, const std::vector<uint64_t> &pcs,
                                   const std::vector<uint64_t> &rb, const uint64_t *hist, const uint64_t *d_hist, uint32_t *err)
 {

@@ -153,8 +153,8 @@ int sample_error(int code, int q, const char *what)
 }
 
 // Device bytes a sample adds to a group: its FASTQ and output, 60 B per read (read table, counts,
-// forest, mate-union lists), 36 B per k-mer position (the k-mer cache while enumerating, two tuple
-// buffers while sorting), its bucket counts and prefix (12 B per bucket).
+// forest, mate-union lists), 36 B per k-mer position (a sorted group's two tuple buffers and marks; a grouped one takes
+// about 24), its bucket counts and prefix (12 B per bucket).
 uint64_t estimate_sample(const char *fq, uint64_t nbytes, int k)
 {
     uint64_t nl[4] = {0, 0, 0, 0};  // the first record's four line ends
@@ -271,7 +271,7 @@ static int run_group(mp_batch *b, const mp_batch_params *p, const mp_batch_sampl
     // once); the parse waits for them, since its small read-backs would queue behind the big copies
     retire(b, older);
     // ---- per upload segment, as its bytes arrive: parse, the samples' and their chunks' first records,
-    // k-mer cache and per-sample bucket counts
+    // per-sample bucket counts
     uint32_t *cc = A.alloc_persistent<uint32_t>((size_t)nseg * NB);
     uint32_t *err = A.alloc_persistent<uint32_t>(1);
     uint64_t *d_srec = A.alloc_persistent<uint64_t>(nseg + nu);  // each segment's sample read offsets (local)

@@ -96,8 +96,8 @@ int mp_job_count(mp_job *job, int k, int min3, const uint64_t *chunk_starts, int
 /* mp_job_load_fastq followed by mp_job_count (without per-chunk bucket counts), with the upload
  * overlapped: for pinned host bytes and the plain variant, the input goes up in segments of whole
  * chunks on a second stream while the job's stream parses and counts the segments already in HBM.
- * Results, errors and the job state afterwards are those of the two calls made one after the other
- * (which is also what runs for pageable bytes, the 3-minimizer variant, or when a segment fails).
+ * Results, errors and the job state afterwards are those of the two calls made one after the other (which is
+ * also what runs for pageable bytes, the 3-minimizer variant, MP_STORE_FASTQ, or when a segment fails).
  * The reference reads each chunk from disk inside genHistograms' count loop (genHistograms.c:82-575);
  * this has no further counterpart there. */
 int mp_job_load_count(mp_job *job, const char *bytes, uint64_t nbytes, const uint64_t *file_sizes, int nfiles,
@@ -121,7 +121,8 @@ typedef struct {
  * unionFindPeReads (:2801), the work-partition planner (:4016-4053), and the enum module
  * getCanonKmers (enumerateKmers.c:127; enumerateKmers_3minimizers.c:129).
  * chunk_first_read: nchunks+1 read ids (fileIndex readId/readIdExtra; last = read count).
- * hist: the 1048577-entry .kmerHist of the same k and variant.  bounds_out: 17 read-id bounds. */
+ * hist: the 1048577-entry .kmerHist of the same reads, k and variant (MP_EFMT when the tuples do not match it).
+ * bounds_out: 17 read-id bounds. */
 int mp_job_partition(mp_job *job, const mp_part_params *p, const uint64_t *chunk_starts,
                      const uint64_t *chunk_first_read, int nchunks, const uint64_t *hist, uint64_t *bounds_out);
 
@@ -246,8 +247,7 @@ typedef struct {
 } mp_server_stats_t;
 
 /* Estimated device bytes of one request (FASTQ, read table, forest, the largest scan's tuple
- * buffers, output, the store of the reads its count pass keeps), from the request size and its first
- * records. */
+ * buffers, output, what the read store asks for), from the request size and its first records. */
 uint64_t mp_request_footprint(const char *fastq, uint64_t nbytes, const mp_request_params *p);
 
 /* slots: worker threads (jobs in flight at most); hbm_budget: bytes the admitted footprints may add
@@ -278,7 +278,8 @@ int mp_job_set_kmer_cache(mp_job *job, int enable);
  * The job's FASTQ bytes stay in device memory for its output, and every pass over the k-mers takes them from those
  * bytes, packing the bases on chip; that is faster than reading stored k-mers (9 bytes per position) or packed reads
  * was, so no store holds device memory beside the FASTQ bytes.  The choice still sets a request's admission footprint
- * (mp_request_footprint) and what mp_job_read_store reports: MP_STORE_FASTQ without a count, after a count whose input
+ * (mp_request_footprint), whether mp_job_load_count overlaps the upload (not with MP_STORE_FASTQ) and what
+ * mp_job_read_store reports: MP_STORE_FASTQ without a count, after a count whose input
  * MP_STORE_PACKED cannot hold (any sequence byte other than A, C, G, T, N), for the 3-minimizer variant, and after the
  * partition.  The results are the same with all three.  No counterpart in the reference, whose stages are separate
  * processes that re-read the FASTQ files. */
@@ -291,8 +292,8 @@ int mp_job_read_store(const mp_job *job);
 /* Most tuples one scan of mp_job_partition holds in HBM at once (0, the default: what the context's
  * budget, or the device, has left at about 32 bytes per tuple; the environment variable
  * MP_SCAN_PIECE_TUPLES overrides both).  A scan of the plain variant with more tuples runs in pieces of
- * consecutive m-mer buckets, swept twice (sort and mischief filter of every piece, then sort and union of
- * every piece), with the same results as the whole scan at once.  The reference has no counterpart: its
+ * consecutive m-mer buckets, swept twice (mischief filter of every piece, then the unions of every piece),
+ * with the same results as the whole scan at once.  The reference has no counterpart: its
  * scans are what bounds its memory (numScans, metapart.c:3720-3791), and a different numScans changes
  * the partitions; pieces inside a scan do not. */
 int mp_job_set_scan_piece_tuples(mp_job *job, uint64_t max_tuples);

@@ -71,4 +71,4 @@ def test_one_long_read_does_not_set_the_time(ctx):
                 job.count(27, np.array([0, len(data)], np.uint64))
                 best = min(best, job.stage_ms()["count"])
             t.append(best)
-    assert t[1] < 3 * t[0], t
+    assert t[1] < 5 * t[0], t  # (8.5 with the tiles that the long read set)
